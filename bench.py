@@ -167,8 +167,8 @@ def algorithmic_bytes(phase: str, r):
     if phase == "sub_partition":       # bucketed k-mers read + written in sub-bucket order, plus the
         # count that sizes the sub-buckets: 1 in 8 keys sampled on a large pass, every key otherwise
         return 16 * O + (O if O >= (64 << 20) else 8 * O)
-    if phase == "smem_count":          # sub-bucket k-mers read, FIRST ones written back and read again, records
-        return 8 * O + 16 * r.low_len + 12 * r.n_records_total
+    if phase == "smem_count":          # sub-bucket k-mers read, records written
+        return 8 * O + 12 * r.n_records_total
     if phase == "insert_high":         # list read (8 B) + slot key read and count update (16 B)
         return 24 * r.high_len
     if phase == "merge_low":
@@ -180,13 +180,18 @@ def algorithmic_bytes(phase: str, r):
         # writing a 12 B record (P * 24 * R).  The most-significant-bits-first
         # sort of 1M-201M records moves less for the same result (a bucket
         # histogram, two scatter passes and the bucket sort: 8R + 3 * 24R)
+        # The shared-memory path sorts each sub-bucket's records on their own:
+        # they are read and written once
         R = r.n_records_total
-        return math.ceil(2 * 31 / 8) * 24 * R
+        return 24 * R if r.smem_passes else math.ceil(2 * 31 / 8) * 24 * R
     if phase == "census":
         return S
     if phase == "scan":
-        # Bloom jobs read the 1-in-8 census tiles and the pre-pass sample
-        # (the first 256 MiB); plain jobs every tile
+        # the shared-memory path reads its census tiles (1 in 32 from 512 MiB
+        # on, else 1 in 8); Bloom jobs on global-memory tables 1 in 8 and the
+        # pre-pass sample (the first 256 MiB); small plain jobs every tile
+        if r.smem_passes:
+            return S // 32 if S >= (512 << 20) else S // 8
         return S // 8 + min(S, 256 << 20) if r.low_len + r.high_len else S
     return 0
 
@@ -875,8 +880,7 @@ def run_ours(args):
 
     # atomic throughput of the table inserts against random-atomicAdd peaks
     # measured here.  The job's own path (shared-memory sub-bucket tables):
-    # one count atomicAdd per non-FIRST occurrence and one per FIRST
-    # occurrence of a k-mer in the table, against random adds on a 16 KiB
+    # one count atomicAdd per occurrence, against random adds on a 32 KiB
     # shared-memory table per block (the sub-bucket table's count array).
     # The global-memory tables (kc_tuning.bloom_smem = 2), timed on one more
     # untimed job: one count atomicAdd per non-FIRST occurrence, against a
@@ -885,14 +889,13 @@ def run_ours(args):
     atomics = None
     sc = phases.index("smem_count")
     if mean_ms[sc] > 0:
-        pk_smem, _ = kc.atomic_peak_shared(16384)
-        adds = r0.high_len + (r0.low_len - r0.low_only)
+        pk_smem, _ = kc.atomic_peak_shared(32768)
+        adds = r0.occurrences
         rate = adds / (mean_ms[sc] / 1000.0)
         atomics = {"kernel": "smem_count", "table_adds_per_s": rate, "unit": "atomics/s",
                    "table_adds_per_job": int(adds), "peak_smem_random": pk_smem, "frac_of_smem_peak": rate / pk_smem,
-                   "note": "count atomicAdds on the shared-memory sub-bucket tables (non-FIRST occurrences and "
-                           "FIRST occurrences found in the table); the kernel also reads and hashes every key "
-                           "and updates the filter slice, so the fraction is a floor on the insert's share"}
+                   "note": "count atomicAdds on the shared-memory sub-bucket tables; the kernel also reads, hashes and "
+                           "compares every key, so the fraction is a floor on the insert's share"}
         prev = counter.tuning["bloom_smem"]
         counter.set_tuning(bloom_smem=2)
         rg = counter.count(input=inp, keep_records=False, **JOB)

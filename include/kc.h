@@ -105,8 +105,9 @@ typedef struct {
     uint32_t k;                   /* 1..128 (reference: <k_len>); batched jobs 1..32 */
     const kc_input *input;        /* non-NULL: use this resident input, ignore files */
     uint32_t count_max;           /* saturation of counts (reference [count_max], default 255) */
-    uint32_t bloom;               /* 1: reference Bloom singleton split (src/BloomFilter.h) */
-    uint64_t memory_gb;           /* reference <memory_limit_gb>, sizes the Bloom filters */
+    uint32_t bloom;               /* 1: reference singleton split (src/BloomFilter.h): low_len, high_len and
+                                     low_only report it; the counts are exact either way */
+    uint64_t memory_gb;           /* reference <memory_limit_gb>, sizes the Bloom filters (kc_tuning.bloom_smem 2) */
     uint32_t filter_min;          /* reference [filter_min]/[filter_max], applied by */
     uint32_t filter_max;          /*   kc_write_tmpdir to the high.bin records */
     uint32_t min_count;           /* records kept: min_count <= count <= max_count */
@@ -149,22 +150,22 @@ typedef struct {
     double run_ms;                /* start -> end (host clock) */
     /* device time per stage (CUDA events on the job's stream):
      * [0] newline census + tile line numbers, [1] SCAN pass, [2] INSERT pass
-     * (plain) or scatter into the root-prefix buckets (Bloom), [3] insert of
-     * the non-FIRST k-mers, [4] merge of the FIRST k-mers, [5] compaction +
-     * histogram, [6] radix sort, [7] queries, [8] Bloom classification,
-     * [9] scatter of the buckets into filter sub-buckets and [10] their
-     * shared-memory Bloom split + count + compaction (Bloom mode, min count
-     * >= 2), [11] packing of the high.bin records (kc_job.pack_high) */
+     * (plain) or scatter into the 256 buckets, [3] insert of the non-FIRST
+     * k-mers, [4] merge of the FIRST k-mers, [5] compaction + histogram, [6]
+     * sort of the records, [7] queries, [8] Bloom classification, [9] scatter
+     * of the buckets into sub-buckets and [10] their count in shared memory
+     * (prefix path), [11] packing of the high.bin records (kc_job.pack_high) */
     double phase_ms[KC_STAGES];
     uint64_t phase_launches[KC_STAGES];   /* kernel launches per stage */
-    uint64_t low_len;             /* Bloom mode: FIRST occurrences (merged after the inserts) */
-    uint64_t high_len;            /* occurrences inserted into root-prefix bucket tables (Bloom mode:
-                                     the non-FIRST ones; large plain jobs: all); 0 for one table */
+    uint64_t low_len;             /* Bloom mode: FIRST occurrences */
+    uint64_t high_len;            /* occurrences counted in bucket or sub-bucket tables (Bloom mode: the
+                                     non-FIRST ones; large plain jobs: all); 0 for one table */
     uint64_t input_bytes;         /* FASTQ bytes of the job */
     uint64_t n_records_total;     /* records on the device (also when keep_records = 0) */
     uint32_t passes;              /* counting passes over ranges of root prefixes (1: the whole job at once) */
-    uint16_t smem_passes;         /* passes counted on the shared-memory sub-bucket path (Bloom mode) */
-    uint16_t smem_fallbacks;      /* passes that left it after a sub-bucket table overflowed */
+    uint16_t smem_passes;         /* passes counted by printed-order prefix in shared memory */
+    uint16_t smem_fallbacks;      /* passes counted on global-memory tables because sub-buckets had more
+                                     distinct k-mers than their tables hold */
     uint32_t region_redos;        /* shared-memory passes counted again because a sub-bucket outgrew the
                                      region estimated from a sample of the pass's keys */
     uint32_t batch_part;          /* batched jobs: the sub-batch (0, 1, ...) the sample was counted in; a
@@ -183,21 +184,20 @@ typedef struct {
                                      default 1.6 */
     uint64_t sort_group_records;  /* records sorted together (kept in L2) by a batch's segmented sort;
                                      default 4M */
-    uint64_t bloom_smem;          /* Bloom jobs with min_count >= 2: 1 counts each filter sub-bucket (a slice
-                                     of at most 2048 blocks, 32 KiB) in shared memory, 2 uses global-memory
-                                     filters and tables; default 1 */
-    uint64_t record_sort;         /* records of jobs with at least 1M of them: 1 sorts most significant bits
-                                     first (bucket scatter + shared-memory sort per bucket), 2 with the
-                                     8-bit LSD radix sort; default 1 */
-    uint64_t sampled_region_keys; /* Bloom passes (shared-memory path) with at least this many k-mers size
+    uint64_t bloom_smem;          /* Bloom jobs and plain jobs from 4 MiB of FASTQ on: 1 partitions the k-mers by
+                                     their first bases and counts each sub-bucket in a shared-memory table
+                                     (no filter: a FIRST occurrence is the one that makes its k-mer's table
+                                     entry), 2 uses global-memory filters and tables; default 1 */
+    uint64_t record_sort;         /* records counted in global-memory tables, from 1M on: 1 sorts most
+                                     significant bits first (bucket scatter + shared-memory sort per bucket),
+                                     2 with the 8-bit LSD radix sort; default 1 */
+    uint64_t sampled_region_keys; /* passes of the shared-memory path with at least this many k-mers size
                                      their sub-buckets from a 1-in-8 sample of the k-mers instead of
                                      counting them all (a sub-bucket that outgrows its estimate sends the
                                      pass back to exact counts); default 64M */
-    uint64_t count_shape;         /* block shape of the shared-memory count: 1 = 512-thread blocks, two per
-                                     SM, filter slices of up to 2048 blocks, 4096-slot tables; 2 = 256-thread
-                                     blocks, four per SM, slices of up to 1024 blocks, 2048-slot tables
-                                     (sub-buckets of half the k-mers); 3, 4 = 1, 2 with table slots from one
-                                     multiply instead of a 64-bit mix; default 1 */
+    uint64_t count_shape;         /* block shape of the shared-memory count: 1, 3 = 512-thread blocks, two per
+                                     SM, 8192-slot tables; 2, 4 = 256-thread blocks, four per SM, 4096-slot
+                                     tables (sub-buckets of half the k-mers); default 1 */
     uint64_t part_shape;          /* the partition's rounds: 1 = 4096 k-mers staged per round (three blocks
                                      per SM), 2 = 2048 (four blocks per SM); default 1 */
     uint64_t scatter_shape;       /* the sub-bucket scatter: 1 = two blocks per SM, 2 = a variant with fewer

@@ -222,8 +222,8 @@ class Result:
     input_bytes: int = 0
     n_records_total: int = 0
     passes: int = 1
-    smem_passes: int = 0      # passes counted per sub-bucket in shared memory (Bloom mode)
-    smem_fallbacks: int = 0   # passes recounted on global-memory tables after a sub-bucket table overflowed
+    smem_passes: int = 0      # passes counted per sub-bucket in shared memory
+    smem_fallbacks: int = 0   # passes counted on global-memory tables after sub-bucket tables overflowed
     region_redos: int = 0     # shared-memory passes counted again after a sub-bucket outgrew its estimated region
     batch_part: int = 0       # batched jobs: the sub-batch the sample was counted in
 
@@ -441,9 +441,9 @@ class KmerCounter:
     def set_tuning(self, bucket_table_factor: float = 0.0, table_factor: float = 0.0, sort_group_records: int = 0,
                    bloom_smem: int = 0, record_sort: int = 0, sampled_region_keys: int = 0, count_shape: int = 0,
                    part_shape: int = 0, scatter_shape: int = 0):
-        """0 (or less) keeps a setting.  bloom_smem: 1 counts Bloom jobs (min
-        count >= 2) per sub-bucket in shared memory, 2 on global-memory tables.
-        record_sort: 1 sorts large jobs' records most significant bits first,
+        """0 (or less) keeps a setting.  bloom_smem: 1 counts Bloom and large
+        plain jobs per sub-bucket in shared memory, 2 on global-memory tables.
+        record_sort: 1 sorts those tables' records most significant bits first,
         2 with the LSD radix sort.  count_shape: the shared-memory count's
         block shape, 1..4; part_shape: the partition's round size, 1 or 2;
         scatter_shape: the sub-bucket scatter's variant, 1 or 2 (kc_tuning in

@@ -8,11 +8,14 @@
 //
 // One job is the reference's counter run followed by its precise tools:
 //   upload (tile-aligned, zero padded)  -> newline census -> tile line numbers
-//   -> SCAN pass (occurrences, HyperLogLog; Bloom pre-pass statistics)
-//   -> plain:  INSERT pass into a table sized from the HyperLogLog estimate
-//      Bloom:  BLOOM pass (reference filter sizing and probes), then insert
-//              the non-FIRST occurrences and merge the FIRST ones back
-//   -> compaction + histogram -> radix sort in printed-string order
+//   -> Bloom jobs and plain ones of some size (the prefix path): a sampled
+//      census -> scatter by the first bases, twice -> every sub-bucket counted
+//      in a shared-memory table, its records sorted on their own
+//      small plain jobs: SCAN (occurrences, HyperLogLog) -> INSERT into a table
+//      sized from the estimate -> compaction + histogram -> radix sort
+//      global-memory tables (kc_tuning.bloom_smem 2): SCAN with the Bloom
+//      pre-pass statistics -> root-prefix buckets -> the reference's filter
+//      -> insert, merge, compaction + histogram -> radix sort
 //   -> queries -> host.
 // All device memory is stream-ordered (cudaMallocAsync on the worker stream)
 // from a pool that keeps freed memory for the next job.
@@ -88,11 +91,17 @@ kc_tuning default_tuning()
 // uploaded in chunks that the census, SCAN and partition follow.
 constexpr uint64_t STREAMED_UPLOAD_MIN_BYTES = 512ull << 20;
 
-// k-mers per sub-bucket the shared-memory Bloom path starts from.  Its table
-// (SUB_TABLE_SLOTS, 4096) holds the distinct non-FIRST k-mers: at 30x
-// coverage with 1% errors about 1k of 24k, a quarter of the table; a
-// sub-bucket with more is cut in two and counted again.
-constexpr uint64_t SUB_KEYS_TARGET = 24 * 1024;
+// The prefix path (kc_tuning.bloom_smem = 1) takes every Bloom job and the
+// plain jobs of at least this many FASTQ bytes; smaller ones keep one table.
+constexpr uint64_t PREFIX_PATH_MIN_BYTES = 4ull << 20;
+
+// Most k-mers per sub-bucket of the prefix path, for its 8192-slot tables:
+// sub-buckets have half to all of it.
+// At 16K the single large job's sub-buckets of 9K k-mers (2.7K distinct) fill
+// a third of a table: count 18.5 ms, scatter 21.0; 8K (half-empty tables swept
+// twice as often, runs of half the length in the scatter) 21.3 and 30.1, 24K
+// (tables that overflow into rounds) 25.3 and 17.1.
+constexpr uint64_t SUB_KEYS_TARGET = 16 * 1024;
 
 // A plain job whose table would hold more slots than this (64 MiB of slots,
 // half of L2) is counted through the root-prefix buckets.
@@ -346,8 +355,13 @@ struct HostStage {
     }
 };
 
-// A root-prefix bucket outgrew the region estimated from the sampled census.
+// A bucket outgrew the region estimated from the sampled census.
 struct CensusOverflow {};
+
+// A sub-bucket of the prefix path holds more distinct k-mers than its rounds
+// can count and its bucket cannot be cut further: the job is counted again on
+// global-memory tables.
+struct SubTablesFull {};
 
 // Device memory one counting pass may use: 70% of the free device memory, the
 // part of this worker's workspace the job has not used yet, and what the
@@ -397,7 +411,7 @@ void pack_high_on_device(Job &job, DevScope &ds, const unsigned long long *keys,
     job.has_packed = true;
 }
 
-void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, const kc_tuning &tn)
+void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, bool global_tables, const kc_tuning &tn)
 {
     const kc_job &P = job.p;
     const uint32_t k = P.k;
@@ -411,14 +425,20 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, c
     static const bool trace_host = getenv("KC_TRACE") && getenv("KC_TRACE")[0] == '1';
     const double th_start = now_ms();
     std::vector<PinnedBlock> inflated;   // gzip files inflated on the host (kept until the job ends)
-    // a Bloom job's one large host file goes up in chunks while the census,
-    // SCAN and partition work on the chunks that have arrived (declared after
-    // the host and device buffers: it drains its copies before they go)
+    // the one large host file of a prefix-path or Bloom job goes up in chunks
+    // while the census, SCAN and partition work on the chunks that have arrived
+    // (declared after the host and device buffers: it drains its copies before
+    // they go)
     ChunkedUpload cu;
     bool streamed = false;
+    // counted by printed-order prefix in shared memory
+    const auto by_prefix = [&](uint64_t bytes) {
+        return tn.bloom_smem == 1 && !global_tables && (P.bloom || bytes >= PREFIX_PATH_MIN_BYTES);
+    };
     if (!in) {
         const std::vector<kc_buffer> files = inflate_inputs(job.files, inflated);
-        streamed = P.bloom && !exact_census && files.size() == 1 && files[0].size >= STREAMED_UPLOAD_MIN_BYTES;
+        streamed = !exact_census && files.size() == 1 && files[0].size >= STREAMED_UPLOAD_MIN_BYTES &&
+                   (P.bloom || by_prefix(files[0].size));
         build_input(local, files.data(), (uint32_t)files.size(), st, &ds, tile_seg_host, nullptr,
                     streamed ? &cu : nullptr);
         in = &local;
@@ -426,6 +446,7 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, c
             fprintf(stderr, "[kc trace] job upload of %zu files enqueued after %.3f ms\n", job.files.size(),
                     now_ms() - th_start);
     }
+    const bool prefix = by_prefix(in->total_bytes);
     // small uploads and read-backs through pinned staging: a pageable copy
     // would hold the host (and, behind a streamed upload, wait for it)
     HostStage hs(st);
@@ -481,11 +502,11 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, c
     };
     clk.begin(0);
     if (streamed) {
-        // first the chunks holding the pre-pass sample (with the 2 MiB chunks
-        // it ends in) and at least a quarter of the file: the bucket census
-        // and the Bloom sizing come from them
+        // first the chunks holding at least a quarter of the file and, for
+        // global-memory filters, the pre-pass sample (with the 2 MiB chunks it
+        // ends in): the bucket census and the Bloom sizing come from them
         const uint64_t need = std::max<uint64_t>(
-            (segs[0].sample_end + PREPASS_CHUNK - 1) / PREPASS_CHUNK * PREPASS_CHUNK, in->total_bytes / 4);
+            prefix ? 0 : (segs[0].sample_end + PREPASS_CHUNK - 1) / PREPASS_CHUNK * PREPASS_CHUNK, in->total_bytes / 4);
         size_t first = cu.ev.size();
         for (size_t c = 0; c < cu.ev.size(); ++c)
             if (cu.tile_end[c] * TILE >= need) {
@@ -525,21 +546,23 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, c
     unsigned long long *qual = nullptr;
     unsigned long long *bucket_hist = nullptr;
     clk.begin(1);
-    if (P.bloom) {
-        a.hll = nullptr;   // the tables are sized from the non-FIRST occurrences instead
+    if (P.bloom || prefix) {
+        a.hll = nullptr;   // no table, or tables sized from the non-FIRST occurrences
+        a.census_by_string = prefix;
         bucket_hist = ds.n<unsigned long long>(N_BUCKETS);
         CK(cudaMemsetAsync(bucket_hist, 0, N_BUCKETS * 8, st));
         a.bucket_hist = bucket_hist;
         // the bucket census reads every 8th tile of large inputs; buckets get
         // regions with headroom and an outgrown region triggers an exact redo
-        a.bucket_sample_mask = (exact_census || T < 512) ? 0 : 7;
+        // (every 32nd from 512 MiB on, where no pre-pass statistics are needed)
+        a.bucket_sample_mask = (exact_census || T < 512) ? 0 : (prefix && T >= 65536 ? 31 : 7);
         if (a.bucket_sample_mask) {
             // only the census tiles and the pre-pass sample of each file are
             // read; the exact occurrence count comes from the partition pass
             std::vector<uint32_t> visit;
             visit.reserve(T / (a.bucket_sample_mask + 1) + 1);
             for (uint32_t i = 0; i < n_seg; ++i) {
-                const uint64_t pre = (segs[i].sample_end + TILE - 1) / TILE;
+                const uint64_t pre = prefix ? 0 : (segs[i].sample_end + TILE - 1) / TILE;
                 for (uint64_t t = segs[i].first_tile; t < segs[i].first_tile + segs[i].n_tiles && t < tiles_ready; ++t)
                     if ((t & a.bucket_sample_mask) == 0 || t - segs[i].first_tile < pre) visit.push_back((uint32_t)t);
             }
@@ -550,21 +573,23 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, c
             a.visit = d_visit;
             a.n_visit = visit.size();
         }
-        int32_t *chunk_lastnl = ds.n<int32_t>(std::max<uint64_t>(n_chunks, 1));
-        uint64_t *d_chunk0 = ds.n<uint64_t>(seg_chunk0.size());
-        prefix_hist = ds.n<uint32_t>(256);
-        qual = ds.n<unsigned long long>(2);
-        CK(cudaMemsetAsync(chunk_lastnl, 0xff, std::max<uint64_t>(n_chunks, 1) * 4, st));
-        CK(cudaMemcpyAsync(d_chunk0, hs.up(seg_chunk0.data(), seg_chunk0.size()), seg_chunk0.size() * 8,
-                           cudaMemcpyHostToDevice, st));
-        CK(cudaMemsetAsync(prefix_hist, 0, 256 * 4, st));
-        CK(cudaMemsetAsync(qual, 0, 16, st));
-        CK(launch_chunk_lastnl(tile_lastnl, in->d_tile_seg, d_segs, d_chunk0, tiles_ready, chunk_lastnl, st));
-        a.prepass = 1;
-        a.chunk_lastnl = chunk_lastnl;
-        a.seg_chunk0 = d_chunk0;
-        a.prefix_hist = prefix_hist;
-        a.qual = qual;
+        if (!prefix) {
+            int32_t *chunk_lastnl = ds.n<int32_t>(std::max<uint64_t>(n_chunks, 1));
+            uint64_t *d_chunk0 = ds.n<uint64_t>(seg_chunk0.size());
+            prefix_hist = ds.n<uint32_t>(256);
+            qual = ds.n<unsigned long long>(2);
+            CK(cudaMemsetAsync(chunk_lastnl, 0xff, std::max<uint64_t>(n_chunks, 1) * 4, st));
+            CK(cudaMemcpyAsync(d_chunk0, hs.up(seg_chunk0.data(), seg_chunk0.size()), seg_chunk0.size() * 8,
+                               cudaMemcpyHostToDevice, st));
+            CK(cudaMemsetAsync(prefix_hist, 0, 256 * 4, st));
+            CK(cudaMemsetAsync(qual, 0, 16, st));
+            CK(launch_chunk_lastnl(tile_lastnl, in->d_tile_seg, d_segs, d_chunk0, tiles_ready, chunk_lastnl, st));
+            a.prepass = 1;
+            a.chunk_lastnl = chunk_lastnl;
+            a.seg_chunk0 = d_chunk0;
+            a.prefix_hist = prefix_hist;
+            a.qual = qual;
+        }
     } else {
         // plain jobs: an exact root-prefix census beside the distinct
         // estimate, for the partitioned path of large tables
@@ -584,7 +609,7 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, c
     unsigned long long *p_c0 = hs.n<unsigned long long>(C_COUNT);
     CK(cudaMemcpyAsync(p_occ, occ, 8, cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(p_hll, hll, HLL_M * 4, cudaMemcpyDeviceToHost, st));
-    if (P.bloom) {
+    if (P.bloom && !prefix) {
         CK(cudaMemcpyAsync(p_ph, prefix_hist, 256 * 4, cudaMemcpyDeviceToHost, st));
         CK(cudaMemcpyAsync(p_qh, qual, 16, cudaMemcpyDeviceToHost, st));
     }
@@ -595,7 +620,7 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, c
     unsigned long long O = *p_occ;
     std::vector<uint32_t> ph(256, 0);
     unsigned long long qh[2] = {0, 0};
-    if (P.bloom) {
+    if (P.bloom && !prefix) {
         ph.assign(p_ph, p_ph + 256);
         qh[0] = p_qh[0];
         qh[1] = p_qh[1];
@@ -612,14 +637,17 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, c
     const double est = hll_estimate(hll_h.data(), HLL_M);
     unsigned long long *hist = ds.n<unsigned long long>(HIST_BINS);
     // counts of HIST_BINS or more go to a list: a k-mer that often needs
-    // HIST_BINS occurrences, so O / HIST_BINS bounds the list (heavily
-    // repeated genomes reach millions of such k-mers)
-    const uint64_t ovf_cap = std::max<uint64_t>(1ull << 20, O / HIST_BINS + 1);
+    // HIST_BINS occurrences, so the FASTQ bytes (more than the occurrences,
+    // which a sampled census has not counted yet) over HIST_BINS bound the list
+    // (heavily repeated genomes reach millions of such k-mers)
+    const uint64_t ovf_cap = std::max<uint64_t>(1ull << 20, in->total_bytes / HIST_BINS + 1);
     uint32_t *ovf = ds.n<uint32_t>(ovf_cap);
     unsigned long long *n_keys = ds.n<unsigned long long>(1);
     CK(cudaMemsetAsync(hist, 0, HIST_BINS * 8, st));
     unsigned long long low_len = 0, high_len = 0;
     uint64_t table_cap = 0;
+    // singletons that are no table entry (the global-memory filters' FIRST-only k-mers)
+    uint64_t untabled = 0;
     job.distinct = job.low_only = 0;
     job.smem_passes = job.smem_fallbacks = job.region_redos = 0;
 
@@ -635,9 +663,7 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, c
     // into_sort_tmp: the records are written into the sort's alternate
     // buffers, from which an odd number of passes ends in rec_keys/rec_counts.
     bool rec_by_bucket = true, rec_in_sort_tmp = false;
-    // the records per value of their keys' top 16 bits, when the count made
-    // it as it wrote them (a one-pass Bloom job): the sort's bucket histogram
-    uint32_t *rec_hist16 = nullptr;
+    bool rec_sorted = false;   // records of the prefix path: in order, as k-mer words
     void *sort_tmp = nullptr;
     auto compact_table = [&](const TableRef &t, uint64_t cap, uint64_t n_low, const unsigned long long *lst,
                              const BucketRanges *low_rg, uint32_t n_low_items, unsigned int *merge_next,
@@ -714,12 +740,13 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, c
         if (!ordered) n_rec = c2.v[C_REC_LEN];
         job.distinct += c2.v[C_DISTINCT] + c2.v[C_LOW_ONLY];
         job.low_only += c2.v[C_LOW_ONLY];
+        untabled += c2.v[C_LOW_ONLY];
     };
 
     // a plain job whose table would not fit in L2 takes the partitioned path
     // too (without the Bloom split): scattered by root prefix, every bucket's
     // sub-table is filled while it sits in L2
-    const bool plain_part = !P.bloom && table_capacity_for(est, tn.table_factor) > PLAIN_PART_MIN_SLOTS;
+    const bool plain_part = prefix || (!P.bloom && table_capacity_for(est, tn.table_factor) > PLAIN_PART_MIN_SLOTS);
     if (!P.bloom && !plain_part) {
         TableRef tr{};
         TableRef *d_tr = ds.n<TableRef>(1);
@@ -768,7 +795,7 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, c
         for (uint32_t b = 0; b < N_BUCKETS; ++b)
             region[b] = exact ? bh[b] : (unsigned long long)std::ceil((double)bh[b] * scale * 1.15) + 8192;
         std::vector<uint64_t> fcap(N_BUCKETS, 0);
-        if (P.bloom) {
+        if (P.bloom && !prefix) {
             // reference sizing (src/main.cpp:41-153) from the pre-pass statistics
             uint8_t avg_q = qh[1] ? (uint8_t)(qh[0] / qh[1]) : 0;
             BloomPlan bp = bloom_plan(ph.data(), avg_q, in->total_bytes, P.memory_gb, k);
@@ -777,7 +804,10 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, c
         // passes over ranges of buckets, each within the device-memory budget
         // of a pass (k-mer arrays, filters, tables, records of its buckets)
         const uint64_t budget = P.pass_bytes ? P.pass_bytes : default_pass_budget(ws);
-        const uint64_t per_occ = P.bloom ? 42 : 48;
+        // prefix path: two key arrays and the counts with room for estimated
+        // sub-bucket regions (1.25 x (8 + 8 + 4)), then at most n / min count records
+        const uint64_t per_occ =
+            prefix ? 25 + (12 + std::max(P.min_count, 1u) - 1) / std::max(P.min_count, 1u) : (P.bloom ? 42 : 48);
         std::vector<std::pair<uint32_t, uint32_t>> ranges;
         {
             uint32_t lo = 0;
@@ -815,11 +845,17 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, c
             // the Bloom split the scattered k-mers are the insert's input
             unsigned long long *list = nullptr, *bits = nullptr, *keys = nullptr;
             unsigned long long list_cap = ocap;
-            if (P.bloom) {
+            uint32_t *tmp_counts = nullptr;
+            if (prefix) {
                 // room for the sub-buckets' estimated regions (their sizes plus
-                // about 15% on a large pass)
+                // about 15% on a large pass); the partitioned keys' array later
+                // takes the records' keys, at the sub-buckets' offsets
                 list_cap = ocap + ocap / 4 + 65536;
                 list = ds.n<unsigned long long>(list_cap);
+                keys = ds.n<unsigned long long>(list_cap);
+                tmp_counts = ds.n<uint32_t>(list_cap);
+            } else if (P.bloom) {
+                list = ds.n<unsigned long long>(ocap);
                 bits = ds.n<unsigned long long>(std::max<unsigned long long>(words, 1));
                 keys = ds.n<unsigned long long>(ocap);
             } else {
@@ -859,18 +895,18 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, c
                 cu.enqueue(cu.ev.size());
                 a.tile0 = 0;
                 a.n_tiles = tiles_ready;
-                CK(launch_extract(MODE_PART, a, 0, st, (uint32_t)tn.part_shape));
+                CK(launch_extract(prefix ? MODE_PARTS : MODE_PART, a, 0, st, (uint32_t)tn.part_shape));
                 while (chunks_done < cu.ev.size()) {
                     const uint64_t t0 = tiles_ready;
                     census_chunks(chunks_done + 1);
                     a.tile0 = t0;
                     a.n_tiles = tiles_ready - t0;
-                    CK(launch_extract(MODE_PART, a, 0, st, (uint32_t)tn.part_shape));
+                    CK(launch_extract(prefix ? MODE_PARTS : MODE_PART, a, 0, st, (uint32_t)tn.part_shape));
                 }
                 a.tile0 = 0;
                 a.n_tiles = T;
             } else {
-                CK(launch_extract(MODE_PART, a, 0, st, (uint32_t)tn.part_shape));
+                CK(launch_extract(prefix ? MODE_PARTS : MODE_PART, a, 0, st, (uint32_t)tn.part_shape));
             }
             clk.end();
             unsigned long long *p_fill = hs.n<unsigned long long>(N_BUCKETS);
@@ -892,35 +928,20 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, c
                 CK(cudaMemcpyAsync(d, hs.up(&r, 1), sizeof(BucketRanges), cudaMemcpyHostToDevice, st));
                 return d;
             };
-            // Bloom jobs whose records need count >= 2: the Bloom split, the
-            // counting and the compaction run per sub-bucket (a slice of its
-            // bucket's filter) in shared memory.  A bucket starts with about
-            // SUB_KEYS_TARGET k-mers per sub-bucket (and slices of at most
-            // SUB_SLICE_BLOCKS blocks); a bucket whose table overflowed is
-            // counted again with twice the sub-buckets, and a bucket that
-            // cannot be cut further sends the pass to the global-memory path.
-            bool sub_done = false;
-            if (P.bloom && P.min_count >= 2 && tn.bloom_smem == 1) {
-                // the count kernel's block shape: its slice and table sizes
-                // set the sub-buckets (a table of 2048 slots takes half the k-mers)
+            // Prefix path: the buckets are cut into sub-buckets by the next bases,
+            // each counted in a shared-memory table, and its records sorted on
+            // their own.  A bucket starts with at most SUB_KEYS_TARGET k-mers per
+            // sub-bucket; one whose sub-buckets no number of rounds fits is cut
+            // into 16 times as many and the pass counted again, and a bucket that
+            // cannot be cut further sends the job to global-memory tables.
+            if (prefix) {
                 const uint32_t shape = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(tn.count_shape, 4));
-                const uint64_t keys_target = SUB_KEYS_TARGET * sub_table_slots(shape) / SUB_TABLE_SLOTS;
+                const uint64_t keys_target = SUB_KEYS_TARGET * sub_table_slots(shape) / sub_table_slots(1);
+                const uint32_t max_sub_k = 2 * k > 8 ? (2 * k >= 20 ? SUB_MAX_PER_BUCKET : 1u << (2 * k - 8)) : 1u;
                 std::vector<uint32_t> nsub(N_BUCKETS, 0);
-                bool eligible = true;
-                for (uint32_t b = lo; b < hi; ++b) {
-                    const uint64_t f = fcap[b];
-                    if (!f || (f & (f - 1))) {
-                        eligible = false;
-                        break;
-                    }
-                    uint64_t want = std::max<uint64_t>(f / sub_slice_blocks(shape), (cfg[b].key_len + keys_target - 1) / keys_target);
-                    want = std::max<uint64_t>(bit_ceil64(want), 1);
-                    if (want > std::min<uint64_t>(f, SUB_MAX_PER_BUCKET)) {
-                        eligible = false;
-                        break;
-                    }
-                    nsub[b] = (uint32_t)want;
-                }
+                for (uint32_t b = lo; b < hi; ++b)
+                    nsub[b] = (uint32_t)std::min<uint64_t>(
+                        bit_ceil64((cfg[b].key_len + keys_target - 1) / keys_target), max_sub_k);
                 // the overflow list's length before the attempts, restored after
                 // a failed one (on the device: no round trip)
                 unsigned long long *ovf_len_saved = ds.n<unsigned long long>(1);
@@ -929,37 +950,33 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, c
                 // its keys instead of counting them all; a sub-bucket that
                 // outgrows its region sends the pass back to exact counts
                 bool exact_regions = false;
-                for (int attempt = 0; eligible && !sub_done; ++attempt) {
+                for (int attempt = 0;; ++attempt) {
                     const DevScope::Mark m0 = ds.mark();
                     std::vector<SubCfg> sc(N_BUCKETS);
                     std::vector<uint8_t> sb;
-                    uint32_t n_sub = 0;
+                    uint32_t n_sub = 0, max_sub = 1;
                     uint64_t pass_keys = 0;
                     for (uint32_t b = lo; b < hi; ++b) {
-                        sc[b].fcap = fcap[b];
                         sc[b].sub_base = n_sub;
                         sc[b].n_sub = nsub[b];
-                        sc[b].slice_shift = (uint32_t)__builtin_ctzll(fcap[b] / nsub[b]);
+                        sc[b].shift = 56 - (uint32_t)__builtin_ctz(nsub[b]);
                         n_sub += nsub[b];
+                        max_sub = std::max(max_sub, nsub[b]);
                         sb.insert(sb.end(), nsub[b], (uint8_t)b);
                         pass_keys += cfg[b].key_len;
                     }
                     SubCfg *d_sc = ds.n<SubCfg>(N_BUCKETS);
-                    uint8_t *d_sb = ds.n<uint8_t>(std::max<uint32_t>(n_sub, 1));
-                    uint32_t *sub_count = ds.n<uint32_t>(std::max<uint32_t>(n_sub, 1));
-                    unsigned long long *sub_off = ds.n<unsigned long long>(std::max<uint32_t>(n_sub, 1));
-                    unsigned long long *sub_cur = ds.n<unsigned long long>(std::max<uint32_t>(n_sub, 1));
-                    unsigned long long *sub_tmp =
-                        ds.n<unsigned long long>(scan_tmp_words(std::max<uint32_t>(n_sub, 1)));
+                    uint8_t *d_sb = ds.n<uint8_t>(n_sub);
+                    uint32_t *sub_count = ds.n<uint32_t>(n_sub);
+                    uint32_t *sub_len = ds.n<uint32_t>(n_sub);
+                    unsigned long long *sub_off = ds.n<unsigned long long>(n_sub);
+                    unsigned long long *sub_cur = ds.n<unsigned long long>(n_sub);
+                    unsigned long long *sub_tmp = ds.n<unsigned long long>(scan_tmp_words(n_sub));
                     unsigned int *sub_next = ds.n<unsigned int>(1);
                     uint32_t *bucket_ovf = ds.n<uint32_t>(N_BUCKETS);
                     unsigned long long *hist_sub = ds.n<unsigned long long>(HIST_BINS);
-                    // a record has count >= 2: at most half the occurrences, and at
-                    // most one table of slots per sub-bucket
-                    const uint64_t rcap = std::max<uint64_t>(
-                        std::min<uint64_t>((uint64_t)n_sub * sub_table_slots(shape), pass_keys / 2 + 1), 1);
-                    unsigned long long *rk = ds.n<unsigned long long>(rcap);
-                    uint32_t *rc = ds.n<uint32_t>(rcap);
+                    const uint32_t unit_cap = 2 * n_sub + 4096;
+                    SubUnit *units = ds.n<SubUnit>((size_t)UNIT_CLASSES * unit_cap);
                     BucketRanges br{};
                     for (uint32_t b = lo; b < hi; ++b) {
                         br.begin[b] = cfg[b].key_base;
@@ -969,29 +986,27 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, c
                     BucketRanges *d_br = upload_ranges(br, n_items);
                     CK(cudaMemcpyAsync(d_sc, hs.up(sc.data(), N_BUCKETS), N_BUCKETS * sizeof(SubCfg),
                                        cudaMemcpyHostToDevice, st));
-                    if (n_sub) CK(cudaMemcpyAsync(d_sb, hs.up(sb.data(), n_sub), n_sub, cudaMemcpyHostToDevice, st));
-                    CK(cudaMemsetAsync(sub_count, 0, std::max<uint32_t>(n_sub, 1) * 4, st));
+                    CK(cudaMemcpyAsync(d_sb, hs.up(sb.data(), n_sub), n_sub, cudaMemcpyHostToDevice, st));
+                    CK(cudaMemsetAsync(sub_count, 0, n_sub * 4ull, st));
                     CK(cudaMemsetAsync(bucket_ovf, 0, N_BUCKETS * 4, st));
                     CK(cudaMemsetAsync(hist_sub, 0, HIST_BINS * 8, st));
-                    CK(cudaMemsetAsync(counters + C_LOW_LEN, 0, 2 * 8, st));   // C_LOW_LEN, C_HIGH_LEN
                     CK(cudaMemsetAsync(counters + C_REC_LEN, 0, 3 * 8, st));   // C_REC_LEN, C_LOW_ONLY, C_DISTINCT
                     CK(cudaMemsetAsync(counters + C_SUB_OVF, 0, 2 * 8, st));   // C_SUB_OVF, C_REGION_OVF
+                    CK(cudaMemsetAsync(counters + C_UNITS, 0, UNIT_CLASSES * 8, st));
                     const bool sampled = !exact_regions && pass_keys >= tn.sampled_region_keys;
                     unsigned long long *sub_end = nullptr;
                     clk.begin(9);
                     if (sampled) {
-                        uint32_t *region = ds.n<uint32_t>(std::max<uint32_t>(n_sub, 1));
-                        sub_end = ds.n<unsigned long long>(std::max<uint32_t>(n_sub, 1));
+                        uint32_t *region = ds.n<uint32_t>(n_sub);
+                        sub_end = ds.n<unsigned long long>(n_sub);
                         CK(launch_subpart_count(keys, d_br, n_items, d_sc, sub_count, st, SUB_REGION_SAMPLE));
                         CK(launch_subpart_regions(sub_count, n_sub, SUB_REGION_SAMPLE, region, sub_off, sub_end, sub_cur,
                                                   sub_tmp, st));
                     } else {
                         CK(launch_subpart_count(keys, d_br, n_items, d_sc, sub_count, st));
                         CK(launch_scan_u32(sub_count, sub_off, n_sub, sub_tmp, st));
-                        if (n_sub)
-                            CK(cudaMemcpyAsync(sub_cur, sub_off, (size_t)n_sub * 8, cudaMemcpyDeviceToDevice, st));
+                        CK(cudaMemcpyAsync(sub_cur, sub_off, (size_t)n_sub * 8, cudaMemcpyDeviceToDevice, st));
                     }
-                    const uint32_t max_sub = *std::max_element(nsub.begin(), nsub.end());
                     BucketRanges bs = br;
                     const uint32_t n_sp_items = fill_item_starts_n(bs, SUB_SCATTER_ITEM_KEYS);
                     BucketRanges *d_bs = ds.n<BucketRanges>(1);
@@ -1003,14 +1018,28 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, c
                                                 counters + C_REGION_OVF, st));
                     clk.end();
                     clk.begin(10);
-                    uint32_t *hb16 = nullptr;
-                    if (!multi && 2 * k >= 24) {
-                        hb16 = ds.n<uint32_t>(1u << 16);
-                        CK(cudaMemsetAsync(hb16, 0, (1u << 16) * 4, st));
-                    }
-                    CK(launch_count_subs(list, sub_off, sub_count, d_sb, n_sub, d_sc, sub_next, count_max,
-                                         P.min_count, P.max_count, rk, rc, rcap, hist_sub, ovf, ovf_cap, counters,
-                                         bucket_ovf, st, hb16, 2 * k - 16, shape));
+                    PrefixCountArgs pc{};
+                    pc.keys = list;
+                    pc.sub_off = sub_off;
+                    pc.sub_count = sub_count;
+                    pc.sub_bucket = d_sb;
+                    pc.sc = d_sc;
+                    pc.n_sub = n_sub;
+                    pc.next_sub = sub_next;
+                    pc.count_max = count_max;
+                    pc.min_count = P.min_count;
+                    pc.max_count = P.max_count;
+                    pc.rec_keys = keys;
+                    pc.rec_counts = tmp_counts;
+                    pc.sub_len = sub_len;
+                    pc.units = units;
+                    pc.unit_cap = unit_cap;
+                    pc.hist = hist_sub;
+                    pc.ovf = ovf;
+                    pc.ovf_cap = ovf_cap;
+                    pc.counters = counters;
+                    pc.bucket_ovf = bucket_ovf;
+                    CK(launch_count_prefix(pc, shape, st));
                     clk.end();
                     if (attempt == 0 && (P.fault_inject & KC_INJECT_TABLE_FULL_ONCE)) {
                         // as if the first bucket's sub-bucket tables had overflowed
@@ -1019,51 +1048,67 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, c
                     }
                     const Counters cs = read_counters(counters, st);
                     check_flags(cs.v[C_FLAGS], "sub-bucket count");
-                    if (cs.v[C_REGION_OVF]) {
-                        // a sub-bucket outgrew its estimated region: count again
-                        // with exact regions (same sub-buckets)
+                    const bool again = cs.v[C_REGION_OVF] || cs.v[C_SUB_OVF];
+                    if (again) {
+                        std::vector<uint32_t> bo(N_BUCKETS);
+                        CK(cudaMemcpyAsync(bo.data(), bucket_ovf, N_BUCKETS * 4, cudaMemcpyDeviceToHost, st));
                         CK(cudaMemcpyAsync(counters + C_OVF_LEN, ovf_len_saved, 8, cudaMemcpyDeviceToDevice, st));
                         CK(cudaStreamSynchronize(st));
                         ds.rewind(m0);
-                        exact_regions = true;
-                        ++job.region_redos;
+                        if (cs.v[C_REGION_OVF]) {
+                            // a sub-bucket outgrew its estimated region (the count
+                            // then leaves the keys alone): exact regions, same
+                            // sub-buckets
+                            exact_regions = true;
+                            ++job.region_redos;
+                        } else {
+                            // buckets with more distinct k-mers than 64 rounds of
+                            // their sub-buckets hold: 16 times the sub-buckets
+                            bool cut = false;
+                            for (uint32_t b = lo; b < hi; ++b) {
+                                if (!bo[b]) continue;
+                                if (nsub[b] * 2 > max_sub_k) throw SubTablesFull{};
+                                nsub[b] = std::min(nsub[b] * 16, max_sub_k);
+                                cut = true;
+                            }
+                            if (!cut) throw SubTablesFull{};
+                            // the records went over the partitioned keys
+                            CK(cudaMemsetAsync(cursor, 0, N_BUCKETS * 8, st));
+                            clk.begin(2);
+                            CK(launch_extract(MODE_PARTS, a, 0, st, (uint32_t)tn.part_shape));
+                            clk.end();
+                        }
                         continue;
                     }
-                    if (cs.v[C_SUB_OVF] == 0) {
-                        CK(launch_add_u64(hist, hist_sub, HIST_BINS, st));
-                        rec_keys = rk;
-                        rec_counts = rc;
-                        n_rec = cs.v[C_REC_LEN];
-                        rec_by_bucket = false;
-                        rec_hist16 = hb16;
-                        job.distinct += cs.v[C_DISTINCT] + cs.v[C_LOW_ONLY];
+                    clk.begin(6);
+                    CK(launch_add_u64(hist, hist_sub, HIST_BINS, st));
+                    n_rec = cs.v[C_REC_LEN];
+                    rec_keys = ds.n<unsigned long long>(std::max<uint64_t>(n_rec, 1));
+                    rec_counts = ds.n<uint32_t>(std::max<uint64_t>(n_rec, 1));
+                    // where each sub-bucket's records go; sub_cur is free again
+                    CK(launch_scan_u32(sub_len, sub_cur, n_sub, sub_tmp, st));
+                    uint32_t n_units[UNIT_CLASSES];
+                    for (uint32_t c = 0; c < UNIT_CLASSES; ++c) n_units[c] = (uint32_t)cs.v[C_UNITS + c];
+                    CK(launch_unit_sort(keys, tmp_counts, sub_off, sub_cur, units, unit_cap, n_units, rec_keys, rec_counts,
+                                        n_rec, k, st));
+                    clk.end();
+                    rec_by_bucket = false;
+                    rec_sorted = true;
+                    job.distinct += cs.v[C_DISTINCT];
+                    if (P.bloom) {
+                        // the split: an occurrence is FIRST when it claims its k-mer's slot
                         job.low_only += cs.v[C_LOW_ONLY];
-                        low_len += cs.v[C_LOW_LEN];
-                        high_len += cs.v[C_HIGH_LEN];
-                        table_cap = std::max<uint64_t>(table_cap, (uint64_t)n_sub * sub_table_slots(shape));
-                        ++job.smem_passes;
-                        sub_done = true;
-                        break;
+                        low_len += cs.v[C_DISTINCT];
+                        high_len += pass_keys - cs.v[C_DISTINCT];
+                    } else {
+                        high_len += pass_keys;
                     }
-                    // buckets that held more distinct repeated k-mers than their
-                    // sub-buckets' tables: twice the sub-buckets next time
-                    std::vector<uint32_t> bo(N_BUCKETS);
-                    CK(cudaMemcpyAsync(bo.data(), bucket_ovf, N_BUCKETS * 4, cudaMemcpyDeviceToHost, st));
-                    CK(cudaMemcpyAsync(counters + C_OVF_LEN, ovf_len_saved, 8, cudaMemcpyDeviceToDevice, st));
-                    CK(cudaStreamSynchronize(st));
-                    ds.rewind(m0);
-                    bool any = false;
-                    for (uint32_t b = lo; b < hi; ++b) {
-                        if (!bo[b]) continue;
-                        any = true;
-                        if ((uint64_t)nsub[b] * 2 > std::min<uint64_t>(fcap[b], SUB_MAX_PER_BUCKET)) eligible = false;
-                        else nsub[b] *= 2;
-                    }
-                    if (!any) eligible = false;
-                    if (!eligible) ++job.smem_fallbacks;
+                    table_cap = std::max<uint64_t>(table_cap, (uint64_t)n_sub * sub_table_slots(shape));
+                    ++job.smem_passes;
+                    break;
                 }
             }
-            if (!sub_done) {
+            if (!prefix) {
                 std::vector<unsigned long long> lh(2 * N_BUCKETS, 0);
                 std::vector<uint32_t> hh;
                 if (P.bloom) {
@@ -1220,13 +1265,15 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, c
     // ---- sort in printed-string order ---------------------------------------
     clk.begin(6);
     bool reversed = false;   // keys back in the k-mer word layout
-    if (n_rec > 1) {
+    if (rec_sorted) {
+        reversed = true;   // sorted by sub-bucket, the passes' ranges in order
+    } else if (n_rec > 1) {
         const uint32_t skip = rec_by_bucket && job.passes <= 1 ? 8u : 0u;
         void *stmp = rec_in_sort_tmp ? sort_tmp : ds.get(record_sort_bytes(n_rec, k));
         if (msd_sort_applies(n_rec, 2 * k) && tn.record_sort != 2) {
             // the sort writes the k-mer words back (pair_reverse) as it stores
             CK(launch_msd_sort(rec_keys, rec_counts, n_rec, 2 * k, stmp, st, counters + C_FLAGS, rec_in_sort_tmp,
-                               true, rec_hist16));
+                               true));
             reversed = true;
         } else {
             CK(launch_radix_sort(rec_keys, rec_counts, n_rec, 2 * k, stmp, st, counters + C_FLAGS, skip,
@@ -1253,7 +1300,7 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, c
         CK(cudaMemcpyAsync(ovf_h.data(), ovf, n_ovf * 4, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
     }
-    hd[1] += job.low_only;   // FIRST-only k-mers have count 1 (count_max >= 1)
+    hd[1] += untabled;   // FIRST-only k-mers have count 1 (count_max >= 1)
     {
         uint32_t lo = P.hist_min, hi = P.hist_max;
         if (hi < lo) hi = lo;
@@ -1763,15 +1810,22 @@ void run_job(Job &job, cudaStream_t st, Workspace &ws, const kc_tuning &tn)
         run_wide_job(job, st, ws, tn);
         return;
     }
-    try {
-        run_job_once(job, st, ws, false, tn);
-    } catch (const CensusOverflow &) {
-        // the sampled census missed a skewed bucket: count every tile instead
+    bool exact_census = false, global_tables = false;
+    for (;;) {
+        try {
+            run_job_once(job, st, ws, exact_census, global_tables, tn);
+            break;
+        } catch (const CensusOverflow &) {
+            // the sampled census missed a skewed bucket: count every tile instead
+            exact_census = true;
+        } catch (const SubTablesFull &) {
+            global_tables = true;
+        }
         CK(cudaStreamSynchronize(st));
         ws.end_job();
         ws.begin_job();
-        run_job_once(job, st, ws, true, tn);
     }
+    if (global_tables) job.smem_fallbacks = job.passes;
 }
 
 // Batched jobs: every sample's files in one device buffer, one SCAN and one
@@ -2366,7 +2420,7 @@ int kc_autotune(kc_handle *h, const kc_job *jobs, uint32_t n_jobs, uint32_t batc
     if (rc == KC_OK) rc = run(cur, cur_ms);
     const double bucket_c[] = {2.0, 3.0, 4.0, 3.0}, table_c[] = {1.3, 1.6, 2.2, 1.6};
     const uint64_t group_c[] = {2ull << 20, 4ull << 20, 8ull << 20, 4ull << 20}, smem_c[] = {1, 2, 1, 1},
-                   sort_c[] = {1, 2, 1, 1}, shape_c[] = {1, 2, 3, 4}, part_c[] = {1, 2, 1, 1},
+                   sort_c[] = {1, 2, 1, 1}, shape_c[] = {1, 2, 1, 1}, part_c[] = {1, 2, 1, 1},
                    scatter_c[] = {1, 2, 1, 1};
     for (int param = 0; param < 8 && rc == KC_OK; ++param)
         for (int c = 0; c < 4 && rc == KC_OK; ++c) {

@@ -324,6 +324,7 @@ template <int MODE, uint32_t SCAP = STAGE_CAP>
 __global__ void __launch_bounds__(EXT_THREADS, MODE == MODE_SCAN ? 5 : (SCAP <= 2048 ? 4 : 3))
     k_extract(ExtractArgs a, uint32_t stage_cap)
 {
+    constexpr bool PART = MODE == MODE_PART || MODE == MODE_PARTS;
     extern __shared__ __align__(128) uint8_t smem[];
     uint8_t *sbuf[2] = {smem, smem + BUF_BYTES};
     uint64_t *s_codes = reinterpret_cast<uint64_t *>(smem + 2 * BUF_BYTES);   // 257 used
@@ -340,8 +341,8 @@ __global__ void __launch_bounds__(EXT_THREADS, MODE == MODE_SCAN ? 5 : (SCAP <= 
     __shared__ __align__(8) uint64_t mbar[2];
     __shared__ uint32_t s_warp[8];
     __shared__ uint32_t s_hist[256];
-    __shared__ uint32_t s_bhist[MODE == MODE_SCAN || MODE == MODE_PART ? 256 : 1];
-    __shared__ unsigned long long s_bpos[MODE == MODE_PART ? 256 : 1];
+    __shared__ uint32_t s_bhist[MODE == MODE_SCAN || PART ? 256 : 1];
+    __shared__ unsigned long long s_bpos[PART ? 256 : 1];
     __shared__ unsigned long long s_bcast[2];
     __shared__ unsigned long long s_boff[MODE == MODE_BLOOM ? 256 : 1];
     __shared__ unsigned long long s_bcap[MODE == MODE_BLOOM ? 256 : 1];
@@ -513,7 +514,10 @@ __global__ void __launch_bounds__(EXT_THREADS, MODE == MODE_SCAN ? 5 : (SCAP <= 
                         const unsigned long long key = f < rc ? f : rc;
                         if (hll_local) hll_add_shared(s_hll, key);
                         else if (a.hll) hll_add_sampled(a.hll + hll_base, key);
-                        if (census) atomicAdd(&s_bhist[key >> 56], 1u);
+                        if (census) {
+                            const unsigned long long ck = a.census_by_string ? ~(f < rc ? rc : f) & kp.topmask : key;
+                            atomicAdd(&s_bhist[ck >> 56], 1u);
+                        }
                         if ((sok >> (q0 + p)) & 1u) atomicAdd(&s_hist[key >> 56], 1u);
                     }
                 }
@@ -551,7 +555,7 @@ __global__ void __launch_bounds__(EXT_THREADS, MODE == MODE_SCAN ? 5 : (SCAP <= 
                     idx += (uint32_t)__popc(e8);
                 }
             }
-            if (MODE == MODE_PART) s_bhist[tid] = 0;
+            if (PART) s_bhist[tid] = 0;
             __syncthreads();
             const uint32_t blo = a.bucket_lo, bhi = a.bucket_hi ? a.bucket_hi : N_BUCKETS;
             for (uint32_t base = 0; base < tot; base += stage_cap) {
@@ -573,9 +577,14 @@ __global__ void __launch_bounds__(EXT_THREADS, MODE == MODE_SCAN ? 5 : (SCAP <= 
                         if ((e8 >> p) & 1u) {
                             if (idx >= base && idx < base + nr) {
                                 const uint64_t f = fwd & kp.topmask;
-                                const unsigned long long key = f < rc ? f : rc;
+                                // the canonical word is the smaller one; its
+                                // string key (first base high) is the complement
+                                // of the other, larger one: rc holds the
+                                // complemented bases in reverse order
+                                const unsigned long long key =
+                                    MODE == MODE_PARTS ? ~(f < rc ? rc : f) & kp.topmask : (f < rc ? f : rc);
                                 s_stage[idx - base] = key;
-                                if (MODE == MODE_PART) {
+                                if (PART) {
                                     // rank inside the tile's share of its bucket (a
                                     // pass of a multi-pass job keeps only its range)
                                     const uint32_t bk = (uint32_t)(key >> 56);
@@ -595,7 +604,7 @@ __global__ void __launch_bounds__(EXT_THREADS, MODE == MODE_SCAN ? 5 : (SCAP <= 
                         bool act = i < nr;
                         warp_insert(act, act ? s_stage[i] : EMPTY_KEY, tr, a.max_probe, flags);
                     }
-                } else if (MODE == MODE_PART) {
+                } else if (PART) {
                     // scatter into the root-prefix buckets (ranks were taken
                     // as the k-mers were formed), one cursor update per bucket;
                     // the round's k-mers are reordered by bucket in shared
@@ -1778,17 +1787,12 @@ __global__ void __launch_bounds__(256) k_merge_buckets(const unsigned long long 
 }
 
 // ---------------------------------------------------------------------------
-// shared-memory sub-bucket path of the Bloom split
+// sub-buckets of the prefix path
 // ---------------------------------------------------------------------------
 
-// Sub-bucket of a k-mer inside its bucket: its filter block (the reference's
-// block = XXH3-128.low64 & (cap - 1), src/BloomFilter.h:215-222) divided by
-// the slice size.
 __device__ __forceinline__ uint32_t sub_of(unsigned long long key, const SubCfg &c)
 {
-    uint64_t lo, hi;
-    xxh3_128_8(key, lo, hi);
-    return (uint32_t)((lo & (c.fcap - 1)) >> c.slice_shift);
+    return (uint32_t)(key >> c.shift) & (c.n_sub - 1);
 }
 
 // Each block counts a contiguous run of work items (bucket-major, so a block
@@ -1956,7 +1960,6 @@ __global__ void __launch_bounds__(SP_THREADS, BPSM) k_subpart_scatter(const unsi
     unsigned long long *s_dst = s_sorted + SUB_SCATTER_ITEM_KEYS;                             // max_sub
     uint32_t *s_cnt = reinterpret_cast<uint32_t *>(s_dst + max_sub);                          // max_sub
     uint32_t *s_start = s_cnt + max_sub;                                                      // max_sub
-    uint16_t *s_sub = reinterpret_cast<uint16_t *>(s_start + max_sub);                        // SUB_SCATTER_ITEM_KEYS
     __shared__ uint32_t s_item0[N_BUCKETS + 1];
     __shared__ uint32_t s_item, s_warp[32];
     const int tid = threadIdx.x;
@@ -2012,9 +2015,7 @@ __global__ void __launch_bounds__(SP_THREADS, BPSM) k_subpart_scatter(const unsi
         for (uint32_t r = 0; r < SP_PER_THREAD; ++r) {
             const uint32_t sub = sr[r] & 0xFFFFu;
             if (sub != 0xFFFFu) {
-                const uint32_t p = s_start[sub] + (sr[r] >> 16);
-                s_sorted[p] = k[r];
-                s_sub[p] = (uint16_t)sub;
+                s_sorted[s_start[sub] + (sr[r] >> 16)] = k[r];
             }
         }
         // destination of sorted index i of sub-bucket s: s_dst[s] + i
@@ -2023,271 +2024,16 @@ __global__ void __launch_bounds__(SP_THREADS, BPSM) k_subpart_scatter(const unsi
             if (j < per && b0 + j < c.n_sub) s_dst[b0 + j] = cur[j] - first[j];
         __syncthreads();
         for (uint32_t i = tid; i < n; i += SP_THREADS) {
-            const uint32_t sb = s_sub[i];
+            const unsigned long long key = s_sorted[i];
+            const uint32_t sb = sub_of(key, c);
             const unsigned long long d = s_dst[sb] + i;
             // estimated regions: a sub-bucket that outgrew its region is
             // reported by its cursor (k_subpart_sizes) and counted exactly
-            if (d < out_cap && (!sub_end || d < sub_end[c.sub_base + sb])) out[d] = s_sorted[i];
+            if (d < out_cap && (!sub_end || d < sub_end[c.sub_base + sb])) out[d] = key;
         }
         for (uint32_t i = tid; i < c.n_sub; i += SP_THREADS) s_cnt[i] = 0;
         __syncthreads();
     }
-}
-
-// Shared-memory counting table of one sub-bucket (2^TBITS slots): linear
-// probing from the key's hash, claims by CAS; a slot only changes from empty
-// to a key.  The home slot is the top TBITS bits of the 64-bit mix
-// (slot_hash), or with FIB of the key times 2^64 / golden ratio (one
-// multiply: placement only, it never affects a count).
-constexpr uint32_t SUB_MAX_PROBE = 512;
-
-template <uint32_t TBITS, bool FIB>
-__device__ __forceinline__ uint32_t sub_table_slot(unsigned long long key)
-{
-    return FIB ? (uint32_t)((key * 0x9E3779B97F4A7C15ULL) >> (64 - TBITS))
-               : (uint32_t)(slot_hash(key) >> (64 - TBITS));
-}
-
-template <uint32_t TBITS, bool FIB>
-__device__ __forceinline__ bool sub_table_add(unsigned long long *tk, uint32_t *tc, unsigned long long key)
-{
-    uint32_t i = sub_table_slot<TBITS, FIB>(key);
-    for (uint32_t n = 0; n < SUB_MAX_PROBE; ++n) {
-        const unsigned long long cur = *(volatile unsigned long long *)&tk[i];
-        if (cur == key) {
-            atomicAdd(&tc[i], 1u);
-            return true;
-        }
-        if (cur == EMPTY_KEY) {
-            const unsigned long long prev = atomicCAS(&tk[i], EMPTY_KEY, key);
-            if (prev == EMPTY_KEY || prev == key) {
-                atomicAdd(&tc[i], 1u);
-                return true;
-            }
-        }
-        i = (i + 1) & ((1u << TBITS) - 1);
-    }
-    return false;
-}
-
-template <uint32_t TBITS, bool FIB>
-__device__ __forceinline__ int sub_table_find(const unsigned long long *tk, unsigned long long key)
-{
-    uint32_t i = sub_table_slot<TBITS, FIB>(key);
-    for (uint32_t n = 0; n < SUB_MAX_PROBE; ++n) {
-        const unsigned long long cur = tk[i];
-        if (cur == key) return (int)i;
-        if (cur == EMPTY_KEY) return -1;
-        i = (i + 1) & ((1u << TBITS) - 1);
-    }
-    return -1;
-}
-
-constexpr uint32_t SUB_PER_THREAD = 4;
-
-// THREADS per block, BPSM blocks per SM, filter slices of at most SLICE
-// blocks, tables of 2^TBITS slots, counts below HBINS histogrammed in shared
-// memory (the two shapes are SubShape 1 and 2 in kc_kernels.cuh).
-template <uint32_t THREADS, uint32_t BPSM, uint32_t SLICE, uint32_t TBITS, uint32_t HBINS, bool FIB>
-__global__ void __launch_bounds__(THREADS, BPSM) k_count_subs(
-    unsigned long long *keys, const unsigned long long *sub_off, const uint32_t *sub_count, const uint8_t *sub_bucket,
-    uint32_t n_sub, const SubCfg *sc, unsigned int *next_sub, uint32_t count_max, uint32_t min_count,
-    uint32_t max_count, unsigned long long *rec_keys, uint32_t *rec_counts, uint64_t rec_cap, unsigned long long *hist,
-    uint32_t *ovf, uint64_t ovf_cap, unsigned long long *counters, uint32_t *bucket_ovf, uint32_t *hb16,
-    uint32_t hb16_shift)
-{
-    extern __shared__ __align__(16) uint8_t cs_smem[];
-    unsigned long long *s_filter = reinterpret_cast<unsigned long long *>(cs_smem);   // 2 * SLICE
-    unsigned long long *s_tk = s_filter + 2 * SLICE;                       // (1u << TBITS)
-    uint32_t *s_tc = reinterpret_cast<uint32_t *>(s_tk + (1u << TBITS));            // (1u << TBITS)
-    uint32_t *s_hist = s_tc + (1u << TBITS);                                        // HBINS
-    unsigned long long *s_queue = reinterpret_cast<unsigned long long *>(s_hist + HBINS);   // (THREADS * SUB_PER_THREAD)
-    __shared__ uint32_t s_warp[32], s_sub, s_lo;   // s_lo: FIRST keys written back
-    __shared__ unsigned long long s_base;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t lt = lanemask_lt();
-    for (uint32_t i = tid; i < HBINS; i += THREADS) s_hist[i] = 0;
-    unsigned long long n_high = 0, n_low = 0, n_low_only = 0, n_distinct = 0;
-    uint32_t n_ovf_subs = 0;
-    bool rec_full = false;
-    for (;;) {
-        if (tid == 0) s_sub = atomicAdd(next_sub, 1u);
-        __syncthreads();
-        const uint32_t sub = s_sub;
-        __syncthreads();
-        if (sub >= n_sub) break;
-        const uint32_t n = sub_count[sub];
-        if (n == 0) continue;
-        const unsigned long long base = sub_off[sub];
-        const uint32_t bucket = sub_bucket[sub];
-        const unsigned long long fcap = sc[bucket].fcap;
-        const uint32_t slice = 1u << sc[bucket].slice_shift;
-        if (tid == 0) s_lo = 0;
-        for (uint32_t i = tid; i < 2 * slice; i += THREADS) s_filter[i] = 0;
-        for (uint32_t i = tid; i < (1u << TBITS); i += THREADS) {
-            s_tk[i] = EMPTY_KEY;
-            s_tc[i] = 0;
-        }
-        __syncthreads();
-        // 1. the reference's two-level Bloom classification (src/BloomFilter.h:233-273)
-        // on the slice; non-FIRST occurrences counted in the table, FIRST ones
-        // written back over the front of the sub-bucket's keys
-        bool full = false;
-        // the next tile's k-mers are loaded while this one is classified (a
-        // tile's FIRST write-back only reaches positions already loaded)
-        unsigned long long kn[SUB_PER_THREAD];
-#pragma unroll
-        for (uint32_t r = 0; r < SUB_PER_THREAD; ++r) {
-            const uint32_t i = r * THREADS + tid;
-            kn[r] = i < n ? __ldcs(&keys[base + i]) : EMPTY_KEY;
-        }
-        __syncthreads();   // the first tile is loaded by every warp before any write-back
-        for (uint32_t t0 = 0; t0 < n; t0 += (THREADS * SUB_PER_THREAD)) {
-            unsigned long long k[SUB_PER_THREAD];
-            uint32_t firsts = 0, highs = 0;
-#pragma unroll
-            for (uint32_t r = 0; r < SUB_PER_THREAD; ++r) {
-                k[r] = kn[r];
-                const uint32_t i = t0 + (THREADS * SUB_PER_THREAD) + r * THREADS + tid;
-                kn[r] = i < n ? __ldcs(&keys[base + i]) : EMPTY_KEY;
-            }
-#pragma unroll
-            for (uint32_t r = 0; r < SUB_PER_THREAD; ++r) {
-                if (t0 + r * THREADS + tid >= n) continue;
-                uint64_t block, m, hi;
-                bloom_probe_hi(k[r], fcap, block, m, hi);
-                unsigned long long *cell = s_filter + 2 * (block & (slice - 1));
-                // a k-mer seen twice already (most of them) needs no update;
-                // otherwise it is FIRST exactly when the seen-once word lacked
-                // its bits (the seen-twice bits are always a subset of the
-                // seen-once bits, so this is the reference's three-way test,
-                // and setting bits already set changes nothing)
-                bool first = false;
-                if ((*(volatile unsigned long long *)&cell[0] & m) != m) {
-                    const unsigned long long old2 = atomicOr(&cell[1], (unsigned long long)m);
-                    first = (old2 & m) != m;
-                    if (!first) atomicOr(&cell[0], (unsigned long long)m);
-                }
-                if (first) firsts |= 1u << r;
-                else highs |= 1u << r;
-            }
-            n_high += (uint64_t)__popc(highs);
-            // the warp's non-FIRST k-mers are queued so that every lane inserts
-            {
-                unsigned long long *q = s_queue + warp * (32 * SUB_PER_THREAD);
-                uint32_t qn = 0;
-#pragma unroll
-                for (uint32_t r = 0; r < SUB_PER_THREAD; ++r) {
-                    const bool h = (highs >> r) & 1u;
-                    const uint32_t b = __ballot_sync(FULL, h);
-                    if (h) q[qn + (uint32_t)__popc(b & lt)] = k[r];
-                    qn += (uint32_t)__popc(b);
-                }
-                __syncwarp();
-                for (uint32_t j = lane; j < qn; j += 32)
-                    if (!sub_table_add<TBITS, FIB>(s_tk, s_tc, q[j])) full = true;
-                __syncwarp();
-            }
-            // FIRST write-back: each warp takes its positions with one
-            // shared-memory atomic.  They lie below the keys classified so
-            // far, i.e. in this tile or earlier ones, whose keys every warp
-            // holds in registers (the barrier at the end of the previous tile
-            // came after every warp's loads of this one)
-            {
-                uint32_t wb[SUB_PER_THREAD], wtot = 0;
-#pragma unroll
-                for (uint32_t r = 0; r < SUB_PER_THREAD; ++r) {
-                    wb[r] = __ballot_sync(FULL, (firsts >> r) & 1u);
-                    wtot += (uint32_t)__popc(wb[r]);
-                }
-                uint32_t wbase = 0;
-                if (lane == 0 && wtot) wbase = atomicAdd(&s_lo, wtot);
-                wbase = __shfl_sync(FULL, wbase, 0);
-                uint32_t before = 0;
-#pragma unroll
-                for (uint32_t r = 0; r < SUB_PER_THREAD; ++r) {
-                    if ((firsts >> r) & 1u) keys[base + wbase + before + (uint32_t)__popc(wb[r] & lt)] = k[r];
-                    before += (uint32_t)__popc(wb[r]);
-                }
-            }
-            n_low += (uint64_t)__popc(firsts);
-            __syncthreads();
-        }
-        if (__syncthreads_or(full)) {
-            if (tid == 0) {
-                ++n_ovf_subs;
-                atomicOr(&bucket_ovf[bucket], 1u);
-            }
-            continue;   // incomplete: the host counts the pass again with more sub-buckets
-        }
-        // 2. FIRST occurrences: a hit adds one to the table count, a miss is a
-        // k-mer seen once (counted, not a record: min_count >= 2)
-        const uint32_t lo_cnt = s_lo;
-        for (uint32_t i0 = tid; i0 < lo_cnt; i0 += THREADS * SUB_PER_THREAD) {
-            unsigned long long kk[SUB_PER_THREAD];
-#pragma unroll
-            for (uint32_t r = 0; r < SUB_PER_THREAD; ++r) {
-                const uint32_t i = i0 + r * THREADS;
-                kk[r] = i < lo_cnt ? __ldcg(&keys[base + i]) : EMPTY_KEY;
-            }
-#pragma unroll
-            for (uint32_t r = 0; r < SUB_PER_THREAD; ++r) {
-                if (i0 + r * THREADS >= lo_cnt) continue;
-                const int sl = sub_table_find<TBITS, FIB>(s_tk, kk[r]);
-                if (sl >= 0) atomicAdd(&s_tc[sl], 1u);
-                else ++n_low_only;
-            }
-        }
-        __syncthreads();
-        // 3. the table's records and histogram
-        uint32_t keep = 0;
-        for (uint32_t i = tid; i < (1u << TBITS); i += THREADS) {
-            if (s_tk[i] == EMPTY_KEY) continue;
-            ++n_distinct;
-            const uint32_t c = s_tc[i] < count_max ? s_tc[i] : count_max;
-            if (c < HBINS) atomicAdd(&s_hist[c], 1u);
-            else if (c < HIST_BINS) atomicAdd(&hist[c], 1ull);
-            else {
-                const unsigned long long q = atomicAdd(&counters[C_OVF_LEN], 1ull);
-                if (q < ovf_cap) ovf[q] = c;
-                else atomicOr(&counters[C_FLAGS], ERR_HIST_OVERFLOW_FULL);
-            }
-            keep += (c >= min_count && c <= max_count) ? 1u : 0u;
-        }
-        uint32_t tk;
-        const uint32_t ok = block_excl_scan_1024(keep, s_warp, tk);
-        if (tid == 0) s_base = tk ? atomicAdd(&counters[C_REC_LEN], (unsigned long long)tk) : 0ull;
-        __syncthreads();
-        unsigned long long q = s_base + ok;
-        for (uint32_t i = tid; i < (1u << TBITS); i += THREADS) {
-            if (s_tk[i] == EMPTY_KEY) continue;
-            const uint32_t c = s_tc[i] < count_max ? s_tc[i] : count_max;
-            if (c < min_count || c > max_count) continue;
-            if (q < rec_cap) {
-                const unsigned long long sk = pair_reverse(s_tk[i]);
-                rec_keys[q] = sk;
-                rec_counts[q] = c;
-                if (hb16) atomicAdd(&hb16[(uint32_t)(sk >> hb16_shift) & 0xFFFFu], 1u);   // the record sort's buckets
-            } else {
-                rec_full = true;
-            }
-            ++q;
-        }
-        __syncthreads();
-    }
-    __syncthreads();
-    for (uint32_t i = tid; i < HBINS; i += THREADS)
-        if (s_hist[i]) atomicAdd(&hist[i], (unsigned long long)s_hist[i]);
-    if (rec_full) atomicOr(&counters[C_FLAGS], ERR_RECORDS_FULL);
-    const unsigned long long v[4] = {n_high, n_low, n_low_only, n_distinct};
-    const int idx[4] = {C_HIGH_LEN, C_LOW_LEN, C_LOW_ONLY, C_DISTINCT};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        unsigned long long x = v[j];
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(FULL, x, o);
-        if ((tid & 31) == 0 && x) atomicAdd(&counters[idx[j]], x);
-    }
-    if (tid == 0 && n_ovf_subs) atomicAdd(&counters[C_SUB_OVF], (unsigned long long)n_ovf_subs);
 }
 
 __global__ void k_hash_batch(const unsigned long long *keys, uint64_t n, unsigned long long *out)
@@ -2427,6 +2173,9 @@ cudaError_t launch_extract(int mode, const ExtractArgs &a, int grid, cudaStream_
     case MODE_PART:
         return part_shape == 2 ? launch_extract_t<MODE_PART, 2048>(a, grid, 2048, st)
                                : launch_extract_t<MODE_PART>(a, grid, STAGE_CAP, st);
+    case MODE_PARTS:
+        return part_shape == 2 ? launch_extract_t<MODE_PARTS, 2048>(a, grid, 2048, st)
+                               : launch_extract_t<MODE_PARTS>(a, grid, STAGE_CAP, st);
     default: return cudaErrorInvalidValue;
     }
 }
@@ -2984,7 +2733,7 @@ cudaError_t launch_subpart_sizes(const unsigned long long *sub_off, const unsign
 
 static size_t subpart_scatter_smem(uint32_t max_sub)
 {
-    return (size_t)SUB_SCATTER_ITEM_KEYS * (8 + 2) + (size_t)max_sub * (8 + 4 + 4);
+    return (size_t)SUB_SCATTER_ITEM_KEYS * 8 + (size_t)max_sub * (8 + 4 + 4);
 }
 
 cudaError_t launch_subpart_scatter(const unsigned long long *keys, const BucketRanges *rg, uint32_t n_items,
@@ -2994,7 +2743,6 @@ cudaError_t launch_subpart_scatter(const unsigned long long *keys, const BucketR
 {
     if (!n_items) return cudaSuccess;
     if (!max_sub || max_sub > SUB_MAX_PER_BUCKET) return cudaErrorInvalidValue;
-    max_sub = (max_sub + 1) & ~1u;   // keeps the 2-byte array after the 4-byte ones aligned
     cudaError_t e = cudaMemsetAsync(next_item, 0, 4, st);
     if (e != cudaSuccess) return e;
     const size_t smem = subpart_scatter_smem(max_sub);
@@ -3009,51 +2757,6 @@ cudaError_t launch_subpart_scatter(const unsigned long long *keys, const BucketR
     note_launch();
     kern<<<grid, SP_THREADS, smem, st>>>(keys, rg, n_items, next_item, sc, sub_cursor, sub_end, out, out_cap, max_sub);
     return cudaGetLastError();
-}
-
-template <uint32_t THREADS, uint32_t BPSM, uint32_t SLICE, uint32_t TBITS, uint32_t HBINS, bool FIB>
-static cudaError_t launch_count_subs_t(unsigned long long *keys, const unsigned long long *sub_off,
-                                       const uint32_t *sub_count, const uint8_t *sub_bucket, uint32_t n_sub,
-                                       const SubCfg *sc, unsigned int *next_sub, uint32_t count_max,
-                                       uint32_t min_count, uint32_t max_count, unsigned long long *rec_keys,
-                                       uint32_t *rec_counts, uint64_t rec_cap, unsigned long long *hist, uint32_t *ovf,
-                                       uint64_t ovf_cap, unsigned long long *counters, uint32_t *bucket_ovf,
-                                       cudaStream_t st, uint32_t *hb16, uint32_t hb16_shift)
-{
-    const size_t smem = (size_t)2 * SLICE * 8 + ((size_t)1 << TBITS) * (8 + 4) + HBINS * 4 +
-                        (size_t)THREADS * SUB_PER_THREAD * 8;
-    auto kern = k_count_subs<THREADS, BPSM, SLICE, TBITS, HBINS, FIB>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    const uint32_t grid = std::min<uint32_t>(n_sub, (uint32_t)sm_count() * BPSM);
-    note_launch();
-    kern<<<grid, THREADS, smem, st>>>(keys, sub_off, sub_count, sub_bucket, n_sub, sc, next_sub, count_max, min_count,
-                                      max_count, rec_keys, rec_counts, rec_cap, hist, ovf, ovf_cap, counters, bucket_ovf,
-                                      hb16, hb16_shift);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_count_subs(unsigned long long *keys, const unsigned long long *sub_off, const uint32_t *sub_count,
-                              const uint8_t *sub_bucket, uint32_t n_sub, const SubCfg *sc, unsigned int *next_sub,
-                              uint32_t count_max, uint32_t min_count, uint32_t max_count, unsigned long long *rec_keys,
-                              uint32_t *rec_counts, uint64_t rec_cap, unsigned long long *hist, uint32_t *ovf,
-                              uint64_t ovf_cap, unsigned long long *counters, uint32_t *bucket_ovf, cudaStream_t st,
-                              uint32_t *hb16, uint32_t hb16_shift, uint32_t shape)
-{
-    if (!n_sub) return cudaSuccess;
-    if (min_count < 2) return cudaErrorInvalidValue;   // singletons are not records on this path
-    cudaError_t e = cudaMemsetAsync(next_sub, 0, 4, st);
-    if (e != cudaSuccess) return e;
-#define KC_COUNT_SUBS_ARGS                                                                                         \
-    keys, sub_off, sub_count, sub_bucket, n_sub, sc, next_sub, count_max, min_count, max_count, rec_keys, rec_counts, \
-        rec_cap, hist, ovf, ovf_cap, counters, bucket_ovf, st, hb16, hb16_shift
-    switch (shape) {
-    case 2: return launch_count_subs_t<256, 4, 1024, 11, 1024, false>(KC_COUNT_SUBS_ARGS);
-    case 3: return launch_count_subs_t<512, 2, 2048, 12, 2048, true>(KC_COUNT_SUBS_ARGS);
-    case 4: return launch_count_subs_t<256, 4, 1024, 11, 1024, true>(KC_COUNT_SUBS_ARGS);
-    default: return launch_count_subs_t<512, 2, 2048, 12, 2048, false>(KC_COUNT_SUBS_ARGS);
-    }
-#undef KC_COUNT_SUBS_ARGS
 }
 
 cudaError_t launch_wait_flag(const unsigned int *flag, uint32_t poll_limit, unsigned long long *flags, cudaStream_t st)

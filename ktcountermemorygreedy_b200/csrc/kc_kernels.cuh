@@ -34,7 +34,7 @@ enum Counter : int {
     C_HIGH_LEN = 2,      // other occurrences (back of the list buffer)
     C_EMIT_LEN = 3,      // plain occurrence list (testing entry point)
     C_REC_LEN = 4,       // output records
-    C_LOW_ONLY = 5,      // low k-mers absent from the table (final count 1)
+    C_LOW_ONLY = 5,      // low k-mers absent from the table (final count 1); prefix path: k-mers seen once
     C_DISTINCT = 6,      // distinct k-mers seen by compaction
     C_OVF_LEN = 7,       // histogram counts >= HIST_BINS
     C_SEL_A = 8,         // query selections
@@ -42,7 +42,8 @@ enum Counter : int {
     C_SUB_OVF = 10,      // sub-buckets whose shared-memory table overflowed
     C_REGION_OVF = 11,   // nonzero: a sub-bucket outgrew its estimated region
     C_KEPT = 12,         // records a counting compaction pass would keep
-    C_COUNT = 16
+    C_UNITS = 16,        // UNIT_CLASSES counts: sort units by size
+    C_COUNT = 24
 };
 
 // One FASTQ file inside a job's device buffer.  Files start on tile
@@ -110,6 +111,7 @@ struct ExtractArgs {
     // root-prefix buckets (single sample): SCAN counts, PART scatters
     unsigned long long *bucket_hist;          // 256 counts (SCAN)
     uint64_t bucket_sample_mask;              // SCAN counts tiles t with (t & mask) == 0
+    int census_by_string;                     // SCAN: buckets by the first four bases (for MODE_PARTS)
     // SCAN over a subset of the tiles: visit[0..n_visit) ascending tile
     // indexes (NULL: every tile); occurrences are then counted on the census
     // tiles only
@@ -122,7 +124,13 @@ struct ExtractArgs {
     const unsigned long long *bucket_end;     // 256 end offsets in `list` (PART)
 };
 
-enum ExtractMode : int { MODE_SCAN = 0, MODE_INSERT = 1, MODE_BLOOM = 2, MODE_EMIT = 3, MODE_PART = 4 };
+// MODE_PART scatters k-mer words by root prefix (the word's top 8 bits, the
+// last four bases), MODE_PARTS string keys (the k bases first-base-high, left
+// aligned) by their first four bases, so that buckets are consecutive ranges
+// of the printed order.
+enum ExtractMode : int {
+    MODE_SCAN = 0, MODE_INSERT = 1, MODE_BLOOM = 2, MODE_EMIT = 3, MODE_PART = 4, MODE_PARTS = 5
+};
 
 constexpr uint32_t WORK_ITEM_KEYS = 2048;   // k-mers per work item (8 per thread)
 constexpr uint32_t BUCKET_HLL_BITS = 10;    // HyperLogLog registers per bucket = 2^10
@@ -151,18 +159,13 @@ uint32_t fill_item_starts(BucketRanges &r);   // sets item0 from len, returns th
 uint32_t fill_item_starts_n(BucketRanges &r, uint64_t item_keys);   // items of item_keys keys
 constexpr uint32_t SUB_SCATTER_ITEM_KEYS = 4096;   // keys per work item of the sub-bucket scatter
 
-// Shared-memory sub-bucket path of the Bloom split: every bucket is cut
-// into n_sub sub-buckets of 2^slice_shift consecutive blocks of its filter (a
-// k-mer's sub-bucket follows from its filter block), so one thread block
-// holds a sub-bucket's filter slice and counting table in shared memory.
-constexpr uint32_t SUB_SLICE_BLOCKS = 2048;     // largest slice (2 words a block): 32 KiB of filter
-constexpr uint32_t SUB_TABLE_BITS = 12;
-constexpr uint32_t SUB_TABLE_SLOTS = 1u << SUB_TABLE_BITS;   // counting-table slots of a sub-bucket
+// Prefix path: the buckets of the string keys' top 8 bits are cut into n_sub
+// sub-buckets each (a power of two) by the bits below, so that one thread
+// block counts a sub-bucket's distinct k-mers in a shared-memory table.
 constexpr uint32_t SUB_MAX_PER_BUCKET = 4096;   // sub-buckets of one bucket
 struct SubCfg {
-    unsigned long long fcap;    // the bucket's filter blocks (a power of two)
-    uint32_t sub_base, n_sub;   // its sub-buckets [sub_base, sub_base + n_sub), n_sub = fcap >> slice_shift
-    uint32_t slice_shift;       // log2 of the blocks of one slice, <= log2(SUB_SLICE_BLOCKS)
+    uint32_t sub_base, n_sub;   // its sub-buckets [sub_base, sub_base + n_sub)
+    uint32_t shift;             // a key's sub-bucket: (key >> shift) & (n_sub - 1)
     uint32_t pad;
 };
 
@@ -296,17 +299,7 @@ cudaError_t launch_select_range(const unsigned long long *keys, const uint32_t *
 // Sub-bucket path.  count: sub_count[sub_base + s] += the keys of bucket b
 // in sub-bucket s.  scatter: every key to out[sub_cursor[its sub-bucket]++]
 // (sub_cursor starts at the exclusive scan of sub_count); its ranges rg are
-// cut into items of SUB_SCATTER_ITEM_KEYS keys (fill_item_starts_n).  count_subs: one
-// block per sub-bucket at a time runs the Bloom split with the filter slice in
-// shared memory, counts the non-FIRST occurrences in a shared-memory table,
-// merges the FIRST ones (written back over the front of the sub-bucket's
-// keys) and appends (and, with hb16, counts every record's printed-order key
-// >> hb16_shift, the record sort's buckets, into hb16[65536]) the table's records (counts saturated at count_max, kept
-// when min_count <= count <= max_count) at rec_keys[C_REC_LEN...]; every
-// table count goes to hist/ovf, the totals to counters (C_REC_LEN,
-// C_LOW_LEN, C_HIGH_LEN, C_LOW_ONLY, C_DISTINCT) and the sub-buckets whose
-// table overflowed to C_SUB_OVF and bucket_ovf[their bucket] (the results
-// are then incomplete).
+// cut into items of SUB_SCATTER_ITEM_KEYS keys (fill_item_starts_n).
 // stride > 1: only every stride-th run of 4 keys is counted (a sample).
 cudaError_t launch_subpart_count(const unsigned long long *keys, const BucketRanges *rg, uint32_t n_items,
                                  const SubCfg *sc, uint32_t *sub_count, cudaStream_t st, uint32_t stride = 1);
@@ -329,19 +322,51 @@ cudaError_t launch_subpart_regions(const uint32_t *sampled, uint32_t n_sub, uint
 cudaError_t launch_subpart_sizes(const unsigned long long *sub_off, const unsigned long long *sub_cursor,
                                  const unsigned long long *sub_end, uint32_t n_sub, uint64_t out_cap, uint32_t *count,
                                  unsigned long long *overflow, cudaStream_t st);
-cudaError_t launch_count_subs(unsigned long long *keys, const unsigned long long *sub_off, const uint32_t *sub_count,
-                              const uint8_t *sub_bucket, uint32_t n_sub, const SubCfg *sc, unsigned int *next_sub,
-                              uint32_t count_max, uint32_t min_count, uint32_t max_count, unsigned long long *rec_keys,
-                              uint32_t *rec_counts, uint64_t rec_cap, unsigned long long *hist, uint32_t *ovf,
-                              uint64_t ovf_cap, unsigned long long *counters, uint32_t *bucket_ovf, cudaStream_t st,
-                              uint32_t *hb16 = nullptr, uint32_t hb16_shift = 0, uint32_t shape = 1);
-// Block shapes of the shared-memory count (kc_tuning.count_shape): 1 and 3
-// run 512-thread blocks, two per SM, filter slices of up to 2048 blocks and
-// 4096-slot tables; 2 and 4 run 256-thread blocks, four per SM, slices of up
-// to 1024 blocks and 2048-slot tables (sub-buckets of half the k-mers).  3
-// and 4 place keys in the table by one multiply instead of the 64-bit mix.
-inline uint32_t sub_slice_blocks(uint32_t shape) { return (shape == 2 || shape == 4) ? 1024u : 2048u; }
-inline uint32_t sub_table_slots(uint32_t shape) { return (shape == 2 || shape == 4) ? 2048u : 4096u; }
+// The shared-memory count of the sub-buckets (kc_count.cu): sub-bucket s's
+// keys are keys[sub_off[s] .. + sub_count[s]).  Its kept records
+// (count_max, min_count, max_count as for the other paths) go to rec_keys /
+// rec_counts from sub_off[s] on, unsorted within each of its sort units;
+// sub_len[s] receives their number.  A unit is the run
+// [off, off + len) of a sub-bucket's records; the units of size class c
+// (len <= UNIT_CAP0 << c) are listed at units[c * unit_cap], C_UNITS + c of
+// them.  Every k-mer's count goes to hist / ovf; totals to counters
+// (C_REC_LEN, C_DISTINCT, C_LOW_ONLY: k-mers seen once).  Sub-buckets that no
+// number of rounds fits, and more units than unit_cap, are counted in
+// C_SUB_OVF (and bucket_ovf[their bucket]): the results are then incomplete.
+constexpr uint32_t UNIT_CAP0 = 1024, UNIT_CLASSES = 4;
+struct SubUnit {
+    uint32_t sub, off, len, pad;
+};
+struct PrefixCountArgs {
+    const unsigned long long *keys, *sub_off;
+    const uint32_t *sub_count;
+    const uint8_t *sub_bucket;   // bucket of each sub-bucket
+    const SubCfg *sc;
+    uint32_t n_sub;
+    unsigned int *next_sub;
+    uint32_t count_max, min_count, max_count;
+    unsigned long long *rec_keys;
+    uint32_t *rec_counts, *sub_len;
+    SubUnit *units;
+    uint32_t unit_cap;
+    unsigned long long *hist;
+    uint32_t *ovf;
+    uint64_t ovf_cap;
+    unsigned long long *counters;
+    uint32_t *bucket_ovf;
+};
+// shape (kc_tuning.count_shape): 1 and 3 run 512-thread blocks, two per SM,
+// with 8192-slot tables; 2 and 4 run 256-thread blocks, four per SM, with
+// 4096-slot tables (sub-buckets of half the k-mers).
+cudaError_t launch_count_prefix(const PrefixCountArgs &a, uint32_t shape, cudaStream_t st);
+inline uint32_t sub_table_slots(uint32_t shape) { return (shape == 2 || shape == 4) ? 4096u : 8192u; }
+// Every unit's records sorted and written, as k-mer words, to out_k / out_v
+// from sub_final[sub] + off on (sub_final: the exclusive scan of sub_len);
+// n_units: units per class (host values).
+cudaError_t launch_unit_sort(const unsigned long long *tk, const uint32_t *tv, const unsigned long long *sub_off,
+                             const unsigned long long *sub_final, const SubUnit *units, uint32_t unit_cap,
+                             const uint32_t *n_units, unsigned long long *out_k, uint32_t *out_v, uint64_t out_cap,
+                             uint32_t k, cudaStream_t st);
 cudaError_t launch_bloom_buckets(const unsigned long long *keys, const BucketRanges *rg, uint32_t n_items,
                                  unsigned int *next_item, const BucketCfg *cfg, unsigned long long *bits,
                                  unsigned long long *out, unsigned long long *low_cnt, unsigned long long *high_cnt,

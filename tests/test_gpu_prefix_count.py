@@ -1,0 +1,95 @@
+"""Counting by printed-order prefix in shared memory (Bloom jobs of any size and
+plain jobs from 4 MiB of FASTQ on), where it can go wrong: k below and at the
+bucket prefix, k-mers that share a long prefix (tables counted in rounds,
+buckets cut again, the global-memory fallback), one k-mer of very many
+occurrences, and sort units of every size class.  Integer work: exact
+comparisons against the oracle."""
+import random
+
+import numpy as np
+import pytest
+
+import oracle_lib as O
+
+pytestmark = pytest.mark.gpu
+U32 = 0xFFFFFFFF
+
+
+@pytest.fixture(scope="module")
+def counter():
+    import ktcountermemorygreedy_b200 as kc
+    with kc.KmerCounter(max_inflight_jobs=1) as c:
+        yield c
+
+
+def _fastq(seqs):
+    return "".join(f"@r{i}\n{s}\n+\n{'I' * len(s)}\n" for i, s in enumerate(seqs)).encode()
+
+
+def _check(c, fq, k, min_count=1, **kw):
+    all_k, all_c = O.exact_records([fq], k, U32)
+    m = all_c >= min_count
+    r = c.count([fq], k=k, count_max=U32, min_count=min_count, hist_max=300, top_n=20, want_le2=True, **kw)
+    assert np.array_equal(r.keys, all_k[m]) and np.array_equal(r.counts, all_c[m])
+    assert r.hist.tolist() == O.histogram(all_c, 1, 300).tolist()
+    assert r.distinct == len(all_k) and r.occurrences == int(all_c.sum(dtype=np.uint64))
+    le = all_c[m] <= 2
+    assert np.array_equal(r.le2_keys, all_k[m][le])
+    if kw.get("bloom"):
+        assert r.low_len + r.high_len == r.occurrences
+    return r
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 8, 10, 13, 21, 31, 32])
+def test_small_and_large_k(counter, k):
+    rnd = random.Random(k)
+    g = "".join(rnd.choice("ACGT") for _ in range(20_000))
+    seqs = [g[i:i + 150] for i in (rnd.randrange(len(g) - 150) for _ in range(3000))] + ["ACGTN" * 20, "A" * 400, "T" * 60]
+    fq = _fastq(seqs)
+    for mc in (1, 2):
+        r = _check(counter, fq, k, mc, bloom=True, memory_gb=1)
+        assert r.smem_passes == 1 and r.smem_fallbacks == 0
+
+
+@pytest.mark.parametrize("prefix,n,fallback", [(4, 60_000, False), (9, 60_000, False), (11, 30_000, False),
+                                               (12, 30_000, True), (14, 60_000, True)])
+@pytest.mark.parametrize("shape", [1, 2])
+def test_many_kmers_of_one_prefix(counter, prefix, n, fallback, shape):
+    """n distinct k-mers that start with the same `prefix` bases, some of them
+    repeated: too many for one sub-bucket's table.  Sub-buckets and rounds
+    tell at most 13 bases apart (8 + 12 + 6 bits), so 12 shared bases leave 4
+    ranges of 7500 k-mers, more than a table takes."""
+    rnd = random.Random(prefix)
+    k = 31
+    p = "AC" + "".join(rnd.choice("ACGT") for _ in range(prefix - 2))
+    # first base A, last base A: the forward strand is the canonical one
+    seqs = list({p + "".join(rnd.choice("ACGT") for _ in range(k - prefix - 1)) + "A" for _ in range(n)})
+    seqs += [seqs[i % 777] for i in range(5000)] + ["".join(rnd.choice("ACGT") for _ in range(150)) for _ in range(200)]
+    rnd.shuffle(seqs)
+    counter.set_tuning(count_shape=shape)
+    for mc in (1, 2):
+        r = _check(counter, _fastq(seqs), k, mc, bloom=True, memory_gb=1)
+        assert (r.smem_fallbacks > 0) == fallback and r.smem_passes == (0 if fallback else 1)
+    counter.set_tuning(count_shape=1)
+
+
+def test_one_kmer_of_many_occurrences(counter):
+    """Poly-A reads: one sub-bucket holds a few million equal keys."""
+    rnd = random.Random(1)
+    seqs = ["A" * 5000] * 500 + ["".join(rnd.choice("ACGT") for _ in range(150)) for _ in range(20_000)]
+    rnd.shuffle(seqs)
+    fq = _fastq(seqs)
+    assert len(fq) > 4 << 20
+    _check(counter, fq, 31)              # a plain job on the prefix path
+    _check(counter, fq, 31, 2, bloom=True, memory_gb=1)
+
+
+@pytest.mark.parametrize("per_bucket", [900, 1100, 2100, 4200, 8100, 16500])
+def test_sort_units_of_every_size(counter, per_bucket):
+    """Distinct k-mers spread over the buckets: records per unit on both sides
+    of each size class's edge."""
+    rng = np.random.default_rng(per_bucket)
+    bases = np.frombuffer(b"ACGT", np.uint8)
+    reads = bases[rng.integers(0, 4, size=(per_bucket * 256 // 118, 150))]
+    fq = b"".join(b"@r\n" + r.tobytes() + b"\n+\n" + b"I" * 150 + b"\n" for r in reads)
+    _check(counter, fq, 31, 1, bloom=True, memory_gb=1)
