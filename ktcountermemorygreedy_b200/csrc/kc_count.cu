@@ -31,8 +31,8 @@ namespace {
 
 constexpr uint32_t FULLW = 0xffffffffu;
 constexpr uint32_t CP_PER_THREAD = 4;       // keys per thread whose first probes are in flight together
-constexpr uint32_t CP_HIST = 1024;          // counts below this are histogrammed in shared memory
-constexpr uint32_t CP_MAX_PROBE = 128;      // a probe this long: the table is taken as full
+constexpr uint32_t CP_HIST = 512;           // counts below this are histogrammed in shared memory
+constexpr uint32_t CP_QUEUE = 64;           // keys a warp has waiting for their next probe
 constexpr uint32_t CP_MAX_ROUNDS = 64;      // rounds a sub-bucket may be cut into
 
 __device__ __forceinline__ uint32_t lanes_below()
@@ -42,18 +42,27 @@ __device__ __forceinline__ uint32_t lanes_below()
     return m;
 }
 
-// Home slot of a key in a table of 2^lg slots: two 32-bit multiplies over its
-// halves (the top bits are the same for a whole sub-bucket, so the low half
-// leads).  Placement only; it never affects a count.
-__device__ __forceinline__ uint32_t slot_of(unsigned long long key, uint32_t lg)
+// Placement hash of a key: two 32-bit multiplies over its halves (the top
+// bits are the same for a whole sub-bucket, so the low half leads).  The top
+// bits are its home slot, an odd number from the next ones its probe step.  It
+// never affects a count.
+__device__ __forceinline__ uint32_t mix_of(unsigned long long key)
 {
-    const uint32_t x = ((uint32_t)key * 0x9E3779B1u + (uint32_t)(key >> 32)) * 0x85EBCA77u;
-    return x >> (32 - lg);
+    return ((uint32_t)key * 0x9E3779B1u + (uint32_t)(key >> 32)) * 0x85EBCA77u;
 }
 
 // Counts one sub-bucket per block at a time.  The keys are inserted into an
 // open-addressing table in shared memory (a slot only changes from empty to a
-// key, by CAS; no barrier between tiles), then one sweep writes the kept
+// key, by CAS; no barrier between tiles): every key looks at its home slot,
+// where most are found and counted; the others wait in the warp's queue until
+// there are 32 of them, so that a probe step (claim, count, or on to the next
+// slot and back into the queue) has all lanes busy.  (Each lane stepping its
+// own keys to the end left 16 of 32 lanes active and 198 warp instructions per
+// 32 keys; with the queue 23 and 172.  A ring that refilled each idle lane at
+// every step took 248: more bookkeeping than probing.)  Bound by instruction
+// issue (72%) and shared-memory wavefronts (63%): 2.4G k-mers of the 20M-read
+// job 18.5 -> 15.6 ms, 480M k-mers with every record kept 3.8 -> 3.15, 25M
+// mostly distinct ones 0.92 -> 0.49.  Then one sweep writes the kept
 // records to the front of the sub-bucket's place in the record arrays,
 // adds every count to the histogram and empties the table for the next
 // sub-bucket.  A table that fills up (more distinct k-mers than it holds) is
@@ -69,6 +78,10 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
     unsigned long long *s_tk = reinterpret_cast<unsigned long long *>(cp_smem);   // 2^TBITS keys
     uint32_t *s_tc = reinterpret_cast<uint32_t *>(s_tk + (1u << TBITS));          // their counts
     uint32_t *s_hist = s_tc + (1u << TBITS);                                      // CP_HIST
+    unsigned long long *q_key =                                                   // CP_QUEUE per warp
+        reinterpret_cast<unsigned long long *>(s_hist + CP_HIST) + (threadIdx.x >> 5) * CP_QUEUE;
+    uint16_t *q_slot = reinterpret_cast<uint16_t *>(s_hist + CP_HIST + 2 * CP_QUEUE * (THREADS / 32)) +
+                       (threadIdx.x >> 5) * CP_QUEUE;
     __shared__ uint32_t s_out, s_full, s_next, s_next_n, s_next_plen;
     __shared__ unsigned long long s_next_off;
     constexpr uint32_t TILE_KEYS = THREADS * CP_PER_THREAD;
@@ -81,7 +94,8 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
         s_tc[i] = 0;
     }
     for (uint32_t i = tid; i < CP_HIST; i += THREADS) s_hist[i] = 0;
-    unsigned long long n_distinct = 0, n_once = 0, n_one = 0, n_kept = 0;
+    uint32_t n_distinct = 0, n_once = 0, n_one = 0;   // per lane: below 2^32 whatever the pass
+    unsigned long long n_kept = 0;
     uint32_t n_ovf_subs = 0, rounds0 = 1;
     bool unit_full = false;
     // thread 0 takes the next sub-bucket while this one is counted
@@ -126,7 +140,40 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
             const uint32_t rmask = rounds - 1;
             const int rsh = 64 - (int)plen - (31 - __clz(rounds));   // rounds == 1: unused
             const bool reread = rd > 0 || failed;
-            bool full = false;
+            // a warp takes at most this many probe steps (a table less than
+            // about five sixths full needs far fewer)
+            const uint32_t hsh = 32 - lg;
+            uint32_t qn = 0, steps = 0, most_steps = 3 * (n / THREADS + 1) + 64;
+            // one more probe of the last `m` queued keys (m <= 32); those that
+            // meet another key stay queued at their next slot
+            auto probe_queue = [&](uint32_t m) {
+                __syncwarp();
+                qn -= m;
+                ++steps;
+                const bool in = lane < (int)m;
+                unsigned long long key = 0;
+                uint32_t slot = 0;
+                bool wait = false;
+                if (in) {
+                    key = q_key[qn + lane];
+                    slot = q_slot[qn + lane];
+                    unsigned long long cur = *(volatile unsigned long long *)&s_tk[slot];
+                    if (cur == EMPTY_KEY) {
+                        cur = atomicCAS(&s_tk[slot], EMPTY_KEY, key);
+                        if (cur == EMPTY_KEY) cur = key;   // claimed
+                    }
+                    wait = cur != key;
+                    if (!wait) atomicAdd(&s_tc[slot], 1u);
+                }
+                const uint32_t w = __ballot_sync(FULLW, wait);
+                if (wait) {
+                    const uint32_t at = qn + (uint32_t)__popc(w & lt);
+                    q_key[at] = key;
+                    q_slot[at] = (uint16_t)((slot + (mix_of(key) >> 3 | 1u)) & smask);
+                }
+                qn += (uint32_t)__popc(w);
+                __syncwarp();
+            };
             for (uint32_t t0 = 0; t0 < n; t0 += TILE_KEYS) {
                 unsigned long long k[CP_PER_THREAD];
                 if (reread) {
@@ -148,36 +195,39 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
                     for (uint32_t r = 0; r < CP_PER_THREAD; ++r)
                         if (((uint32_t)(k[r] >> rsh) & rmask) != rd) k[r] = EMPTY_KEY;
                 }
+                // the home slots: most keys are there already and only counted
                 uint32_t slot[CP_PER_THREAD];
                 unsigned long long cur[CP_PER_THREAD];
 #pragma unroll
                 for (uint32_t r = 0; r < CP_PER_THREAD; ++r) {
-                    slot[r] = slot_of(k[r], lg);
+                    slot[r] = mix_of(k[r]) >> hsh;
                     cur[r] = *(volatile unsigned long long *)&s_tk[slot[r]];
                 }
 #pragma unroll
                 for (uint32_t r = 0; r < CP_PER_THREAD; ++r) {
-                    if (k[r] == EMPTY_KEY) continue;
-                    for (uint32_t p = 0;;) {
-                        if (cur[r] == EMPTY_KEY) {
-                            cur[r] = atomicCAS(&s_tk[slot[r]], EMPTY_KEY, k[r]);
-                            if (cur[r] == EMPTY_KEY) cur[r] = k[r];   // claimed
+                    const bool in = k[r] != EMPTY_KEY, hit = in && cur[r] == k[r];
+                    if (hit) atomicAdd(&s_tc[slot[r]], 1u);
+                    const uint32_t w = __ballot_sync(FULLW, in && !hit);
+                    if (in && !hit) {
+                        const uint32_t at = qn + (uint32_t)__popc(w & lt);
+                        q_key[at] = k[r];
+                        q_slot[at] = (uint16_t)slot[r];
+                    }
+                    qn += (uint32_t)__popc(w);
+                    // below 32 again before the next keys come (the queue holds 64)
+                    while (qn >= 32) {
+                        if (steps > most_steps) {
+                            qn = 0;   // full: counted again anyway
+                            s_full = 1;
+                        } else {
+                            probe_queue(32);
                         }
-                        if (cur[r] == k[r]) {
-                            atomicAdd(&s_tc[slot[r]], 1u);
-                            break;
-                        }
-                        if (++p == CP_MAX_PROBE) {
-                            full = true;
-                            break;
-                        }
-                        slot[r] = (slot[r] + 1) & smask;
-                        cur[r] = *(volatile unsigned long long *)&s_tk[slot[r]];
                     }
                 }
-                if (full) s_full = 1;
-                if (*(volatile uint32_t *)&s_full) break;
+                if (__any_sync(FULLW, *(volatile uint32_t *)&s_full != 0)) break;
             }
+            while (qn && steps <= most_steps) probe_queue(qn < 32 ? qn : 32);
+            if (qn) s_full = 1;
             __syncthreads();
             if (s_full) {
                 // emptied and counted again over half the range
@@ -205,38 +255,49 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
             }
             // the sweep: records out, histogram, table emptied
             const unsigned long long out = base + off;
-            for (uint32_t i0 = 0; i0 <= smask; i0 += THREADS) {
-                const uint32_t i = i0 + tid;
-                unsigned long long key = EMPTY_KEY;
-                uint32_t c = 0;
-                bool keep = false;
-                if (i <= smask) key = s_tk[i];
-                if (key != EMPTY_KEY) {
-                    const uint32_t raw = s_tc[i];
-                    s_tk[i] = EMPTY_KEY;
-                    s_tc[i] = 0;
-                    ++n_distinct;
-                    n_once += raw == 1;
-                    c = raw < a.count_max ? raw : a.count_max;
-                    if (c == 1) ++n_one;   // most k-mers of many inputs: one shared bin would serialize
-                    else if (c < CP_HIST) atomicAdd(&s_hist[c], 1u);
-                    else if (c < HIST_BINS) atomicAdd(&a.hist[c], 1ull);
-                    else {
-                        const unsigned long long q = atomicAdd(&a.counters[C_OVF_LEN], 1ull);
-                        if (q < a.ovf_cap) a.ovf[q] = c;
-                        else atomicOr(&a.counters[C_FLAGS], ERR_HIST_OVERFLOW_FULL);
+            for (uint32_t i0 = 0; i0 <= smask; i0 += 2 * THREADS) {
+                const uint32_t i = i0 + 2 * tid;   // two slots a thread
+                ulonglong2 kk = make_ulonglong2(EMPTY_KEY, EMPTY_KEY);
+                uint32_t c[2] = {0, 0};
+                bool keep[2] = {false, false};
+                if (i <= smask) kk = *reinterpret_cast<const ulonglong2 *>(&s_tk[i]);
+                const unsigned long long key[2] = {kk.x, kk.y};
+                if (kk.x != EMPTY_KEY || kk.y != EMPTY_KEY) {
+                    const uint2 raw2 = *reinterpret_cast<const uint2 *>(&s_tc[i]);
+                    *reinterpret_cast<ulonglong2 *>(&s_tk[i]) = make_ulonglong2(EMPTY_KEY, EMPTY_KEY);
+                    *reinterpret_cast<uint2 *>(&s_tc[i]) = make_uint2(0u, 0u);
+                    const uint32_t raw[2] = {raw2.x, raw2.y};
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        if (key[j] == EMPTY_KEY) continue;
+                        ++n_distinct;
+                        n_once += raw[j] == 1;
+                        c[j] = raw[j] < a.count_max ? raw[j] : a.count_max;
+                        if (c[j] == 1) ++n_one;   // most k-mers of many inputs: one shared bin would serialize
+                        else if (c[j] < CP_HIST) atomicAdd(&s_hist[c[j]], 1u);
+                        else if (c[j] < HIST_BINS) atomicAdd(&a.hist[c[j]], 1ull);
+                        else {
+                            const unsigned long long q = atomicAdd(&a.counters[C_OVF_LEN], 1ull);
+                            if (q < a.ovf_cap) a.ovf[q] = c[j];
+                            else atomicOr(&a.counters[C_FLAGS], ERR_HIST_OVERFLOW_FULL);
+                        }
+                        keep[j] = c[j] >= a.min_count && c[j] <= a.max_count;
                     }
-                    keep = c >= a.min_count && c <= a.max_count;
                 }
-                const uint32_t b = __ballot_sync(FULLW, keep);
-                if (b) {
+                const uint32_t b0 = __ballot_sync(FULLW, keep[0]), b1 = __ballot_sync(FULLW, keep[1]);
+                if (b0 | b1) {
                     uint32_t w = 0;
-                    if (lane == 0) w = atomicAdd(&s_out, (uint32_t)__popc(b));
+                    if (lane == 0) w = atomicAdd(&s_out, (uint32_t)(__popc(b0) + __popc(b1)));
                     w = __shfl_sync(FULLW, w, 0);
-                    if (keep) {
-                        const unsigned long long q = out + w + (uint32_t)__popc(b & lt);
-                        a.rec_keys[q] = key;
-                        a.rec_counts[q] = c;
+                    if (keep[0]) {
+                        const unsigned long long q = out + w + (uint32_t)__popc(b0 & lt);
+                        a.rec_keys[q] = key[0];
+                        a.rec_counts[q] = c[0];
+                    }
+                    if (keep[1]) {
+                        const unsigned long long q = out + w + (uint32_t)(__popc(b0) + __popc(b1 & lt));
+                        a.rec_keys[q] = key[1];
+                        a.rec_counts[q] = c[1];
                     }
                 }
             }
@@ -408,7 +469,7 @@ int n_sms()
 template <uint32_t THREADS, uint32_t BPSM, uint32_t TBITS>
 cudaError_t launch_count_prefix_t(const PrefixCountArgs &a, cudaStream_t st)
 {
-    const size_t smem = ((size_t)1 << TBITS) * 12 + CP_HIST * 4;
+    const size_t smem = ((size_t)1 << TBITS) * 12 + CP_HIST * 4 + (THREADS / 32) * CP_QUEUE * 10;
     auto kern = k_count_prefix<THREADS, BPSM, TBITS>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;

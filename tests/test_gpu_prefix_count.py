@@ -52,13 +52,13 @@ def test_small_and_large_k(counter, k):
 
 
 @pytest.mark.parametrize("prefix,n,fallback", [(4, 60_000, False), (9, 60_000, False), (11, 30_000, False),
-                                               (12, 30_000, True), (14, 60_000, True)])
+                                               (12, 40_000, True), (14, 60_000, True)])
 @pytest.mark.parametrize("shape", [1, 2])
 def test_many_kmers_of_one_prefix(counter, prefix, n, fallback, shape):
     """n distinct k-mers that start with the same `prefix` bases, some of them
     repeated: too many for one sub-bucket's table.  Sub-buckets and rounds
     tell at most 13 bases apart (8 + 12 + 6 bits), so 12 shared bases leave 4
-    ranges of 7500 k-mers, more than a table takes."""
+    ranges of 10000 k-mers, more than a table has slots."""
     rnd = random.Random(prefix)
     k = 31
     p = "AC" + "".join(rnd.choice("ACGT") for _ in range(prefix - 2))
