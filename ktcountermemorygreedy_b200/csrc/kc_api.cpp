@@ -922,8 +922,8 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
             CK(cudaMemcpyAsync(d_cfg_b, hs.up(cfg.data(), N_BUCKETS), N_BUCKETS * sizeof(BucketCfg),
                                cudaMemcpyHostToDevice, st));
             // each bucket-major launch gets its 256 ranges, not a list of items
-            auto upload_ranges = [&](BucketRanges &r, uint32_t &n_items) {
-                n_items = fill_item_starts(r);
+            auto upload_ranges = [&](BucketRanges &r, uint32_t &n_items, uint64_t item_keys = WORK_ITEM_KEYS) {
+                n_items = fill_item_starts_n(r, item_keys);
                 BucketRanges *d = ds.n<BucketRanges>(1);
                 CK(cudaMemcpyAsync(d, hs.up(&r, 1), sizeof(BucketRanges), cudaMemcpyHostToDevice, st));
                 return d;
@@ -982,8 +982,11 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
                         br.begin[b] = cfg[b].key_base;
                         br.len[b] = cfg[b].key_len;
                     }
-                    uint32_t n_items = 0;
-                    BucketRanges *d_br = upload_ranges(br, n_items);
+                    const bool sampled = !exact_regions && pass_keys >= tn.sampled_region_keys;
+                    const uint32_t stride = sampled ? SUB_REGION_SAMPLE : 1;
+                    uint32_t n_items = 0, n_sp_items = 0;
+                    BucketRanges *d_br = upload_ranges(br, n_items, SUB_COUNT_KEYS * stride);
+                    BucketRanges *d_bs = upload_ranges(br, n_sp_items, sub_scatter_item_keys(max_sub));
                     CK(cudaMemcpyAsync(d_sc, hs.up(sc.data(), N_BUCKETS), N_BUCKETS * sizeof(SubCfg),
                                        cudaMemcpyHostToDevice, st));
                     CK(cudaMemcpyAsync(d_sb, hs.up(sb.data(), n_sub), n_sub, cudaMemcpyHostToDevice, st));
@@ -993,24 +996,19 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
                     CK(cudaMemsetAsync(counters + C_REC_LEN, 0, 3 * 8, st));   // C_REC_LEN, C_LOW_ONLY, C_DISTINCT
                     CK(cudaMemsetAsync(counters + C_SUB_OVF, 0, 2 * 8, st));   // C_SUB_OVF, C_REGION_OVF
                     CK(cudaMemsetAsync(counters + C_UNITS, 0, UNIT_CLASSES * 8, st));
-                    const bool sampled = !exact_regions && pass_keys >= tn.sampled_region_keys;
                     unsigned long long *sub_end = nullptr;
                     clk.begin(9);
                     if (sampled) {
                         uint32_t *region = ds.n<uint32_t>(n_sub);
                         sub_end = ds.n<unsigned long long>(n_sub);
-                        CK(launch_subpart_count(keys, d_br, n_items, d_sc, sub_count, st, SUB_REGION_SAMPLE));
-                        CK(launch_subpart_regions(sub_count, n_sub, SUB_REGION_SAMPLE, region, sub_off, sub_end, sub_cur,
+                        CK(launch_subpart_count(keys, d_br, n_items, d_sc, sub_count, st, stride));
+                        CK(launch_subpart_regions(sub_count, n_sub, stride, region, sub_off, sub_end, sub_cur,
                                                   sub_tmp, st));
                     } else {
                         CK(launch_subpart_count(keys, d_br, n_items, d_sc, sub_count, st));
                         CK(launch_scan_u32(sub_count, sub_off, n_sub, sub_tmp, st));
                         CK(cudaMemcpyAsync(sub_cur, sub_off, (size_t)n_sub * 8, cudaMemcpyDeviceToDevice, st));
                     }
-                    BucketRanges bs = br;
-                    const uint32_t n_sp_items = fill_item_starts_n(bs, SUB_SCATTER_ITEM_KEYS);
-                    BucketRanges *d_bs = ds.n<BucketRanges>(1);
-                    CK(cudaMemcpyAsync(d_bs, hs.up(&bs, 1), sizeof(BucketRanges), cudaMemcpyHostToDevice, st));
                     CK(launch_subpart_scatter(keys, d_bs, n_sp_items, sub_next, d_sc, sub_cur, list, list_cap, max_sub,
                                               st, sub_end, (uint32_t)tn.scatter_shape));
                     if (sampled)

@@ -1796,8 +1796,16 @@ __device__ __forceinline__ uint32_t sub_of(unsigned long long key, const SubCfg 
 }
 
 // Each block counts a contiguous run of work items (bucket-major, so a block
-// meets one or two buckets) in a shared histogram, flushed per bucket.
-constexpr uint32_t SPC_PER_THREAD = WORK_ITEM_KEYS / 256;
+// meets one or two buckets) in a shared histogram, flushed per bucket.  An
+// item is SUB_COUNT_KEYS keys per stride: with stride > 1 only every stride-th
+// run of 16 keys (one 128-byte line) is counted, a sample.  Sampling single
+// lines rather than whole work items keeps the sampled count of a sub-bucket
+// close to binomial: a work item holds several keys of each sub-bucket, and
+// sampling items would multiply the count's variance by about that number.
+// Either way a thread's SPC_PER_THREAD loads of an item are in flight together
+// (the sample read one key per thread and item, a 32-byte sector of every
+// eighth: 2.0 ms for 2.4G keys).
+constexpr uint32_t SPC_PER_THREAD = SUB_COUNT_KEYS / 256;
 __global__ void __launch_bounds__(256) k_subpart_count(const unsigned long long *keys, const BucketRanges *rg,
                                                        uint32_t n_items, const SubCfg *sc, uint32_t *sub_count,
                                                        uint32_t stride)
@@ -1812,7 +1820,7 @@ __global__ void __launch_bounds__(256) k_subpart_count(const unsigned long long 
     uint32_t cur = N_BUCKETS;
     SubCfg c{};
     for (uint32_t it = it0; it < it1; ++it) {
-        const WorkItem w = work_item(rg, s_item0, it);
+        const WorkItem w = work_item_n(rg, s_item0, it, SUB_COUNT_KEYS * stride);
         if (w.bucket != cur) {
             if (cur != N_BUCKETS) {
                 __syncthreads();
@@ -1826,31 +1834,16 @@ __global__ void __launch_bounds__(256) k_subpart_count(const unsigned long long 
             cur = w.bucket;
             c = sc[cur];
         }
-        if (stride > 1) {
-            // a sample: every stride-th run of 4 keys (one 32-byte sector).
-            // Sampling single sectors rather than whole work items keeps the
-            // sampled count of a sub-bucket close to binomial: a work item
-            // holds several keys of each sub-bucket, and sampling items would
-            // multiply the count's variance by about that number.
-            for (unsigned long long j = tid;; j += 256) {
-                const unsigned long long i = w.begin + 4ull * stride * (j >> 2) + (j & 3);
-                if (i >= w.end) break;
-                atomicAdd(&s_h[sub_of(__ldcs(&keys[i]), c)], 1u);
-            }
-            continue;
-        }
-        // a work item is 8 keys per thread: their loads are issued together
-        for (unsigned long long i0 = w.begin + tid; i0 < w.end; i0 += 256 * SPC_PER_THREAD) {
-            unsigned long long kk[SPC_PER_THREAD];
+        unsigned long long kk[SPC_PER_THREAD];
 #pragma unroll
-            for (uint32_t r = 0; r < SPC_PER_THREAD; ++r) {
-                const unsigned long long i = i0 + r * 256;
-                kk[r] = i < w.end ? __ldcs(&keys[i]) : 0ull;
-            }
-#pragma unroll
-            for (uint32_t r = 0; r < SPC_PER_THREAD; ++r)
-                if (i0 + r * 256 < w.end) atomicAdd(&s_h[sub_of(kk[r], c)], 1u);
+        for (uint32_t r = 0; r < SPC_PER_THREAD; ++r) {
+            const uint32_t j = r * 256 + tid;
+            const unsigned long long i = w.begin + 16ull * stride * (j >> 4) + (j & 15);
+            kk[r] = i < w.end ? __ldcs(&keys[i]) : EMPTY_KEY;
         }
+#pragma unroll
+        for (uint32_t r = 0; r < SPC_PER_THREAD; ++r)
+            if (kk[r] != EMPTY_KEY) atomicAdd(&s_h[sub_of(kk[r], c)], 1u);
     }
     __syncthreads();
     if (cur != N_BUCKETS)
@@ -1859,7 +1852,7 @@ __global__ void __launch_bounds__(256) k_subpart_count(const unsigned long long 
 }
 
 // Regions of the sub-buckets estimated from a 1-in-stride sample of the
-// keys (sectors of 4 keys): n = stride * sampled count, region = n +
+// keys (lines of 16 keys): n = stride * sampled count, region = n +
 // 20 sqrt(n) + 64; the estimate's standard deviation is about
 // sqrt(stride * n), under 2.9 sqrt(n) for stride 8, so the margin is about
 // 7 of them.
@@ -1930,22 +1923,25 @@ __device__ __forceinline__ uint32_t block_excl_scan_1024(uint32_t v, uint32_t *s
     return base + x - v;
 }
 
-// One work item (SUB_SCATTER_ITEM_KEYS keys of one bucket) per round: the
-// keys are ranked by sub-bucket in shared memory, every sub-bucket of the
-// item takes its range with one cursor update, and the item's keys are
-// written reordered by sub-bucket (consecutive threads store consecutive
-// addresses).  Items are larger than the other bucket kernels' so that a
-// sub-bucket's run in an item spans several sectors.
-constexpr uint32_t SP_THREADS = 512;
-constexpr uint32_t SP_PER_THREAD = SUB_SCATTER_ITEM_KEYS / SP_THREADS;
-constexpr uint32_t SP_MAX_BINS = (SUB_MAX_PER_BUCKET + SP_THREADS - 1) / SP_THREADS;   // sub-buckets per thread
-static_assert(SUB_SCATTER_ITEM_KEYS % SP_THREADS == 0 && SUB_SCATTER_ITEM_KEYS <= 65536, "item layout");
-
-// MAXB: sub-buckets per thread in the rank scan (the cursor updates held in
-// registers until after the reorder); launches whose buckets have at most
-// 2 * SP_THREADS sub-buckets use MAXB = 2 and fit three blocks per SM.
-template <uint32_t MAXB, uint32_t BPSM>
-__global__ void __launch_bounds__(SP_THREADS, BPSM) k_subpart_scatter(const unsigned long long *keys,
+// One work item (ITEM keys of one bucket) per round: the keys are ranked by
+// sub-bucket in shared memory, every sub-bucket of the item takes its range
+// with one cursor update, and the item's keys are written reordered by
+// sub-bucket (consecutive threads store consecutive addresses).  Items are
+// larger than the other bucket kernels' so that a sub-bucket's run in an item
+// spans several sectors.  Thread 0 takes the next item while this one is
+// ranked, and its keys are loaded while this one's are written.  Estimated
+// regions are checked once per sub-bucket and item, by the thread that moves
+// its cursor; only an item that holds an outgrown one checks every key.
+// KPT: keys per thread; MAXB: sub-buckets per thread in the rank scan (the
+// cursor updates held in registers until after the reorder).  An item's work
+// is partly per key and partly per sub-bucket (count, scan, cursor), and its
+// stores are runs of ITEM / n_sub keys, so buckets of many sub-buckets want
+// large items: 2.4G keys in up to 2048 sub-buckets a bucket take 17.0 ms with
+// items of 4096 keys, 13.9 with 6144 (two blocks per SM) and 12.4 with 16384
+// (one block of 1024 threads); 480M keys in up to 512 sub-buckets 2.2, 1.9 and
+// 2.4 ms.
+template <uint32_t THREADS, uint32_t KPT, uint32_t MAXB, uint32_t BPSM>
+__global__ void __launch_bounds__(THREADS, BPSM) k_subpart_scatter(const unsigned long long *keys,
                                                                       const BucketRanges *rg, uint32_t n_items,
                                                                       unsigned int *next_item, const SubCfg *sc,
                                                                       unsigned long long *sub_cursor,
@@ -1953,86 +1949,121 @@ __global__ void __launch_bounds__(SP_THREADS, BPSM) k_subpart_scatter(const unsi
                                                                       unsigned long long *out, uint64_t out_cap,
                                                                       uint32_t max_sub)
 {
+    constexpr uint32_t ITEM = KPT * THREADS;
+    static_assert(ITEM <= 65536, "ranks take 16 bits");
     // shared arrays per sub-bucket hold max_sub entries (the most of any
     // bucket of the launch)
     extern __shared__ __align__(16) uint8_t sp_smem[];
-    unsigned long long *s_sorted = reinterpret_cast<unsigned long long *>(sp_smem);          // SUB_SCATTER_ITEM_KEYS
-    unsigned long long *s_dst = s_sorted + SUB_SCATTER_ITEM_KEYS;                             // max_sub
-    uint32_t *s_cnt = reinterpret_cast<uint32_t *>(s_dst + max_sub);                          // max_sub
-    uint32_t *s_start = s_cnt + max_sub;                                                      // max_sub
+    unsigned long long *s_sorted = reinterpret_cast<unsigned long long *>(sp_smem);   // ITEM
+    unsigned long long *s_dst = s_sorted + ITEM;                                      // max_sub
+    uint32_t *s_cnt = reinterpret_cast<uint32_t *>(s_dst + max_sub);                  // max_sub: counts, then starts
     __shared__ uint32_t s_item0[N_BUCKETS + 1];
-    __shared__ uint32_t s_item, s_warp[32];
+    __shared__ uint32_t s_warp[32], s_over;
+    __shared__ unsigned long long s_begin;
+    __shared__ uint32_t s_n, s_shift, s_nsub, s_base;
     const int tid = threadIdx.x;
-    for (uint32_t i = tid; i < max_sub; i += SP_THREADS) s_cnt[i] = 0;
+    for (uint32_t i = tid; i < max_sub; i += THREADS) s_cnt[i] = 0;
     load_item_starts(rg, s_item0);
-    uint32_t it;
-    while (next_work(next_item, n_items, &s_item, it)) {
-        const WorkItem w = work_item_n(rg, s_item0, it, SUB_SCATTER_ITEM_KEYS);
-        const SubCfg c = sc[w.bucket];
-        const uint32_t n = (uint32_t)(w.end - w.begin);
-        unsigned long long k[SP_PER_THREAD];
-        uint32_t sr[SP_PER_THREAD];   // rank << 16 | sub (sub 0xFFFF: no key)
-#pragma unroll
-        for (uint32_t r = 0; r < SP_PER_THREAD; ++r) {
-            const uint32_t i = r * SP_THREADS + tid;
-            if (i < n) k[r] = __ldcs(&keys[w.begin + i]);
+    auto take_next = [&]() {
+        const uint32_t it = atomicAdd(next_item, 1u);
+        s_n = 0;
+        if (it < n_items) {
+            const WorkItem w = work_item_n(rg, s_item0, it, ITEM);
+            const SubCfg c = sc[w.bucket];
+            s_begin = w.begin;
+            s_n = (uint32_t)(w.end - w.begin);
+            s_shift = c.shift - 32;   // sub-buckets follow the key's upper half: shift >= 44
+            s_nsub = c.n_sub;
+            s_base = c.sub_base;
         }
+    };
+    if (tid == 0) {
+        s_over = 0;
+        take_next();
+    }
+    __syncthreads();
+    unsigned long long k[KPT];
+    uint32_t n = s_n;
 #pragma unroll
-        for (uint32_t r = 0; r < SP_PER_THREAD; ++r) {
-            const uint32_t i = r * SP_THREADS + tid;
-            sr[r] = 0xFFFFu;
-            if (i < n) {
-                const uint32_t sub = sub_of(k[r], c);
+    for (uint32_t r = 0; r < KPT; ++r)
+        if (r * THREADS + tid < n) k[r] = __ldcs(&keys[s_begin + r * THREADS + tid]);
+    while (n) {
+        const uint32_t shift = s_shift, n_sub = s_nsub, base = s_base, smask = n_sub - 1;
+        uint32_t sr[KPT];   // rank << 16 | sub
+#pragma unroll
+        for (uint32_t r = 0; r < KPT; ++r)
+            if (r * THREADS + tid < n) {
+                const uint32_t sub = ((uint32_t)(k[r] >> 32) >> shift) & smask;
                 sr[r] = (atomicAdd(&s_cnt[sub], 1u) << 16) | sub;
             }
-        }
         __syncthreads();
+        if (tid == 0) take_next();
         // exclusive scan of the n_sub counts, a few per thread
-        const uint32_t per = (c.n_sub + SP_THREADS - 1) / SP_THREADS, b0 = tid * per;
-        uint32_t local = 0;
-        for (uint32_t j = 0; j < per; ++j)
-            if (b0 + j < c.n_sub) local += s_cnt[b0 + j];
-        uint32_t tot;
-        uint32_t run = block_excl_scan_1024(local, s_warp, tot);
+        const uint32_t per = (n_sub + THREADS - 1) / THREADS, b0 = tid * per;
+        uint32_t cnt[MAXB], local = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < MAXB; ++j) {
+            cnt[j] = j < per && b0 + j < n_sub ? s_cnt[b0 + j] : 0u;
+            local += cnt[j];
+        }
         // the sub-buckets' cursor updates are in flight during the reorder
         // and consumed only after it
         unsigned long long cur[MAXB];
-        uint32_t first[MAXB];
-#pragma unroll
-        for (uint32_t j = 0; j < MAXB; ++j) {
-            const uint32_t s = b0 + j;
-            cur[j] = 0ull;
-            first[j] = run;
-            if (j < per && s < c.n_sub) {
-                const uint32_t cnt = s_cnt[s];
-                s_start[s] = run;
-                if (cnt) cur[j] = atomicAdd(&sub_cursor[c.sub_base + s], (unsigned long long)cnt);
-                run += cnt;
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (uint32_t r = 0; r < SP_PER_THREAD; ++r) {
-            const uint32_t sub = sr[r] & 0xFFFFu;
-            if (sub != 0xFFFFu) {
-                s_sorted[s_start[sub] + (sr[r] >> 16)] = k[r];
-            }
-        }
-        // destination of sorted index i of sub-bucket s: s_dst[s] + i
 #pragma unroll
         for (uint32_t j = 0; j < MAXB; ++j)
-            if (j < per && b0 + j < c.n_sub) s_dst[b0 + j] = cur[j] - first[j];
+            cur[j] = cnt[j] ? atomicAdd(&sub_cursor[base + b0 + j], (unsigned long long)cnt[j]) : 0ull;
+        uint32_t tot;
+        const uint32_t run0 = block_excl_scan_1024(local, s_warp, tot);
+        uint32_t run = run0;
+#pragma unroll
+        for (uint32_t j = 0; j < MAXB; ++j)
+            if (j < per && b0 + j < n_sub) {
+                s_cnt[b0 + j] = run;
+                run += cnt[j];
+            }
         __syncthreads();
-        for (uint32_t i = tid; i < n; i += SP_THREADS) {
-            const unsigned long long key = s_sorted[i];
-            const uint32_t sb = sub_of(key, c);
-            const unsigned long long d = s_dst[sb] + i;
-            // estimated regions: a sub-bucket that outgrew its region is
-            // reported by its cursor (k_subpart_sizes) and counted exactly
-            if (d < out_cap && (!sub_end || d < sub_end[c.sub_base + sb])) out[d] = key;
+#pragma unroll
+        for (uint32_t r = 0; r < KPT; ++r)
+            if (r * THREADS + tid < n) s_sorted[s_cnt[sr[r] & 0xFFFFu] + (sr[r] >> 16)] = k[r];
+        const uint32_t nn = s_n;
+        const unsigned long long nb = s_begin;
+#pragma unroll
+        for (uint32_t r = 0; r < KPT; ++r)
+            if (r * THREADS + tid < nn) k[r] = __ldcs(&keys[nb + r * THREADS + tid]);
+        // destination of sorted index i of sub-bucket s: s_dst[s] + i
+        run = run0;
+#pragma unroll
+        for (uint32_t j = 0; j < MAXB; ++j) {
+            if (cnt[j]) {
+                s_dst[b0 + j] = cur[j] - run;
+                if (sub_end) {
+                    const unsigned long long e = sub_end[base + b0 + j];
+                    if (cur[j] + cnt[j] > (e < out_cap ? e : out_cap)) s_over = 1;
+                }
+            }
+            run += cnt[j];
         }
-        for (uint32_t i = tid; i < c.n_sub; i += SP_THREADS) s_cnt[i] = 0;
         __syncthreads();
+        if (!s_over) {
+#pragma unroll 4
+            for (uint32_t i = tid; i < n; i += THREADS) {
+                const unsigned long long key = s_sorted[i];
+                out[s_dst[((uint32_t)(key >> 32) >> shift) & smask] + i] = key;
+            }
+        } else {
+            // a sub-bucket that outgrew its region is reported by its cursor
+            // (k_subpart_sizes) and counted exactly
+            for (uint32_t i = tid; i < n; i += THREADS) {
+                const unsigned long long key = s_sorted[i];
+                const uint32_t sub = ((uint32_t)(key >> 32) >> shift) & smask;
+                const unsigned long long d = s_dst[sub] + i;
+                if (d < out_cap && d < sub_end[base + sub]) out[d] = key;
+            }
+        }
+        for (uint32_t i = tid; i < n_sub; i += THREADS) s_cnt[i] = 0;
+        n = nn;
+        __syncthreads();
+        if (tid == 0) s_over = 0;   // set again only after the next item's first barrier
     }
 }
 
@@ -2650,8 +2681,6 @@ uint32_t fill_item_starts_n(BucketRanges &r, uint64_t item_keys)
     return n;
 }
 
-uint32_t fill_item_starts(BucketRanges &r) { return fill_item_starts_n(r, WORK_ITEM_KEYS); }
-
 cudaError_t launch_bloom_buckets(const unsigned long long *keys, const BucketRanges *rg, uint32_t n_items,
                                  unsigned int *next_item, const BucketCfg *cfg, unsigned long long *bits,
                                  unsigned long long *out, unsigned long long *low_cnt, unsigned long long *high_cnt,
@@ -2731,9 +2760,23 @@ cudaError_t launch_subpart_sizes(const unsigned long long *sub_off, const unsign
     return cudaGetLastError();
 }
 
-static size_t subpart_scatter_smem(uint32_t max_sub)
+template <uint32_t THREADS, uint32_t KPT, uint32_t MAXB, uint32_t BPSM>
+static cudaError_t launch_subpart_scatter_t(const unsigned long long *keys, const BucketRanges *rg, uint32_t n_items,
+                                            unsigned int *next_item, const SubCfg *sc, unsigned long long *sub_cursor,
+                                            unsigned long long *out, uint64_t out_cap, uint32_t max_sub,
+                                            cudaStream_t st, const unsigned long long *sub_end)
 {
-    return (size_t)SUB_SCATTER_ITEM_KEYS * 8 + (size_t)max_sub * (8 + 4 + 4);
+    const size_t smem = (size_t)KPT * THREADS * 8 + (size_t)max_sub * (8 + 4);
+    auto kern = k_subpart_scatter<THREADS, KPT, MAXB, BPSM>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, THREADS, smem) != cudaSuccess || per_sm < 1)
+        per_sm = 1;
+    const uint32_t grid = std::min<uint32_t>(n_items, (uint32_t)(sm_count() * per_sm));
+    note_launch();
+    kern<<<grid, THREADS, smem, st>>>(keys, rg, n_items, next_item, sc, sub_cursor, sub_end, out, out_cap, max_sub);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_subpart_scatter(const unsigned long long *keys, const BucketRanges *rg, uint32_t n_items,
@@ -2745,18 +2788,13 @@ cudaError_t launch_subpart_scatter(const unsigned long long *keys, const BucketR
     if (!max_sub || max_sub > SUB_MAX_PER_BUCKET) return cudaErrorInvalidValue;
     cudaError_t e = cudaMemsetAsync(next_item, 0, 4, st);
     if (e != cudaSuccess) return e;
-    const size_t smem = subpart_scatter_smem(max_sub);
-    auto kern = (scatter_shape == 2 && max_sub <= 2 * SP_THREADS) ? k_subpart_scatter<2, 3>
-                                                                  : k_subpart_scatter<SP_MAX_BINS, 2>;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, SP_THREADS, smem) != cudaSuccess || per_sm < 1)
-        per_sm = 1;
-    const uint32_t grid = std::min<uint32_t>(n_items, (uint32_t)(sm_count() * per_sm));
-    note_launch();
-    kern<<<grid, SP_THREADS, smem, st>>>(keys, rg, n_items, next_item, sc, sub_cursor, sub_end, out, out_cap, max_sub);
-    return cudaGetLastError();
+#define KC_SCATTER_ARGS keys, rg, n_items, next_item, sc, sub_cursor, out, out_cap, max_sub, st, sub_end
+    if (sub_scatter_item_keys(max_sub) == 16384)
+        return max_sub > 2048 ? launch_subpart_scatter_t<1024, 16, 4, 1>(KC_SCATTER_ARGS)
+                              : launch_subpart_scatter_t<1024, 16, 2, 1>(KC_SCATTER_ARGS);
+    return scatter_shape == 2 ? launch_subpart_scatter_t<512, 12, 2, 3>(KC_SCATTER_ARGS)
+                              : launch_subpart_scatter_t<512, 12, 2, 2>(KC_SCATTER_ARGS);
+#undef KC_SCATTER_ARGS
 }
 
 cudaError_t launch_wait_flag(const unsigned int *flag, uint32_t poll_limit, unsigned long long *flags, cudaStream_t st)

@@ -155,9 +155,12 @@ struct BucketRanges {
     unsigned long long begin[N_BUCKETS], len[N_BUCKETS];
     uint32_t item0[N_BUCKETS + 1];
 };
-uint32_t fill_item_starts(BucketRanges &r);   // sets item0 from len, returns the number of items
-uint32_t fill_item_starts_n(BucketRanges &r, uint64_t item_keys);   // items of item_keys keys
-constexpr uint32_t SUB_SCATTER_ITEM_KEYS = 4096;   // keys per work item of the sub-bucket scatter
+// sets item0 from len for items of item_keys keys, returns the number of items
+uint32_t fill_item_starts_n(BucketRanges &r, uint64_t item_keys);
+constexpr uint32_t SUB_COUNT_KEYS = 2048;   // keys per work item and stride of the sub-bucket count
+// keys per work item of the sub-bucket scatter: larger items where a bucket
+// has many sub-buckets (k_subpart_scatter)
+inline uint32_t sub_scatter_item_keys(uint32_t max_sub) { return max_sub > 1024 ? 16384u : 6144u; }
 
 // Prefix path: the buckets of the string keys' top 8 bits are cut into n_sub
 // sub-buckets each (a power of two) by the bits below, so that one thread
@@ -298,9 +301,10 @@ cudaError_t launch_select_range(const unsigned long long *keys, const uint32_t *
 // Bucket-major kernels of the partitioned pipeline; each resets *next_item.
 // Sub-bucket path.  count: sub_count[sub_base + s] += the keys of bucket b
 // in sub-bucket s.  scatter: every key to out[sub_cursor[its sub-bucket]++]
-// (sub_cursor starts at the exclusive scan of sub_count); its ranges rg are
-// cut into items of SUB_SCATTER_ITEM_KEYS keys (fill_item_starts_n).
-// stride > 1: only every stride-th run of 4 keys is counted (a sample).
+// (sub_cursor starts at the exclusive scan of sub_count).  The count's ranges
+// rg are cut into items of SUB_COUNT_KEYS * stride keys, the scatter's into
+// items of sub_scatter_item_keys(max_sub) keys (fill_item_starts_n).
+// stride > 1: only every stride-th run of 16 keys is counted (a sample).
 cudaError_t launch_subpart_count(const unsigned long long *keys, const BucketRanges *rg, uint32_t n_items,
                                  const SubCfg *sc, uint32_t *sub_count, cudaStream_t st, uint32_t stride = 1);
 // sub_end non-NULL: the sub-buckets' regions are estimates and a key is
