@@ -198,8 +198,7 @@ typedef struct {
     uint64_t count_shape;         /* block shape of the shared-memory count: 1, 3 = 512-thread blocks, two per
                                      SM, 8192-slot tables; 2, 4 = 256-thread blocks, four per SM, 4096-slot
                                      tables (sub-buckets of half the k-mers); default 1 */
-    uint64_t part_shape;          /* the partition's rounds: 1 = 4096 k-mers staged per round (three blocks
-                                     per SM), 2 = 2048 (four blocks per SM); default 1 */
+    uint64_t part_shape;          /* 1 or 2; kept for callers that set it: the partition has one shape */
     uint64_t scatter_shape;       /* the sub-bucket scatter: 1 = two blocks per SM, 2 = a variant with fewer
                                      registers, three per SM (passes whose buckets have at most 1024
                                      sub-buckets); default 1 */

@@ -445,7 +445,7 @@ class KmerCounter:
         plain jobs per sub-bucket in shared memory, 2 on global-memory tables.
         record_sort: 1 sorts those tables' records most significant bits first,
         2 with the LSD radix sort.  count_shape: the shared-memory count's
-        block shape, 1..4; part_shape: the partition's round size, 1 or 2;
+        block shape, 1..4; part_shape: 1 or 2, no effect any more;
         scatter_shape: the sub-bucket scatter's variant, 1 or 2 (kc_tuning in
         include/kc.h)."""
         t = kc_tuning()

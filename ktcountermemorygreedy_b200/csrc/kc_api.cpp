@@ -895,18 +895,18 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
                 cu.enqueue(cu.ev.size());
                 a.tile0 = 0;
                 a.n_tiles = tiles_ready;
-                CK(launch_extract(prefix ? MODE_PARTS : MODE_PART, a, 0, st, (uint32_t)tn.part_shape));
+                CK(launch_part(prefix, k, a, st));
                 while (chunks_done < cu.ev.size()) {
                     const uint64_t t0 = tiles_ready;
                     census_chunks(chunks_done + 1);
                     a.tile0 = t0;
                     a.n_tiles = tiles_ready - t0;
-                    CK(launch_extract(prefix ? MODE_PARTS : MODE_PART, a, 0, st, (uint32_t)tn.part_shape));
+                    CK(launch_part(prefix, k, a, st));
                 }
                 a.tile0 = 0;
                 a.n_tiles = T;
             } else {
-                CK(launch_extract(prefix ? MODE_PARTS : MODE_PART, a, 0, st, (uint32_t)tn.part_shape));
+                CK(launch_part(prefix, k, a, st));
             }
             clk.end();
             unsigned long long *p_fill = hs.n<unsigned long long>(N_BUCKETS);
@@ -1073,7 +1073,7 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
                             // the records went over the partitioned keys
                             CK(cudaMemsetAsync(cursor, 0, N_BUCKETS * 8, st));
                             clk.begin(2);
-                            CK(launch_extract(MODE_PARTS, a, 0, st, (uint32_t)tn.part_shape));
+                            CK(launch_part(true, k, a, st));
                             clk.end();
                         }
                         continue;
@@ -2418,7 +2418,7 @@ int kc_autotune(kc_handle *h, const kc_job *jobs, uint32_t n_jobs, uint32_t batc
     if (rc == KC_OK) rc = run(cur, cur_ms);
     const double bucket_c[] = {2.0, 3.0, 4.0, 3.0}, table_c[] = {1.3, 1.6, 2.2, 1.6};
     const uint64_t group_c[] = {2ull << 20, 4ull << 20, 8ull << 20, 4ull << 20}, smem_c[] = {1, 2, 1, 1},
-                   sort_c[] = {1, 2, 1, 1}, shape_c[] = {1, 2, 1, 1}, part_c[] = {1, 2, 1, 1},
+                   sort_c[] = {1, 2, 1, 1}, shape_c[] = {1, 2, 1, 1}, part_c[] = {1, 1, 1, 1},
                    scatter_c[] = {1, 2, 1, 1};
     for (int param = 0; param < 8 && rc == KC_OK; ++param)
         for (int c = 0; c < 4 && rc == KC_OK; ++c) {

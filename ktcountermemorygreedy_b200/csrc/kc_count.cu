@@ -2,7 +2,7 @@
 // shared memory, and the sort of the resulting records.
 //
 // The occurrences arrive partitioned twice, into 256 buckets by their first
-// four bases and into sub-buckets by the next bases (k_extract<MODE_PARTS>,
+// four bases and into sub-buckets by the next bases (launch_part by string,
 // k_subpart_scatter), as string keys: the k bases first-base-high, left
 // aligned.  So the sub-buckets are consecutive ranges of the printed order:
 // once every sub-bucket's distinct k-mers are counted and sorted on their own,

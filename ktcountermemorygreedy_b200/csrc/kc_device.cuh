@@ -38,10 +38,18 @@ __device__ __forceinline__ uint64_t slot_hash(uint64_t x)
 // FASTQ bytes
 // ---------------------------------------------------------------------------
 
-// Bit i of the result is bit 0 of byte i of x (x's bytes hold 0 or 1).
-__device__ __forceinline__ uint32_t byte_bits4(uint32_t x)
+// Top byte of the result: bits 0..3 are bit 0 of the bytes of x, bits 4..7
+// bit 0 of the bytes of y (all bytes hold 0 or 1; the products' other terms
+// stay below bit 24 or leave the word, and never carry).
+__device__ __forceinline__ uint32_t byte_bits8(uint32_t x, uint32_t y)
 {
-    return (x * 0x01020408u) >> 24 & 0xFu;
+    return (x + (y << 4)) * 0x01020408u;
+}
+
+// The top bytes of four words.
+__device__ __forceinline__ uint32_t top_bytes(uint32_t a, uint32_t b, uint32_t c, uint32_t d)
+{
+    return __byte_perm(__byte_perm(a, b, 0x0073), __byte_perm(c, d, 0x0073), 0x5410);
 }
 
 // 2-bit codes (A0 C1 G2 T/U3, case-insensitive, as the reference's
@@ -57,28 +65,24 @@ __device__ __forceinline__ void classify32(const uint8_t *p, uint64_t &codes, ui
     const uint4 a = *reinterpret_cast<const uint4 *>(p);
     const uint4 b = *reinterpret_cast<const uint4 *>(p + 16);
     const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    uint64_t c = 0;
-    uint32_t v = 0, n = 0;
+    uint32_t c[8], v[8], n[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const uint32_t x = w[i];
         // newline bytes: zero bytes of x ^ 0x0a0a0a0a (exact, no borrow)
         const uint32_t z = x ^ 0x0a0a0a0au;
         const uint32_t nz = (((z & 0x7f7f7f7fu) + 0x7f7f7f7fu) | z) & 0x80808080u;   // 0x80 where byte != 0
-        n |= byte_bits4((~nz & 0x80808080u) >> 7) << (4 * i);
+        n[i] = (~nz & 0x80808080u) >> 7;
         const uint32_t u = x & 0xdfdfdfdfu;
         const uint32_t x0 = u, x1 = u >> 1, x2 = u >> 2, x3 = u >> 3, x4 = u >> 4, x6 = u >> 6, x7 = u >> 7;
-        const uint32_t ok = x6 & ~x7 & ~x3 & ((~x4 & x0 & ~(x2 & ~x1)) | (x4 & x2 & ~x1)) & 0x01010101u;
-        v |= byte_bits4(ok) << (4 * i);
-        // four 2-bit codes, one per byte, packed into 8 bits
-        const uint32_t c4 = ((u >> 1) & 0x03030303u) ^ ((u >> 2) & 0x01010101u);
-        const uint32_t c2 = c4 | (c4 >> 6);                       // bytes 0 and 2 hold two codes each
-        const uint32_t c8 = (c2 & 0xfu) | ((c2 >> 12) & 0xf0u);
-        c |= (uint64_t)c8 << (8 * i);
+        v[i] = x6 & ~x7 & ~x3 & ((~x4 & x0 & ~(x2 & ~x1)) | (x4 & x2 & ~x1)) & 0x01010101u;
+        // four 2-bit codes, one per byte, packed into the top byte (the
+        // product's other terms do not reach it and never carry)
+        c[i] = (((u >> 1) & 0x03030303u) ^ ((u >> 2) & 0x01010101u)) * 0x01041040u;
     }
-    codes = c;
-    valid = v;
-    nl = n;
+    codes = (uint64_t)top_bytes(c[4], c[5], c[6], c[7]) << 32 | top_bytes(c[0], c[1], c[2], c[3]);
+    valid = top_bytes(byte_bits8(v[0], v[1]), byte_bits8(v[2], v[3]), byte_bits8(v[4], v[5]), byte_bits8(v[6], v[7]));
+    nl = top_bytes(byte_bits8(n[0], n[1]), byte_bits8(n[2], n[3]), byte_bits8(n[4], n[5]), byte_bits8(n[6], n[7]));
 }
 
 __device__ __forceinline__ uint32_t range_mask(uint32_t a, uint32_t b)
@@ -103,6 +107,21 @@ __device__ __forceinline__ uint32_t line_mask(uint64_t line0, uint32_t nl, uint3
     }
     if ((cur & 3) == want) m |= range_mask(pos, 32);
     return m;
+}
+
+// Bit b (b >= 32) of the result is set when bits b-k+1 .. b of g are all set.
+__device__ __forceinline__ uint32_t run_ends(uint64_t g, uint32_t k)
+{
+    uint64_t r1 = g, r2 = r1 & (r1 << 1), r4 = r2 & (r2 << 2), r8 = r4 & (r4 << 4), r16 = r8 & (r8 << 8);
+    uint64_t acc = ~0ULL;
+    uint32_t sh = 0;
+    if (k & 32) { acc &= r16 & (r16 << 16); sh = 32; }
+    if (k & 16) { acc &= r16 << sh; sh += 16; }
+    if (k & 8) { acc &= r8 << sh; sh += 8; }
+    if (k & 4) { acc &= r4 << sh; sh += 4; }
+    if (k & 2) { acc &= r2 << sh; sh += 2; }
+    if (k & 1) { acc &= r1 << sh; sh += 1; }
+    return (uint32_t)(acc >> 32);
 }
 
 // ---------------------------------------------------------------------------

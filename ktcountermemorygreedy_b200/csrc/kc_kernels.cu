@@ -69,21 +69,6 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t *s_warp
     return base + x - v;
 }
 
-// Bit b (b >= 32) of the result is set when bits b-k+1 .. b of g are all set.
-__device__ __forceinline__ uint32_t run_ends(uint64_t g, uint32_t k)
-{
-    uint64_t r1 = g, r2 = r1 & (r1 << 1), r4 = r2 & (r2 << 2), r8 = r4 & (r4 << 4), r16 = r8 & (r8 << 8);
-    uint64_t acc = ~0ULL;
-    uint32_t sh = 0;
-    if (k & 32) { acc &= r16 & (r16 << 16); sh = 32; }
-    if (k & 16) { acc &= r16 << sh; sh += 16; }
-    if (k & 8) { acc &= r8 << sh; sh += 8; }
-    if (k & 4) { acc &= r4 << sh; sh += 4; }
-    if (k & 2) { acc &= r2 << sh; sh += 2; }
-    if (k & 1) { acc &= r1 << sh; sh += 1; }
-    return (uint32_t)(acc >> 32);
-}
-
 struct KParams {
     uint32_t k;
     uint64_t kmask;     // low 2k bits
@@ -317,14 +302,9 @@ __global__ void k_chunk_lastnl(const int32_t *tile_lastnl, const uint32_t *tile_
 // extraction
 // ---------------------------------------------------------------------------
 
-// SCAP: the most k-mers staged per round (the PART reorder holds SCAP /
-// EXT_THREADS of them per thread in registers); a PART launch with
-// SCAP = 2048 fits four blocks per SM instead of three.
-template <int MODE, uint32_t SCAP = STAGE_CAP>
-__global__ void __launch_bounds__(EXT_THREADS, MODE == MODE_SCAN ? 5 : (SCAP <= 2048 ? 4 : 3))
-    k_extract(ExtractArgs a, uint32_t stage_cap)
+template <int MODE>
+__global__ void __launch_bounds__(EXT_THREADS, MODE == MODE_SCAN ? 5 : 3) k_extract(ExtractArgs a, uint32_t stage_cap)
 {
-    constexpr bool PART = MODE == MODE_PART || MODE == MODE_PARTS;
     extern __shared__ __align__(128) uint8_t smem[];
     uint8_t *sbuf[2] = {smem, smem + BUF_BYTES};
     uint64_t *s_codes = reinterpret_cast<uint64_t *>(smem + 2 * BUF_BYTES);   // 257 used
@@ -334,15 +314,10 @@ __global__ void __launch_bounds__(EXT_THREADS, MODE == MODE_SCAN ? 5 : (SCAP <= 
     uint32_t *s_hll = reinterpret_cast<uint32_t *>(s_good + 264);   // SCAN mode: registers of sample 0
     const bool hll_local = MODE == MODE_SCAN && a.hll && a.hll_local;
 
-    // staged modes: (segment, position) of each window, then (PART mode) the
-    // rank of each staged k-mer inside its bucket's share of the tile
-    uint16_t *s_rank = reinterpret_cast<uint16_t *>(s_stage + stage_cap);
-
     __shared__ __align__(8) uint64_t mbar[2];
     __shared__ uint32_t s_warp[8];
     __shared__ uint32_t s_hist[256];
-    __shared__ uint32_t s_bhist[MODE == MODE_SCAN || PART ? 256 : 1];
-    __shared__ unsigned long long s_bpos[PART ? 256 : 1];
+    __shared__ uint32_t s_bhist[MODE == MODE_SCAN ? 256 : 1];
     __shared__ unsigned long long s_bcast[2];
     __shared__ unsigned long long s_boff[MODE == MODE_BLOOM ? 256 : 1];
     __shared__ unsigned long long s_bcap[MODE == MODE_BLOOM ? 256 : 1];
@@ -555,9 +530,7 @@ __global__ void __launch_bounds__(EXT_THREADS, MODE == MODE_SCAN ? 5 : (SCAP <= 
                     idx += (uint32_t)__popc(e8);
                 }
             }
-            if (PART) s_bhist[tid] = 0;
             __syncthreads();
-            const uint32_t blo = a.bucket_lo, bhi = a.bucket_hi ? a.bucket_hi : N_BUCKETS;
             for (uint32_t base = 0; base < tot; base += stage_cap) {
                 const uint32_t nr = min(stage_cap, tot - base);
                 for (uint32_t ci = tid; ci < n_chunks; ci += EXT_THREADS) {
@@ -577,20 +550,8 @@ __global__ void __launch_bounds__(EXT_THREADS, MODE == MODE_SCAN ? 5 : (SCAP <= 
                         if ((e8 >> p) & 1u) {
                             if (idx >= base && idx < base + nr) {
                                 const uint64_t f = fwd & kp.topmask;
-                                // the canonical word is the smaller one; its
-                                // string key (first base high) is the complement
-                                // of the other, larger one: rc holds the
-                                // complemented bases in reverse order
-                                const unsigned long long key =
-                                    MODE == MODE_PARTS ? ~(f < rc ? rc : f) & kp.topmask : (f < rc ? f : rc);
+                                const unsigned long long key = f < rc ? f : rc;
                                 s_stage[idx - base] = key;
-                                if (PART) {
-                                    // rank inside the tile's share of its bucket (a
-                                    // pass of a multi-pass job keeps only its range)
-                                    const uint32_t bk = (uint32_t)(key >> 56);
-                                    s_rank[idx - base] =
-                                        (bk >= blo && bk < bhi) ? (uint16_t)atomicAdd(&s_bhist[bk], 1u) : (uint16_t)0xFFFFu;
-                                }
                             }
                             ++idx;
                         }
@@ -603,53 +564,6 @@ __global__ void __launch_bounds__(EXT_THREADS, MODE == MODE_SCAN ? 5 : (SCAP <= 
                         uint32_t i = r0 + tid;
                         bool act = i < nr;
                         warp_insert(act, act ? s_stage[i] : EMPTY_KEY, tr, a.max_probe, flags);
-                    }
-                } else if (PART) {
-                    // scatter into the root-prefix buckets (ranks were taken
-                    // as the k-mers were formed), one cursor update per bucket;
-                    // the round's k-mers are reordered by bucket in shared
-                    // memory, so that consecutive threads store consecutive
-                    // addresses of one bucket's region (a warp's store then
-                    // touches a few sectors instead of one per k-mer)
-                    uint32_t tot_b;
-                    const uint32_t c = s_bhist[tid];
-                    s_bhist[tid] = 0;   // the next round's ranks (emission is done)
-                    const uint32_t bstart = block_excl_scan(c, s_warp, tot_b);
-                    s_hist[tid] = bstart;
-                    // this tile's range of bucket tid: the cursor update is in
-                    // flight during the reorder and consumed only after it
-                    const unsigned long long cur = c ? atomicAdd(&a.bucket_cursor[tid], (unsigned long long)c) : 0ull;
-                    __syncthreads();
-                    unsigned long long kr[SCAP / EXT_THREADS];
-#pragma unroll
-                    for (uint32_t r = 0; r < SCAP / EXT_THREADS; ++r) {
-                        const uint32_t i = tid + r * EXT_THREADS;
-                        if (i < nr && s_rank[i] != 0xFFFFu) {
-                            kr[r] = s_stage[i];
-                            s_rank[i] = (uint16_t)(s_hist[(uint32_t)(kr[r] >> 56)] + s_rank[i]);
-                        }
-                    }
-                    __syncthreads();
-#pragma unroll
-                    for (uint32_t r = 0; r < SCAP / EXT_THREADS; ++r) {
-                        const uint32_t i = tid + r * EXT_THREADS;
-                        if (i < nr && s_rank[i] != 0xFFFFu) s_stage[s_rank[i]] = kr[r];
-                    }
-                    // destination of sorted index i of bucket b: s_bpos[b] + i,
-                    // written while i < s_hist[b] (inside the bucket's region
-                    // and the list: a bucket that outgrows its estimated
-                    // region is reported by its cursor and redone)
-                    {
-                        const unsigned long long bp = c ? a.bucket_base[tid] + cur - bstart : 0ull;
-                        s_bpos[tid] = bp;
-                        const unsigned long long lim = a.bucket_end[tid] < a.list_cap ? a.bucket_end[tid] : a.list_cap;
-                        s_hist[tid] = lim > bp ? (uint32_t)(lim - bp < 0xFFFFFFFFull ? lim - bp : 0xFFFFFFFFull) : 0u;
-                    }
-                    __syncthreads();
-                    for (uint32_t i = tid; i < tot_b; i += EXT_THREADS) {
-                        const unsigned long long key = s_stage[i];
-                        const uint32_t b = (uint32_t)(key >> 56);
-                        if (i < s_hist[b]) a.list[s_bpos[b] + i] = key;
                     }
                 } else if (MODE == MODE_EMIT) {
                     if (tid == 0) s_bcast[0] = atomicAdd(&a.counters[C_EMIT_LEN], (unsigned long long)nr);
@@ -2146,7 +2060,6 @@ size_t extract_smem_bytes_for(int mode, uint32_t stage_cap)
     size_t b = 2 * BUF_BYTES + 264 * 8 * 2 + 264 * 4;
     if (mode != MODE_SCAN) b += (size_t)stage_cap * 8;
     else b += HLL_M * 4;
-    if (mode != MODE_SCAN) b += (size_t)stage_cap * 2;
     return b;
 }
 
@@ -2171,11 +2084,11 @@ cudaError_t launch_chunk_lastnl(const int32_t *tile_lastnl, const uint32_t *tile
     return cudaGetLastError();
 }
 
-template <int M, uint32_t SCAP = STAGE_CAP>
+template <int M>
 static cudaError_t launch_extract_t(const ExtractArgs &a, int grid, uint32_t stage_cap, cudaStream_t st)
 {
     size_t smem = extract_smem_bytes_for(M, stage_cap);
-    auto kern = k_extract<M, SCAP>;
+    auto kern = k_extract<M>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     if (grid <= 0) {
@@ -2193,7 +2106,7 @@ static cudaError_t launch_extract_t(const ExtractArgs &a, int grid, uint32_t sta
     return cudaGetLastError();
 }
 
-cudaError_t launch_extract(int mode, const ExtractArgs &a, int grid, cudaStream_t st, uint32_t part_shape)
+cudaError_t launch_extract(int mode, const ExtractArgs &a, int grid, cudaStream_t st)
 {
     if (!a.n_tiles) return cudaSuccess;
     switch (mode) {
@@ -2201,12 +2114,6 @@ cudaError_t launch_extract(int mode, const ExtractArgs &a, int grid, cudaStream_
     case MODE_INSERT: return launch_extract_t<MODE_INSERT>(a, grid, STAGE_CAP, st);
     case MODE_BLOOM: return launch_extract_t<MODE_BLOOM>(a, grid, STAGE_CAP, st);
     case MODE_EMIT: return launch_extract_t<MODE_EMIT>(a, grid, STAGE_CAP, st);
-    case MODE_PART:
-        return part_shape == 2 ? launch_extract_t<MODE_PART, 2048>(a, grid, 2048, st)
-                               : launch_extract_t<MODE_PART>(a, grid, STAGE_CAP, st);
-    case MODE_PARTS:
-        return part_shape == 2 ? launch_extract_t<MODE_PARTS, 2048>(a, grid, 2048, st)
-                               : launch_extract_t<MODE_PARTS>(a, grid, STAGE_CAP, st);
     default: return cudaErrorInvalidValue;
     }
 }

@@ -108,29 +108,23 @@ struct ExtractArgs {
     // emit / bloom / part output list
     unsigned long long *list;
     unsigned long long list_cap;
-    // root-prefix buckets (single sample): SCAN counts, PART scatters
+    // buckets (single sample): SCAN counts, launch_part scatters
     unsigned long long *bucket_hist;          // 256 counts (SCAN)
     uint64_t bucket_sample_mask;              // SCAN counts tiles t with (t & mask) == 0
-    int census_by_string;                     // SCAN: buckets by the first four bases (for MODE_PARTS)
+    int census_by_string;                     // SCAN: buckets by the first four bases (for launch_part by string)
     // SCAN over a subset of the tiles: visit[0..n_visit) ascending tile
     // indexes (NULL: every tile); occurrences are then counted on the census
     // tiles only
     const uint32_t *visit;
     uint64_t n_visit;
-    uint32_t bucket_lo, bucket_hi;            // PART keeps buckets lo <= b < hi (hi 0: all)
+    uint32_t bucket_lo, bucket_hi;            // launch_part keeps buckets lo <= b < hi (hi 0: all)
     uint64_t tile0;                           // without visit: tiles tile0 .. tile0 + n_tiles - 1
-    unsigned long long *bucket_cursor;        // 256 fill levels (PART)
-    const unsigned long long *bucket_base;    // 256 start offsets in `list` (PART)
-    const unsigned long long *bucket_end;     // 256 end offsets in `list` (PART)
+    unsigned long long *bucket_cursor;        // 256 fill levels (launch_part)
+    const unsigned long long *bucket_base;    // 256 start offsets in `list` (launch_part)
+    const unsigned long long *bucket_end;     // 256 end offsets in `list` (launch_part)
 };
 
-// MODE_PART scatters k-mer words by root prefix (the word's top 8 bits, the
-// last four bases), MODE_PARTS string keys (the k bases first-base-high, left
-// aligned) by their first four bases, so that buckets are consecutive ranges
-// of the printed order.
-enum ExtractMode : int {
-    MODE_SCAN = 0, MODE_INSERT = 1, MODE_BLOOM = 2, MODE_EMIT = 3, MODE_PART = 4, MODE_PARTS = 5
-};
+enum ExtractMode : int { MODE_SCAN = 0, MODE_INSERT = 1, MODE_BLOOM = 2, MODE_EMIT = 3 };
 
 constexpr uint32_t WORK_ITEM_KEYS = 2048;   // k-mers per work item (8 per thread)
 constexpr uint32_t BUCKET_HLL_BITS = 10;    // HyperLogLog registers per bucket = 2^10
@@ -187,9 +181,13 @@ cudaError_t launch_newlines(const uint8_t *buf, uint64_t n_tiles, uint32_t *tile
 cudaError_t launch_chunk_lastnl(const int32_t *tile_lastnl, const uint32_t *tile_seg, const Seg *segs,
                                 const uint64_t *seg_chunk0, uint64_t n_tiles, int32_t *chunk_lastnl,
                                 cudaStream_t st);
-// part_shape (MODE_PART, kc_tuning.part_shape): 1 stages 4096 k-mers a round
-// (three blocks per SM), 2 stages 2048 (four blocks per SM).
-cudaError_t launch_extract(int mode, const ExtractArgs &a, int grid, cudaStream_t st, uint32_t part_shape = 1);
+cudaError_t launch_extract(int mode, const ExtractArgs &a, int grid, cudaStream_t st);
+// The partition (kc_part.cu): every k-mer of k bases to its bucket's region of
+// a.list, the buckets by root prefix (the word's top 8 bits, the last four
+// bases), or, as string keys (the k bases first-base-high, left aligned), by
+// their first four bases, so that buckets are consecutive ranges of the printed
+// order.
+cudaError_t launch_part(bool by_string, uint32_t k, const ExtractArgs &a, cudaStream_t st);
 
 // Exclusive prefix sum of n 32-bit values into 64-bit outputs.  tmp must
 // hold scan_tmp_words(n) 64-bit words.

@@ -1,0 +1,317 @@
+// kc_part.cu -- the partition of a job's k-mers (k <= 32) into 256 buckets:
+// the FASTQ tiles are read once, every window of k valid bases becomes its
+// canonical k-mer, and the k-mers are scattered by their first four bases (as
+// string keys, for the counting by printed-order prefix) or by root prefix (as
+// k-mer words, the reference's get_root_prefix, for global-memory tables).
+#include <algorithm>
+
+#include "kc_device.cuh"
+#include "kc_kernels.cuh"
+
+namespace kc {
+
+namespace {
+
+constexpr uint32_t FULLW = 0xffffffffu;
+constexpr uint32_t PT_THREADS = 256;                 // one 32-byte segment per thread
+constexpr uint32_t PT_BUF = TILE + HALO;             // 8224, a multiple of 16
+constexpr uint32_t PT_SEGS = PT_THREADS + 1;         // the halo segment first
+constexpr uint32_t PT_CHUNK = 16;                    // positions a thread rolls along
+constexpr uint32_t PT_STAGE = PT_THREADS * PT_CHUNK; // most k-mers of a round
+
+struct PartSmem {
+    uint8_t tile[PT_BUF];
+    unsigned long long codes[PT_SEGS + 7];   // 2-bit codes of a segment's bytes
+    uint32_t good[PT_SEGS + 7];              // valid bases in sequence lines
+    uint32_t chunk[2 * PT_THREADS];          // chunks holding window ends
+    unsigned long long stage[PT_STAGE];      // a round's k-mers in bucket order
+};
+
+// Sum of the first `warp` of eight values.
+__device__ __forceinline__ uint32_t sum_before(const uint32_t *s, int warp, uint32_t &total)
+{
+    const uint4 a = *reinterpret_cast<const uint4 *>(s), b = *reinterpret_cast<const uint4 *>(s + 4);
+    const uint32_t v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    uint32_t before = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+        before += w < warp ? v[w] : 0u;
+        all += v[w];
+    }
+    total = all;
+    return before;
+}
+
+__device__ __forceinline__ uint32_t warp_inclusive(uint32_t v, int lane)
+{
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(FULLW, v, o);
+        if (lane >= o) v += y;
+    }
+    return v;
+}
+
+// One tile per block at a time.  Bytes are classified per 32-byte segment;
+// the 16-position chunks holding window ends are listed (header and quality
+// lines have none), and a thread rolls the forward and reverse-complement
+// words along one chunk, keeping its k-mers in registers while their ranks in
+// their buckets come from shared-memory counters.  The k-mers are then
+// written once to shared memory, in bucket order, and from there in runs of
+// one bucket.  The next tile's bytes arrive while this one's k-mers are formed
+// and written (the tile buffer is free once classified).
+//
+// Bound by instruction issue (58%) and shared-memory wavefronts (56%).  A
+// kernel that staged the k-mers unsorted in shared memory first (stores 64
+// bytes apart, 16 to a bank), rolled chunks of 8 with 64-bit shifts by variable
+// amounts, read the file's data and line numbers when a tile had arrived and
+// checked every k-mer against its bucket's region took 172 warp instructions
+// per 32 k-mers at three blocks per SM, this one 122 at four: 2.4G k-mers of
+// 150-base reads 21.2 -> 13.7 ms, 480M 4.25 -> 2.74, 25M 0.23 -> 0.15.
+//
+// W: k > 16 (words reach into both halves; below, the upper half holds all).
+template <bool STRING, bool W>
+__global__ void __launch_bounds__(PT_THREADS, 4) k_part(ExtractArgs a)
+{
+    extern __shared__ __align__(128) uint8_t pt_smem[];
+    PartSmem &s = *reinterpret_cast<PartSmem *>(pt_smem);
+    __shared__ __align__(8) uint64_t mbar;
+    __shared__ __align__(16) uint32_t s_wnl[8], s_wbk[8];
+    __shared__ uint32_t s_hist[N_BUCKETS], s_start[N_BUCKETS], s_lim[N_BUCKETS];
+    __shared__ unsigned long long *s_ptr[N_BUCKETS];
+    __shared__ uint32_t s_nch, s_over;
+
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    uint64_t u = blockIdx.x;
+    if (u >= a.n_tiles) return;
+    uint32_t lt;
+    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
+    if (tid == 0) {
+        mbar_init(&mbar, 1);
+        fence_mbar_init();
+        s_over = 0;
+    }
+    s_hist[tid] = 0;
+    __syncthreads();
+    if (tid == 0) {
+        mbar_expect_tx(&mbar, PT_BUF);
+        bulk_load(s.tile, a.buf + (a.tile0 + u) * TILE - HALO, PT_BUF, &mbar);
+    }
+    const uint32_t blo = a.bucket_lo, bhi = a.bucket_hi ? a.bucket_hi : N_BUCKETS;
+    const bool all_buckets = blo == 0 && bhi == N_BUCKETS;
+    // the file a tile lies in and its first line's number (mod 4 is all that
+    // counts) are read a tile ahead; the file's own data when it changes
+    uint32_t seg_next = a.tile_seg[a.tile0 + u], seg_cur = 0xFFFFFFFFu;
+    uint32_t line_next = (uint32_t)a.tile_prefix[a.tile0 + u], line_file = 0, k = 0;
+    uint64_t first_tile = 0;
+    for (uint32_t iter = 0; u < a.n_tiles; u += gridDim.x, ++iter) {
+        const uint64_t t = a.tile0 + u;
+        if (tid == 0) s_nch = 0;
+        if (seg_next != seg_cur) {
+            seg_cur = seg_next;
+            first_tile = a.segs[seg_cur].first_tile;
+            k = a.segs[seg_cur].k;
+            line_file = (uint32_t)a.tile_prefix[first_tile];
+        }
+        const uint32_t line0 = line_next - line_file;
+        const bool ok = mbar_wait(&mbar, iter & 1);
+        if (__syncthreads_or(!ok)) {
+            if (tid == 0) atomicOr(&a.counters[C_FLAGS], ERR_WAIT_TIMEOUT);
+            return;
+        }
+        const bool first = t == first_tile;
+        const uint32_t fs = 64 - 2 * k;
+
+        // ---- segments: codes, valid bases, lines
+        uint64_t codes;
+        uint32_t valid, nl;
+        classify32(s.tile + HALO + 32 * tid, codes, valid, nl);
+        const uint32_t own_nl = (uint32_t)__popc(nl);
+        const uint32_t inc_nl = warp_inclusive(own_nl, lane);
+        if (lane == 31) s_wnl[warp] = inc_nl;
+        s.codes[tid + 1] = codes;
+        if (warp == 0) {
+            // the halo segment (the end of the file's previous tile), a byte per lane
+            const uint32_t b = s.tile[lane], up = b & 0xDFu;
+            const bool v = up == 'A' || up == 'C' || up == 'G' || up == 'T' || up == 'U';
+            const uint32_t c = ((up >> 1) & 3u) ^ ((up >> 2) & 1u);
+            const uint32_t hn = __ballot_sync(FULLW, b == '\n'), hv = __ballot_sync(FULLW, v);
+            const uint32_t lo = __reduce_or_sync(FULLW, lane < 16 ? c << (2 * lane) : 0u);
+            const uint32_t hi = __reduce_or_sync(FULLW, lane >= 16 ? c << (2 * (lane - 16)) : 0u);
+            if (lane == 0) {
+                s.codes[0] = ((uint64_t)hi << 32) | lo;
+                s.good[0] = first ? 0u : hv & line_mask(line0 - (uint32_t)__popc(hn), hn, 1);
+            }
+        }
+        __syncthreads();
+        uint32_t tot_nl;
+        const uint32_t before_nl = sum_before(s_wnl, warp, tot_nl);
+        s.good[tid + 1] = valid & line_mask(line0 + before_nl + inc_nl - own_nl, nl, 1);
+        __syncthreads();
+        // classified: the tile buffer takes the next tile
+        if (u + gridDim.x < a.n_tiles) {
+            if (tid == 0) {
+                fence_proxy_async_smem();
+                mbar_expect_tx(&mbar, PT_BUF);
+                bulk_load(s.tile, a.buf + (t + gridDim.x) * TILE - HALO, PT_BUF, &mbar);
+            }
+            seg_next = a.tile_seg[t + gridDim.x];
+            line_next = (uint32_t)a.tile_prefix[t + gridDim.x];
+        }
+
+        // ---- chunks holding ends of windows of k valid bases, in any order
+        const uint32_t ends = run_ends((uint64_t)s.good[tid] | ((uint64_t)s.good[tid + 1] << 32), k);
+        {
+            const uint32_t e0 = ends & 0xFFFFu, e1 = ends >> 16;
+            const uint32_t b0 = __ballot_sync(FULLW, e0 != 0), b1 = __ballot_sync(FULLW, e1 != 0);
+            uint32_t at = 0;
+            if (lane == 0 && (b0 | b1)) at = atomicAdd(&s_nch, (uint32_t)(__popc(b0) + __popc(b1)));
+            at = __shfl_sync(FULLW, at, 0);
+            if (e0) s.chunk[at + (uint32_t)__popc(b0 & lt)] = ((uint32_t)tid << 17) | e0;
+            if (e1) s.chunk[at + (uint32_t)(__popc(b0) + __popc(b1 & lt))] = ((uint32_t)tid << 17) | 0x10000u | e1;
+        }
+        __syncthreads();
+        const uint32_t n_ch = s_nch;
+        const uint64_t topmask = k >= 32 ? ~0ULL : ~0ULL << fs;
+        const uint32_t tm_hi = (uint32_t)(topmask >> 32), tm_lo = (uint32_t)topmask;
+
+        for (uint32_t r0 = 0; r0 < n_ch; r0 += PT_THREADS) {
+            uint32_t e = 0;
+            uint32_t kh[PT_CHUNK], kl[PT_CHUNK], rk[PT_CHUNK / 2];
+            if (r0 + tid < n_ch) {
+                const uint32_t ch = s.chunk[r0 + tid];
+                e = ch & 0xFFFFu;
+                const uint32_t sgm = ch >> 17;
+                const uint64_t prev = s.codes[sgm], cur = s.codes[sgm + 1];
+                const bool half = (ch & 0x10000u) != 0;
+                // the window ending just before the chunk: forward word (base
+                // i at bit 64-2k+2i, stale bits below) and, from it, the
+                // reverse complement's
+                const uint32_t cw = half ? (uint32_t)(cur >> 32) : (uint32_t)cur;   // the chunk's 16 codes
+                uint32_t fh = half ? (uint32_t)cur : (uint32_t)(prev >> 32);
+                uint32_t fl = half ? (uint32_t)(prev >> 32) : (uint32_t)prev;
+                const uint64_t rc0 = ~(pair_reverse(((uint64_t)fh << 32) | fl) << fs) & topmask;
+                uint32_t rh = (uint32_t)(rc0 >> 32), rl = (uint32_t)rc0;
+                // complemented codes at the bits where the roll takes them in
+                const uint64_t nc = (uint64_t)(~cw) << (W ? fs : fs - 32);
+                const uint32_t nc_hi = (uint32_t)(nc >> 32), nc_lo = (uint32_t)nc;
+                const uint32_t in_mask = 3u << (W ? fs : fs - 32);
+#pragma unroll
+                for (uint32_t p = 0; p < PT_CHUNK; ++p) {
+                    const uint32_t in = __funnelshift_r(nc_lo, nc_hi, 2 * p) & in_mask;
+                    if (W) {
+                        fl = __funnelshift_r(fl, fh, 2);
+                        rh = __funnelshift_l(rl, rh, 2);
+                        rl = (rl << 2) | in;
+                    } else {
+                        rh = (rh << 2) | in;
+                    }
+                    fh = (fh >> 2) | ((cw << (30 - 2 * p)) & 0xC0000000u);
+                    // the canonical word is the smaller one; the string key of
+                    // the canonical strand is the complement of the larger one
+                    const uint32_t xh = W ? fh : fh & tm_hi, xl = W ? fl & tm_lo : 0u;
+                    const bool less = W ? (((uint64_t)xh << 32) | xl) < (((uint64_t)rh << 32) | rl) : xh < rh;
+                    if (STRING) {
+                        kh[p] = W ? ~(less ? rh : xh) : ~(less ? rh : xh) & tm_hi;
+                        kl[p] = W ? ~(less ? rl : xl) & tm_lo : 0u;
+                    } else {
+                        kh[p] = less ? xh : rh;
+                        kl[p] = W ? (less ? xl : rl) : 0u;
+                    }
+                }
+                if (!all_buckets) {
+#pragma unroll
+                    for (uint32_t p = 0; p < PT_CHUNK; ++p) {
+                        const uint32_t b = kh[p] >> 24;
+                        if (b < blo || b >= bhi) e &= ~(1u << p);
+                    }
+                }
+#pragma unroll
+                for (uint32_t p = 0; p < PT_CHUNK; ++p) {
+                    uint32_t r = 0;
+                    if ((e >> p) & 1u) r = atomicAdd(&s_hist[kh[p] >> 24], 1u);
+                    if (p & 1) rk[p / 2] |= r << 16;
+                    else rk[p / 2] = r;
+                }
+            }
+            __syncthreads();
+            // bucket starts; the cursor update is in flight while the k-mers
+            // are placed
+            const uint32_t c = s_hist[tid];
+            s_hist[tid] = 0;
+            const unsigned long long cur = c ? atomicAdd(&a.bucket_cursor[tid], (unsigned long long)c) : 0ull;
+            const uint32_t inc = warp_inclusive(c, lane);
+            if (lane == 31) s_wbk[warp] = inc;
+            __syncthreads();
+            uint32_t n;
+            const uint32_t start = sum_before(s_wbk, warp, n) + inc - c;
+            s_start[tid] = start;
+            __syncthreads();
+#pragma unroll
+            for (uint32_t p = 0; p < PT_CHUNK; ++p)
+                if ((e >> p) & 1u)
+                    s.stage[s_start[kh[p] >> 24] + ((rk[p / 2] >> (16 * (p & 1))) & 0xFFFFu)] =
+                        ((unsigned long long)kh[p] << 32) | kl[p];
+            // sorted index i of bucket b goes to s_ptr[b] + i; a bucket that
+            // outgrows its estimated region is reported by its cursor and
+            // redone, and only its region's part is written
+            if (c) {
+                const unsigned long long at = a.bucket_base[tid] + cur;
+                const unsigned long long end = a.bucket_end[tid] < a.list_cap ? a.bucket_end[tid] : a.list_cap;
+                s_ptr[tid] = a.list + at - start;
+                s_lim[tid] = start + (uint32_t)(at >= end ? 0ull : (end - at < c ? end - at : c));
+                if (at + c > end) s_over = 1;
+            }
+            __syncthreads();
+            if (!s_over) {
+#pragma unroll 4
+                for (uint32_t i = tid; i < n; i += PT_THREADS) {
+                    const unsigned long long key = s.stage[i];
+                    s_ptr[key >> 56][i] = key;
+                }
+            } else {
+                for (uint32_t i = tid; i < n; i += PT_THREADS) {
+                    const unsigned long long key = s.stage[i];
+                    const uint32_t b = (uint32_t)(key >> 56);
+                    if (i < s_lim[b]) s_ptr[b][i] = key;
+                }
+            }
+            if (r0 + PT_THREADS < n_ch) __syncthreads();   // another round: its ranks and stage follow
+        }
+        // s_over stays set: the launch is redone as a whole
+    }
+}
+
+int part_sms()
+{
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return n > 0 ? n : 148;
+}
+
+template <bool STRING, bool W>
+cudaError_t launch_part_t(const ExtractArgs &a, cudaStream_t st)
+{
+    auto kern = k_part<STRING, W>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PartSmem));
+    if (e != cudaSuccess) return e;
+    int per_sm = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, PT_THREADS, sizeof(PartSmem));
+    if (e != cudaSuccess) return e;
+    const uint64_t grid = std::min<uint64_t>(a.n_tiles, (uint64_t)part_sms() * std::max(per_sm, 1));
+    note_kernel_launch();
+    kern<<<(unsigned)grid, PT_THREADS, sizeof(PartSmem), st>>>(a);
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t launch_part(bool by_string, uint32_t k, const ExtractArgs &a, cudaStream_t st)
+{
+    if (!a.n_tiles) return cudaSuccess;
+    if (k > 16) return by_string ? launch_part_t<true, true>(a, st) : launch_part_t<false, true>(a, st);
+    return by_string ? launch_part_t<true, false>(a, st) : launch_part_t<false, false>(a, st);
+}
+
+}  // namespace kc
