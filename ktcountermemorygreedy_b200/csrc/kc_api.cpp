@@ -1312,9 +1312,7 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
     // ---- queries --------------------------------------------------------------
     if (P.top_n || P.want_le2) {
         clk.begin(7);
-        uint32_t *flags = ds.n<uint32_t>(std::max<uint64_t>(n_rec, 1));
-        unsigned long long *pos = ds.n<unsigned long long>(std::max<uint64_t>(n_rec, 1));
-        unsigned long long *qtmp = ds.n<unsigned long long>(scan_tmp_words(std::max<uint64_t>(n_rec, 1)));
+        void *qtmp = ds.get(select_tmp_bytes(n_rec));
         if (P.top_n && n_rec) {
             // threshold from the histogram restricted to the record range
             auto count_at = [&](uint64_t c) -> uint64_t { return c < HIST_BINS ? hd[c] : 0; };
@@ -1338,27 +1336,18 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
                     if (c == 0) break;
                 }
             }
-            // strictly above the threshold
+            // the records above the threshold, and the first ones at it
             unsigned long long *ak = ds.n<unsigned long long>(P.top_n);
             uint32_t *ac = ds.n<uint32_t>(P.top_n);
             unsigned long long *bk = ds.n<unsigned long long>(P.top_n);
             uint32_t *bc = ds.n<uint32_t>(P.top_n);
-            uint64_t n_above = 0, n_at = 0;
-            if (thr < 0xffffffffu) {
-                CK(launch_select_range(rec_keys, rec_counts, n_rec, thr + 1, 0xffffffffu, P.top_n, ak, ac, flags, pos,
-                                       qtmp, counters, C_SEL_A, st));
-            } else {
-                CK(cudaMemsetAsync(&counters[C_SEL_A], 0, 8, st));
-            }
-            Counters ca = read_counters(counters, st);
-            n_above = std::min<uint64_t>(ca.v[C_SEL_A], P.top_n);
-            uint64_t need = P.top_n - n_above;
-            if (need) {
-                CK(launch_select_range(rec_keys, rec_counts, n_rec, thr, thr, need, bk, bc, flags, pos, qtmp, counters,
-                                       C_SEL_B, st));
-                Counters cb = read_counters(counters, st);
-                n_at = std::min<uint64_t>(cb.v[C_SEL_B], need);
-            }
+            const SelectRange at_thr{thr, thr, P.top_n, bk, bc, C_SEL_B};
+            const SelectRange sel[2] = {at_thr, SelectRange{thr + 1, 0xffffffffu, P.top_n, ak, ac, C_SEL_A}};
+            CK(cudaMemsetAsync(&counters[C_SEL_A], 0, 8, st));
+            CK(launch_select(rec_keys, rec_counts, n_rec, sel, thr < 0xffffffffu ? 2 : 1, qtmp, counters, st));
+            const Counters ca = read_counters(counters, st);
+            const uint64_t n_above = std::min<uint64_t>(ca.v[C_SEL_A], P.top_n);
+            const uint64_t n_at = std::min<uint64_t>(ca.v[C_SEL_B], P.top_n - n_above);
             std::vector<uint64_t> tk(n_above), tk2(n_at);
             std::vector<uint32_t> tc(n_above), tc2(n_at);
             if (n_above) {
@@ -1381,8 +1370,8 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
         if (P.want_le2 && n_rec) {
             unsigned long long *lk = ds.n<unsigned long long>(n_rec);
             uint32_t *lc = ds.n<uint32_t>(n_rec);
-            CK(launch_select_range(rec_keys, rec_counts, n_rec, 0, 2, n_rec, lk, lc, flags, pos, qtmp, counters, C_SEL_A,
-                                   st));
+            const SelectRange sel{0, 2, n_rec, lk, lc, C_SEL_A};
+            CK(launch_select(rec_keys, rec_counts, n_rec, &sel, 1, qtmp, counters, st));
             Counters cl = read_counters(counters, st);
             uint64_t nl = std::min<uint64_t>(cl.v[C_SEL_A], n_rec);
             job.le2.allocate(nl);
@@ -1678,17 +1667,13 @@ void run_wide_job(Job &job, cudaStream_t st, Workspace &ws, const kc_tuning &tn)
     // ---- queries: record positions selected by count, their keys gathered --------
     if ((P.top_n || P.want_le2) && n_rec) {
         clk.begin(7);
-        unsigned long long *idx = ds.n<unsigned long long>(n_rec);
-        CK(launch_iota_u64(idx, n_rec, st));
-        uint32_t *flags = ds.n<uint32_t>(n_rec);
-        unsigned long long *pos = ds.n<unsigned long long>(n_rec);
-        unsigned long long *qtmp = ds.n<unsigned long long>(scan_tmp_words(n_rec));
+        void *qtmp = ds.get(select_tmp_bytes(n_rec));
         auto select = [&](uint32_t lo, uint32_t hi, uint64_t limit, int ctr, std::vector<uint64_t> &keys_out,
                           std::vector<uint32_t> &counts_out) {
             unsigned long long *si = ds.n<unsigned long long>(std::max<uint64_t>(limit, 1));
             uint32_t *scn = ds.n<uint32_t>(std::max<uint64_t>(limit, 1));
-            CK(cudaMemsetAsync(&counters[ctr], 0, 8, st));
-            CK(launch_select_range(idx, sc, n_rec, lo, hi, limit, si, scn, flags, pos, qtmp, counters, ctr, st));
+            const SelectRange sel{lo, hi, limit, si, scn, ctr};   // record positions
+            CK(launch_select(nullptr, sc, n_rec, &sel, 1, qtmp, counters, st));
             Counters cs = read_counters(counters, st);
             const uint64_t m = std::min<uint64_t>(cs.v[ctr], limit);
             unsigned long long *rows = ds.n<unsigned long long>(std::max<uint64_t>(m, 1) * nw);

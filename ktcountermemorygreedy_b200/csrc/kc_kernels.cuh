@@ -289,12 +289,21 @@ void note_kernel_launch();
 
 cudaError_t launch_pair_reverse(unsigned long long *keys, uint64_t n, cudaStream_t st);
 
-// Stable selection of records whose count satisfies lo <= c <= hi: writes the
-// selected keys/counts in input order.  Uses the scan temp space.
-cudaError_t launch_select_range(const unsigned long long *keys, const uint32_t *counts, uint64_t n, uint32_t lo,
-                                uint32_t hi, uint64_t limit, unsigned long long *out_keys, uint32_t *out_counts,
-                                uint32_t *flags, unsigned long long *pos, unsigned long long *tmp,
-                                unsigned long long *counters, int counter_idx, cudaStream_t st);
+// Stable selection of the records whose count lies in one of one or two
+// ranges: a range's first `limit` records go, in input order, to out_keys /
+// out_counts, and their full number to counters[counter].  keys NULL: the
+// records' indexes are written in place of their keys.  counts must be 16-byte
+// aligned; tmp holds select_tmp_bytes(n) bytes.
+struct SelectRange {
+    uint32_t lo, hi;
+    uint64_t limit;
+    unsigned long long *out_keys;
+    uint32_t *out_counts;
+    int counter;
+};
+size_t select_tmp_bytes(uint64_t n);
+cudaError_t launch_select(const unsigned long long *keys, const uint32_t *counts, uint64_t n, const SelectRange *ranges,
+                          uint32_t n_ranges, void *tmp, unsigned long long *counters, cudaStream_t st);
 
 // Bucket-major kernels of the partitioned pipeline; each resets *next_item.
 // Sub-bucket path.  count: sub_count[sub_base + s] += the keys of bucket b

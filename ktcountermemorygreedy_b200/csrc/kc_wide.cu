@@ -581,12 +581,6 @@ __global__ void k_iota_u32(uint32_t *p, uint64_t n)
         p[i] = (uint32_t)i;
 }
 
-__global__ void k_iota_u64(unsigned long long *p, uint64_t n)
-{
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        p[i] = i;
-}
-
 // skey[i] = word w of record perm[i], its 2-bit groups reversed (printed order)
 template <uint32_t N>
 __global__ void k_wide_sort_word(const unsigned long long *keys, const uint32_t *perm, uint64_t n, uint32_t w,
@@ -783,14 +777,6 @@ cudaError_t launch_pack_high(uint32_t k, const unsigned long long *keys, const u
     if (k <= 32) k_pack_write<1><<<g, 256, 0, st>>>(keys, counts, flags, pos, n, full, tail, count_bytes, out, n_bytes);
     else if (k <= 64) k_pack_write<2><<<g, 256, 0, st>>>(keys, counts, flags, pos, n, full, tail, count_bytes, out, n_bytes);
     else k_pack_write<4><<<g, 256, 0, st>>>(keys, counts, flags, pos, n, full, tail, count_bytes, out, n_bytes);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_iota_u64(unsigned long long *p, uint64_t n, cudaStream_t st)
-{
-    if (!n) return cudaSuccess;
-    note_kernel_launch();
-    k_iota_u64<<<wide_grid(n, 256), 256, 0, st>>>(p, n);
     return cudaGetLastError();
 }
 

@@ -88,8 +88,6 @@ cudaError_t launch_wide_sort(uint32_t k, const unsigned long long *keys, const u
 // out rows i = keys rows idx[i] (idx: record positions as 64-bit words).
 cudaError_t launch_wide_gather_rows(uint32_t k, const unsigned long long *keys, const unsigned long long *idx,
                                     uint64_t n, unsigned long long *out, cudaStream_t st);
-// 0, 1, 2, ... n - 1
-cudaError_t launch_iota_u64(unsigned long long *p, uint64_t n, cudaStream_t st);
 
 // high.bin bytes of sorted records (src/FinalDrainWriter.h:71-88): for each
 // record whose count c has c + 1 >= filter_min and c <= filter_max

@@ -93,3 +93,22 @@ def test_sort_units_of_every_size(counter, per_bucket):
     reads = bases[rng.integers(0, 4, size=(per_bucket * 256 // 118, 150))]
     fq = b"".join(b"@r\n" + r.tobytes() + b"\n+\n" + b"I" * 150 + b"\n" for r in reads)
     _check(counter, fq, 31, 1, bloom=True, memory_gb=1)
+
+
+@pytest.mark.parametrize("n", [1, 3, 1023, 4095, 4096, 4097, 8193])
+@pytest.mark.parametrize("k", [31, 47])
+def test_queries_at_chunk_edges(counter, n, k):
+    """n records around the selection's chunks (4096 counts, four per load),
+    with 1, 2 or 3 occurrences: top-N of several N and the count <= 2 set."""
+    rnd = random.Random(n)
+    g = "".join(rnd.choice("ACGT") for _ in range(n + k - 1))
+    kmers = [g[i:i + k] for i in range(n)]
+    seqs = [g] + [kmers[i] for i in range(n) if i % 3 != 0] + [kmers[i] for i in range(n) if i % 7 == 1]
+    fq = _fastq(seqs)
+    want_k, want_c = (O.exact_records if k <= 32 else O.exact_records_wide)([fq], k, U32)
+    assert len(want_c) == n
+    order = np.argsort(-want_c.astype(np.int64), kind="stable")
+    for top in (1, 7, n, n + 5):
+        r = counter.count([fq], k=k, count_max=U32, top_n=top, want_le2=True)
+        assert np.array_equal(r.top_keys, want_k[order[:top]]) and np.array_equal(r.top_counts, want_c[order[:top]])
+        assert np.array_equal(r.le2_keys, want_k[want_c <= 2]) and np.array_equal(r.le2_counts, want_c[want_c <= 2])
