@@ -31,6 +31,7 @@
 #include <cstdio>
 #include <cstring>
 #include <deque>
+#include <functional>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -382,6 +383,217 @@ uint64_t default_pass_budget(Workspace &ws)
     }
     cudaGetLastError();
     return (uint64_t)(0.7 * (double)(free_b + ws_free + pool_slack));
+}
+
+// One counting pass of the prefix path: partitioned string keys -> sorted
+// records, histograms and totals.  The buckets are cut into sub-buckets by the
+// next bases, each counted in a shared-memory table, and its records sorted on
+// their own.  A bucket starts with at most SUB_KEYS_TARGET k-mers per
+// sub-bucket; one whose sub-buckets no number of rounds fits is cut into 16
+// times as many and the pass counted again, and a bucket that cannot be cut
+// further is reported by SubTablesFull.
+struct PrefixPass {
+    uint32_t words = 1;                 // 64-bit words per key
+    uint32_t lo = 0, hi = 0;            // its buckets; their keys are cfg[b].key_base, key_len
+    uint32_t base_bits = 8;             // bits of the first word that a bucket's keys share
+    const BucketCfg *cfg = nullptr;
+    std::vector<SubCfg> sc;             // per bucket: k, group and count limits
+    uint32_t n_groups = 1, hist_bins = 0;
+    unsigned long long *hist = nullptr; // hist_bins per group, added to
+    uint32_t *ovf = nullptr;
+    unsigned long long *ovf64 = nullptr;
+    uint64_t ovf_cap = 0;
+    unsigned long long *counters = nullptr;
+    // the partitioned keys, whose array then takes the unsorted records' keys,
+    // room for the keys in sub-bucket order, and the records' counts: list_cap
+    // entries each
+    unsigned long long *keys = nullptr, *list = nullptr;
+    uint32_t *tmp_counts = nullptr;
+    uint64_t list_cap = 0;
+    uint32_t fault_inject = 0;
+    std::function<void()> repartition;  // fills keys again, as they were
+    // results
+    unsigned long long *rec_keys = nullptr;
+    uint32_t *rec_counts = nullptr;
+    uint64_t n_rec = 0, n_keys = 0, table_cap = 0;
+    uint32_t region_redos = 0;
+    std::vector<unsigned long long> totals;   // per group: distinct k-mers, k-mers seen once, records
+};
+
+// Entries of a pass's arrays for n keys: room for the sub-buckets' estimated
+// regions (their sizes plus about 15% on a large pass).
+uint64_t prefix_list_cap(uint64_t n) { return n + n / 4 + 65536; }
+
+void count_by_prefix(PrefixPass &pp, DevScope &ds, HostStage &hs, PhaseClock &clk, const kc_tuning &tn, cudaStream_t st)
+{
+    const uint32_t lo = pp.lo, hi = pp.hi, N = pp.words;
+    unsigned long long *counters = pp.counters;
+    const uint32_t shape = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(tn.count_shape, 4));
+    const uint64_t keys_target = SUB_KEYS_TARGET * sub_table_slots(N, shape) / sub_table_slots(1, 1);
+    std::vector<uint32_t> nsub(N_BUCKETS, 0), max_nsub(N_BUCKETS, 1);
+    for (uint32_t b = lo; b < hi; ++b) {
+        const uint32_t word_bits = std::min(2 * pp.sc[b].k, 64u);
+        if (word_bits > pp.base_bits)
+            max_nsub[b] = 1u << std::min<uint32_t>(word_bits - pp.base_bits, 31u - (uint32_t)__builtin_clz(SUB_MAX_PER_BUCKET));
+        nsub[b] = (uint32_t)std::min<uint64_t>(bit_ceil64((pp.cfg[b].key_len + keys_target - 1) / keys_target), max_nsub[b]);
+    }
+    // the overflow list's length before the attempts, restored after a failed
+    // one (on the device: no round trip)
+    unsigned long long *ovf_len_saved = ds.n<unsigned long long>(1);
+    CK(cudaMemcpyAsync(ovf_len_saved, counters + C_OVF_LEN, 8, cudaMemcpyDeviceToDevice, st));
+    // a large pass sizes the sub-buckets' regions from a sample of its keys
+    // instead of counting them all; a sub-bucket that outgrows its region sends
+    // the pass back to exact counts
+    bool exact_regions = false;
+    for (int attempt = 0;; ++attempt) {
+        const DevScope::Mark m0 = ds.mark();
+        std::vector<uint8_t> sb;
+        uint32_t n_sub = 0, max_sub = 1;
+        pp.n_keys = 0;
+        BucketRanges br{};
+        for (uint32_t b = lo; b < hi; ++b) {
+            const uint32_t lg = (uint32_t)__builtin_ctz(nsub[b]);
+            SubCfg &c = pp.sc[b];
+            c.sub_base = n_sub;
+            c.n_sub = nsub[b];
+            c.plen = pp.base_bits + lg;
+            c.shift = std::min(64 - c.plen, 63u);   // one sub-bucket: any shift will do
+            n_sub += nsub[b];
+            max_sub = std::max(max_sub, nsub[b]);
+            sb.insert(sb.end(), nsub[b], (uint8_t)b);
+            pp.n_keys += pp.cfg[b].key_len;
+            br.begin[b] = pp.cfg[b].key_base;
+            br.len[b] = pp.cfg[b].key_len;
+        }
+        SubCfg *d_sc = ds.n<SubCfg>(N_BUCKETS);
+        uint8_t *d_sb = ds.n<uint8_t>(n_sub);
+        uint32_t *sub_count = ds.n<uint32_t>(n_sub);
+        uint32_t *sub_len = ds.n<uint32_t>(n_sub);
+        unsigned long long *sub_off = ds.n<unsigned long long>(n_sub);
+        unsigned long long *sub_cur = ds.n<unsigned long long>(n_sub);
+        unsigned long long *sub_tmp = ds.n<unsigned long long>(scan_tmp_words(n_sub));
+        unsigned int *sub_next = ds.n<unsigned int>(1);
+        uint32_t *bucket_ovf = ds.n<uint32_t>(N_BUCKETS);
+        const size_t hist_n = (size_t)pp.n_groups * pp.hist_bins;
+        unsigned long long *hist_sub = ds.n<unsigned long long>(hist_n);
+        unsigned long long *totals = ds.n<unsigned long long>(3 * pp.n_groups);
+        const uint32_t unit_cap = 2 * n_sub + 4096;
+        SubUnit *units = ds.n<SubUnit>((size_t)UNIT_CLASSES * unit_cap);
+        const bool sampled = !exact_regions && pp.n_keys >= tn.sampled_region_keys;
+        const uint32_t stride = sampled ? SUB_REGION_SAMPLE : 1;
+        // each bucket-major launch gets its 256 ranges, not a list of items
+        auto upload_ranges = [&](uint32_t &n_items, uint64_t item_keys) {
+            n_items = fill_item_starts_n(br, item_keys);
+            BucketRanges *d = ds.n<BucketRanges>(1);
+            CK(cudaMemcpyAsync(d, hs.up(&br, 1), sizeof(BucketRanges), cudaMemcpyHostToDevice, st));
+            return d;
+        };
+        uint32_t n_items = 0, n_sp_items = 0;
+        BucketRanges *d_br = upload_ranges(n_items, SUB_COUNT_KEYS * stride);
+        BucketRanges *d_bs = upload_ranges(n_sp_items, sub_scatter_item_keys(max_sub, N));
+        CK(cudaMemcpyAsync(d_sc, hs.up(pp.sc.data(), N_BUCKETS), N_BUCKETS * sizeof(SubCfg), cudaMemcpyHostToDevice, st));
+        CK(cudaMemcpyAsync(d_sb, hs.up(sb.data(), n_sub), n_sub, cudaMemcpyHostToDevice, st));
+        CK(cudaMemsetAsync(sub_count, 0, n_sub * 4ull, st));
+        CK(cudaMemsetAsync(bucket_ovf, 0, N_BUCKETS * 4, st));
+        CK(cudaMemsetAsync(hist_sub, 0, hist_n * 8, st));
+        CK(cudaMemsetAsync(totals, 0, 3ull * pp.n_groups * 8, st));
+        CK(cudaMemsetAsync(counters + C_SUB_OVF, 0, 2 * 8, st));   // C_SUB_OVF, C_REGION_OVF
+        CK(cudaMemsetAsync(counters + C_UNITS, 0, UNIT_CLASSES * 8, st));
+        unsigned long long *sub_end = nullptr;
+        clk.begin(9);
+        if (sampled) {
+            uint32_t *region = ds.n<uint32_t>(n_sub);
+            sub_end = ds.n<unsigned long long>(n_sub);
+            CK(launch_subpart_count(pp.keys, d_br, n_items, d_sc, sub_count, N, st, stride));
+            CK(launch_subpart_regions(sub_count, n_sub, stride, region, sub_off, sub_end, sub_cur, sub_tmp, st));
+        } else {
+            CK(launch_subpart_count(pp.keys, d_br, n_items, d_sc, sub_count, N, st));
+            CK(launch_scan_u32(sub_count, sub_off, n_sub, sub_tmp, st));
+            CK(cudaMemcpyAsync(sub_cur, sub_off, (size_t)n_sub * 8, cudaMemcpyDeviceToDevice, st));
+        }
+        CK(launch_subpart_scatter(pp.keys, d_bs, n_sp_items, sub_next, d_sc, sub_cur, pp.list, pp.list_cap, max_sub, N, st,
+                                  sub_end, (uint32_t)tn.scatter_shape));
+        if (sampled)
+            CK(launch_subpart_sizes(sub_off, sub_cur, sub_end, n_sub, pp.list_cap, sub_count, counters + C_REGION_OVF, st));
+        clk.end();
+        clk.begin(10);
+        PrefixCountArgs pc{};
+        pc.keys = pp.list;
+        pc.sub_off = sub_off;
+        pc.sub_count = sub_count;
+        pc.sub_bucket = d_sb;
+        pc.sc = d_sc;
+        pc.n_sub = n_sub;
+        pc.next_sub = sub_next;
+        pc.rec_keys = pp.keys;
+        pc.rec_counts = pp.tmp_counts;
+        pc.sub_len = sub_len;
+        pc.units = units;
+        pc.unit_cap = unit_cap;
+        pc.hist_bins = pp.hist_bins;
+        pc.hist = hist_sub;
+        pc.totals = totals;
+        pc.ovf = pp.ovf;
+        pc.ovf64 = pp.ovf64;
+        pc.ovf_cap = pp.ovf_cap;
+        pc.counters = counters;
+        pc.bucket_ovf = bucket_ovf;
+        CK(launch_count_prefix(pc, N, shape, st));
+        clk.end();
+        if (attempt == 0 && (pp.fault_inject & KC_INJECT_TABLE_FULL_ONCE)) {
+            // as if the first bucket's sub-bucket tables had overflowed
+            CK(cudaMemsetAsync(bucket_ovf + lo, 0x01, 1, st));
+            CK(launch_or_flags(counters + C_SUB_OVF, 1ull, st));
+        }
+        unsigned long long *p_tot = hs.n<unsigned long long>(3 * pp.n_groups);
+        CK(cudaMemcpyAsync(p_tot, totals, 3ull * pp.n_groups * 8, cudaMemcpyDeviceToHost, st));
+        const Counters cs = read_counters(counters, st);
+        check_flags(cs.v[C_FLAGS], "sub-bucket count");
+        if (cs.v[C_REGION_OVF] || cs.v[C_SUB_OVF]) {
+            std::vector<uint32_t> bo(N_BUCKETS);
+            CK(cudaMemcpyAsync(bo.data(), bucket_ovf, N_BUCKETS * 4, cudaMemcpyDeviceToHost, st));
+            CK(cudaMemcpyAsync(counters + C_OVF_LEN, ovf_len_saved, 8, cudaMemcpyDeviceToDevice, st));
+            CK(cudaStreamSynchronize(st));
+            ds.rewind(m0);
+            if (cs.v[C_REGION_OVF]) {
+                // a sub-bucket outgrew its estimated region (the count then
+                // leaves the keys alone): exact regions, same sub-buckets
+                exact_regions = true;
+                ++pp.region_redos;
+            } else {
+                // buckets with more distinct k-mers than 64 rounds of their
+                // sub-buckets hold: 16 times the sub-buckets
+                bool cut = false;
+                for (uint32_t b = lo; b < hi; ++b) {
+                    if (!bo[b]) continue;
+                    if (nsub[b] * 2 > max_nsub[b]) throw SubTablesFull{};
+                    nsub[b] = std::min(nsub[b] * 16, max_nsub[b]);
+                    cut = true;
+                }
+                if (!cut) throw SubTablesFull{};
+                clk.begin(2);
+                pp.repartition();   // the records went over the partitioned keys
+                clk.end();
+            }
+            continue;
+        }
+        pp.totals.assign(p_tot, p_tot + 3 * pp.n_groups);
+        pp.n_rec = 0;
+        for (uint32_t g = 0; g < pp.n_groups; ++g) pp.n_rec += pp.totals[3 * g + 2];
+        clk.begin(6);
+        CK(launch_add_u64(pp.hist, hist_sub, hist_n, st));
+        pp.rec_keys = ds.n<unsigned long long>(std::max<uint64_t>(pp.n_rec, 1) * N);
+        pp.rec_counts = ds.n<uint32_t>(std::max<uint64_t>(pp.n_rec, 1));
+        // where each sub-bucket's records go; sub_cur is free again
+        CK(launch_scan_u32(sub_len, sub_cur, n_sub, sub_tmp, st));
+        uint32_t n_units[UNIT_CLASSES];
+        for (uint32_t c = 0; c < UNIT_CLASSES; ++c) n_units[c] = (uint32_t)cs.v[C_UNITS + c];
+        CK(launch_unit_sort(N, pp.keys, pp.tmp_counts, sub_off, sub_cur, units, unit_cap, n_units, pp.rec_keys,
+                            pp.rec_counts, pp.n_rec, st));
+        clk.end();
+        pp.table_cap = (uint64_t)n_sub * sub_table_slots(N, shape);
+        return;
+    }
 }
 
 // kc_job.pack_high: the high.bin bytes of the job's sorted records (k-mer
@@ -847,10 +1059,7 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
             unsigned long long list_cap = ocap;
             uint32_t *tmp_counts = nullptr;
             if (prefix) {
-                // room for the sub-buckets' estimated regions (their sizes plus
-                // about 15% on a large pass); the partitioned keys' array later
-                // takes the records' keys, at the sub-buckets' offsets
-                list_cap = ocap + ocap / 4 + 65536;
+                list_cap = prefix_list_cap(ocap);
                 list = ds.n<unsigned long long>(list_cap);
                 keys = ds.n<unsigned long long>(list_cap);
                 tmp_counts = ds.n<uint32_t>(list_cap);
@@ -922,189 +1131,57 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
             CK(cudaMemcpyAsync(d_cfg_b, hs.up(cfg.data(), N_BUCKETS), N_BUCKETS * sizeof(BucketCfg),
                                cudaMemcpyHostToDevice, st));
             // each bucket-major launch gets its 256 ranges, not a list of items
-            auto upload_ranges = [&](BucketRanges &r, uint32_t &n_items, uint64_t item_keys = WORK_ITEM_KEYS) {
-                n_items = fill_item_starts_n(r, item_keys);
+            auto upload_ranges = [&](BucketRanges &r, uint32_t &n_items) {
+                n_items = fill_item_starts_n(r, WORK_ITEM_KEYS);
                 BucketRanges *d = ds.n<BucketRanges>(1);
                 CK(cudaMemcpyAsync(d, hs.up(&r, 1), sizeof(BucketRanges), cudaMemcpyHostToDevice, st));
                 return d;
             };
-            // Prefix path: the buckets are cut into sub-buckets by the next bases,
-            // each counted in a shared-memory table, and its records sorted on
-            // their own.  A bucket starts with at most SUB_KEYS_TARGET k-mers per
-            // sub-bucket; one whose sub-buckets no number of rounds fits is cut
-            // into 16 times as many and the pass counted again, and a bucket that
-            // cannot be cut further sends the job to global-memory tables.
             if (prefix) {
-                const uint32_t shape = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(tn.count_shape, 4));
-                const uint64_t keys_target = SUB_KEYS_TARGET * sub_table_slots(shape) / sub_table_slots(1);
-                const uint32_t max_sub_k = 2 * k > 8 ? (2 * k >= 20 ? SUB_MAX_PER_BUCKET : 1u << (2 * k - 8)) : 1u;
-                std::vector<uint32_t> nsub(N_BUCKETS, 0);
-                for (uint32_t b = lo; b < hi; ++b)
-                    nsub[b] = (uint32_t)std::min<uint64_t>(
-                        bit_ceil64((cfg[b].key_len + keys_target - 1) / keys_target), max_sub_k);
-                // the overflow list's length before the attempts, restored after
-                // a failed one (on the device: no round trip)
-                unsigned long long *ovf_len_saved = ds.n<unsigned long long>(1);
-                CK(cudaMemcpyAsync(ovf_len_saved, counters + C_OVF_LEN, 8, cudaMemcpyDeviceToDevice, st));
-                // a large pass sizes the sub-buckets' regions from a sample of
-                // its keys instead of counting them all; a sub-bucket that
-                // outgrows its region sends the pass back to exact counts
-                bool exact_regions = false;
-                for (int attempt = 0;; ++attempt) {
-                    const DevScope::Mark m0 = ds.mark();
-                    std::vector<SubCfg> sc(N_BUCKETS);
-                    std::vector<uint8_t> sb;
-                    uint32_t n_sub = 0, max_sub = 1;
-                    uint64_t pass_keys = 0;
-                    for (uint32_t b = lo; b < hi; ++b) {
-                        sc[b].sub_base = n_sub;
-                        sc[b].n_sub = nsub[b];
-                        sc[b].shift = 56 - (uint32_t)__builtin_ctz(nsub[b]);
-                        n_sub += nsub[b];
-                        max_sub = std::max(max_sub, nsub[b]);
-                        sb.insert(sb.end(), nsub[b], (uint8_t)b);
-                        pass_keys += cfg[b].key_len;
-                    }
-                    SubCfg *d_sc = ds.n<SubCfg>(N_BUCKETS);
-                    uint8_t *d_sb = ds.n<uint8_t>(n_sub);
-                    uint32_t *sub_count = ds.n<uint32_t>(n_sub);
-                    uint32_t *sub_len = ds.n<uint32_t>(n_sub);
-                    unsigned long long *sub_off = ds.n<unsigned long long>(n_sub);
-                    unsigned long long *sub_cur = ds.n<unsigned long long>(n_sub);
-                    unsigned long long *sub_tmp = ds.n<unsigned long long>(scan_tmp_words(n_sub));
-                    unsigned int *sub_next = ds.n<unsigned int>(1);
-                    uint32_t *bucket_ovf = ds.n<uint32_t>(N_BUCKETS);
-                    unsigned long long *hist_sub = ds.n<unsigned long long>(HIST_BINS);
-                    const uint32_t unit_cap = 2 * n_sub + 4096;
-                    SubUnit *units = ds.n<SubUnit>((size_t)UNIT_CLASSES * unit_cap);
-                    BucketRanges br{};
-                    for (uint32_t b = lo; b < hi; ++b) {
-                        br.begin[b] = cfg[b].key_base;
-                        br.len[b] = cfg[b].key_len;
-                    }
-                    const bool sampled = !exact_regions && pass_keys >= tn.sampled_region_keys;
-                    const uint32_t stride = sampled ? SUB_REGION_SAMPLE : 1;
-                    uint32_t n_items = 0, n_sp_items = 0;
-                    BucketRanges *d_br = upload_ranges(br, n_items, SUB_COUNT_KEYS * stride);
-                    BucketRanges *d_bs = upload_ranges(br, n_sp_items, sub_scatter_item_keys(max_sub));
-                    CK(cudaMemcpyAsync(d_sc, hs.up(sc.data(), N_BUCKETS), N_BUCKETS * sizeof(SubCfg),
-                                       cudaMemcpyHostToDevice, st));
-                    CK(cudaMemcpyAsync(d_sb, hs.up(sb.data(), n_sub), n_sub, cudaMemcpyHostToDevice, st));
-                    CK(cudaMemsetAsync(sub_count, 0, n_sub * 4ull, st));
-                    CK(cudaMemsetAsync(bucket_ovf, 0, N_BUCKETS * 4, st));
-                    CK(cudaMemsetAsync(hist_sub, 0, HIST_BINS * 8, st));
-                    CK(cudaMemsetAsync(counters + C_REC_LEN, 0, 3 * 8, st));   // C_REC_LEN, C_LOW_ONLY, C_DISTINCT
-                    CK(cudaMemsetAsync(counters + C_SUB_OVF, 0, 2 * 8, st));   // C_SUB_OVF, C_REGION_OVF
-                    CK(cudaMemsetAsync(counters + C_UNITS, 0, UNIT_CLASSES * 8, st));
-                    unsigned long long *sub_end = nullptr;
-                    clk.begin(9);
-                    if (sampled) {
-                        uint32_t *region = ds.n<uint32_t>(n_sub);
-                        sub_end = ds.n<unsigned long long>(n_sub);
-                        CK(launch_subpart_count(keys, d_br, n_items, d_sc, sub_count, st, stride));
-                        CK(launch_subpart_regions(sub_count, n_sub, stride, region, sub_off, sub_end, sub_cur,
-                                                  sub_tmp, st));
-                    } else {
-                        CK(launch_subpart_count(keys, d_br, n_items, d_sc, sub_count, st));
-                        CK(launch_scan_u32(sub_count, sub_off, n_sub, sub_tmp, st));
-                        CK(cudaMemcpyAsync(sub_cur, sub_off, (size_t)n_sub * 8, cudaMemcpyDeviceToDevice, st));
-                    }
-                    CK(launch_subpart_scatter(keys, d_bs, n_sp_items, sub_next, d_sc, sub_cur, list, list_cap, max_sub,
-                                              st, sub_end, (uint32_t)tn.scatter_shape));
-                    if (sampled)
-                        CK(launch_subpart_sizes(sub_off, sub_cur, sub_end, n_sub, list_cap, sub_count,
-                                                counters + C_REGION_OVF, st));
-                    clk.end();
-                    clk.begin(10);
-                    PrefixCountArgs pc{};
-                    pc.keys = list;
-                    pc.sub_off = sub_off;
-                    pc.sub_count = sub_count;
-                    pc.sub_bucket = d_sb;
-                    pc.sc = d_sc;
-                    pc.n_sub = n_sub;
-                    pc.next_sub = sub_next;
-                    pc.count_max = count_max;
-                    pc.min_count = P.min_count;
-                    pc.max_count = P.max_count;
-                    pc.rec_keys = keys;
-                    pc.rec_counts = tmp_counts;
-                    pc.sub_len = sub_len;
-                    pc.units = units;
-                    pc.unit_cap = unit_cap;
-                    pc.hist = hist_sub;
-                    pc.ovf = ovf;
-                    pc.ovf_cap = ovf_cap;
-                    pc.counters = counters;
-                    pc.bucket_ovf = bucket_ovf;
-                    CK(launch_count_prefix(pc, shape, st));
-                    clk.end();
-                    if (attempt == 0 && (P.fault_inject & KC_INJECT_TABLE_FULL_ONCE)) {
-                        // as if the first bucket's sub-bucket tables had overflowed
-                        CK(cudaMemsetAsync(bucket_ovf + lo, 0x01, 1, st));
-                        CK(launch_or_flags(counters + C_SUB_OVF, 1ull, st));
-                    }
-                    const Counters cs = read_counters(counters, st);
-                    check_flags(cs.v[C_FLAGS], "sub-bucket count");
-                    const bool again = cs.v[C_REGION_OVF] || cs.v[C_SUB_OVF];
-                    if (again) {
-                        std::vector<uint32_t> bo(N_BUCKETS);
-                        CK(cudaMemcpyAsync(bo.data(), bucket_ovf, N_BUCKETS * 4, cudaMemcpyDeviceToHost, st));
-                        CK(cudaMemcpyAsync(counters + C_OVF_LEN, ovf_len_saved, 8, cudaMemcpyDeviceToDevice, st));
-                        CK(cudaStreamSynchronize(st));
-                        ds.rewind(m0);
-                        if (cs.v[C_REGION_OVF]) {
-                            // a sub-bucket outgrew its estimated region (the count
-                            // then leaves the keys alone): exact regions, same
-                            // sub-buckets
-                            exact_regions = true;
-                            ++job.region_redos;
-                        } else {
-                            // buckets with more distinct k-mers than 64 rounds of
-                            // their sub-buckets hold: 16 times the sub-buckets
-                            bool cut = false;
-                            for (uint32_t b = lo; b < hi; ++b) {
-                                if (!bo[b]) continue;
-                                if (nsub[b] * 2 > max_sub_k) throw SubTablesFull{};
-                                nsub[b] = std::min(nsub[b] * 16, max_sub_k);
-                                cut = true;
-                            }
-                            if (!cut) throw SubTablesFull{};
-                            // the records went over the partitioned keys
-                            CK(cudaMemsetAsync(cursor, 0, N_BUCKETS * 8, st));
-                            clk.begin(2);
-                            CK(launch_part(true, k, a, st));
-                            clk.end();
-                        }
-                        continue;
-                    }
-                    clk.begin(6);
-                    CK(launch_add_u64(hist, hist_sub, HIST_BINS, st));
-                    n_rec = cs.v[C_REC_LEN];
-                    rec_keys = ds.n<unsigned long long>(std::max<uint64_t>(n_rec, 1));
-                    rec_counts = ds.n<uint32_t>(std::max<uint64_t>(n_rec, 1));
-                    // where each sub-bucket's records go; sub_cur is free again
-                    CK(launch_scan_u32(sub_len, sub_cur, n_sub, sub_tmp, st));
-                    uint32_t n_units[UNIT_CLASSES];
-                    for (uint32_t c = 0; c < UNIT_CLASSES; ++c) n_units[c] = (uint32_t)cs.v[C_UNITS + c];
-                    CK(launch_unit_sort(keys, tmp_counts, sub_off, sub_cur, units, unit_cap, n_units, rec_keys, rec_counts,
-                                        n_rec, k, st));
-                    clk.end();
-                    rec_by_bucket = false;
-                    rec_sorted = true;
-                    job.distinct += cs.v[C_DISTINCT];
-                    if (P.bloom) {
-                        // the split: an occurrence is FIRST when it claims its k-mer's slot
-                        job.low_only += cs.v[C_LOW_ONLY];
-                        low_len += cs.v[C_DISTINCT];
-                        high_len += pass_keys - cs.v[C_DISTINCT];
-                    } else {
-                        high_len += pass_keys;
-                    }
-                    table_cap = std::max<uint64_t>(table_cap, (uint64_t)n_sub * sub_table_slots(shape));
-                    ++job.smem_passes;
-                    break;
+                PrefixPass pp;
+                pp.words = 1;
+                pp.lo = lo;
+                pp.hi = hi;
+                pp.base_bits = 8;
+                pp.cfg = cfg.data();
+                SubCfg lim{};
+                lim.k = k;
+                lim.count_max = count_max;
+                lim.min_count = P.min_count;
+                lim.max_count = P.max_count;
+                pp.sc.assign(N_BUCKETS, lim);
+                pp.hist = hist;
+                pp.hist_bins = HIST_BINS;
+                pp.ovf = ovf;
+                pp.ovf_cap = ovf_cap;
+                pp.counters = counters;
+                pp.keys = keys;
+                pp.list = list;
+                pp.tmp_counts = tmp_counts;
+                pp.list_cap = list_cap;
+                pp.fault_inject = P.fault_inject;
+                pp.repartition = [&] {
+                    CK(cudaMemsetAsync(cursor, 0, N_BUCKETS * 8, st));
+                    CK(launch_part(true, k, a, st));
+                };
+                count_by_prefix(pp, ds, hs, clk, tn, st);
+                rec_keys = pp.rec_keys;
+                rec_counts = pp.rec_counts;
+                n_rec = pp.n_rec;
+                rec_by_bucket = false;
+                rec_sorted = true;
+                job.distinct += pp.totals[0];
+                if (P.bloom) {
+                    // the split: an occurrence is FIRST when it claims its k-mer's slot
+                    job.low_only += pp.totals[1];
+                    low_len += pp.totals[0];
+                    high_len += pp.n_keys - pp.totals[0];
+                } else {
+                    high_len += pp.n_keys;
                 }
+                table_cap = std::max(table_cap, pp.table_cap);
+                job.region_redos += pp.region_redos;
+                ++job.smem_passes;
             }
             if (!prefix) {
                 std::vector<unsigned long long> lh(2 * N_BUCKETS, 0);
@@ -1411,7 +1488,10 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
 // src/main.cpp:617-633)
 // ---------------------------------------------------------------------------
 //
-// One job: upload -> newline census -> SCAN (occurrences, HyperLogLog,
+// Jobs of some size take the prefix path with N-word string keys: a sampled
+// census per first four bases -> per pass over a range of those: partition ->
+// sub-buckets -> count and sort in shared memory.
+// The others: upload -> newline census -> SCAN (occurrences, HyperLogLog,
 // occurrences per root prefix) -> per pass over a range of root prefixes:
 // INSERT into an N-word table sized from the estimate (regrown when full) ->
 // compaction (count, then records + histogram) -> sort of all records in
@@ -1420,7 +1500,7 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
 // memory until the final sort.  The Bloom split (kc_job.bloom) only chooses
 // which occurrences the reference keeps in memory; the counts are exact
 // either way, so these jobs count every occurrence in the table.
-void run_wide_job(Job &job, cudaStream_t st, Workspace &ws, const kc_tuning &tn)
+void run_wide_job(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, bool global_tables, const kc_tuning &tn)
 {
     const kc_job &P = job.p;
     const uint32_t k = P.k, nw = key_words(k);
@@ -1472,11 +1552,27 @@ void run_wide_job(Job &job, cudaStream_t st, Workspace &ws, const kc_tuning &tn)
         CK(launch_wait_flag(reinterpret_cast<const unsigned int *>(counters + C_COUNT - 1), 1024, counters + C_FLAGS,
                             st));
 
+    const bool prefix = tn.bloom_smem == 1 && !global_tables && in->total_bytes >= PREFIX_PATH_MIN_BYTES;
+    job.smem_passes = job.smem_fallbacks = job.region_redos = 0;
+    job.distinct = 0;
+
     // ---- SCAN: occurrences, distinct estimate, root-prefix histogram ---------
+    // (prefix path: occurrences per first four bases of every 8th tile, every
+    // 32nd from 512 MiB on)
     unsigned long long *scan_out = ds.n<unsigned long long>(1 + N_BUCKETS);   // occurrences, 256 bucket counts
     uint32_t *hll = ds.n<uint32_t>(HLL_M);
     CK(cudaMemsetAsync(scan_out, 0, (1 + N_BUCKETS) * 8, st));
     CK(cudaMemsetAsync(hll, 0, HLL_M * 4, st));
+    ExtractArgs pa{};
+    pa.buf = in->buf;
+    pa.n_tiles = T;
+    pa.tile_prefix = reinterpret_cast<const uint64_t *>(tile_prefix);
+    pa.tile_seg = in->d_tile_seg;
+    pa.segs = d_segs;
+    pa.counters = counters;
+    pa.occ = scan_out;
+    pa.bucket_hist = scan_out + 1;
+    pa.bucket_sample_mask = exact_census || T < 512 ? 0 : (T >= 65536 ? 31 : 7);
     WideArgs a{};
     a.buf = in->buf;
     a.n_tiles = T;
@@ -1488,7 +1584,8 @@ void run_wide_job(Job &job, cudaStream_t st, Workspace &ws, const kc_tuning &tn)
     a.bucket_hist = scan_out + 1;
     a.hll = hll;
     clk.begin(1);
-    CK(launch_wide_extract(WMODE_SCAN, k, a, st));
+    if (prefix) CK(launch_part_wide(true, k, pa, st));
+    else CK(launch_wide_extract(WMODE_SCAN, k, a, st));
     clk.end();
     unsigned long long *h_scan = hs.n<unsigned long long>(1 + N_BUCKETS);
     uint32_t *h_hll = hs.n<uint32_t>(HLL_M);
@@ -1496,11 +1593,18 @@ void run_wide_job(Job &job, cudaStream_t st, Workspace &ws, const kc_tuning &tn)
     CK(cudaMemcpyAsync(h_hll, hll, HLL_M * 4, cudaMemcpyDeviceToHost, st));
     Counters c0 = read_counters(counters, st);
     check_flags(c0.v[C_FLAGS], "scan");
-    const uint64_t O = h_scan[0];
+    uint64_t O = h_scan[0];
     std::vector<uint64_t> bh(h_scan + 1, h_scan + 1 + N_BUCKETS);
     const double est = hll_estimate(h_hll, HLL_M);
     job.occurrences = O;
     check_cancel(job, "after the scan");
+    const bool exact = !prefix || pa.bucket_sample_mask == 0;
+    if (!exact && O < 65536) throw CensusOverflow{};   // too thin a sample
+    if (!exact)   // each bucket's region: its share of the census, and some
+        for (auto &x : bh)
+            x = (uint64_t)std::ceil((double)x * 1.15 * (double)T /
+                                    (double)((T + pa.bucket_sample_mask) / (pa.bucket_sample_mask + 1))) +
+                8192;
 
     // ---- passes over ranges of root prefixes ------------------------------------
     // a pass holds its table (slots per estimated distinct k-mer at the
@@ -1515,7 +1619,11 @@ void run_wide_job(Job &job, cudaStream_t st, Workspace &ws, const kc_tuning &tn)
         uint64_t need = 0;
         for (uint32_t b = 0; b < N_BUCKETS; ++b) {
             const double share = O ? (double)bh[b] / (double)O : 0.0;
-            const uint64_t nb = (uint64_t)(share * est * (factor * slot_bytes + rec_bytes)) + 4096;
+            // prefix path: two key arrays and the counts with room for
+            // estimated sub-bucket regions, then at most n / min count records
+            const uint64_t per_key = 20ull * nw + 5 + rec_bytes / std::max(P.min_count, 1u) + 1;
+            const uint64_t nb = prefix ? bh[b] * per_key + 4096
+                                       : (uint64_t)(share * est * (factor * slot_bytes + rec_bytes)) + 4096;
             if (b > lo && need + nb > budget) {
                 ranges.push_back({lo, b});
                 lo = b;
@@ -1528,14 +1636,109 @@ void run_wide_job(Job &job, cudaStream_t st, Workspace &ws, const kc_tuning &tn)
     const bool multi = ranges.size() > 1;
     unsigned long long *hist = ds.n<unsigned long long>(HIST_BINS);
     CK(cudaMemsetAsync(hist, 0, HIST_BINS * 8, st));
-    const uint64_t ovf_cap = std::max<uint64_t>(1ull << 20, (uint64_t)(est / HIST_BINS) + 1);
+    const uint64_t ovf_cap = std::max<uint64_t>(
+        1ull << 20, prefix ? in->total_bytes / HIST_BINS + 1 : (uint64_t)(est / HIST_BINS) + 1);
     uint32_t *ovf = ds.n<uint32_t>(ovf_cap);
     std::vector<std::unique_ptr<HostRecords>> spilled;
     uint64_t n_rec = 0, inserted_total = 0, table_cap = 0;
     unsigned long long *rec_keys = nullptr;
     uint32_t *rec_counts = nullptr;
     bool injected_full = false;
+    // a pass's records: to pinned host memory when there are more passes
+    auto park = [&](const unsigned long long *rk, const uint32_t *rc, uint64_t kept, const DevScope::Mark &mk) {
+        auto hr = std::make_unique<HostRecords>();
+        hr->allocate(kept, nw);
+        if (kept) {
+            CK(cudaMemcpyAsync(hr->keys(), rk, kept * nw * 8, cudaMemcpyDeviceToHost, st));
+            CK(cudaMemcpyAsync(hr->counts(), rc, kept * 4, cudaMemcpyDeviceToHost, st));
+        }
+        Counters cw = read_counters(counters, st);
+        check_flags(cw.v[C_FLAGS], "compaction");
+        n_rec += kept;
+        spilled.push_back(std::move(hr));
+        ds.rewind(mk);
+    };
     for (const auto &rg : ranges) {
+        if (!prefix) break;
+        const DevScope::Mark mk = ds.mark();
+        check_cancel(job, "before a counting pass");
+        std::vector<BucketCfg> cfg(N_BUCKETS);
+        std::vector<unsigned long long> bb(2 * N_BUCKETS, 0);
+        uint64_t off = 0;
+        for (uint32_t b = rg.first; b < rg.second; ++b) {
+            cfg[b].key_base = bb[b] = off;
+            off += bh[b];
+            bb[N_BUCKETS + b] = off;
+        }
+        const uint64_t ocap = std::max<uint64_t>(off, 1), list_cap = prefix_list_cap(ocap);
+        unsigned long long *list = ds.n<unsigned long long>(list_cap * nw);
+        unsigned long long *keys = ds.n<unsigned long long>(list_cap * nw);
+        uint32_t *tmp_counts = ds.n<uint32_t>(list_cap);
+        unsigned long long *cursor = ds.n<unsigned long long>(N_BUCKETS);
+        unsigned long long *bbase = ds.n<unsigned long long>(2 * N_BUCKETS);
+        CK(cudaMemcpyAsync(bbase, hs.up(bb.data(), bb.size()), 2 * N_BUCKETS * 8, cudaMemcpyHostToDevice, st));
+        pa.list = keys;
+        pa.list_cap = ocap;
+        pa.bucket_cursor = cursor;
+        pa.bucket_base = bbase;
+        pa.bucket_end = bbase + N_BUCKETS;
+        pa.bucket_lo = rg.first;
+        pa.bucket_hi = rg.second;
+        auto partition = [&] {
+            CK(cudaMemsetAsync(cursor, 0, N_BUCKETS * 8, st));
+            CK(launch_part_wide(false, k, pa, st));
+        };
+        clk.begin(2);
+        partition();
+        clk.end();
+        unsigned long long *p_fill = hs.n<unsigned long long>(N_BUCKETS);
+        CK(cudaMemcpyAsync(p_fill, cursor, N_BUCKETS * 8, cudaMemcpyDeviceToHost, st));
+        const Counters cp = read_counters(counters, st);
+        check_flags(cp.v[C_FLAGS], "partition");
+        for (uint32_t b = rg.first; b < rg.second; ++b) {
+            if (p_fill[b] > bh[b]) throw CensusOverflow{};
+            cfg[b].key_len = p_fill[b];
+            inserted_total += p_fill[b];
+        }
+        PrefixPass pp;
+        pp.words = nw;
+        pp.lo = rg.first;
+        pp.hi = rg.second;
+        pp.base_bits = 8;
+        pp.cfg = cfg.data();
+        SubCfg lim{};
+        lim.k = k;
+        lim.count_max = P.count_max;
+        lim.min_count = P.min_count;
+        lim.max_count = P.max_count;
+        pp.sc.assign(N_BUCKETS, lim);
+        pp.hist = hist;
+        pp.hist_bins = HIST_BINS;
+        pp.ovf = ovf;
+        pp.ovf_cap = ovf_cap;
+        pp.counters = counters;
+        pp.keys = keys;
+        pp.list = list;
+        pp.tmp_counts = tmp_counts;
+        pp.list_cap = list_cap;
+        pp.fault_inject = P.fault_inject;
+        pp.repartition = partition;
+        count_by_prefix(pp, ds, hs, clk, tn, st);
+        job.distinct += pp.totals[0];
+        job.region_redos += pp.region_redos;
+        ++job.smem_passes;
+        table_cap = std::max(table_cap, pp.table_cap);
+        if (multi) {
+            park(pp.rec_keys, pp.rec_counts, pp.n_rec, mk);
+        } else {
+            n_rec = pp.n_rec;
+            rec_keys = pp.rec_keys;
+            rec_counts = pp.rec_counts;
+        }
+    }
+    if (prefix && !exact) O = job.occurrences = inserted_total;
+    for (const auto &rg : ranges) {
+        if (prefix) break;
         const DevScope::Mark mk = ds.mark();
         uint64_t occ_r = 0;
         for (uint32_t b = rg.first; b < rg.second; ++b) occ_r += bh[b];
@@ -1590,17 +1793,7 @@ void run_wide_job(Job &job, cudaStream_t st, Workspace &ws, const kc_tuning &tn)
         clk.end();
         (void)rec0;
         if (multi) {
-            auto hr = std::make_unique<HostRecords>();
-            hr->allocate(kept, nw);
-            if (kept) {
-                CK(cudaMemcpyAsync(hr->keys(), rk, kept * nw * 8, cudaMemcpyDeviceToHost, st));
-                CK(cudaMemcpyAsync(hr->counts(), rc, kept * 4, cudaMemcpyDeviceToHost, st));
-            }
-            Counters cw = read_counters(counters, st);
-            check_flags(cw.v[C_FLAGS], "compaction");
-            n_rec += kept;
-            spilled.push_back(std::move(hr));
-            ds.rewind(mk);
+            park(rk, rc, kept, mk);
         } else {
             n_rec = kept;
             rec_keys = rk;
@@ -1629,9 +1822,11 @@ void run_wide_job(Job &job, cudaStream_t st, Workspace &ws, const kc_tuning &tn)
 
     // ---- sort in printed-string order -----------------------------------------
     clk.begin(6);
-    unsigned long long *sk = ds.n<unsigned long long>(std::max<uint64_t>(n_rec, 1) * nw);
-    uint32_t *sc = ds.n<uint32_t>(std::max<uint64_t>(n_rec, 1));
-    {
+    unsigned long long *sk = rec_keys;   // prefix path: sorted, the passes' ranges in order
+    uint32_t *sc = rec_counts;
+    if (!prefix) {
+        sk = ds.n<unsigned long long>(std::max<uint64_t>(n_rec, 1) * nw);
+        sc = ds.n<uint32_t>(std::max<uint64_t>(n_rec, 1));
         void *stmp = ds.get(wide_sort_tmp_bytes(n_rec));
         CK(launch_wide_sort(k, rec_keys, rec_counts, n_rec, sk, sc, stmp, counters + C_FLAGS, st));
         ds.release(stmp);
@@ -1647,7 +1842,7 @@ void run_wide_job(Job &job, cudaStream_t st, Workspace &ws, const kc_tuning &tn)
     Counters c2{};
     std::memcpy(c2.v, p_c2, sizeof(c2.v));
     check_flags(c2.v[C_FLAGS], "sort");
-    job.distinct = c2.v[C_DISTINCT];
+    if (!prefix) job.distinct = c2.v[C_DISTINCT];
     std::vector<unsigned long long> hd(p_hd, p_hd + HIST_BINS);
     const uint64_t n_ovf = std::min<uint64_t>(c2.v[C_OVF_LEN], ovf_cap);
     std::vector<uint32_t> ovf_h(n_ovf);
@@ -1789,14 +1984,11 @@ uint64_t reserve_for(const kc_job &p, uint64_t resident_bytes)
 
 void run_job(Job &job, cudaStream_t st, Workspace &ws, const kc_tuning &tn)
 {
-    if (job.p.k > 32) {
-        run_wide_job(job, st, ws, tn);
-        return;
-    }
     bool exact_census = false, global_tables = false;
     for (;;) {
         try {
-            run_job_once(job, st, ws, exact_census, global_tables, tn);
+            if (job.p.k > 32) run_wide_job(job, st, ws, exact_census, global_tables, tn);
+            else run_job_once(job, st, ws, exact_census, global_tables, tn);
             break;
         } catch (const CensusOverflow &) {
             // the sampled census missed a skewed bucket: count every tile instead

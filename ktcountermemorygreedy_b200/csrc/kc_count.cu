@@ -1,10 +1,10 @@
-// kc_count.cu -- counting of k-mers (k <= 32) by printed-order prefix, in
-// shared memory, and the sort of the resulting records.
+// kc_count.cu -- counting of k-mers by printed-order prefix, in shared memory,
+// and the sort of the resulting records.
 //
 // The occurrences arrive partitioned twice, into 256 buckets by their first
 // four bases and into sub-buckets by the next bases (launch_part by string,
 // k_subpart_scatter), as string keys: the k bases first-base-high, left
-// aligned.  So the sub-buckets are consecutive ranges of the printed order:
+// aligned, in one, two or four 64-bit words.  So the sub-buckets are consecutive ranges of the printed order:
 // once every sub-bucket's distinct k-mers are counted and sorted on their own,
 // all records are in order and no sort of the whole set is left.
 //
@@ -20,6 +20,10 @@
 // min count 2) count 27.1 -> 18.5 ms and sort 7.1 -> 1.2 ms; 4M reads with
 // every k-mer kept (480M k-mers, 145M records) insert + compaction 11.8 ms ->
 // scatter + count 6.8 ms, sort 11.9 -> 1.7 ms.
+// k > 32, against an N-word table in HBM probed straight from the extraction and
+// one stable LSD sort per word: 2M reads at k = 63 (176M k-mers) scan, insert,
+// compaction and sort 26.2 ms -> census, partition, count and sort 7.0 ms; 500k
+// reads at k = 127 (29M records) 25.8 -> 5.1 ms.
 #include <algorithm>
 
 #include "kc_device.cuh"
@@ -30,7 +34,6 @@ namespace kc {
 namespace {
 
 constexpr uint32_t FULLW = 0xffffffffu;
-constexpr uint32_t CP_PER_THREAD = 4;       // keys per thread whose first probes are in flight together
 constexpr uint32_t CP_HIST = 512;           // counts below this are histogrammed in shared memory
 constexpr uint32_t CP_QUEUE = 64;           // keys a warp has waiting for their next probe
 constexpr uint32_t CP_MAX_ROUNDS = 64;      // rounds a sub-bucket may be cut into
@@ -42,14 +45,81 @@ __device__ __forceinline__ uint32_t lanes_below()
     return m;
 }
 
-// Placement hash of a key: two 32-bit multiplies over its halves (the top
-// bits are the same for a whole sub-bucket, so the low half leads).  The top
-// bits are its home slot, an odd number from the next ones its probe step.  It
-// never affects a count.
-__device__ __forceinline__ uint32_t mix_of(unsigned long long key)
+template <uint32_t N>
+struct KeyN {
+    unsigned long long w[N];
+    __device__ __forceinline__ bool operator==(const KeyN &o) const
+    {
+        bool e = w[0] == o.w[0];
+#pragma unroll
+        for (uint32_t i = 1; i < N; ++i) e = e && w[i] == o.w[i];
+        return e;
+    }
+};
+
+// Key i of an array of N-word keys: one 8- or 16-byte access per word (pair).
+template <uint32_t N, class INDEX, class LOAD>
+__device__ __forceinline__ KeyN<N> load_key(const unsigned long long *p, INDEX i, LOAD load)
 {
-    return ((uint32_t)key * 0x9E3779B1u + (uint32_t)(key >> 32)) * 0x85EBCA77u;
+    KeyN<N> k;
+    if constexpr (N == 1) {
+        k.w[0] = load(p + i);
+    } else {
+        const ulonglong2 *q = reinterpret_cast<const ulonglong2 *>(p + i * N);
+#pragma unroll
+        for (uint32_t j = 0; j < N / 2; ++j) {
+            const ulonglong2 v = load(q + j);
+            k.w[2 * j] = v.x;
+            k.w[2 * j + 1] = v.y;
+        }
+    }
+    return k;
 }
+
+template <uint32_t N, class INDEX>
+__device__ __forceinline__ void store_key(unsigned long long *p, INDEX i, const KeyN<N> &k)
+{
+    if constexpr (N == 1) {
+        p[i] = k.w[0];
+    } else {
+        ulonglong2 *q = reinterpret_cast<ulonglong2 *>(p + i * N);
+#pragma unroll
+        for (uint32_t j = 0; j < N / 2; ++j) q[j] = make_ulonglong2(k.w[2 * j], k.w[2 * j + 1]);
+    }
+}
+
+struct LoadStream {
+    template <class T>
+    __device__ __forceinline__ T operator()(const T *p) const { return __ldcs(p); }
+};
+struct LoadL2 {
+    template <class T>
+    __device__ __forceinline__ T operator()(const T *p) const { return __ldcg(p); }
+};
+struct LoadPlain {
+    template <class T>
+    __device__ __forceinline__ T operator()(const T *p) const { return *p; }
+};
+
+// Placement hash of a key: two 32-bit multiplies over its halves (the top
+// bits are the same for a whole sub-bucket, so the low half leads), two more
+// per further word.  The top bits are its home slot, an odd number from the
+// next ones its probe step.  It never affects a count.
+template <uint32_t N>
+__device__ __forceinline__ uint32_t mix_of(const KeyN<N> &k)
+{
+    uint32_t h = 0;
+#pragma unroll
+    for (uint32_t i = N - 1; i > 0; --i)
+        h = ((h ^ (uint32_t)k.w[i]) * 0x9E3779B1u + (uint32_t)(k.w[i] >> 32)) * 0xC2B2AE3Du;
+    return ((h ^ (uint32_t)k.w[0]) * 0x9E3779B1u + (uint32_t)(k.w[0] >> 32)) * 0x85EBCA77u;
+}
+
+// Slots of two- and four-word keys: the count word says what state a slot is
+// in.  A slot is claimed by one CAS of that word, its key written and then
+// published; another thread compares keys only in published slots, and meets a
+// claimed one again at its next probe step.
+constexpr uint32_t SLOT_CLAIMED = 1u << 31, SLOT_PUBLISHED = 1u << 30, SLOT_COUNT = SLOT_PUBLISHED - 1;
 
 // Counts one sub-bucket per block at a time.  The keys are inserted into an
 // open-addressing table in shared memory (a slot only changes from empty to a
@@ -70,34 +140,35 @@ __device__ __forceinline__ uint32_t mix_of(unsigned long long key)
 // (quarters, ... at most CP_MAX_ROUNDS), each round reading the keys again
 // from L2; a round's records lie after the earlier rounds' ones, and are a
 // sort unit of their own.  The next sub-bucket's first keys are loaded before
-// the sweep.
-template <uint32_t THREADS, uint32_t BPSM, uint32_t TBITS>
+// the sweep.  Histogram and totals go to the sub-bucket's group.
+template <uint32_t N, uint32_t THREADS, uint32_t BPSM, uint32_t TBITS>
 __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs a)
 {
+    constexpr uint32_t SLOTS = 1u << TBITS, PER_THREAD = N == 1 ? 3 : 4 / N;   // keys whose home slots are read together
+    constexpr uint32_t TILE_KEYS = THREADS * PER_THREAD, WARPS = THREADS / 32;
     extern __shared__ __align__(16) uint8_t cp_smem[];
-    unsigned long long *s_tk = reinterpret_cast<unsigned long long *>(cp_smem);   // 2^TBITS keys
-    uint32_t *s_tc = reinterpret_cast<uint32_t *>(s_tk + (1u << TBITS));          // their counts
-    uint32_t *s_hist = s_tc + (1u << TBITS);                                      // CP_HIST
-    unsigned long long *q_key =                                                   // CP_QUEUE per warp
-        reinterpret_cast<unsigned long long *>(s_hist + CP_HIST) + (threadIdx.x >> 5) * CP_QUEUE;
-    uint16_t *q_slot = reinterpret_cast<uint16_t *>(s_hist + CP_HIST + 2 * CP_QUEUE * (THREADS / 32)) +
+    unsigned long long *s_tk = reinterpret_cast<unsigned long long *>(cp_smem);   // SLOTS keys
+    uint32_t *s_tc = reinterpret_cast<uint32_t *>(s_tk + N * SLOTS);              // their counts (N > 1: and states)
+    uint32_t *s_hist = s_tc + SLOTS;                                              // CP_HIST
+    unsigned long long *q_key =                                                   // CP_QUEUE keys per warp
+        reinterpret_cast<unsigned long long *>(s_hist + CP_HIST) + (threadIdx.x >> 5) * (CP_QUEUE * N);
+    uint16_t *q_slot = reinterpret_cast<uint16_t *>(s_hist + CP_HIST + 2 * N * CP_QUEUE * WARPS) +
                        (threadIdx.x >> 5) * CP_QUEUE;
-    __shared__ uint32_t s_out, s_full, s_next, s_next_n, s_next_plen;
-    __shared__ unsigned long long s_next_off;
-    constexpr uint32_t TILE_KEYS = THREADS * CP_PER_THREAD;
+    __shared__ uint32_t s_out, s_full, s_next, s_next_n;
+    __shared__ unsigned long long s_next_off, s_kept;   // s_kept, s_ovf, s_group: only thread 0 writes them
+    __shared__ uint32_t s_ovf, s_group;
+    __shared__ SubCfg s_cfg[2];   // this sub-bucket's and the next one's
     const int tid = threadIdx.x, lane = tid & 31;
     const uint32_t lt = lanes_below();
     // sub-buckets that outgrew their regions are incomplete: nothing is counted
     if (a.counters[C_REGION_OVF]) return;
-    for (uint32_t i = tid; i < (1u << TBITS); i += THREADS) {
-        s_tk[i] = EMPTY_KEY;
+    for (uint32_t i = tid; i < SLOTS; i += THREADS) {
+        if (N == 1) s_tk[i] = EMPTY_KEY;
         s_tc[i] = 0;
     }
     for (uint32_t i = tid; i < CP_HIST; i += THREADS) s_hist[i] = 0;
-    uint32_t n_distinct = 0, n_once = 0, n_one = 0;   // per lane: below 2^32 whatever the pass
-    unsigned long long n_kept = 0;
-    uint32_t n_ovf_subs = 0, rounds0 = 1;
-    bool unit_full = false;
+    uint32_t n_distinct = 0, n_once = 0, n_one = 0;   // per lane and group: below 2^32 whatever the pass
+    uint32_t rounds0 = 1, par = 1;
     // thread 0 takes the next sub-bucket while this one is counted
     auto take_next = [&]() {
         const uint32_t s = atomicAdd(a.next_sub, 1u);
@@ -105,44 +176,80 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
         if (s < a.n_sub) {
             s_next_n = a.sub_count[s];
             s_next_off = a.sub_off[s];
-            s_next_plen = 8 + (31 - __clz(a.sc[a.sub_bucket[s]].n_sub));
+            s_cfg[par ^ 1] = a.sc[a.sub_bucket[s]];
         }
     };
     if (tid == 0) {
         s_out = 0;
         s_full = 0;
+        s_kept = 0;
+        s_ovf = 0;
         take_next();
+        s_group = s_next < a.n_sub ? s_cfg[0].group : 0u;
     }
     __syncthreads();
-    unsigned long long kn[CP_PER_THREAD];
-    uint32_t sub = s_next, n = 0, plen = 0;
+    // the first tile of keys of a sub-bucket
+    KeyN<N> kn[PER_THREAD];
+    auto load_first = [&](unsigned long long off, uint32_t cnt) {
+#pragma unroll
+        for (uint32_t r = 0; r < PER_THREAD; ++r)
+            if (r * THREADS + tid < cnt) kn[r] = load_key<N>(a.keys, off + r * THREADS + tid, LoadStream());
+    };
+    uint32_t sub = s_next, n = 0;
     unsigned long long base = 0;
+    par = 0;
     if (sub < a.n_sub) {
         n = s_next_n;
         base = s_next_off;
-        plen = s_next_plen;
-#pragma unroll
-        for (uint32_t r = 0; r < CP_PER_THREAD; ++r) {
-            const uint32_t i = r * THREADS + tid;
-            kn[r] = i < n ? __ldcs(&a.keys[base + i]) : EMPTY_KEY;
-        }
+        load_first(base, n);
     }
+    // a group's histogram and totals; the block starts over
+    auto flush = [&]() {
+        __syncthreads();
+        const uint32_t group = s_group;
+        unsigned long long *hist = a.hist + (unsigned long long)group * a.hist_bins;
+        for (uint32_t i = tid; i < CP_HIST; i += THREADS)
+            if (s_hist[i]) {
+                atomicAdd(&hist[i], (unsigned long long)s_hist[i]);
+                s_hist[i] = 0;
+            }
+        unsigned long long s[3] = {n_distinct, n_once, n_one};
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+            for (int o = 16; o > 0; o >>= 1) s[j] += __shfl_down_sync(FULLW, s[j], o);
+        if (lane == 0) {
+            if (s[0]) atomicAdd(&a.totals[3ull * group], s[0]);
+            if (s[1]) atomicAdd(&a.totals[3ull * group + 1], s[1]);
+            if (s[2]) atomicAdd(&hist[1], s[2]);
+        }
+        n_distinct = n_once = n_one = 0;
+        if (tid == 0) {
+            if (s_kept) atomicAdd(&a.totals[3ull * group + 2], s_kept);
+            s_kept = 0;
+        }
+    };
     while (sub < a.n_sub) {
+        const SubCfg &cfg = s_cfg[par];
+        if (cfg.group != s_group) {
+            flush();
+            __syncthreads();
+            if (tid == 0) s_group = cfg.group;
+        }
         __syncthreads();   // s_next* read by all; the table is empty
         if (tid == 0) take_next();
         // slots for twice the keys where that is less than the whole table
         uint32_t lg = n > 1 ? 33 - __clz(n - 1) : 1;
         lg = lg < 9 ? 9 : (lg > TBITS ? TBITS : lg);
-        const uint32_t smask = (1u << lg) - 1;
+        const uint32_t smask = (1u << lg) - 1, hsh = 32 - lg;
         uint32_t rounds = rounds0, rd = 0, off = 0, most = 0;
         bool failed = false;
-        while (rd < rounds) {
+        const bool too_many = N > 1 && n >= SLOT_COUNT;   // a count could run into the state bits
+        while (rd < rounds && !too_many) {
             const uint32_t rmask = rounds - 1;
-            const int rsh = 64 - (int)plen - (31 - __clz(rounds));   // rounds == 1: unused
+            const int rsh = 64 - (int)cfg.plen - (31 - __clz(rounds));   // rounds == 1: unused
             const bool reread = rd > 0 || failed;
-            // a warp takes at most this many probe steps (a table less than
-            // about five sixths full needs far fewer)
-            const uint32_t hsh = 32 - lg;
+            // a warp takes at most this many probe steps (a table that is not
+            // nearly full needs far fewer)
             uint32_t qn = 0, steps = 0, most_steps = 3 * (n / THREADS + 1) + 64;
             // one more probe of the last `m` queued keys (m <= 32); those that
             // meet another key stay queued at their next slot
@@ -150,67 +257,100 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
                 __syncwarp();
                 qn -= m;
                 ++steps;
-                const bool in = lane < (int)m;
-                unsigned long long key = 0;
+                KeyN<N> key;
                 uint32_t slot = 0;
                 bool wait = false;
-                if (in) {
-                    key = q_key[qn + lane];
+                if (lane < (int)m) {
+                    key = load_key<N>(q_key, qn + lane, LoadPlain());
                     slot = q_slot[qn + lane];
-                    unsigned long long cur = *(volatile unsigned long long *)&s_tk[slot];
-                    if (cur == EMPTY_KEY) {
-                        cur = atomicCAS(&s_tk[slot], EMPTY_KEY, key);
-                        if (cur == EMPTY_KEY) cur = key;   // claimed
+                    if constexpr (N == 1) {
+                        unsigned long long cur = *(volatile unsigned long long *)&s_tk[slot];
+                        if (cur == EMPTY_KEY) {
+                            cur = atomicCAS(&s_tk[slot], EMPTY_KEY, key.w[0]);
+                            if (cur == EMPTY_KEY) cur = key.w[0];   // claimed
+                        }
+                        wait = cur != key.w[0];
+                        if (!wait) atomicAdd(&s_tc[slot], 1u);
+                    } else {
+                        uint32_t st = *(volatile uint32_t *)&s_tc[slot];
+                        wait = true;
+                        if (st == 0) {
+                            st = atomicCAS(&s_tc[slot], 0u, SLOT_CLAIMED | 1u);
+                            if (st == 0) {
+                                volatile unsigned long long *d = s_tk + N * slot;
+#pragma unroll
+                                for (uint32_t j = 0; j < N; ++j) d[j] = key.w[j];
+                                __threadfence_block();   // the key before the state
+                                atomicOr(&s_tc[slot], SLOT_PUBLISHED);
+                                wait = false;
+                            }
+                        }
+                        if (st & SLOT_PUBLISHED) {
+                            __threadfence_block();
+                            if (load_key<N>(s_tk, slot, LoadPlain()) == key) {
+                                atomicAdd(&s_tc[slot], 1u);
+                                wait = false;
+                            } else {
+                                slot = (slot + (mix_of<N>(key) >> 3 | 1u)) & smask;
+                            }
+                        }
                     }
-                    wait = cur != key;
-                    if (!wait) atomicAdd(&s_tc[slot], 1u);
                 }
                 const uint32_t w = __ballot_sync(FULLW, wait);
                 if (wait) {
                     const uint32_t at = qn + (uint32_t)__popc(w & lt);
-                    q_key[at] = key;
-                    q_slot[at] = (uint16_t)((slot + (mix_of(key) >> 3 | 1u)) & smask);
+                    store_key<N>(q_key, at, key);
+                    q_slot[at] = (uint16_t)(N == 1 ? (slot + (mix_of<N>(key) >> 3 | 1u)) & smask : slot);
                 }
                 qn += (uint32_t)__popc(w);
                 __syncwarp();
             };
             for (uint32_t t0 = 0; t0 < n; t0 += TILE_KEYS) {
-                unsigned long long k[CP_PER_THREAD];
+                KeyN<N> k[PER_THREAD];
+                bool in[PER_THREAD];
+#pragma unroll
+                for (uint32_t r = 0; r < PER_THREAD; ++r) in[r] = t0 + r * THREADS + tid < n;
                 if (reread) {
 #pragma unroll
-                    for (uint32_t r = 0; r < CP_PER_THREAD; ++r) {
-                        const uint32_t i = t0 + r * THREADS + tid;
-                        k[r] = i < n ? __ldcg(&a.keys[base + i]) : EMPTY_KEY;
-                    }
+                    for (uint32_t r = 0; r < PER_THREAD; ++r)
+                        if (in[r]) k[r] = load_key<N>(a.keys, base + t0 + r * THREADS + tid, LoadL2());
                 } else {
 #pragma unroll
-                    for (uint32_t r = 0; r < CP_PER_THREAD; ++r) {
+                    for (uint32_t r = 0; r < PER_THREAD; ++r) {
                         k[r] = kn[r];
                         const uint32_t i = t0 + TILE_KEYS + r * THREADS + tid;
-                        kn[r] = i < n ? __ldcs(&a.keys[base + i]) : EMPTY_KEY;
+                        if (i < n) kn[r] = load_key<N>(a.keys, base + i, LoadStream());
                     }
                 }
                 if (rounds > 1) {
 #pragma unroll
-                    for (uint32_t r = 0; r < CP_PER_THREAD; ++r)
-                        if (((uint32_t)(k[r] >> rsh) & rmask) != rd) k[r] = EMPTY_KEY;
+                    for (uint32_t r = 0; r < PER_THREAD; ++r)
+                        in[r] = in[r] && ((uint32_t)(k[r].w[0] >> rsh) & rmask) == rd;
                 }
                 // the home slots: most keys are there already and only counted
-                uint32_t slot[CP_PER_THREAD];
-                unsigned long long cur[CP_PER_THREAD];
+                uint32_t slot[PER_THREAD];
+                bool hit[PER_THREAD];
 #pragma unroll
-                for (uint32_t r = 0; r < CP_PER_THREAD; ++r) {
-                    slot[r] = mix_of(k[r]) >> hsh;
-                    cur[r] = *(volatile unsigned long long *)&s_tk[slot[r]];
+                for (uint32_t r = 0; r < PER_THREAD; ++r) {
+                    slot[r] = mix_of<N>(k[r]) >> hsh;
+                    if constexpr (N == 1) {
+                        hit[r] = *(volatile unsigned long long *)&s_tk[slot[r]] == k[r].w[0];
+                    } else {
+                        hit[r] = false;
+                        if (in[r] && (*(volatile uint32_t *)&s_tc[slot[r]] & SLOT_PUBLISHED)) {
+                            __threadfence_block();
+                            hit[r] = load_key<N>(s_tk, slot[r], LoadPlain()) == k[r];
+                        }
+                    }
                 }
 #pragma unroll
-                for (uint32_t r = 0; r < CP_PER_THREAD; ++r) {
-                    const bool in = k[r] != EMPTY_KEY, hit = in && cur[r] == k[r];
-                    if (hit) atomicAdd(&s_tc[slot[r]], 1u);
-                    const uint32_t w = __ballot_sync(FULLW, in && !hit);
-                    if (in && !hit) {
+                for (uint32_t r = 0; r < PER_THREAD; ++r) {
+                    if (in[r] && hit[r]) atomicAdd(&s_tc[slot[r]], 1u);
+                    const bool wait = in[r] && !hit[r];
+                    const uint32_t w = __ballot_sync(FULLW, wait);
+                    if (wait) {
                         const uint32_t at = qn + (uint32_t)__popc(w & lt);
-                        q_key[at] = k[r];
+                        store_key<N>(q_key, at, k[r]);
                         q_slot[at] = (uint16_t)slot[r];
                     }
                     qn += (uint32_t)__popc(w);
@@ -233,7 +373,7 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
                 // emptied and counted again over half the range
                 __syncthreads();
                 for (uint32_t i = tid; i <= smask; i += THREADS) {
-                    s_tk[i] = EMPTY_KEY;
+                    if (N == 1) s_tk[i] = EMPTY_KEY;
                     s_tc[i] = 0;
                 }
                 if (tid == 0) s_full = 0;
@@ -241,47 +381,55 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
                 failed = true;
                 rounds *= 2;
                 rd *= 2;
-                if (rounds > CP_MAX_ROUNDS || (int)plen + (31 - __clz(rounds)) > 64) break;
+                if (rounds > CP_MAX_ROUNDS || (int)cfg.plen + (31 - __clz(rounds)) > 64) break;
                 continue;
             }
-            if (rd + 1 == rounds) {
-                // the next sub-bucket's first keys arrive during the sweep
-                const uint32_t nn = s_next < a.n_sub ? s_next_n : 0u;
-#pragma unroll
-                for (uint32_t r = 0; r < CP_PER_THREAD; ++r) {
-                    const uint32_t i = r * THREADS + tid;
-                    kn[r] = i < nn ? __ldcs(&a.keys[s_next_off + i]) : EMPTY_KEY;
-                }
-            }
-            // the sweep: records out, histogram, table emptied
+            // the next sub-bucket's first keys arrive during the sweep
+            if (rd + 1 == rounds) load_first(s_next_off, s_next < a.n_sub ? s_next_n : 0u);
+            // the sweep: records out, histogram, table emptied; two slots a thread
             const unsigned long long out = base + off;
+            const uint32_t cmax = cfg.count_max, keep_lo = cfg.min_count, keep_hi = cfg.max_count;
             for (uint32_t i0 = 0; i0 <= smask; i0 += 2 * THREADS) {
-                const uint32_t i = i0 + 2 * tid;   // two slots a thread
-                ulonglong2 kk = make_ulonglong2(EMPTY_KEY, EMPTY_KEY);
-                uint32_t c[2] = {0, 0};
+                const uint32_t i = i0 + 2 * tid;
+                uint32_t raw[2] = {0, 0}, c[2] = {0, 0};
                 bool keep[2] = {false, false};
-                if (i <= smask) kk = *reinterpret_cast<const ulonglong2 *>(&s_tk[i]);
-                const unsigned long long key[2] = {kk.x, kk.y};
-                if (kk.x != EMPTY_KEY || kk.y != EMPTY_KEY) {
-                    const uint2 raw2 = *reinterpret_cast<const uint2 *>(&s_tc[i]);
-                    *reinterpret_cast<ulonglong2 *>(&s_tk[i]) = make_ulonglong2(EMPTY_KEY, EMPTY_KEY);
+                KeyN<N> key[2];
+                bool used = false;
+                if constexpr (N == 1) {
+                    key[0].w[0] = key[1].w[0] = EMPTY_KEY;
+                    if (i <= smask) {
+                        const ulonglong2 kk = *reinterpret_cast<const ulonglong2 *>(&s_tk[i]);
+                        key[0].w[0] = kk.x;
+                        key[1].w[0] = kk.y;
+                    }
+                    used = key[0].w[0] != EMPTY_KEY || key[1].w[0] != EMPTY_KEY;
+                }
+                if (N == 1 ? used : i <= smask) {
+                    const uint2 r2 = *reinterpret_cast<const uint2 *>(&s_tc[i]);
+                    raw[0] = r2.x;
+                    raw[1] = r2.y;
+                }
+                if (raw[0] | raw[1]) {
                     *reinterpret_cast<uint2 *>(&s_tc[i]) = make_uint2(0u, 0u);
-                    const uint32_t raw[2] = {raw2.x, raw2.y};
+                    if constexpr (N == 1)
+                        *reinterpret_cast<ulonglong2 *>(&s_tk[i]) = make_ulonglong2(EMPTY_KEY, EMPTY_KEY);
 #pragma unroll
                     for (int j = 0; j < 2; ++j) {
-                        if (key[j] == EMPTY_KEY) continue;
+                        if (N > 1) raw[j] &= SLOT_COUNT;
+                        if (raw[j] == 0) continue;
                         ++n_distinct;
                         n_once += raw[j] == 1;
-                        c[j] = raw[j] < a.count_max ? raw[j] : a.count_max;
+                        c[j] = raw[j] < cmax ? raw[j] : cmax;
                         if (c[j] == 1) ++n_one;   // most k-mers of many inputs: one shared bin would serialize
                         else if (c[j] < CP_HIST) atomicAdd(&s_hist[c[j]], 1u);
-                        else if (c[j] < HIST_BINS) atomicAdd(&a.hist[c[j]], 1ull);
+                        else if (c[j] < a.hist_bins) atomicAdd(&a.hist[(unsigned long long)s_group * a.hist_bins + c[j]], 1ull);
                         else {
                             const unsigned long long q = atomicAdd(&a.counters[C_OVF_LEN], 1ull);
-                            if (q < a.ovf_cap) a.ovf[q] = c[j];
-                            else atomicOr(&a.counters[C_FLAGS], ERR_HIST_OVERFLOW_FULL);
+                            if (q >= a.ovf_cap) atomicOr(&a.counters[C_FLAGS], ERR_HIST_OVERFLOW_FULL);
+                            else if (a.ovf64) a.ovf64[q] = ((unsigned long long)s_group << 32) | c[j];
+                            else a.ovf[q] = c[j];
                         }
-                        keep[j] = c[j] >= a.min_count && c[j] <= a.max_count;
+                        keep[j] = c[j] >= keep_lo && c[j] <= keep_hi;
                     }
                 }
                 const uint32_t b0 = __ballot_sync(FULLW, keep[0]), b1 = __ballot_sync(FULLW, keep[1]);
@@ -289,16 +437,14 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
                     uint32_t w = 0;
                     if (lane == 0) w = atomicAdd(&s_out, (uint32_t)(__popc(b0) + __popc(b1)));
                     w = __shfl_sync(FULLW, w, 0);
-                    if (keep[0]) {
-                        const unsigned long long q = out + w + (uint32_t)__popc(b0 & lt);
-                        a.rec_keys[q] = key[0];
-                        a.rec_counts[q] = c[0];
-                    }
-                    if (keep[1]) {
-                        const unsigned long long q = out + w + (uint32_t)(__popc(b0) + __popc(b1 & lt));
-                        a.rec_keys[q] = key[1];
-                        a.rec_counts[q] = c[1];
-                    }
+                    const uint32_t at[2] = {w + (uint32_t)__popc(b0 & lt), w + (uint32_t)(__popc(b0) + __popc(b1 & lt))};
+#pragma unroll
+                    for (int j = 0; j < 2; ++j)
+                        if (keep[j]) {
+                            if (N > 1) key[j] = load_key<N>(s_tk, i + j, LoadPlain());
+                            store_key<N>(a.rec_keys, out + at[j], key[j]);
+                            a.rec_counts[out + at[j]] = c[j];
+                        }
                 }
             }
             __syncthreads();
@@ -307,11 +453,12 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
             if (tid == 0) {
                 s_out = 0;
                 if (len) {
-                    const uint32_t cls = len <= UNIT_CAP0 ? 0 : (len <= 2 * UNIT_CAP0 ? 1 : (len <= 4 * UNIT_CAP0 ? 2 : 3));
+                    constexpr uint32_t CAP0 = unit_cap0(N);
+                    const uint32_t cls = len <= CAP0 ? 0 : (len <= 2 * CAP0 ? 1 : (len <= 4 * CAP0 ? 2 : 3));
                     const unsigned long long u = atomicAdd(&a.counters[C_UNITS + cls], 1ull);
-                    if (u < a.unit_cap) a.units[cls * (uint64_t)a.unit_cap + u] = SubUnit{sub, off, len, 0u};
-                    else unit_full = true;
-                    n_kept += len;
+                    if (u < a.unit_cap) a.units[cls * (uint64_t)a.unit_cap + u] = SubUnit{sub, off, len, cfg.k};
+                    else ++s_ovf;   // more sort units than the lists hold: counted as an overflow
+                    s_kept += len;
                 }
             }
             off += len;
@@ -322,96 +469,90 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
         if (tid == 0) {
             a.sub_len[sub] = off;
             if (gave_up) {
-                ++n_ovf_subs;
+                ++s_ovf;
                 atomicOr(&a.bucket_ovf[a.sub_bucket[sub]], 1u);
             }
         }
         // sub-buckets are alike: the next one starts with as many rounds,
         // or with half as many when no round came near the table's size
-        rounds0 = gave_up ? 1u : (rounds > 1 && most < (1u << TBITS) / 4 ? rounds / 2 : rounds);
-        if (gave_up) {
-            const uint32_t nn = s_next < a.n_sub ? s_next_n : 0u;
-#pragma unroll
-            for (uint32_t r = 0; r < CP_PER_THREAD; ++r) {
-                const uint32_t i = r * THREADS + tid;
-                kn[r] = i < nn ? __ldcs(&a.keys[s_next_off + i]) : EMPTY_KEY;
-            }
-        }
+        rounds0 = gave_up ? 1u : (rounds > 1 && most < SLOTS / 4 ? rounds / 2 : rounds);
+        if (too_many) __syncthreads();   // thread 0 has taken the next sub-bucket
+        if (gave_up) load_first(s_next_off, s_next < a.n_sub ? s_next_n : 0u);
         sub = s_next;
         n = s_next_n;
         base = s_next_off;
-        plen = s_next_plen;
+        par ^= 1;
     }
-    __syncthreads();
-    for (uint32_t i = tid; i < CP_HIST; i += THREADS)
-        if (s_hist[i]) atomicAdd(&a.hist[i], (unsigned long long)s_hist[i]);
-    if (tid == 0 && unit_full) n_ovf_subs += 1;   // more sort units than the lists hold: counted as an overflow
-    unsigned long long s[4] = {n_distinct, n_once, n_one, n_kept};
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-        for (int o = 16; o > 0; o >>= 1) s[j] += __shfl_down_sync(FULLW, s[j], o);
-    if (lane == 0) {
-        if (s[0]) atomicAdd(&a.counters[C_DISTINCT], s[0]);
-        if (s[1]) atomicAdd(&a.counters[C_LOW_ONLY], s[1]);
-        if (s[2]) atomicAdd(&a.hist[1], s[2]);
-        if (s[3]) atomicAdd(&a.counters[C_REC_LEN], s[3]);
-    }
-    if (tid == 0 && n_ovf_subs) atomicAdd(&a.counters[C_SUB_OVF], (unsigned long long)n_ovf_subs);
+    flush();
+    if (tid == 0 && s_ovf) atomicAdd(&a.counters[C_SUB_OVF], (unsigned long long)s_ovf);
 }
 
 // Sorts the records of one unit (a sub-bucket, or one round of it: at most
 // CAP records of one range of the printed order) per block at a time and
 // writes them, as k-mer words, to their final place.  The keys come into
 // shared memory once; their indexes are placed by the 2^LGB values of the bits
-// below the unit's common prefix (the xor of all its keys says where that
-// ends), then each record finds its rank inside its run of a few records by
-// comparing itself with the run's other keys: no lane waits for another,
-// unlike an insertion sort per run.  The counts are read where they are
-// written (a unit's counts stay in L1).
-template <uint32_t THREADS, uint32_t CAP, uint32_t LGB>
+// below the unit's common prefix (the xor of all its keys says in which word
+// and where that ends), then each record finds its rank inside its run of a few
+// records by comparing itself with the run's other keys: no lane waits for
+// another, unlike an insertion sort per run.  The counts are read where they
+// are written (a unit's counts stay in L1).
+template <uint32_t N, uint32_t THREADS, uint32_t CAP, uint32_t LGB>
 __global__ void __launch_bounds__(THREADS) k_unit_sort(const unsigned long long *tk, const uint32_t *tv,
                                                        const unsigned long long *sub_off,
                                                        const unsigned long long *sub_final, const SubUnit *units,
                                                        uint32_t n_units, unsigned long long *out_k, uint32_t *out_v,
-                                                       uint64_t out_cap, uint32_t kshift)
+                                                       uint64_t out_cap)
 {
     constexpr uint32_t NB = 1u << LGB, PER = NB / THREADS, WARPS = THREADS / 32;
     static_assert(NB % THREADS == 0 && CAP <= 65536, "layout");
     extern __shared__ __align__(16) uint8_t us_smem[];
-    unsigned long long *s_keys = reinterpret_cast<unsigned long long *>(us_smem);   // CAP
-    uint32_t *s_start = reinterpret_cast<uint32_t *>(s_keys + CAP);                 // NB + 1 (+ 3: alignment)
-    uint16_t *s_idx = reinterpret_cast<uint16_t *>(s_start + NB + 4);               // CAP
-    __shared__ uint32_t s_warp[WARPS], s_xlo, s_xhi;
+    unsigned long long *s_keys = reinterpret_cast<unsigned long long *>(us_smem);   // CAP keys
+    uint32_t *s_start = reinterpret_cast<uint32_t *>(s_keys + N * CAP);             // NB
+    uint16_t *s_idx = reinterpret_cast<uint16_t *>(s_start + NB);                   // CAP
+    __shared__ uint32_t s_warp[WARPS], s_xor[2 * N];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (uint32_t ui = blockIdx.x; ui < n_units; ui += gridDim.x) {
         const SubUnit u = units[ui];
         const uint32_t m = u.len < CAP ? u.len : CAP;
         const unsigned long long src = sub_off[u.sub] + u.off, dst = sub_final[u.sub] + u.off;
-        if (tid == 0) {
-            s_xlo = s_xhi = 0;
-            s_start[NB] = m;
-        }
+        if (tid < 2 * (int)N) s_xor[tid] = 0;
 #pragma unroll
         for (uint32_t j = 0; j < PER; ++j) s_start[j * THREADS + tid] = 0;
         __syncthreads();
         // common prefix: the bits in which no key differs from the first
-        const unsigned long long k0 = __ldg(&tk[src]);
-        unsigned long long x = 0;
+        const KeyN<N> k0 = load_key<N>(tk, src, LoadPlain());
+        unsigned long long x[N];
+#pragma unroll
+        for (uint32_t j = 0; j < N; ++j) x[j] = 0;
 #pragma unroll 4
         for (uint32_t i = tid; i < m; i += THREADS) {
-            const unsigned long long key = __ldcs(&tk[src + i]);
-            s_keys[i] = key;
-            x |= key ^ k0;
+            const KeyN<N> key = load_key<N>(tk, src + i, LoadStream());
+            store_key<N>(s_keys, i, key);
+#pragma unroll
+            for (uint32_t j = 0; j < N; ++j) x[j] |= key.w[j] ^ k0.w[j];
         }
-        const uint32_t xh = __reduce_or_sync(FULLW, (uint32_t)(x >> 32)), xl = __reduce_or_sync(FULLW, (uint32_t)x);
-        if (lane == 0) {
-            if (xh) atomicOr(&s_xhi, xh);
-            if (xl) atomicOr(&s_xlo, xl);
+#pragma unroll
+        for (uint32_t j = 0; j < N; ++j) {
+            const uint32_t xh = __reduce_or_sync(FULLW, (uint32_t)(x[j] >> 32)), xl = __reduce_or_sync(FULLW, (uint32_t)x[j]);
+            if (lane == 0) {
+                if (xh) atomicOr(&s_xor[2 * j], xh);
+                if (xl) atomicOr(&s_xor[2 * j + 1], xl);
+            }
         }
         __syncthreads();
-        const int pre = __clzll(((unsigned long long)s_xhi << 32) | s_xlo);   // 64: one record
+        // the first word in which keys differ, and the digit below its common bits
+        uint32_t dw = 0;
+        unsigned long long diff = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < N; ++j)
+            if (!diff) {
+                diff = ((unsigned long long)s_xor[2 * j] << 32) | s_xor[2 * j + 1];
+                dw = j;
+            }
+        const int pre = __clzll(diff);   // 64: one record
         const int dsh = 64 - pre - (int)LGB > 0 ? 64 - pre - (int)LGB : 0;
-        for (uint32_t i = tid; i < m; i += THREADS) atomicAdd(&s_start[(uint32_t)(s_keys[i] >> dsh) & (NB - 1)], 1u);
+        auto digit = [&](uint32_t i) { return (uint32_t)(s_keys[N * i + dw] >> dsh) & (NB - 1); };
+        for (uint32_t i = tid; i < m; i += THREADS) atomicAdd(&s_start[digit(i)], 1u);
         __syncthreads();
         // exclusive scan of the NB counts, PER consecutive ones per thread
         uint32_t c[PER], own = 0;
@@ -439,18 +580,51 @@ __global__ void __launch_bounds__(THREADS) k_unit_sort(const unsigned long long 
         }
         __syncthreads();
         // placing moves each start to its run's end: run d is [end of run d - 1, end of run d)
-        for (uint32_t i = tid; i < m; i += THREADS)
-            s_idx[atomicAdd(&s_start[(uint32_t)(s_keys[i] >> dsh) & (NB - 1)], 1u)] = (uint16_t)i;
+        for (uint32_t i = tid; i < m; i += THREADS) s_idx[atomicAdd(&s_start[digit(i)], 1u)] = (uint16_t)i;
         __syncthreads();
         for (uint32_t p = tid; p < m; p += THREADS) {
-            const uint32_t i = s_idx[p];
-            const unsigned long long key = s_keys[i];
-            const uint32_t d = (uint32_t)(key >> dsh) & (NB - 1);
+            const uint32_t i = s_idx[p], d = digit(i);
             const uint32_t lo = d ? s_start[d - 1] : 0u, hi = s_start[d];
             uint32_t rank = lo;
-            for (uint32_t j = lo; j < hi; ++j) rank += s_keys[s_idx[j]] < key ? 1u : 0u;
+            if constexpr (N == 1) {
+                const unsigned long long key = s_keys[i];
+                for (uint32_t j = lo; j < hi; ++j) rank += s_keys[s_idx[j]] < key ? 1u : 0u;
+            } else {
+                // the words before dw are the same in all keys
+                const unsigned long long kd = s_keys[N * i + dw];
+                for (uint32_t j = lo; j < hi; ++j) {
+                    const unsigned long long *o = s_keys + N * s_idx[j];
+                    bool less = o[dw] < kd;
+                    if (o[dw] == kd) {
+                        for (uint32_t w = dw + 1; w < N; ++w) {
+                            const unsigned long long ow = o[w], mw = s_keys[N * i + w];
+                            if (ow != mw) {
+                                less = ow < mw;
+                                break;
+                            }
+                        }
+                    }
+                    rank += less ? 1u : 0u;
+                }
+            }
             if (dst + rank < out_cap) {
-                out_k[dst + rank] = pair_reverse(key) << kshift;
+                // string order back to k-mer words: word w holds the 32 bases
+                // ending 32w before the last, newest at the top
+                KeyN<N> key;
+#pragma unroll
+                for (uint32_t w = 0; w < N; ++w) {
+                    const int b = (int)u.k - 32 * (int)(w + 1);   // first base of the word
+                    unsigned long long v = 0;
+                    if (b >= 0) {
+                        const uint32_t o = 2 * (b & 31);
+                        v = s_keys[N * i + (b >> 5)] << o;
+                        if (o) v |= s_keys[N * i + (b >> 5) + 1] >> (64 - o);
+                    } else if (b > -32) {
+                        v = s_keys[N * i] >> (-2 * b);
+                    }
+                    key.w[w] = pair_reverse(v);
+                }
+                store_key<N>(out_k, dst + rank, key);
                 out_v[dst + rank] = __ldg(&tv[src + i]);
             }
         }
@@ -466,11 +640,11 @@ int n_sms()
     return n > 0 ? n : 148;
 }
 
-template <uint32_t THREADS, uint32_t BPSM, uint32_t TBITS>
+template <uint32_t N, uint32_t THREADS, uint32_t BPSM, uint32_t TBITS>
 cudaError_t launch_count_prefix_t(const PrefixCountArgs &a, cudaStream_t st)
 {
-    const size_t smem = ((size_t)1 << TBITS) * 12 + CP_HIST * 4 + (THREADS / 32) * CP_QUEUE * 10;
-    auto kern = k_count_prefix<THREADS, BPSM, TBITS>;
+    const size_t smem = ((size_t)1 << TBITS) * (8 * N + 4) + CP_HIST * 4 + (THREADS / 32) * CP_QUEUE * (8 * N + 2);
+    auto kern = k_count_prefix<N, THREADS, BPSM, TBITS>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     note_kernel_launch();
@@ -478,14 +652,14 @@ cudaError_t launch_count_prefix_t(const PrefixCountArgs &a, cudaStream_t st)
     return cudaGetLastError();
 }
 
-template <uint32_t THREADS, uint32_t CAP, uint32_t LGB>
+template <uint32_t N, uint32_t THREADS, uint32_t CAP, uint32_t LGB>
 cudaError_t launch_unit_sort_t(const unsigned long long *tk, const uint32_t *tv, const unsigned long long *sub_off,
                                const unsigned long long *sub_final, const SubUnit *units, uint32_t n_units,
-                               unsigned long long *out_k, uint32_t *out_v, uint64_t out_cap, uint32_t k, cudaStream_t st)
+                               unsigned long long *out_k, uint32_t *out_v, uint64_t out_cap, cudaStream_t st)
 {
     if (!n_units) return cudaSuccess;
-    const size_t smem = (size_t)CAP * 10 + ((size_t)(1u << LGB) + 4) * 4;
-    auto kern = k_unit_sort<THREADS, CAP, LGB>;
+    const size_t smem = (size_t)CAP * (8 * N + 2) + (size_t)(1u << LGB) * 4;
+    auto kern = k_unit_sort<N, THREADS, CAP, LGB>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
@@ -493,38 +667,55 @@ cudaError_t launch_unit_sort_t(const unsigned long long *tk, const uint32_t *tv,
         per_sm = 1;
     note_kernel_launch();
     kern<<<std::min<uint32_t>(n_units, (uint32_t)(n_sms() * per_sm)), THREADS, smem, st>>>(
-        tk, tv, sub_off, sub_final, units, n_units, out_k, out_v, out_cap, 64 - 2 * k);
+        tk, tv, sub_off, sub_final, units, n_units, out_k, out_v, out_cap);
     return cudaGetLastError();
+}
+
+template <uint32_t N>
+cudaError_t launch_unit_sort_n(const unsigned long long *tk, const uint32_t *tv, const unsigned long long *sub_off,
+                               const unsigned long long *sub_final, const SubUnit *units, uint32_t unit_cap,
+                               const uint32_t *n_units, unsigned long long *out_k, uint32_t *out_v, uint64_t out_cap,
+                               cudaStream_t st)
+{
+    constexpr uint32_t C = unit_cap0(N);
+    static_assert(UNIT_CLASSES == 4, "one launch per class");
+    cudaError_t e = launch_unit_sort_t<N, 256, C, 9>(tk, tv, sub_off, sub_final, units, n_units[0], out_k, out_v, out_cap,
+                                                     st);
+    if (e == cudaSuccess)
+        e = launch_unit_sort_t<N, 256, 2 * C, 10>(tk, tv, sub_off, sub_final, units + unit_cap, n_units[1], out_k, out_v,
+                                                  out_cap, st);
+    if (e == cudaSuccess)
+        e = launch_unit_sort_t<N, 512, 4 * C, 11>(tk, tv, sub_off, sub_final, units + 2ull * unit_cap, n_units[2], out_k,
+                                                  out_v, out_cap, st);
+    if (e == cudaSuccess)
+        e = launch_unit_sort_t<N, 512, 8 * C, 11>(tk, tv, sub_off, sub_final, units + 3ull * unit_cap, n_units[3], out_k,
+                                                  out_v, out_cap, st);
+    return e;
 }
 
 }  // namespace
 
-cudaError_t launch_count_prefix(const PrefixCountArgs &a, uint32_t shape, cudaStream_t st)
+cudaError_t launch_count_prefix(const PrefixCountArgs &a, uint32_t words, uint32_t shape, cudaStream_t st)
 {
     if (!a.n_sub) return cudaSuccess;
     cudaError_t e = cudaMemsetAsync(a.next_sub, 0, 4, st);
     if (e != cudaSuccess) return e;
-    return (shape == 2 || shape == 4) ? launch_count_prefix_t<256, 4, 12>(a, st) : launch_count_prefix_t<512, 2, 13>(a, st);
+    const bool small = shape == 2 || shape == 4;
+    if (words == 1) return small ? launch_count_prefix_t<1, 256, 4, 12>(a, st) : launch_count_prefix_t<1, 512, 2, 13>(a, st);
+    if (words == 2) return small ? launch_count_prefix_t<2, 256, 4, 11>(a, st) : launch_count_prefix_t<2, 512, 2, 12>(a, st);
+    return small ? launch_count_prefix_t<4, 256, 4, 10>(a, st) : launch_count_prefix_t<4, 512, 2, 11>(a, st);
 }
 
-cudaError_t launch_unit_sort(const unsigned long long *tk, const uint32_t *tv, const unsigned long long *sub_off,
-                             const unsigned long long *sub_final, const SubUnit *units, uint32_t unit_cap,
-                             const uint32_t *n_units, unsigned long long *out_k, uint32_t *out_v, uint64_t out_cap,
-                             uint32_t k, cudaStream_t st)
+cudaError_t launch_unit_sort(uint32_t words, const unsigned long long *tk, const uint32_t *tv,
+                             const unsigned long long *sub_off, const unsigned long long *sub_final,
+                             const SubUnit *units, uint32_t unit_cap, const uint32_t *n_units,
+                             unsigned long long *out_k, uint32_t *out_v, uint64_t out_cap, cudaStream_t st)
 {
-    static_assert(UNIT_CAP0 == 1024 && UNIT_CLASSES == 4, "one launch per class");
-    cudaError_t e = launch_unit_sort_t<256, 1024, 9>(tk, tv, sub_off, sub_final, units, n_units[0], out_k, out_v, out_cap,
-                                                     k, st);
-    if (e == cudaSuccess)
-        e = launch_unit_sort_t<256, 2048, 10>(tk, tv, sub_off, sub_final, units + unit_cap, n_units[1], out_k, out_v,
-                                              out_cap, k, st);
-    if (e == cudaSuccess)
-        e = launch_unit_sort_t<512, 4096, 11>(tk, tv, sub_off, sub_final, units + 2ull * unit_cap, n_units[2], out_k,
-                                              out_v, out_cap, k, st);
-    if (e == cudaSuccess)
-        e = launch_unit_sort_t<512, 8192, 11>(tk, tv, sub_off, sub_final, units + 3ull * unit_cap, n_units[3], out_k,
-                                              out_v, out_cap, k, st);
-    return e;
+    if (words == 1)
+        return launch_unit_sort_n<1>(tk, tv, sub_off, sub_final, units, unit_cap, n_units, out_k, out_v, out_cap, st);
+    if (words == 2)
+        return launch_unit_sort_n<2>(tk, tv, sub_off, sub_final, units, unit_cap, n_units, out_k, out_v, out_cap, st);
+    return launch_unit_sort_n<4>(tk, tv, sub_off, sub_final, units, unit_cap, n_units, out_k, out_v, out_cap, st);
 }
 
 }  // namespace kc

@@ -1805,7 +1805,7 @@ __device__ __forceinline__ uint32_t sub_of(unsigned long long key, const SubCfg 
 constexpr uint32_t SPC_PER_THREAD = SUB_COUNT_KEYS / 256;
 __global__ void __launch_bounds__(256) k_subpart_count(const unsigned long long *keys, const BucketRanges *rg,
                                                        uint32_t n_items, const SubCfg *sc, uint32_t *sub_count,
-                                                       uint32_t stride)
+                                                       uint32_t stride, uint32_t words)
 {
     __shared__ uint32_t s_item0[N_BUCKETS + 1];
     __shared__ uint32_t s_h[SUB_MAX_PER_BUCKET];
@@ -1832,15 +1832,17 @@ __global__ void __launch_bounds__(256) k_subpart_count(const unsigned long long 
             c = sc[cur];
         }
         unsigned long long kk[SPC_PER_THREAD];
+        bool in[SPC_PER_THREAD];
 #pragma unroll
         for (uint32_t r = 0; r < SPC_PER_THREAD; ++r) {
             const uint32_t j = r * 256 + tid;
             const unsigned long long i = w.begin + 16ull * stride * (j >> 4) + (j & 15);
-            kk[r] = i < w.end ? __ldcs(&keys[i]) : EMPTY_KEY;
+            in[r] = i < w.end;
+            kk[r] = in[r] ? __ldcs(&keys[i * words]) : 0ull;
         }
 #pragma unroll
         for (uint32_t r = 0; r < SPC_PER_THREAD; ++r)
-            if (kk[r] != EMPTY_KEY) atomicAdd(&s_h[sub_of(kk[r], c)], 1u);
+            if (in[r]) atomicAdd(&s_h[sub_of(kk[r], c)], 1u);
     }
     __syncthreads();
     if (cur != N_BUCKETS)
@@ -1920,6 +1922,58 @@ __device__ __forceinline__ uint32_t block_excl_scan_1024(uint32_t v, uint32_t *s
     return base + x - v;
 }
 
+// N-word keys, moved 16 bytes at a time from two words on.
+template <uint32_t N>
+struct WordsN {
+    unsigned long long w[N];
+};
+
+template <uint32_t N>
+__device__ __forceinline__ WordsN<N> stream_words(const unsigned long long *p, unsigned long long i)
+{
+    WordsN<N> k;
+    if constexpr (N == 1) {
+        k.w[0] = __ldcs(p + i);
+    } else {
+#pragma unroll
+        for (uint32_t j = 0; j < N / 2; ++j) {
+            const ulonglong2 v = __ldcs(reinterpret_cast<const ulonglong2 *>(p + i * N) + j);
+            k.w[2 * j] = v.x;
+            k.w[2 * j + 1] = v.y;
+        }
+    }
+    return k;
+}
+
+template <uint32_t N>
+__device__ __forceinline__ WordsN<N> get_words(const unsigned long long *p, unsigned long long i)
+{
+    WordsN<N> k;
+    if constexpr (N == 1) {
+        k.w[0] = p[i];
+    } else {
+#pragma unroll
+        for (uint32_t j = 0; j < N / 2; ++j) {
+            const ulonglong2 v = reinterpret_cast<const ulonglong2 *>(p + i * N)[j];
+            k.w[2 * j] = v.x;
+            k.w[2 * j + 1] = v.y;
+        }
+    }
+    return k;
+}
+
+template <uint32_t N>
+__device__ __forceinline__ void put_words(unsigned long long *p, unsigned long long i, const WordsN<N> &k)
+{
+    if constexpr (N == 1) {
+        p[i] = k.w[0];
+    } else {
+#pragma unroll
+        for (uint32_t j = 0; j < N / 2; ++j)
+            reinterpret_cast<ulonglong2 *>(p + i * N)[j] = make_ulonglong2(k.w[2 * j], k.w[2 * j + 1]);
+    }
+}
+
 // One work item (ITEM keys of one bucket) per round: the keys are ranked by
 // sub-bucket in shared memory, every sub-bucket of the item takes its range
 // with one cursor update, and the item's keys are written reordered by
@@ -1937,7 +1991,7 @@ __device__ __forceinline__ uint32_t block_excl_scan_1024(uint32_t v, uint32_t *s
 // items of 4096 keys, 13.9 with 6144 (two blocks per SM) and 12.4 with 16384
 // (one block of 1024 threads); 480M keys in up to 512 sub-buckets 2.2, 1.9 and
 // 2.4 ms.
-template <uint32_t THREADS, uint32_t KPT, uint32_t MAXB, uint32_t BPSM>
+template <uint32_t N, uint32_t THREADS, uint32_t KPT, uint32_t MAXB, uint32_t BPSM>
 __global__ void __launch_bounds__(THREADS, BPSM) k_subpart_scatter(const unsigned long long *keys,
                                                                       const BucketRanges *rg, uint32_t n_items,
                                                                       unsigned int *next_item, const SubCfg *sc,
@@ -1951,8 +2005,8 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_subpart_scatter(const unsigne
     // shared arrays per sub-bucket hold max_sub entries (the most of any
     // bucket of the launch)
     extern __shared__ __align__(16) uint8_t sp_smem[];
-    unsigned long long *s_sorted = reinterpret_cast<unsigned long long *>(sp_smem);   // ITEM
-    unsigned long long *s_dst = s_sorted + ITEM;                                      // max_sub
+    unsigned long long *s_sorted = reinterpret_cast<unsigned long long *>(sp_smem);   // ITEM keys
+    unsigned long long *s_dst = s_sorted + N * ITEM;                                  // max_sub
     uint32_t *s_cnt = reinterpret_cast<uint32_t *>(s_dst + max_sub);                  // max_sub: counts, then starts
     __shared__ uint32_t s_item0[N_BUCKETS + 1];
     __shared__ uint32_t s_warp[32], s_over;
@@ -1969,7 +2023,7 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_subpart_scatter(const unsigne
             const SubCfg c = sc[w.bucket];
             s_begin = w.begin;
             s_n = (uint32_t)(w.end - w.begin);
-            s_shift = c.shift - 32;   // sub-buckets follow the key's upper half: shift >= 44
+            s_shift = c.shift - 32;   // sub-buckets follow the first word's upper half
             s_nsub = c.n_sub;
             s_base = c.sub_base;
         }
@@ -1979,18 +2033,18 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_subpart_scatter(const unsigne
         take_next();
     }
     __syncthreads();
-    unsigned long long k[KPT];
+    WordsN<N> k[KPT];
     uint32_t n = s_n;
 #pragma unroll
     for (uint32_t r = 0; r < KPT; ++r)
-        if (r * THREADS + tid < n) k[r] = __ldcs(&keys[s_begin + r * THREADS + tid]);
+        if (r * THREADS + tid < n) k[r] = stream_words<N>(keys, s_begin + r * THREADS + tid);
     while (n) {
         const uint32_t shift = s_shift, n_sub = s_nsub, base = s_base, smask = n_sub - 1;
         uint32_t sr[KPT];   // rank << 16 | sub
 #pragma unroll
         for (uint32_t r = 0; r < KPT; ++r)
             if (r * THREADS + tid < n) {
-                const uint32_t sub = ((uint32_t)(k[r] >> 32) >> shift) & smask;
+                const uint32_t sub = ((uint32_t)(k[r].w[0] >> 32) >> shift) & smask;
                 sr[r] = (atomicAdd(&s_cnt[sub], 1u) << 16) | sub;
             }
         __syncthreads();
@@ -2021,12 +2075,12 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_subpart_scatter(const unsigne
         __syncthreads();
 #pragma unroll
         for (uint32_t r = 0; r < KPT; ++r)
-            if (r * THREADS + tid < n) s_sorted[s_cnt[sr[r] & 0xFFFFu] + (sr[r] >> 16)] = k[r];
+            if (r * THREADS + tid < n) put_words<N>(s_sorted, s_cnt[sr[r] & 0xFFFFu] + (sr[r] >> 16), k[r]);
         const uint32_t nn = s_n;
         const unsigned long long nb = s_begin;
 #pragma unroll
         for (uint32_t r = 0; r < KPT; ++r)
-            if (r * THREADS + tid < nn) k[r] = __ldcs(&keys[nb + r * THREADS + tid]);
+            if (r * THREADS + tid < nn) k[r] = stream_words<N>(keys, nb + r * THREADS + tid);
         // destination of sorted index i of sub-bucket s: s_dst[s] + i
         run = run0;
 #pragma unroll
@@ -2044,17 +2098,17 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_subpart_scatter(const unsigne
         if (!s_over) {
 #pragma unroll 4
             for (uint32_t i = tid; i < n; i += THREADS) {
-                const unsigned long long key = s_sorted[i];
-                out[s_dst[((uint32_t)(key >> 32) >> shift) & smask] + i] = key;
+                const WordsN<N> key = get_words<N>(s_sorted, i);
+                put_words<N>(out, s_dst[((uint32_t)(key.w[0] >> 32) >> shift) & smask] + i, key);
             }
         } else {
             // a sub-bucket that outgrew its region is reported by its cursor
             // (k_subpart_sizes) and counted exactly
             for (uint32_t i = tid; i < n; i += THREADS) {
-                const unsigned long long key = s_sorted[i];
-                const uint32_t sub = ((uint32_t)(key >> 32) >> shift) & smask;
+                const WordsN<N> key = get_words<N>(s_sorted, i);
+                const uint32_t sub = ((uint32_t)(key.w[0] >> 32) >> shift) & smask;
                 const unsigned long long d = s_dst[sub] + i;
-                if (d < out_cap && d < sub_end[base + sub]) out[d] = key;
+                if (d < out_cap && d < sub_end[base + sub]) put_words<N>(out, d, key);
             }
         }
         for (uint32_t i = tid; i < n_sub; i += THREADS) s_cnt[i] = 0;
@@ -2739,7 +2793,8 @@ cudaError_t launch_merge_buckets(const unsigned long long *keys, const BucketRan
 }
 
 cudaError_t launch_subpart_count(const unsigned long long *keys, const BucketRanges *rg, uint32_t n_items,
-                                 const SubCfg *sc, uint32_t *sub_count, cudaStream_t st, uint32_t stride)
+                                 const SubCfg *sc, uint32_t *sub_count, uint32_t words, cudaStream_t st,
+                                 uint32_t stride)
 {
     if (!n_items) return cudaSuccess;
     int per_sm = 0;
@@ -2747,7 +2802,7 @@ cudaError_t launch_subpart_count(const unsigned long long *keys, const BucketRan
         per_sm = 1;
     const uint32_t grid = std::min<uint32_t>(n_items, (uint32_t)(sm_count() * per_sm));
     note_launch();
-    k_subpart_count<<<grid, 256, 0, st>>>(keys, rg, n_items, sc, sub_count, stride < 1 ? 1u : stride);
+    k_subpart_count<<<grid, 256, 0, st>>>(keys, rg, n_items, sc, sub_count, stride < 1 ? 1u : stride, words);
     return cudaGetLastError();
 }
 
@@ -2775,14 +2830,14 @@ cudaError_t launch_subpart_sizes(const unsigned long long *sub_off, const unsign
     return cudaGetLastError();
 }
 
-template <uint32_t THREADS, uint32_t KPT, uint32_t MAXB, uint32_t BPSM>
+template <uint32_t N, uint32_t THREADS, uint32_t KPT, uint32_t MAXB, uint32_t BPSM>
 static cudaError_t launch_subpart_scatter_t(const unsigned long long *keys, const BucketRanges *rg, uint32_t n_items,
                                             unsigned int *next_item, const SubCfg *sc, unsigned long long *sub_cursor,
                                             unsigned long long *out, uint64_t out_cap, uint32_t max_sub,
                                             cudaStream_t st, const unsigned long long *sub_end)
 {
-    const size_t smem = (size_t)KPT * THREADS * 8 + (size_t)max_sub * (8 + 4);
-    auto kern = k_subpart_scatter<THREADS, KPT, MAXB, BPSM>;
+    const size_t smem = (size_t)KPT * THREADS * N * 8 + (size_t)max_sub * (8 + 4);
+    auto kern = k_subpart_scatter<N, THREADS, KPT, MAXB, BPSM>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
@@ -2794,22 +2849,32 @@ static cudaError_t launch_subpart_scatter_t(const unsigned long long *keys, cons
     return cudaGetLastError();
 }
 
+template <uint32_t N>
+static cudaError_t launch_subpart_scatter_n(const unsigned long long *keys, const BucketRanges *rg, uint32_t n_items,
+                                            unsigned int *next_item, const SubCfg *sc, unsigned long long *sub_cursor,
+                                            unsigned long long *out, uint64_t out_cap, uint32_t max_sub,
+                                            cudaStream_t st, const unsigned long long *sub_end, uint32_t scatter_shape)
+{
+#define KC_SCATTER_ARGS keys, rg, n_items, next_item, sc, sub_cursor, out, out_cap, max_sub, st, sub_end
+    if (max_sub > 1024)   // sub_scatter_item_keys: 16384 / N keys
+        return max_sub > 2048 ? launch_subpart_scatter_t<N, 1024, 16 / N, 4, 1>(KC_SCATTER_ARGS)
+                              : launch_subpart_scatter_t<N, 1024, 16 / N, 2, 1>(KC_SCATTER_ARGS);
+    return scatter_shape == 2 ? launch_subpart_scatter_t<N, 512, 12 / N, 2, 3>(KC_SCATTER_ARGS)
+                              : launch_subpart_scatter_t<N, 512, 12 / N, 2, 2>(KC_SCATTER_ARGS);
+#undef KC_SCATTER_ARGS
+}
+
 cudaError_t launch_subpart_scatter(const unsigned long long *keys, const BucketRanges *rg, uint32_t n_items,
                                    unsigned int *next_item, const SubCfg *sc, unsigned long long *sub_cursor,
-                                   unsigned long long *out, uint64_t out_cap, uint32_t max_sub, cudaStream_t st,
-                                   const unsigned long long *sub_end, uint32_t scatter_shape)
+                                   unsigned long long *out, uint64_t out_cap, uint32_t max_sub, uint32_t words,
+                                   cudaStream_t st, const unsigned long long *sub_end, uint32_t scatter_shape)
 {
     if (!n_items) return cudaSuccess;
     if (!max_sub || max_sub > SUB_MAX_PER_BUCKET) return cudaErrorInvalidValue;
     cudaError_t e = cudaMemsetAsync(next_item, 0, 4, st);
     if (e != cudaSuccess) return e;
-#define KC_SCATTER_ARGS keys, rg, n_items, next_item, sc, sub_cursor, out, out_cap, max_sub, st, sub_end
-    if (sub_scatter_item_keys(max_sub) == 16384)
-        return max_sub > 2048 ? launch_subpart_scatter_t<1024, 16, 4, 1>(KC_SCATTER_ARGS)
-                              : launch_subpart_scatter_t<1024, 16, 2, 1>(KC_SCATTER_ARGS);
-    return scatter_shape == 2 ? launch_subpart_scatter_t<512, 12, 2, 3>(KC_SCATTER_ARGS)
-                              : launch_subpart_scatter_t<512, 12, 2, 2>(KC_SCATTER_ARGS);
-#undef KC_SCATTER_ARGS
+    auto f = words == 1 ? launch_subpart_scatter_n<1> : (words == 2 ? launch_subpart_scatter_n<2> : launch_subpart_scatter_n<4>);
+    return f(keys, rg, n_items, next_item, sc, sub_cursor, out, out_cap, max_sub, st, sub_end, scatter_shape);
 }
 
 cudaError_t launch_wait_flag(const unsigned int *flag, uint32_t poll_limit, unsigned long long *flags, cudaStream_t st)

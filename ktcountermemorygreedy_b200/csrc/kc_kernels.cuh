@@ -154,16 +154,23 @@ uint32_t fill_item_starts_n(BucketRanges &r, uint64_t item_keys);
 constexpr uint32_t SUB_COUNT_KEYS = 2048;   // keys per work item and stride of the sub-bucket count
 // keys per work item of the sub-bucket scatter: larger items where a bucket
 // has many sub-buckets (k_subpart_scatter)
-inline uint32_t sub_scatter_item_keys(uint32_t max_sub) { return max_sub > 1024 ? 16384u : 6144u; }
+inline uint32_t sub_scatter_item_keys(uint32_t max_sub, uint32_t words)
+{
+    return (max_sub > 1024 ? 16384u : 6144u) / words;
+}
 
-// Prefix path: the buckets of the string keys' top 8 bits are cut into n_sub
-// sub-buckets each (a power of two) by the bits below, so that one thread
-// block counts a sub-bucket's distinct k-mers in a shared-memory table.
+// Prefix path: up to 256 buckets of string keys (of one, two or four words),
+// cut into n_sub sub-buckets each (a power of two) by bits of the keys' first
+// word, so that one thread block counts a sub-bucket's distinct k-mers in a
+// shared-memory table.
 constexpr uint32_t SUB_MAX_PER_BUCKET = 4096;   // sub-buckets of one bucket
 struct SubCfg {
     uint32_t sub_base, n_sub;   // its sub-buckets [sub_base, sub_base + n_sub)
-    uint32_t shift;             // a key's sub-bucket: (key >> shift) & (n_sub - 1)
-    uint32_t pad;
+    uint32_t shift;             // a key's sub-bucket: (first word >> shift) & (n_sub - 1); 32..63
+    uint32_t plen;              // bits that all keys of a sub-bucket share
+    uint32_t k;
+    uint32_t group;             // histogram and totals its counts go to
+    uint32_t count_max, min_count, max_count;
 };
 
 // Per-bucket state of the partitioned pipeline.
@@ -188,6 +195,10 @@ cudaError_t launch_extract(int mode, const ExtractArgs &a, int grid, cudaStream_
 // their first four bases, so that buckets are consecutive ranges of the printed
 // order.
 cudaError_t launch_part(bool by_string, uint32_t k, const ExtractArgs &a, cudaStream_t st);
+// The same for k = 33..128: string keys of two or four words (offsets and
+// regions count keys).  census: the k-mers of every (bucket_sample_mask + 1)-th
+// tile are counted in a.bucket_hist and a.occ instead.
+cudaError_t launch_part_wide(bool census, uint32_t k, const ExtractArgs &a, cudaStream_t st);
 
 // Exclusive prefix sum of n 32-bit values into 64-bit outputs.  tmp must
 // hold scan_tmp_words(n) 64-bit words.
@@ -310,16 +321,19 @@ cudaError_t launch_select(const unsigned long long *keys, const uint32_t *counts
 // in sub-bucket s.  scatter: every key to out[sub_cursor[its sub-bucket]++]
 // (sub_cursor starts at the exclusive scan of sub_count).  The count's ranges
 // rg are cut into items of SUB_COUNT_KEYS * stride keys, the scatter's into
-// items of sub_scatter_item_keys(max_sub) keys (fill_item_starts_n).
+// items of sub_scatter_item_keys(max_sub, words) keys (fill_item_starts_n).
+// Keys have `words` 64-bit words; all ranges, offsets and sizes count keys.
 // stride > 1: only every stride-th run of 16 keys is counted (a sample).
 cudaError_t launch_subpart_count(const unsigned long long *keys, const BucketRanges *rg, uint32_t n_items,
-                                 const SubCfg *sc, uint32_t *sub_count, cudaStream_t st, uint32_t stride = 1);
+                                 const SubCfg *sc, uint32_t *sub_count, uint32_t words, cudaStream_t st,
+                                 uint32_t stride = 1);
 // sub_end non-NULL: the sub-buckets' regions are estimates and a key is
 // written only inside its sub-bucket's region [.., sub_end[s]).
 cudaError_t launch_subpart_scatter(const unsigned long long *keys, const BucketRanges *rg, uint32_t n_items,
                                    unsigned int *next_item, const SubCfg *sc, unsigned long long *sub_cursor,
-                                   unsigned long long *out, uint64_t out_cap, uint32_t max_sub, cudaStream_t st,
-                                   const unsigned long long *sub_end = nullptr, uint32_t scatter_shape = 1);
+                                   unsigned long long *out, uint64_t out_cap, uint32_t max_sub, uint32_t words,
+                                   cudaStream_t st, const unsigned long long *sub_end = nullptr,
+                                   uint32_t scatter_shape = 1);
 // scatter_shape 2 (kc_tuning.scatter_shape): launches whose buckets have at
 // most 1024 sub-buckets run a variant with fewer registers, three blocks per SM.
 // Estimated regions from a 1-in-stride sampled count: region (u32 per
@@ -334,19 +348,21 @@ cudaError_t launch_subpart_sizes(const unsigned long long *sub_off, const unsign
                                  const unsigned long long *sub_end, uint32_t n_sub, uint64_t out_cap, uint32_t *count,
                                  unsigned long long *overflow, cudaStream_t st);
 // The shared-memory count of the sub-buckets (kc_count.cu): sub-bucket s's
-// keys are keys[sub_off[s] .. + sub_count[s]).  Its kept records
-// (count_max, min_count, max_count as for the other paths) go to rec_keys /
-// rec_counts from sub_off[s] on, unsorted within each of its sort units;
-// sub_len[s] receives their number.  A unit is the run
-// [off, off + len) of a sub-bucket's records; the units of size class c
-// (len <= UNIT_CAP0 << c) are listed at units[c * unit_cap], C_UNITS + c of
-// them.  Every k-mer's count goes to hist / ovf; totals to counters
-// (C_REC_LEN, C_DISTINCT, C_LOW_ONLY: k-mers seen once).  Sub-buckets that no
-// number of rounds fits, and more units than unit_cap, are counted in
-// C_SUB_OVF (and bucket_ovf[their bucket]): the results are then incomplete.
-constexpr uint32_t UNIT_CAP0 = 1024, UNIT_CLASSES = 4;
+// keys are keys[sub_off[s] .. + sub_count[s]).  Its kept records (limits of its
+// bucket's SubCfg) go to rec_keys / rec_counts from sub_off[s] on, unsorted
+// within each of its sort units; sub_len[s] receives their number.  A unit is
+// the run [off, off + len) of a sub-bucket's records; the units of size class c
+// (len <= unit_cap0(words) << c) are listed at units[c * unit_cap], C_UNITS + c
+// of them.  Every k-mer's count goes to the group's histogram (hist_bins bins
+// at hist + group * hist_bins; larger counts to ovf, or with their group to
+// ovf64), totals to totals[3 * group ..]: distinct k-mers, k-mers seen once,
+// records.  Sub-buckets that no number of rounds fits, and more units than
+// unit_cap, are counted in C_SUB_OVF (and bucket_ovf[their bucket]): the
+// results are then incomplete.
+constexpr uint32_t UNIT_CLASSES = 4;
+__host__ __device__ constexpr uint32_t unit_cap0(uint32_t words) { return 1024u / words; }
 struct SubUnit {
-    uint32_t sub, off, len, pad;
+    uint32_t sub, off, len, k;
 };
 struct PrefixCountArgs {
     const unsigned long long *keys, *sub_off;
@@ -355,29 +371,33 @@ struct PrefixCountArgs {
     const SubCfg *sc;
     uint32_t n_sub;
     unsigned int *next_sub;
-    uint32_t count_max, min_count, max_count;
     unsigned long long *rec_keys;
     uint32_t *rec_counts, *sub_len;
     SubUnit *units;
-    uint32_t unit_cap;
-    unsigned long long *hist;
+    uint32_t unit_cap, hist_bins;
+    unsigned long long *hist, *totals;
     uint32_t *ovf;
+    unsigned long long *ovf64;
     uint64_t ovf_cap;
     unsigned long long *counters;
     uint32_t *bucket_ovf;
 };
 // shape (kc_tuning.count_shape): 1 and 3 run 512-thread blocks, two per SM,
-// with 8192-slot tables; 2 and 4 run 256-thread blocks, four per SM, with
-// 4096-slot tables (sub-buckets of half the k-mers).
-cudaError_t launch_count_prefix(const PrefixCountArgs &a, uint32_t shape, cudaStream_t st);
-inline uint32_t sub_table_slots(uint32_t shape) { return (shape == 2 || shape == 4) ? 4096u : 8192u; }
+// with tables of 8192, 4096 or 2048 slots for keys of 1, 2 or 4 words; 2 and 4
+// run 256-thread blocks, four per SM, with half the slots (sub-buckets of half
+// the k-mers).
+cudaError_t launch_count_prefix(const PrefixCountArgs &a, uint32_t words, uint32_t shape, cudaStream_t st);
+inline uint32_t sub_table_slots(uint32_t words, uint32_t shape)
+{
+    return ((shape == 2 || shape == 4) ? 4096u : 8192u) / words;
+}
 // Every unit's records sorted and written, as k-mer words, to out_k / out_v
 // from sub_final[sub] + off on (sub_final: the exclusive scan of sub_len);
 // n_units: units per class (host values).
-cudaError_t launch_unit_sort(const unsigned long long *tk, const uint32_t *tv, const unsigned long long *sub_off,
-                             const unsigned long long *sub_final, const SubUnit *units, uint32_t unit_cap,
-                             const uint32_t *n_units, unsigned long long *out_k, uint32_t *out_v, uint64_t out_cap,
-                             uint32_t k, cudaStream_t st);
+cudaError_t launch_unit_sort(uint32_t words, const unsigned long long *tk, const uint32_t *tv,
+                             const unsigned long long *sub_off, const unsigned long long *sub_final,
+                             const SubUnit *units, uint32_t unit_cap, const uint32_t *n_units,
+                             unsigned long long *out_k, uint32_t *out_v, uint64_t out_cap, cudaStream_t st);
 cudaError_t launch_bloom_buckets(const unsigned long long *keys, const BucketRanges *rg, uint32_t n_items,
                                  unsigned int *next_item, const BucketCfg *cfg, unsigned long long *bits,
                                  unsigned long long *out, unsigned long long *low_cnt, unsigned long long *high_cnt,

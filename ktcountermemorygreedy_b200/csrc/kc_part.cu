@@ -1,12 +1,13 @@
-// kc_part.cu -- the partition of a job's k-mers (k <= 32) into 256 buckets:
-// the FASTQ tiles are read once, every window of k valid bases becomes its
-// canonical k-mer, and the k-mers are scattered by their first four bases (as
-// string keys, for the counting by printed-order prefix) or by root prefix (as
-// k-mer words, the reference's get_root_prefix, for global-memory tables).
+// kc_part.cu -- the partition of a job's k-mers into 256 buckets: the FASTQ
+// tiles are read once, every window of k valid bases becomes its canonical
+// k-mer, and the k-mers are scattered by their first four bases (as string
+// keys, for the counting by printed-order prefix) or by root prefix (as k-mer
+// words, the reference's get_root_prefix, for global-memory tables; k <= 32).
 #include <algorithm>
 
 #include "kc_device.cuh"
 #include "kc_kernels.cuh"
+#include "kc_wide.cuh"
 
 namespace kc {
 
@@ -282,6 +283,276 @@ __global__ void __launch_bounds__(PT_THREADS, 4) k_part(ExtractArgs a)
     }
 }
 
+// k = 33..128: the same partition of kmer<N> string keys, N = 2 or 4 words.
+// The tile comes with the 128 bytes before it; a chunk is 16 / N positions, so
+// that a thread's k-mers fill as many registers as above.  A window's words
+// are rolled one base at a time: the forward array (newest base at the top of
+// word 0, older ones towards word LAST) moves down by two bits across its
+// words, the reverse complement (first base's complement at the top of word 0)
+// up.  The canonical array is the lexicographically smaller one
+// (src/GetKmer.h:181-206), and the string key of its strand is the complement
+// of the other, larger one, word by word, as for one word.
+//
+// CENSUS: only every (bucket_sample_mask + 1)-th tile is read and its k-mers
+// are counted per bucket (and in *occ), not written.
+constexpr uint32_t WP_HALO_SEGS = WIDE_HALO / 32;
+constexpr uint32_t WP_SEGS = PT_THREADS + WP_HALO_SEGS;
+constexpr uint32_t WP_BUF = TILE + WIDE_HALO;   // 8320, a multiple of 16
+
+struct WidePartSmem {
+    uint8_t tile[WP_BUF];
+    unsigned long long codes[WP_SEGS + 4], rcodes[WP_SEGS + 4];   // rcodes: complemented codes, first at the top
+    uint32_t good[WP_SEGS + 4];
+    uint32_t chunk[8 * PT_THREADS];
+    unsigned long long stage[PT_STAGE];   // PT_STAGE / N keys
+};
+
+template <uint32_t N, uint32_t LAST, bool CENSUS>
+__global__ void __launch_bounds__(PT_THREADS, 3) k_part_wide(ExtractArgs a)
+{
+    constexpr uint32_t CH = 16 / N, PER_SEG = 32 / CH;   // positions of a chunk, chunks of a segment
+    extern __shared__ __align__(128) uint8_t pt_smem[];
+    WidePartSmem &s = *reinterpret_cast<WidePartSmem *>(pt_smem);
+    __shared__ __align__(8) uint64_t mbar;
+    __shared__ __align__(16) uint32_t s_wnl[8], s_wbk[8];
+    __shared__ uint32_t s_hist[N_BUCKETS], s_start[N_BUCKETS], s_lim[N_BUCKETS];
+    __shared__ unsigned long long *s_ptr[N_BUCKETS];
+    __shared__ uint32_t s_nch, s_over;
+
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint64_t step = CENSUS ? a.bucket_sample_mask + 1 : 1;   // tiles between two visited ones
+    const uint64_t n_visit = (a.n_tiles + step - 1) / step;
+    uint64_t u = blockIdx.x;
+    if (u >= n_visit) return;
+    uint32_t lt;
+    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
+    if (tid == 0) {
+        mbar_init(&mbar, 1);
+        fence_mbar_init();
+        s_over = 0;
+        s.codes[WP_SEGS] = 0;
+        s.rcodes[WP_SEGS] = 0;
+    }
+    s_hist[tid] = 0;
+    __syncthreads();
+    if (tid == 0) {
+        mbar_expect_tx(&mbar, WP_BUF);
+        bulk_load(s.tile, a.buf + u * step * TILE - WIDE_HALO, WP_BUF, &mbar);
+    }
+    const uint32_t blo = a.bucket_lo, bhi = a.bucket_hi ? a.bucket_hi : N_BUCKETS;
+    const bool all_buckets = blo == 0 && bhi == N_BUCKETS;
+    uint32_t seg_next = a.tile_seg[u * step], seg_cur = 0xFFFFFFFFu;
+    uint32_t line_next = (uint32_t)a.tile_prefix[u * step], line_file = 0, k = 0;
+    uint64_t first_tile = 0;
+    unsigned long long n_occ = 0;
+    for (uint32_t iter = 0; u < n_visit; u += gridDim.x, ++iter) {
+        const uint64_t t = u * step;
+        if (tid == 0) s_nch = 0;
+        if (seg_next != seg_cur) {
+            seg_cur = seg_next;
+            first_tile = a.segs[seg_cur].first_tile;
+            k = a.segs[seg_cur].k;
+            line_file = (uint32_t)a.tile_prefix[first_tile];
+        }
+        const uint32_t line0 = line_next - line_file;
+        const bool ok = mbar_wait(&mbar, iter & 1);
+        if (__syncthreads_or(!ok)) {
+            if (tid == 0) atomicOr(&a.counters[C_FLAGS], ERR_WAIT_TIMEOUT);
+            return;
+        }
+        const bool first = t == first_tile;
+        const uint32_t rem = k % 32, fs = rem ? 64 - 2 * rem : 0;   // unused low bits of word LAST
+        const uint64_t back_mask = ~0ULL << fs;
+
+        // ---- segments: codes, valid bases, lines
+        uint64_t codes;
+        uint32_t valid, nl;
+        classify32(s.tile + WIDE_HALO + 32 * tid, codes, valid, nl);
+        const uint32_t own_nl = (uint32_t)__popc(nl);
+        const uint32_t inc_nl = warp_inclusive(own_nl, lane);
+        if (lane == 31) s_wnl[warp] = inc_nl;
+        s.codes[WP_HALO_SEGS + tid] = codes;
+        s.rcodes[WP_HALO_SEGS + tid] = pair_reverse(~codes);
+        if (warp == 7) {
+            // the halo: the end of the file's previous tile (nothing for a
+            // file's first one); line numbers counted back from the tile's first
+            uint64_t hc = 0;
+            uint32_t hv = 0, hn = 0;
+            if (lane < (int)WP_HALO_SEGS && !first) classify32(s.tile + 32 * lane, hc, hv, hn);
+            uint32_t x = (uint32_t)__popc(hn);
+            x += __shfl_down_sync(FULLW, x, 1);
+            x += __shfl_down_sync(FULLW, x, 2);   // lane j: newlines of halo segments j..3
+            if (lane < (int)WP_HALO_SEGS) {
+                s.codes[lane] = hc;
+                s.rcodes[lane] = pair_reverse(~hc);
+                s.good[lane] = first ? 0u : hv & line_mask(line0 - x, hn, 1);
+            }
+        }
+        __syncthreads();
+        uint32_t tot_nl;
+        const uint32_t before_nl = sum_before(s_wnl, warp, tot_nl);
+        s.good[WP_HALO_SEGS + tid] = valid & line_mask(line0 + before_nl + inc_nl - own_nl, nl, 1);
+        __syncthreads();
+        if (u + gridDim.x < n_visit) {
+            const uint64_t tn = t + (uint64_t)gridDim.x * step;
+            if (tid == 0) {
+                fence_proxy_async_smem();
+                mbar_expect_tx(&mbar, WP_BUF);
+                bulk_load(s.tile, a.buf + tn * TILE - WIDE_HALO, WP_BUF, &mbar);
+            }
+            seg_next = a.tile_seg[tn];
+            line_next = (uint32_t)a.tile_prefix[tn];
+        }
+
+        // ---- window ends: k > 32, so a window that ends in this segment
+        // holds all its positions before that, and as many before it as are
+        // missing to k
+        uint32_t ends = 0;
+        {
+            const uint32_t g = s.good[WP_HALO_SEGS + tid];
+            uint32_t run = 0;
+            bool open = true;
+#pragma unroll
+            for (uint32_t j = 1; j <= WP_HALO_SEGS; ++j) {
+                const uint32_t gj = s.good[WP_HALO_SEGS + tid - j];
+                if (open) run += gj == FULLW ? 32u : (uint32_t)__clz(~gj);
+                open = open && gj == FULLW;
+            }
+            const uint32_t lead = g == FULLW ? 32u : (uint32_t)__ffs(~g) - 1u;   // valid bases the segment starts with
+            const uint32_t from = k - 1 > run ? k - 1 - run : 0u;
+            if (from < lead) ends = range_mask(from, lead);
+        }
+        n_occ += (unsigned long long)__popc(ends);
+        {
+            uint32_t cnt = 0, b[PER_SEG];
+#pragma unroll
+            for (uint32_t q = 0; q < PER_SEG; ++q) {
+                b[q] = __ballot_sync(FULLW, (ends >> (CH * q)) & ((1u << CH) - 1u));
+                cnt += (uint32_t)__popc(b[q]);
+            }
+            uint32_t at = 0;
+            if (lane == 0 && cnt) at = atomicAdd(&s_nch, cnt);
+            at = __shfl_sync(FULLW, at, 0);
+#pragma unroll
+            for (uint32_t q = 0; q < PER_SEG; ++q) {
+                const uint32_t e = (ends >> (CH * q)) & ((1u << CH) - 1u);
+                if (e) s.chunk[at + (uint32_t)__popc(b[q] & lt)] = ((uint32_t)tid << 16) | (q << 8) | e;
+                at += (uint32_t)__popc(b[q]);
+            }
+        }
+        __syncthreads();
+        const uint32_t n_ch = s_nch;
+
+        for (uint32_t r0 = 0; r0 < n_ch; r0 += PT_THREADS) {
+            uint32_t e = 0;
+            unsigned long long key[CH][N];
+            uint32_t rk[CH];
+            if (r0 + tid < n_ch) {
+                const uint32_t ch = s.chunk[r0 + tid];
+                e = ch & 0xFFu;
+                const uint32_t p0 = 32 * (WP_HALO_SEGS + (ch >> 16)) + CH * ((ch >> 8) & 0xFFu);   // the chunk's first position
+                // the window ending just before the chunk
+                uint64_t f[LAST + 1], r[LAST + 1];
+#pragma unroll
+                for (uint32_t w = 0; w <= LAST; ++w) {
+                    const uint32_t en = p0 - 1 - 32 * w, es = en >> 5, eo = en & 31;
+                    f[w] = eo == 31 ? s.codes[es] : (s.codes[es - 1] >> (2 * eo + 2)) | (s.codes[es] << (62 - 2 * eo));
+                    const uint32_t st = p0 - k + 32 * w, ss = st >> 5, so = st & 31;
+                    r[w] = so == 0 ? s.rcodes[ss] : (s.rcodes[ss] << (2 * so)) | (s.rcodes[ss + 1] >> (64 - 2 * so));
+                }
+                r[LAST] &= back_mask;
+                const uint32_t cw = (uint32_t)(s.codes[p0 >> 5] >> (2 * (p0 & 31)));   // the chunk's codes
+#pragma unroll
+                for (uint32_t p = 0; p < CH; ++p) {
+                    const uint64_t c = (cw >> (2 * p)) & 3u;
+#pragma unroll
+                    for (uint32_t w = LAST; w > 0; --w) f[w] = (f[w] >> 2) | (f[w - 1] << 62);
+                    f[0] = (f[0] >> 2) | (c << 62);
+#pragma unroll
+                    for (uint32_t w = 0; w < LAST; ++w) r[w] = (r[w] << 2) | (r[w + 1] >> 62);
+                    r[LAST] = (r[LAST] << 2) | ((c ^ 3u) << fs);
+                    const uint64_t fl = f[LAST] & back_mask;
+                    // the larger array, complemented
+                    bool less = false, decided = false;
+#pragma unroll
+                    for (uint32_t w = 0; w <= LAST; ++w) {
+                        const uint64_t x = w == LAST ? fl : f[w];
+                        if (!decided && x != r[w]) {
+                            decided = true;
+                            less = x < r[w];
+                        }
+                    }
+#pragma unroll
+                    for (uint32_t w = 0; w < N; ++w) {
+                        if (w > LAST) key[p][w] = 0;
+                        else {
+                            const uint64_t x = w == LAST ? fl : f[w];
+                            key[p][w] = ~(less ? r[w] : x) & (w == LAST ? back_mask : ~0ULL);
+                        }
+                    }
+                }
+                if (!all_buckets) {
+#pragma unroll
+                    for (uint32_t p = 0; p < CH; ++p) {
+                        const uint32_t b = (uint32_t)(key[p][0] >> 56);
+                        if (b < blo || b >= bhi) e &= ~(1u << p);
+                    }
+                }
+#pragma unroll
+                for (uint32_t p = 0; p < CH; ++p) {
+                    rk[p] = 0;
+                    if ((e >> p) & 1u) rk[p] = atomicAdd(&s_hist[key[p][0] >> 56], 1u);
+                }
+            }
+            if (CENSUS) continue;   // counted; s_hist is added up at the end
+            __syncthreads();
+            const uint32_t c = s_hist[tid];
+            s_hist[tid] = 0;
+            const unsigned long long cur = c ? atomicAdd(&a.bucket_cursor[tid], (unsigned long long)c) : 0ull;
+            const uint32_t inc = warp_inclusive(c, lane);
+            if (lane == 31) s_wbk[warp] = inc;
+            __syncthreads();
+            uint32_t n;
+            const uint32_t start = sum_before(s_wbk, warp, n) + inc - c;
+            s_start[tid] = start;
+            __syncthreads();
+#pragma unroll
+            for (uint32_t p = 0; p < CH; ++p)
+                if ((e >> p) & 1u) {
+                    ulonglong2 *d = reinterpret_cast<ulonglong2 *>(s.stage + N * (s_start[key[p][0] >> 56] + rk[p]));
+#pragma unroll
+                    for (uint32_t w = 0; w < N; w += 2) d[w / 2] = make_ulonglong2(key[p][w], key[p][w + 1]);
+                }
+            if (c) {
+                const unsigned long long at = a.bucket_base[tid] + cur;
+                const unsigned long long end = a.bucket_end[tid] < a.list_cap ? a.bucket_end[tid] : a.list_cap;
+                s_ptr[tid] = a.list + N * at - N * (unsigned long long)start;
+                s_lim[tid] = start + (uint32_t)(at >= end ? 0ull : (end - at < c ? end - at : c));
+                if (at + c > end) s_over = 1;
+            }
+            __syncthreads();
+            const bool over = s_over != 0;
+            for (uint32_t i = tid; i < n; i += PT_THREADS) {
+                const ulonglong2 *q = reinterpret_cast<const ulonglong2 *>(s.stage + N * i);
+                const ulonglong2 v = q[0];
+                const uint32_t b = (uint32_t)(v.x >> 56);
+                if (over && i >= s_lim[b]) continue;
+                ulonglong2 *d = reinterpret_cast<ulonglong2 *>(s_ptr[b] + N * (unsigned long long)i);
+                d[0] = v;
+#pragma unroll
+                for (uint32_t w = 1; w < N / 2; ++w) d[w] = q[w];
+            }
+            if (r0 + PT_THREADS < n_ch) __syncthreads();   // another round: its ranks and stage follow
+        }
+        if (CENSUS) __syncthreads();   // the chunk list is read before the next tile's
+    }
+    if (CENSUS) {
+        for (int o = 16; o > 0; o >>= 1) n_occ += __shfl_down_sync(FULLW, n_occ, o);
+        if (lane == 0 && n_occ) atomicAdd(a.occ, n_occ);
+        if (s_hist[tid]) atomicAdd(&a.bucket_hist[tid], (unsigned long long)s_hist[tid]);
+    }
+}
+
 int part_sms()
 {
     int dev = 0, n = 0;
@@ -305,6 +576,22 @@ cudaError_t launch_part_t(const ExtractArgs &a, cudaStream_t st)
     return cudaGetLastError();
 }
 
+template <uint32_t N, uint32_t LAST, bool CENSUS>
+cudaError_t launch_part_wide_t(const ExtractArgs &a, cudaStream_t st)
+{
+    auto kern = k_part_wide<N, LAST, CENSUS>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WidePartSmem));
+    if (e != cudaSuccess) return e;
+    int per_sm = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, PT_THREADS, sizeof(WidePartSmem));
+    if (e != cudaSuccess) return e;
+    const uint64_t step = CENSUS ? a.bucket_sample_mask + 1 : 1;
+    const uint64_t grid = std::min<uint64_t>((a.n_tiles + step - 1) / step, (uint64_t)part_sms() * std::max(per_sm, 1));
+    note_kernel_launch();
+    kern<<<(unsigned)grid, PT_THREADS, sizeof(WidePartSmem), st>>>(a);
+    return cudaGetLastError();
+}
+
 }  // namespace
 
 cudaError_t launch_part(bool by_string, uint32_t k, const ExtractArgs &a, cudaStream_t st)
@@ -312,6 +599,15 @@ cudaError_t launch_part(bool by_string, uint32_t k, const ExtractArgs &a, cudaSt
     if (!a.n_tiles) return cudaSuccess;
     if (k > 16) return by_string ? launch_part_t<true, true>(a, st) : launch_part_t<false, true>(a, st);
     return by_string ? launch_part_t<true, false>(a, st) : launch_part_t<false, false>(a, st);
+}
+
+cudaError_t launch_part_wide(bool census, uint32_t k, const ExtractArgs &a, cudaStream_t st)
+{
+    if (!a.n_tiles) return cudaSuccess;
+    if (k <= 32 || k > 128) return cudaErrorInvalidValue;
+    if (k <= 64) return census ? launch_part_wide_t<2, 1, true>(a, st) : launch_part_wide_t<2, 1, false>(a, st);
+    if (k <= 96) return census ? launch_part_wide_t<4, 2, true>(a, st) : launch_part_wide_t<4, 2, false>(a, st);
+    return census ? launch_part_wide_t<4, 3, true>(a, st) : launch_part_wide_t<4, 3, false>(a, st);
 }
 
 }  // namespace kc

@@ -112,3 +112,80 @@ def test_queries_at_chunk_edges(counter, n, k):
         r = counter.count([fq], k=k, count_max=U32, top_n=top, want_le2=True)
         assert np.array_equal(r.top_keys, want_k[order[:top]]) and np.array_equal(r.top_counts, want_c[order[:top]])
         assert np.array_equal(r.le2_keys, want_k[want_c <= 2]) and np.array_equal(r.le2_counts, want_c[want_c <= 2])
+
+
+def _wide_reads(seed, n, lo, hi, genome):
+    rnd = random.Random(seed)
+    g = "".join(rnd.choice("ACGT") for _ in range(genome))
+    comp = str.maketrans("ACGT", "TGCA")
+    seqs = []
+    for _ in range(n):
+        ln = rnd.randint(lo, hi)
+        i = rnd.randrange(genome - ln)
+        s = list(g[i:i + ln])
+        for j in range(ln):
+            if rnd.random() < 0.004:
+                s[j] = rnd.choice("ACGTN")
+        s = "".join(s)
+        seqs.append(s.translate(comp)[::-1] if rnd.random() < 0.5 else s)
+    return seqs
+
+
+def _check_wide(c, files, k, min_count=1, **kw):
+    all_k, all_c = O.exact_records_wide(files, k, U32)
+    m = all_c >= min_count
+    r = c.count(files, k=k, count_max=U32, min_count=min_count, hist_max=300, top_n=20, want_le2=True, **kw)
+    assert np.array_equal(r.keys, all_k[m]) and np.array_equal(r.counts, all_c[m])
+    assert r.hist.tolist() == O.histogram(all_c, 1, 300).tolist()
+    assert r.distinct == len(all_k) and r.occurrences == int(all_c.sum(dtype=np.uint64))
+    order = np.argsort(-all_c[m].astype(np.int64), kind="stable")[:20]
+    assert np.array_equal(r.top_keys, all_k[m][order])
+    return r
+
+
+@pytest.mark.parametrize("k", [33, 34, 47, 48, 63, 64, 65, 66, 80, 95, 96, 97, 112, 127, 128])
+def test_wide_kmers(counter, k):
+    """Two- and four-word k-mers on the prefix path: every remainder of k at a
+    word's edge, ragged reads of both strands with N bases in two files, long
+    lines across tiles, palindromes."""
+    seqs = _wide_reads(k, 14_000, 130, 250, 60_000)
+    rnd = random.Random(5)
+    half = "".join(rnd.choice("ACGT") for _ in range(70))
+    pal = half + half.translate(str.maketrans("ACGT", "TGCA"))[::-1]
+    seqs += [pal, pal, "A" * 300, "T" * 200, "".join(rnd.choice("ACGT") for _ in range(30_000))]
+    rnd.shuffle(seqs)
+    files = [_fastq(seqs[:9000]), _fastq(seqs[9000:])]
+    assert sum(len(f) for f in files) > 4 << 20
+    for mc in (1, 2):
+        r = _check_wide(counter, files, k, mc)
+        assert r.smem_passes == 1 and r.smem_fallbacks == 0
+
+
+@pytest.mark.parametrize("k", [55, 101])
+def test_wide_kmers_in_passes_and_shapes(counter, k):
+    files = [_fastq(_wide_reads(k, 14_000, 140, 250, 400_000))]
+    for shape in (1, 2):
+        counter.set_tuning(count_shape=shape, scatter_shape=shape, sampled_region_keys=1)
+        one = _check_wide(counter, files, k)
+        many = _check_wide(counter, files, k, pass_bytes=32 << 20)
+        assert one.passes == 1 and many.passes > 1 and many.smem_passes == many.passes
+    counter.set_tuning(count_shape=1, scatter_shape=1, sampled_region_keys=64 << 20)
+
+
+@pytest.mark.parametrize("k,prefix,fallback", [(63, 10, False), (63, 40, True), (127, 10, False), (127, 100, True)])
+def test_many_wide_kmers_of_one_prefix(counter, k, prefix, fallback):
+    rnd = random.Random(prefix)
+    p = "AC" + "".join(rnd.choice("ACGT") for _ in range(prefix - 2))
+    seqs = list({p + "".join(rnd.choice("ACGT") for _ in range(k - prefix - 1)) + "A" for _ in range(30_000)})
+    seqs += [seqs[i % 777] for i in range(3000)] + ["".join(rnd.choice("ACGT") for _ in range(150)) for _ in range(2000)]
+    rnd.shuffle(seqs)
+    r = _check_wide(counter, [_fastq(seqs)], k)
+    assert (r.smem_fallbacks > 0) == fallback and (r.smem_passes == 0) == fallback
+
+
+def test_wide_table_full_once_is_cut_and_counted_again(counter):
+    import ktcountermemorygreedy_b200 as kc
+    files = [_fastq(_wide_reads(9, 14_000, 140, 250, 100_000))]
+    for k in (31, 63, 127):
+        check = _check_wide if k > 32 else lambda c, f, kk, **kw: _check(c, f[0], kk, **kw)
+        check(counter, files, k, fault_inject=kc.INJECT_TABLE_FULL_ONCE)
