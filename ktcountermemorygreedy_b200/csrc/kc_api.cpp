@@ -104,6 +104,17 @@ constexpr uint64_t PREFIX_PATH_MIN_BYTES = 4ull << 20;
 // (tables that overflow into rounds) 25.3 and 17.1.
 constexpr uint64_t SUB_KEYS_TARGET = 16 * 1024;
 
+// The same where k-mers repeat little or sub-buckets are few: a batch's samples
+// (each sequenced far less deeply than a single large job's) and passes below
+// SUB_SMALL_PASS_KEYS, whose 9K-key sub-buckets would be fewer than eight for
+// each of the 296 resident blocks.  Half to all of 6144 keys fit a table even if
+// all are distinct, where 9K take a failed round and two more: count of a
+// 92M-k-mer batch 3.12 -> 2.26 ms, of 25M k-mers of reads 0.49 -> 0.36, of 20M of
+// assembled sequence 0.56 -> 0.31.  (92M k-mers of one job with 2.8 occurrences
+// each: 0.70 at 16K, 1.01 at 6144.)  A batch's sub-buckets are too small for
+// regions sized from a sample.
+constexpr uint64_t SUB_KEYS_SMALL = 6144, SUB_SMALL_PASS_KEYS = 32ull << 20;
+
 // A plain job whose table would hold more slots than this (64 MiB of slots,
 // half of L2) is counted through the root-prefix buckets.
 constexpr uint64_t PLAIN_PART_MIN_SLOTS = 1ull << 22;
@@ -388,8 +399,8 @@ uint64_t default_pass_budget(Workspace &ws)
 // One counting pass of the prefix path: partitioned string keys -> sorted
 // records, histograms and totals.  The buckets are cut into sub-buckets by the
 // next bases, each counted in a shared-memory table, and its records sorted on
-// their own.  A bucket starts with at most SUB_KEYS_TARGET k-mers per
-// sub-bucket; one whose sub-buckets no number of rounds fits is cut into 16
+// their own.  A bucket (a batch's sample, base_bits 0) starts with at most
+// SUB_KEYS_TARGET or SUB_KEYS_SMALL k-mers per sub-bucket; one whose sub-buckets no number of rounds fits is cut into 16
 // times as many and the pass counted again, and a bucket that cannot be cut
 // further is reported by SubTablesFull.
 struct PrefixPass {
@@ -415,8 +426,8 @@ struct PrefixPass {
     // results
     unsigned long long *rec_keys = nullptr;
     uint32_t *rec_counts = nullptr;
-    uint64_t n_rec = 0, n_keys = 0, table_cap = 0;
-    uint32_t region_redos = 0;
+    uint64_t n_rec = 0, n_keys = 0, table_cap = 0, ovf_len = 0;
+    uint32_t n_sub = 0, region_redos = 0;
     std::vector<unsigned long long> totals;   // per group: distinct k-mers, k-mers seen once, records
 };
 
@@ -429,7 +440,12 @@ void count_by_prefix(PrefixPass &pp, DevScope &ds, HostStage &hs, PhaseClock &cl
     const uint32_t lo = pp.lo, hi = pp.hi, N = pp.words;
     unsigned long long *counters = pp.counters;
     const uint32_t shape = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(tn.count_shape, 4));
-    const uint64_t keys_target = SUB_KEYS_TARGET * sub_table_slots(N, shape) / sub_table_slots(1, 1);
+    uint64_t pass_keys = 0;
+    for (uint32_t b = lo; b < hi; ++b) pass_keys += pp.cfg[b].key_len;
+    const bool batch = pp.base_bits == 0;
+    const bool small_subs = batch || (N == 1 && pass_keys < SUB_SMALL_PASS_KEYS);
+    const uint64_t keys_target =
+        (small_subs ? SUB_KEYS_SMALL : SUB_KEYS_TARGET) * sub_table_slots(N, shape) / sub_table_slots(1, 1);
     std::vector<uint32_t> nsub(N_BUCKETS, 0), max_nsub(N_BUCKETS, 1);
     for (uint32_t b = lo; b < hi; ++b) {
         const uint32_t word_bits = std::min(2 * pp.sc[b].k, 64u);
@@ -479,7 +495,7 @@ void count_by_prefix(PrefixPass &pp, DevScope &ds, HostStage &hs, PhaseClock &cl
         unsigned long long *totals = ds.n<unsigned long long>(3 * pp.n_groups);
         const uint32_t unit_cap = 2 * n_sub + 4096;
         SubUnit *units = ds.n<SubUnit>((size_t)UNIT_CLASSES * unit_cap);
-        const bool sampled = !exact_regions && pp.n_keys >= tn.sampled_region_keys;
+        const bool sampled = !exact_regions && !batch && pp.n_keys >= tn.sampled_region_keys;
         const uint32_t stride = sampled ? SUB_REGION_SAMPLE : 1;
         // each bucket-major launch gets its 256 ranges, not a list of items
         auto upload_ranges = [&](uint32_t &n_items, uint64_t item_keys) {
@@ -578,6 +594,7 @@ void count_by_prefix(PrefixPass &pp, DevScope &ds, HostStage &hs, PhaseClock &cl
             continue;
         }
         pp.totals.assign(p_tot, p_tot + 3 * pp.n_groups);
+        pp.ovf_len = cs.v[C_OVF_LEN];
         pp.n_rec = 0;
         for (uint32_t g = 0; g < pp.n_groups; ++g) pp.n_rec += pp.totals[3 * g + 2];
         clk.begin(6);
@@ -591,6 +608,7 @@ void count_by_prefix(PrefixPass &pp, DevScope &ds, HostStage &hs, PhaseClock &cl
         CK(launch_unit_sort(N, pp.keys, pp.tmp_counts, sub_off, sub_cur, units, unit_cap, n_units, pp.rec_keys,
                             pp.rec_counts, pp.n_rec, st));
         clk.end();
+        pp.n_sub = n_sub;
         pp.table_cap = (uint64_t)n_sub * sub_table_slots(N, shape);
         return;
     }
@@ -1104,18 +1122,18 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
                 cu.enqueue(cu.ev.size());
                 a.tile0 = 0;
                 a.n_tiles = tiles_ready;
-                CK(launch_part(prefix, k, a, st));
+                CK(launch_part(prefix ? PART_BY_STRING : PART_BY_ROOT, k, a, st));
                 while (chunks_done < cu.ev.size()) {
                     const uint64_t t0 = tiles_ready;
                     census_chunks(chunks_done + 1);
                     a.tile0 = t0;
                     a.n_tiles = tiles_ready - t0;
-                    CK(launch_part(prefix, k, a, st));
+                    CK(launch_part(prefix ? PART_BY_STRING : PART_BY_ROOT, k, a, st));
                 }
                 a.tile0 = 0;
                 a.n_tiles = T;
             } else {
-                CK(launch_part(prefix, k, a, st));
+                CK(launch_part(prefix ? PART_BY_STRING : PART_BY_ROOT, k, a, st));
             }
             clk.end();
             unsigned long long *p_fill = hs.n<unsigned long long>(N_BUCKETS);
@@ -1162,7 +1180,7 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
                 pp.fault_inject = P.fault_inject;
                 pp.repartition = [&] {
                     CK(cudaMemsetAsync(cursor, 0, N_BUCKETS * 8, st));
-                    CK(launch_part(true, k, a, st));
+                    CK(launch_part(PART_BY_STRING, k, a, st));
                 };
                 count_by_prefix(pp, ds, hs, clk, tn, st);
                 rec_keys = pp.rec_keys;
@@ -2003,10 +2021,13 @@ void run_job(Job &job, cudaStream_t st, Workspace &ws, const kc_tuning &tn)
     if (global_tables) job.smem_fallbacks = job.passes;
 }
 
-// Batched jobs: every sample's files in one device buffer, one SCAN and one
+// Batched jobs: every sample's files in one device buffer and one SCAN launch
+// over all tiles, which counts every sample's k-mers.  Then the prefix path
+// with the samples as buckets; or, for what it cannot hold (global_tables), one
 // INSERT launch over all tiles (each tile counts into its sample's table in a
 // shared slot arena), one batched compaction, one segmented radix sort.
-void run_batch(std::vector<std::shared_ptr<Job>> &jobs, cudaStream_t st, Workspace &ws, const kc_tuning &tn)
+void run_batch_once(std::vector<std::shared_ptr<Job>> &jobs, cudaStream_t st, Workspace &ws, bool global_tables,
+                    const kc_tuning &tn)
 {
     const uint32_t n = (uint32_t)jobs.size();
     if (n > MAX_BATCH) throw KcError{KC_ERR_INVALID, "more than 4096 jobs in one batch"};
@@ -2069,7 +2090,8 @@ void run_batch(std::vector<std::shared_ptr<Job>> &jobs, cudaStream_t st, Workspa
     a.segs = d_segs;
     a.counters = counters;
     a.occ = occ;
-    a.hll = hll;
+    const bool prefix = tn.bloom_smem == 1 && !global_tables;
+    a.hll = prefix ? nullptr : hll;   // the prefix path needs no table sizes
     a.hll_local = n == 1;
     clk.begin(1);
     CK(launch_extract(MODE_SCAN, a, 0, st));
@@ -2081,143 +2103,249 @@ void run_batch(std::vector<std::shared_ptr<Job>> &jobs, cudaStream_t st, Workspa
     Counters c0 = read_counters(counters, st);
     check_flags(c0.v[C_FLAGS], "scan");
 
-    std::vector<uint64_t> caps(n);
-    for (uint32_t i = 0; i < n; ++i) {
-        // one sample: exact registers; several: a 1-in-64 hash sample
-        double e = hll_estimate(&hll_h[(size_t)i * HLL_M], HLL_M);
-        if (n > 1)
-            e = std::max((double)(1u << BATCH_HLL_SAMPLE_BITS) * e, (double)std::min<unsigned long long>(occ_h[i], 4096));
-        e = std::min(e, (double)occ_h[i]);
-        caps[i] = table_capacity_for(e, tn.table_factor);
-    }
-    std::vector<SampleCfg> cfg(n);
-    Slot *arena = nullptr;
-    uint64_t total_slots = 0;
-    SampleCfg *d_cfg = ds.n<SampleCfg>(n);
-    TableRef *d_tables = ds.n<TableRef>(n);
-    for (int attempt = 0;; ++attempt) {
-        total_slots = 0;
-        for (uint32_t i = 0; i < n; ++i) {
-            cfg[i] = SampleCfg{};
-            cfg[i].slot_base = total_slots;
-            cfg[i].slot_cap = caps[i];
-            cfg[i].count_max = jobs[i]->p.count_max;
-            cfg[i].min_count = jobs[i]->p.min_count;
-            cfg[i].max_count = jobs[i]->p.max_count;
-            cfg[i].k = jobs[i]->p.k;
-            total_slots += caps[i];
-        }
-        if (arena) ds.release(arena);
-        arena = static_cast<Slot *>(ds.get(total_slots * sizeof(Slot)));
-        CK(launch_init_slots(arena, total_slots, st));
-        std::vector<TableRef> trs(n);
-        for (uint32_t i = 0; i < n; ++i) trs[i] = TableRef{arena + cfg[i].slot_base, caps[i] - 1};
-        CK(cudaMemcpyAsync(d_tables, trs.data(), n * sizeof(TableRef), cudaMemcpyHostToDevice, st));
-        CK(cudaMemsetAsync(counters, 0, 8, st));
-        a.tables = d_tables;
-        a.max_probe = 1u << 16;
-        clk.begin(2);
-        CK(launch_extract(MODE_INSERT, a, 0, st));
-        clk.end();
-        Counters c = read_counters(counters, st);
-        check_flags(c.v[C_FLAGS], "insert");
-        if (!(c.v[C_FLAGS] & ERR_TABLE_FULL)) break;
-        if (attempt >= 3) throw KcError{KC_ERR_DEVICE, "counting table overflow"};
-        for (auto &cp : caps) cp *= 2;
-    }
-    CK(cudaMemcpyAsync(d_cfg, cfg.data(), n * sizeof(SampleCfg), cudaMemcpyHostToDevice, st));
-    // compaction in chunks of slots of one sample: count the records of every
-    // chunk, scan the counts (the samples' records end up packed in sample
-    // order), then write each chunk's records at its offset
-    std::vector<uint32_t> chunk0(n + 1, 0);
-    uint64_t n_chunks = 0;
-    for (uint32_t i = 0; i < n; ++i) {
-        chunk0[i] = (uint32_t)n_chunks;
-        n_chunks += compact_chunks_of(cfg[i].slot_cap);
-    }
-    chunk0[n] = (uint32_t)n_chunks;
-    uint32_t *d_chunk0 = ds.n<uint32_t>(n + 1);
-    uint32_t *chunk_keep = ds.n<uint32_t>(std::max<uint64_t>(n_chunks, 1));
-    unsigned long long *chunk_pos = ds.n<unsigned long long>(std::max<uint64_t>(n_chunks, 1));
-    unsigned long long *ctmp = ds.n<unsigned long long>(scan_tmp_words(std::max<uint64_t>(n_chunks, 1)));
-    unsigned long long *distinct = ds.n<unsigned long long>(n);
-    CK(cudaMemcpyAsync(d_chunk0, chunk0.data(), (n + 1) * 4, cudaMemcpyHostToDevice, st));
-    CK(cudaMemsetAsync(distinct, 0, (size_t)n * 8, st));
-    clk.begin(5);
-    CK(launch_compact_chunks(arena, d_cfg, d_chunk0, n, n_chunks, chunk_keep, nullptr, nullptr, nullptr, nullptr,
-                             nullptr, 0, distinct, counters, 1, st));
-    CK(launch_scan_u32(chunk_keep, chunk_pos, n_chunks, ctmp, st));
-    clk.end();
-    std::vector<unsigned long long> dist_h(n), pos_h(n_chunks);
-    uint32_t last_keep = 0;
-    CK(cudaMemcpyAsync(dist_h.data(), distinct, (size_t)n * 8, cudaMemcpyDeviceToHost, st));
-    if (n_chunks) {
-        CK(cudaMemcpyAsync(pos_h.data(), chunk_pos, n_chunks * 8, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(&last_keep, chunk_keep + n_chunks - 1, 4, cudaMemcpyDeviceToHost, st));
-    }
-    CK(cudaStreamSynchronize(st));
-    const uint64_t total_rec = n_chunks ? pos_h[n_chunks - 1] + last_keep : 0;
-    std::vector<unsigned long long> len_h(n);
-    for (uint32_t i = 0; i < n; ++i) {
-        cfg[i].rec_base = chunk0[i] < n_chunks ? pos_h[chunk0[i]] : total_rec;
-        const uint64_t next = chunk0[i + 1] < n_chunks ? pos_h[chunk0[i + 1]] : total_rec;
-        len_h[i] = next - cfg[i].rec_base;
-        cfg[i].rec_cap = len_h[i];
-    }
-    unsigned long long *rec_keys = ds.n<unsigned long long>(std::max<uint64_t>(total_rec, 1));
-    uint32_t *rec_counts = ds.n<uint32_t>(std::max<uint64_t>(total_rec, 1));
+    std::vector<uint64_t> caps(n), len_h(n, 0);
+    std::vector<unsigned long long> dist_h(n, 0);
     unsigned long long *hist = ds.n<unsigned long long>((size_t)n * HIST_BINS_BATCH);
+    CK(cudaMemsetAsync(hist, 0, (size_t)n * HIST_BINS_BATCH * 8, st));
     uint64_t occ_total = 0;
     for (uint32_t i = 0; i < n; ++i) occ_total += occ_h[i];
     // counts of HIST_BINS_BATCH or more go to a list, bounded by the
     // occurrences over HIST_BINS_BATCH
     const uint64_t ovf_cap = std::max<uint64_t>(1ull << 20, occ_total / HIST_BINS_BATCH + 1);
     unsigned long long *ovf = ds.n<unsigned long long>(ovf_cap);
-    CK(cudaMemsetAsync(hist, 0, (size_t)n * HIST_BINS_BATCH * 8, st));
-    clk.begin(5);
-    CK(launch_compact_chunks(arena, d_cfg, d_chunk0, n, n_chunks, chunk_keep, chunk_pos, rec_keys, rec_counts, hist,
-                             ovf, ovf_cap, nullptr, counters, 0, st));
-    clk.end();
-    Counters c2 = read_counters(counters, st);
-    check_flags(c2.v[C_FLAGS], "compact");
+    std::vector<unsigned long long> ovf_h;   // sample << 32 | count
+    // a sample's records to its job
+    const auto records_out = [&](uint32_t i, const unsigned long long *keys, const uint32_t *counts) {
+        Job &j = *jobs[i];
+        if (!j.p.keep_records) return;
+        j.recs.allocate(len_h[i]);
+        if (!len_h[i]) return;
+        CK(cudaMemcpyAsync(j.recs.keys(), keys, len_h[i] * 8, cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(j.recs.counts(), counts, len_h[i] * 4, cudaMemcpyDeviceToHost, st));
+    };
+    if (prefix) {
+        // up to 256 samples at a time, as many as a pass's memory holds: each
+        // sample is one bucket, and its k-mers' string keys are cut into
+        // sub-buckets by their first bases
+        HostStage hs(st);
+        const uint64_t budget = default_pass_budget(ws);
+        const auto bytes_of = [&](uint32_t i) {
+            const uint64_t m = std::max(jobs[i]->p.min_count, 1u);
+            return occ_h[i] * (25 + (12 + m - 1) / m);
+        };
+        for (uint32_t lo = 0; lo < n;) {
+            uint64_t need = bytes_of(lo);
+            if (need > budget) throw SubTablesFull{};   // its table of distinct k-mers may be smaller
+            uint32_t hi = lo + 1;
+            while (hi < n && hi - lo < N_BUCKETS && need + bytes_of(hi) <= budget) need += bytes_of(hi++);
+            const uint32_t ng = hi - lo;
+            const DevScope::Mark mk = ds.mark();
+            std::vector<BucketCfg> cfg(N_BUCKETS);
+            std::vector<unsigned long long> bb(2 * N_BUCKETS, 0);
+            unsigned long long off = 0;
+            PrefixPass pp;
+            pp.sc.assign(N_BUCKETS, SubCfg{});
+            for (uint32_t b = 0; b < ng; ++b) {
+                const kc_job &P = jobs[lo + b]->p;
+                cfg[b].key_base = bb[b] = off;
+                cfg[b].key_len = occ_h[lo + b];
+                off += occ_h[lo + b];
+                bb[N_BUCKETS + b] = off;
+                pp.sc[b].k = P.k;
+                pp.sc[b].group = b;
+                pp.sc[b].count_max = P.count_max;
+                pp.sc[b].min_count = P.min_count;
+                pp.sc[b].max_count = P.max_count;
+            }
+            const uint64_t ocap = std::max<uint64_t>(off, 1);
+            pp.list_cap = prefix_list_cap(ocap);
+            pp.list = ds.n<unsigned long long>(pp.list_cap);
+            pp.keys = ds.n<unsigned long long>(pp.list_cap);
+            pp.tmp_counts = ds.n<uint32_t>(pp.list_cap);
+            unsigned long long *cursor = ds.n<unsigned long long>(N_BUCKETS);
+            unsigned long long *bbase = ds.n<unsigned long long>(2 * N_BUCKETS);
+            CK(cudaMemcpyAsync(bbase, hs.up(bb.data(), bb.size()), 2 * N_BUCKETS * 8, cudaMemcpyHostToDevice, st));
+            // the samples' tiles are consecutive
+            uint64_t t0 = T, t1 = 0;
+            for (const auto &sg : segs)
+                if (sg.sample >= lo && sg.sample < hi) {
+                    t0 = std::min<uint64_t>(t0, sg.first_tile);
+                    t1 = std::max<uint64_t>(t1, sg.first_tile + sg.n_tiles);
+                }
+            a.list = pp.keys;
+            a.list_cap = ocap;
+            a.bucket_cursor = cursor;
+            a.bucket_base = bbase;
+            a.bucket_end = bbase + N_BUCKETS;
+            a.sample0 = lo;
+            a.tile0 = t0;
+            a.n_tiles = t1 > t0 ? t1 - t0 : 0;
+            pp.repartition = [&] {
+                CK(cudaMemsetAsync(cursor, 0, N_BUCKETS * 8, st));
+                CK(launch_part(PART_BY_SAMPLE, max_k, a, st));
+            };
+            clk.begin(2);
+            pp.repartition();
+            clk.end();
+            unsigned long long *p_fill = hs.n<unsigned long long>(N_BUCKETS);
+            CK(cudaMemcpyAsync(p_fill, cursor, N_BUCKETS * 8, cudaMemcpyDeviceToHost, st));
+            CK(cudaMemsetAsync(counters + C_OVF_LEN, 0, 8, st));
+            pp.hi = ng;
+            pp.base_bits = 0;
+            pp.cfg = cfg.data();
+            pp.n_groups = ng;
+            pp.hist = hist + (size_t)lo * HIST_BINS_BATCH;
+            pp.hist_bins = HIST_BINS_BATCH;
+            pp.ovf64 = ovf;
+            pp.ovf_cap = ovf_cap;
+            pp.counters = counters;
+            count_by_prefix(pp, ds, hs, clk, tn, st);
+            if (hi == n) CK(cudaEventRecord(ev1, st));
+            uint64_t at = 0;
+            for (uint32_t b = 0; b < ng; ++b) {
+                if (p_fill[b] != occ_h[lo + b])
+                    throw KcError{KC_ERR_DEVICE, "sample census does not add up to its k-mers"};
+                dist_h[lo + b] = pp.totals[3 * b];
+                len_h[lo + b] = pp.totals[3 * b + 2];
+                caps[lo + b] = (uint64_t)pp.sc[b].n_sub * (pp.table_cap / std::max(pp.n_sub, 1u));
+                records_out(lo + b, pp.rec_keys + at, pp.rec_counts + at);
+                at += len_h[lo + b];
+                jobs[lo + b]->smem_passes = 1;
+            }
+            const size_t n_ovf = (size_t)std::min<uint64_t>(pp.ovf_len, ovf_cap), o0 = ovf_h.size();
+            if (n_ovf) {
+                ovf_h.resize(o0 + n_ovf);
+                CK(cudaMemcpyAsync(ovf_h.data() + o0, ovf, n_ovf * 8, cudaMemcpyDeviceToHost, st));
+                CK(cudaStreamSynchronize(st));
+                for (size_t i = o0; i < ovf_h.size(); ++i) ovf_h[i] += (unsigned long long)lo << 32;
+            }
+            ds.rewind(mk);   // the copies of the records are before what follows on the stream
+            lo = hi;
+        }
+    } else {
+        for (uint32_t i = 0; i < n; ++i) {
+            // one sample: exact registers; several: a 1-in-64 hash sample
+            double e = hll_estimate(&hll_h[(size_t)i * HLL_M], HLL_M);
+            if (n > 1)
+                e = std::max((double)(1u << BATCH_HLL_SAMPLE_BITS) * e, (double)std::min<unsigned long long>(occ_h[i], 4096));
+            e = std::min(e, (double)occ_h[i]);
+            caps[i] = table_capacity_for(e, tn.table_factor);
+        }
+        std::vector<SampleCfg> cfg(n);
+        Slot *arena = nullptr;
+        uint64_t total_slots = 0;
+        SampleCfg *d_cfg = ds.n<SampleCfg>(n);
+        TableRef *d_tables = ds.n<TableRef>(n);
+        for (int attempt = 0;; ++attempt) {
+            total_slots = 0;
+            for (uint32_t i = 0; i < n; ++i) {
+                cfg[i] = SampleCfg{};
+                cfg[i].slot_base = total_slots;
+                cfg[i].slot_cap = caps[i];
+                cfg[i].count_max = jobs[i]->p.count_max;
+                cfg[i].min_count = jobs[i]->p.min_count;
+                cfg[i].max_count = jobs[i]->p.max_count;
+                cfg[i].k = jobs[i]->p.k;
+                total_slots += caps[i];
+            }
+            if (arena) ds.release(arena);
+            arena = static_cast<Slot *>(ds.get(total_slots * sizeof(Slot)));
+            CK(launch_init_slots(arena, total_slots, st));
+            std::vector<TableRef> trs(n);
+            for (uint32_t i = 0; i < n; ++i) trs[i] = TableRef{arena + cfg[i].slot_base, caps[i] - 1};
+            CK(cudaMemcpyAsync(d_tables, trs.data(), n * sizeof(TableRef), cudaMemcpyHostToDevice, st));
+            CK(cudaMemsetAsync(counters, 0, 8, st));
+            a.tables = d_tables;
+            a.max_probe = 1u << 16;
+            clk.begin(2);
+            CK(launch_extract(MODE_INSERT, a, 0, st));
+            clk.end();
+            Counters c = read_counters(counters, st);
+            check_flags(c.v[C_FLAGS], "insert");
+            if (!(c.v[C_FLAGS] & ERR_TABLE_FULL)) break;
+            if (attempt >= 3) throw KcError{KC_ERR_DEVICE, "counting table overflow"};
+            for (auto &cp : caps) cp *= 2;
+        }
+        CK(cudaMemcpyAsync(d_cfg, cfg.data(), n * sizeof(SampleCfg), cudaMemcpyHostToDevice, st));
+        // compaction in chunks of slots of one sample: count the records of every
+        // chunk, scan the counts (the samples' records end up packed in sample
+        // order), then write each chunk's records at its offset
+        std::vector<uint32_t> chunk0(n + 1, 0);
+        uint64_t n_chunks = 0;
+        for (uint32_t i = 0; i < n; ++i) {
+            chunk0[i] = (uint32_t)n_chunks;
+            n_chunks += compact_chunks_of(cfg[i].slot_cap);
+        }
+        chunk0[n] = (uint32_t)n_chunks;
+        uint32_t *d_chunk0 = ds.n<uint32_t>(n + 1);
+        uint32_t *chunk_keep = ds.n<uint32_t>(std::max<uint64_t>(n_chunks, 1));
+        unsigned long long *chunk_pos = ds.n<unsigned long long>(std::max<uint64_t>(n_chunks, 1));
+        unsigned long long *ctmp = ds.n<unsigned long long>(scan_tmp_words(std::max<uint64_t>(n_chunks, 1)));
+        unsigned long long *distinct = ds.n<unsigned long long>(n);
+        CK(cudaMemcpyAsync(d_chunk0, chunk0.data(), (n + 1) * 4, cudaMemcpyHostToDevice, st));
+        CK(cudaMemsetAsync(distinct, 0, (size_t)n * 8, st));
+        clk.begin(5);
+        CK(launch_compact_chunks(arena, d_cfg, d_chunk0, n, n_chunks, chunk_keep, nullptr, nullptr, nullptr, nullptr,
+                                 nullptr, 0, distinct, counters, 1, st));
+        CK(launch_scan_u32(chunk_keep, chunk_pos, n_chunks, ctmp, st));
+        clk.end();
+        std::vector<unsigned long long> pos_h(n_chunks);
+        uint32_t last_keep = 0;
+        CK(cudaMemcpyAsync(dist_h.data(), distinct, (size_t)n * 8, cudaMemcpyDeviceToHost, st));
+        if (n_chunks) {
+            CK(cudaMemcpyAsync(pos_h.data(), chunk_pos, n_chunks * 8, cudaMemcpyDeviceToHost, st));
+            CK(cudaMemcpyAsync(&last_keep, chunk_keep + n_chunks - 1, 4, cudaMemcpyDeviceToHost, st));
+        }
+        CK(cudaStreamSynchronize(st));
+        const uint64_t total_rec = n_chunks ? pos_h[n_chunks - 1] + last_keep : 0;
+        for (uint32_t i = 0; i < n; ++i) {
+            cfg[i].rec_base = chunk0[i] < n_chunks ? pos_h[chunk0[i]] : total_rec;
+            const uint64_t next = chunk0[i + 1] < n_chunks ? pos_h[chunk0[i + 1]] : total_rec;
+            len_h[i] = next - cfg[i].rec_base;
+            cfg[i].rec_cap = len_h[i];
+        }
+        unsigned long long *rec_keys = ds.n<unsigned long long>(std::max<uint64_t>(total_rec, 1));
+        uint32_t *rec_counts = ds.n<uint32_t>(std::max<uint64_t>(total_rec, 1));
+        clk.begin(5);
+        CK(launch_compact_chunks(arena, d_cfg, d_chunk0, n, n_chunks, chunk_keep, chunk_pos, rec_keys, rec_counts, hist,
+                                 ovf, ovf_cap, nullptr, counters, 0, st));
+        clk.end();
+        Counters c2 = read_counters(counters, st);
+        check_flags(c2.v[C_FLAGS], "compact");
 
-    std::vector<uint64_t> seg_start(n), seg_len(n);
-    for (uint32_t i = 0; i < n; ++i) {
-        seg_start[i] = cfg[i].rec_base;
-        seg_len[i] = len_h[i];
+        std::vector<uint64_t> seg_start(n), seg_len(n);
+        for (uint32_t i = 0; i < n; ++i) {
+            seg_start[i] = cfg[i].rec_base;
+            seg_len[i] = len_h[i];
+        }
+        clk.begin(6);
+        if (total_rec > 1) {
+            void *stmp = ds.get(sort_tmp_bytes_segmented(total_rec, seg_len.data(), n));
+            std::vector<uint32_t> seg_bits(n);
+            for (uint32_t i = 0; i < n; ++i) seg_bits[i] = 2 * cfg[i].k;
+            CK(launch_radix_sort_segmented(rec_keys, rec_counts, total_rec, seg_start.data(), seg_len.data(), n, 2 * max_k,
+                                           stmp, st, counters + C_FLAGS, seg_bits.data(), tn.sort_group_records));
+            ds.release(stmp);
+        }
+        CK(launch_pair_reverse(rec_keys, total_rec, st));
+        clk.end();
+        CK(cudaEventRecord(ev1, st));
+        check_flags(read_counters(counters, st).v[C_FLAGS], "sort");
+
+        const uint64_t n_ovf = std::min<uint64_t>(c2.v[C_OVF_LEN], ovf_cap);
+        ovf_h.resize(n_ovf);
+        if (n_ovf) CK(cudaMemcpyAsync(ovf_h.data(), ovf, n_ovf * 8, cudaMemcpyDeviceToHost, st));
+        for (uint32_t i = 0; i < n; ++i) records_out(i, rec_keys + cfg[i].rec_base, rec_counts + cfg[i].rec_base);
     }
-    clk.begin(6);
-    if (total_rec > 1) {
-        void *stmp = ds.get(sort_tmp_bytes_segmented(total_rec, seg_len.data(), n));
-        std::vector<uint32_t> seg_bits(n);
-        for (uint32_t i = 0; i < n; ++i) seg_bits[i] = 2 * cfg[i].k;
-        CK(launch_radix_sort_segmented(rec_keys, rec_counts, total_rec, seg_start.data(), seg_len.data(), n, 2 * max_k,
-                                       stmp, st, counters + C_FLAGS, seg_bits.data(), tn.sort_group_records));
-        ds.release(stmp);
-    }
-    CK(launch_pair_reverse(rec_keys, total_rec, st));
-    clk.end();
-    CK(cudaEventRecord(ev1, st));
-    check_flags(read_counters(counters, st).v[C_FLAGS], "sort");
 
     std::vector<unsigned long long> hist_h((size_t)n * HIST_BINS_BATCH);
     CK(cudaMemcpyAsync(hist_h.data(), hist, hist_h.size() * 8, cudaMemcpyDeviceToHost, st));
-    const uint64_t n_ovf = std::min<uint64_t>(c2.v[C_OVF_LEN], ovf_cap);
-    std::vector<unsigned long long> ovf_h(n_ovf);
-    if (n_ovf) CK(cudaMemcpyAsync(ovf_h.data(), ovf, n_ovf * 8, cudaMemcpyDeviceToHost, st));
     for (uint32_t i = 0; i < n; ++i) {
         Job &j = *jobs[i];
         j.n_records_total = len_h[i];
         j.input_bytes = 0;
         for (size_t f = 0; f < files.size(); ++f)   // sizes after gzip inflation
             if (fsample[f] == i) j.input_bytes += files[f].size;
-        if (!j.p.keep_records) continue;
-        j.recs.allocate(len_h[i]);
-        if (len_h[i]) {
-            CK(cudaMemcpyAsync(j.recs.keys(), rec_keys + cfg[i].rec_base, len_h[i] * 8, cudaMemcpyDeviceToHost, st));
-            CK(cudaMemcpyAsync(j.recs.counts(), rec_counts + cfg[i].rec_base, len_h[i] * 4, cudaMemcpyDeviceToHost,
-                               st));
-        }
     }
     const double th1 = now_ms();
     CK(cudaStreamSynchronize(st));
@@ -2246,6 +2374,23 @@ void run_batch(std::vector<std::shared_ptr<Job>> &jobs, cudaStream_t st, Workspa
         uint32_t smp = (uint32_t)(e >> 32), c = (uint32_t)e;
         Job &j = *jobs[smp];
         if (c >= j.p.hist_min && c <= j.p.hist_max) j.hist[c - j.p.hist_min]++;
+    }
+}
+
+void run_batch(std::vector<std::shared_ptr<Job>> &jobs, cudaStream_t st, Workspace &ws, const kc_tuning &tn)
+{
+    try {
+        run_batch_once(jobs, st, ws, false, tn);
+    } catch (const SubTablesFull &) {
+        // a sample whose sub-buckets fit no table, or no pass's memory
+        CK(cudaStreamSynchronize(st));
+        ws.end_job();
+        ws.begin_job();
+        run_batch_once(jobs, st, ws, true, tn);
+        for (auto &j : jobs) {
+            j->smem_passes = 0;
+            ++j->smem_fallbacks;
+        }
     }
 }
 

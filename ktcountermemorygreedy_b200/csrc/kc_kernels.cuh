@@ -118,6 +118,7 @@ struct ExtractArgs {
     const uint32_t *visit;
     uint64_t n_visit;
     uint32_t bucket_lo, bucket_hi;            // launch_part keeps buckets lo <= b < hi (hi 0: all)
+    uint32_t sample0;                         // launch_part by sample: the first bucket's sample
     uint64_t tile0;                           // without visit: tiles tile0 .. tile0 + n_tiles - 1
     unsigned long long *bucket_cursor;        // 256 fill levels (launch_part)
     const unsigned long long *bucket_base;    // 256 start offsets in `list` (launch_part)
@@ -190,11 +191,12 @@ cudaError_t launch_chunk_lastnl(const int32_t *tile_lastnl, const uint32_t *tile
                                 cudaStream_t st);
 cudaError_t launch_extract(int mode, const ExtractArgs &a, int grid, cudaStream_t st);
 // The partition (kc_part.cu): every k-mer of k bases to its bucket's region of
-// a.list, the buckets by root prefix (the word's top 8 bits, the last four
-// bases), or, as string keys (the k bases first-base-high, left aligned), by
-// their first four bases, so that buckets are consecutive ranges of the printed
-// order.
-cudaError_t launch_part(bool by_string, uint32_t k, const ExtractArgs &a, cudaStream_t st);
+// a.list: as words by root prefix (the word's top 8 bits, the last four bases),
+// as string keys (the k bases first-base-high, left aligned) by their first four
+// bases, so that buckets are consecutive ranges of the printed order, or as
+// string keys by sample (bucket = the file's sample - a.sample0, k the file's).
+enum PartBy : int { PART_BY_ROOT = 0, PART_BY_STRING = 1, PART_BY_SAMPLE = 2 };
+cudaError_t launch_part(PartBy by, uint32_t k, const ExtractArgs &a, cudaStream_t st);
 // The same for k = 33..128: string keys of two or four words (offsets and
 // regions count keys).  census: the k-mers of every (bucket_sample_mask + 1)-th
 // tile are counted in a.bucket_hist and a.occ instead.

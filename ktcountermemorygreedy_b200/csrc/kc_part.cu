@@ -70,10 +70,14 @@ __device__ __forceinline__ uint32_t warp_inclusive(uint32_t v, int lane)
 // per 32 k-mers at three blocks per SM, this one 122 at four: 2.4G k-mers of
 // 150-base reads 21.2 -> 13.7 ms, 480M 4.25 -> 2.74, 25M 0.23 -> 0.15.
 //
+// BY: what a bucket is (PartBy).  By sample all k-mers of a tile have one
+// bucket, and their places follow from a scan of the threads' counts.
 // W: k > 16 (words reach into both halves; below, the upper half holds all).
-template <bool STRING, bool W>
+// By sample k differs from tile to tile, and W tells every case apart itself.
+template <int BY, bool W>
 __global__ void __launch_bounds__(PT_THREADS, 4) k_part(ExtractArgs a)
 {
+    constexpr bool STRING = BY != PART_BY_ROOT, SAMPLE = BY == PART_BY_SAMPLE;
     extern __shared__ __align__(128) uint8_t pt_smem[];
     PartSmem &s = *reinterpret_cast<PartSmem *>(pt_smem);
     __shared__ __align__(8) uint64_t mbar;
@@ -103,7 +107,7 @@ __global__ void __launch_bounds__(PT_THREADS, 4) k_part(ExtractArgs a)
     // the file a tile lies in and its first line's number (mod 4 is all that
     // counts) are read a tile ahead; the file's own data when it changes
     uint32_t seg_next = a.tile_seg[a.tile0 + u], seg_cur = 0xFFFFFFFFu;
-    uint32_t line_next = (uint32_t)a.tile_prefix[a.tile0 + u], line_file = 0, k = 0;
+    uint32_t line_next = (uint32_t)a.tile_prefix[a.tile0 + u], line_file = 0, k = 0, sample = 0;
     uint64_t first_tile = 0;
     for (uint32_t iter = 0; u < a.n_tiles; u += gridDim.x, ++iter) {
         const uint64_t t = a.tile0 + u;
@@ -112,6 +116,7 @@ __global__ void __launch_bounds__(PT_THREADS, 4) k_part(ExtractArgs a)
             seg_cur = seg_next;
             first_tile = a.segs[seg_cur].first_tile;
             k = a.segs[seg_cur].k;
+            if (SAMPLE) sample = a.segs[seg_cur].sample - a.sample0;
             line_file = (uint32_t)a.tile_prefix[first_tile];
         }
         const uint32_t line0 = line_next - line_file;
@@ -194,13 +199,20 @@ __global__ void __launch_bounds__(PT_THREADS, 4) k_part(ExtractArgs a)
                 const uint64_t rc0 = ~(pair_reverse(((uint64_t)fh << 32) | fl) << fs) & topmask;
                 uint32_t rh = (uint32_t)(rc0 >> 32), rl = (uint32_t)rc0;
                 // complemented codes at the bits where the roll takes them in
-                const uint64_t nc = (uint64_t)(~cw) << (W ? fs : fs - 32);
+                // (by sample with k <= 16 that is the upper half)
+                const bool upper = SAMPLE && fs >= 32;
+                const uint32_t in_sh = !W || upper ? fs - 32 : fs;
+                const uint64_t nc = (uint64_t)(~cw) << in_sh;
                 const uint32_t nc_hi = (uint32_t)(nc >> 32), nc_lo = (uint32_t)nc;
-                const uint32_t in_mask = 3u << (W ? fs : fs - 32);
+                const uint32_t in_mask = 3u << in_sh;
 #pragma unroll
                 for (uint32_t p = 0; p < PT_CHUNK; ++p) {
                     const uint32_t in = __funnelshift_r(nc_lo, nc_hi, 2 * p) & in_mask;
-                    if (W) {
+                    if (SAMPLE) {
+                        fl = __funnelshift_r(fl, fh, 2);
+                        rh = __funnelshift_l(rl, rh, 2) | (upper ? in : 0u);
+                        rl = (rl << 2) | (upper ? 0u : in);
+                    } else if (W) {
                         fl = __funnelshift_r(fl, fh, 2);
                         rh = __funnelshift_l(rl, rh, 2);
                         rl = (rl << 2) | in;
@@ -210,30 +222,54 @@ __global__ void __launch_bounds__(PT_THREADS, 4) k_part(ExtractArgs a)
                     fh = (fh >> 2) | ((cw << (30 - 2 * p)) & 0xC0000000u);
                     // the canonical word is the smaller one; the string key of
                     // the canonical strand is the complement of the larger one
-                    const uint32_t xh = W ? fh : fh & tm_hi, xl = W ? fl & tm_lo : 0u;
+                    const uint32_t xh = W && !SAMPLE ? fh : fh & tm_hi, xl = W ? fl & tm_lo : 0u;
                     const bool less = W ? (((uint64_t)xh << 32) | xl) < (((uint64_t)rh << 32) | rl) : xh < rh;
                     if (STRING) {
-                        kh[p] = W ? ~(less ? rh : xh) : ~(less ? rh : xh) & tm_hi;
+                        kh[p] = W && !SAMPLE ? ~(less ? rh : xh) : ~(less ? rh : xh) & tm_hi;
                         kl[p] = W ? ~(less ? rl : xl) & tm_lo : 0u;
                     } else {
                         kh[p] = less ? xh : rh;
                         kl[p] = W ? (less ? xl : rl) : 0u;
                     }
                 }
-                if (!all_buckets) {
+                if (!SAMPLE && !all_buckets) {
 #pragma unroll
                     for (uint32_t p = 0; p < PT_CHUNK; ++p) {
                         const uint32_t b = kh[p] >> 24;
                         if (b < blo || b >= bhi) e &= ~(1u << p);
                     }
                 }
+                if (!SAMPLE) {
 #pragma unroll
-                for (uint32_t p = 0; p < PT_CHUNK; ++p) {
-                    uint32_t r = 0;
-                    if ((e >> p) & 1u) r = atomicAdd(&s_hist[kh[p] >> 24], 1u);
-                    if (p & 1) rk[p / 2] |= r << 16;
-                    else rk[p / 2] = r;
+                    for (uint32_t p = 0; p < PT_CHUNK; ++p) {
+                        uint32_t r = 0;
+                        if ((e >> p) & 1u) r = atomicAdd(&s_hist[kh[p] >> 24], 1u);
+                        if (p & 1) rk[p / 2] |= r << 16;
+                        else rk[p / 2] = r;
+                    }
                 }
+            }
+            if (SAMPLE) {
+                const uint32_t own = (uint32_t)__popc(e), inc = warp_inclusive(own, lane);
+                if (lane == 31) s_wbk[warp] = inc;
+                __syncthreads();
+                uint32_t n;
+                uint32_t at = sum_before(s_wbk, warp, n) + inc - own;
+                if (tid == 0) {
+                    const unsigned long long cur = a.bucket_base[sample] + atomicAdd(&a.bucket_cursor[sample], (unsigned long long)n);
+                    const unsigned long long end = a.bucket_end[sample] < a.list_cap ? a.bucket_end[sample] : a.list_cap;
+                    s_ptr[0] = a.list + cur;
+                    s_lim[0] = cur >= end ? 0u : (uint32_t)(end - cur < n ? end - cur : n);
+                }
+#pragma unroll
+                for (uint32_t p = 0; p < PT_CHUNK; ++p)
+                    if ((e >> p) & 1u) s.stage[at++] = ((unsigned long long)kh[p] << 32) | kl[p];
+                __syncthreads();
+                const uint32_t lim = s_lim[0];
+                unsigned long long *out = s_ptr[0];
+                for (uint32_t i = tid; i < lim; i += PT_THREADS) out[i] = s.stage[i];
+                if (r0 + PT_THREADS < n_ch) __syncthreads();
+                continue;
             }
             __syncthreads();
             // bucket starts; the cursor update is in flight while the k-mers
@@ -561,10 +597,10 @@ int part_sms()
     return n > 0 ? n : 148;
 }
 
-template <bool STRING, bool W>
+template <int BY, bool W>
 cudaError_t launch_part_t(const ExtractArgs &a, cudaStream_t st)
 {
-    auto kern = k_part<STRING, W>;
+    auto kern = k_part<BY, W>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PartSmem));
     if (e != cudaSuccess) return e;
     int per_sm = 0;
@@ -594,11 +630,13 @@ cudaError_t launch_part_wide_t(const ExtractArgs &a, cudaStream_t st)
 
 }  // namespace
 
-cudaError_t launch_part(bool by_string, uint32_t k, const ExtractArgs &a, cudaStream_t st)
+cudaError_t launch_part(PartBy by, uint32_t k, const ExtractArgs &a, cudaStream_t st)
 {
     if (!a.n_tiles) return cudaSuccess;
-    if (k > 16) return by_string ? launch_part_t<true, true>(a, st) : launch_part_t<false, true>(a, st);
-    return by_string ? launch_part_t<true, false>(a, st) : launch_part_t<false, false>(a, st);
+    if (by == PART_BY_SAMPLE) return launch_part_t<PART_BY_SAMPLE, true>(a, st);
+    if (k > 16)
+        return by == PART_BY_STRING ? launch_part_t<PART_BY_STRING, true>(a, st) : launch_part_t<PART_BY_ROOT, true>(a, st);
+    return by == PART_BY_STRING ? launch_part_t<PART_BY_STRING, false>(a, st) : launch_part_t<PART_BY_ROOT, false>(a, st);
 }
 
 cudaError_t launch_part_wide(bool census, uint32_t k, const ExtractArgs &a, cudaStream_t st)

@@ -189,3 +189,47 @@ def test_wide_table_full_once_is_cut_and_counted_again(counter):
     for k in (31, 63, 127):
         check = _check_wide if k > 32 else lambda c, f, kk, **kw: _check(c, f[0], kk, **kw)
         check(counter, files, k, fault_inject=kc.INJECT_TABLE_FULL_ONCE)
+
+
+def _check_batch(counter, samples, ks, **kw):
+    fqs = [_fastq(s) for s in samples]
+    rs = counter.count_batch([[f] for f in fqs], ks, count_max=U32, hist_max=9000, **kw)
+    for f, k, r in zip(fqs, ks, rs):
+        all_k, all_c = O.exact_records([f], k, U32)
+        m = all_c >= kw.get("min_count", 1)
+        assert np.array_equal(r.keys, all_k[m]) and np.array_equal(r.counts, all_c[m])
+        assert r.hist.tolist() == O.histogram(all_c, 1, 9000).tolist()
+        assert r.distinct == len(all_k) and r.occurrences == int(all_c.sum(dtype=np.uint64))
+    return rs
+
+
+@pytest.mark.parametrize("min_count", [1, 2])
+@pytest.mark.parametrize("n", [1, 2, 255, 256, 257])
+def test_batch_of_samples(counter, n, min_count):
+    """Samples as buckets: every k, up to and beyond the samples of one pass,
+    empty samples, samples without a window of k bases, several tiles long,
+    and k-mers with more occurrences than the dense histogram holds (the list
+    then carries the sample) in the first and the last sample."""
+    rnd = random.Random(n)
+    g = "".join(rnd.choice("ACGT") for _ in range(4000))
+    samples = []
+    for i in range(n):
+        reads = [g[j:j + 120] for j in (rnd.randrange(len(g) - 120) for _ in range(rnd.choice((0, 1, 5, 200))))]
+        samples.append(reads + ["ACGTN" * 3, "C" * 40] if i % 5 else reads)
+    samples[0] = samples[0] + ["A" * 5000, "T" * 300]
+    samples[-1] = samples[-1] + ["AC" * 2500]
+    rs = _check_batch(counter, samples, [1 + (7 * i + n) % 32 for i in range(n)], min_count=min_count)
+    assert all(r.smem_passes == 1 and r.smem_fallbacks == 0 for r in rs)
+
+
+@pytest.mark.parametrize("prefix,fallback", [(3, False), (7, False), (11, True)])
+def test_batch_sample_of_one_prefix(counter, prefix, fallback):
+    """One sample's k-mers share their first bases: sub-buckets and rounds tell
+    at most 9 bases apart, so 11 leave one range of all k-mers, and the whole
+    batch is counted in global-memory tables."""
+    rnd = random.Random(prefix)
+    p = "AC" + "".join(rnd.choice("ACGT") for _ in range(prefix - 2))
+    skew = list({p + "".join(rnd.choice("ACGT") for _ in range(30 - prefix)) + "A" for _ in range(60_000)})
+    plain = ["".join(rnd.choice("ACGT") for _ in range(150)) for _ in range(300)]
+    rs = _check_batch(counter, [plain, skew + skew[:999], plain[:50]], [21, 31, 32])
+    assert all((r.smem_fallbacks > 0) == fallback and r.smem_passes == (0 if fallback else 1) for r in rs)
