@@ -164,6 +164,12 @@ bool is_gzip(const kc_buffer &b);
 uint64_t gzip_size_hint(const kc_buffer &b);
 std::vector<kc_buffer> inflate_inputs(const std::vector<kc_buffer> &files, std::vector<PinnedBlock> &hold);
 
+// Copies of a caller's arrays.  Pageable memory of some size goes through pinned
+// chunks filled or emptied by several threads; both return when done with the
+// host's side (copy_in: the device's too).
+void copy_in(void *dev, const void *host, size_t bytes, cudaStream_t st);    // throws KcError
+void copy_out(void *host, const void *dev, size_t bytes, cudaStream_t st);   // throws KcError
+
 // (key, count) records of one job in a pinned block; a key is `words`
 // 64-bit words (kmer<N>, N = 1, 2 or 4).
 struct HostRecords {

@@ -34,13 +34,13 @@ int merge_wide(const uint64_t *high_keys, const uint32_t *high_counts, uint64_t 
     if (n_high) {
         unsigned long long *hk = ds.n<unsigned long long>(n_high * nw);
         uint32_t *hc = ds.n<uint32_t>(n_high);
-        CK(cudaMemcpyAsync(hk, high_keys, n_high * nw * 8, cudaMemcpyHostToDevice, st));
-        CK(cudaMemcpyAsync(hc, high_counts, n_high * 4, cudaMemcpyHostToDevice, st));
+        copy_in(hk, high_keys, n_high * nw * 8, st);
+        copy_in(hc, high_counts, n_high * 4, st);
         CK(launch_wide_insert_pairs(k, hk, hc, 0, n_high, t, mp, counters, st));
     }
     if (n_low) {
         unsigned long long *lk = ds.n<unsigned long long>(n_low * nw);
-        CK(cudaMemcpyAsync(lk, low_keys, n_low * nw * 8, cudaMemcpyHostToDevice, st));
+        copy_in(lk, low_keys, n_low * nw * 8, st);
         CK(launch_wide_insert_pairs(k, lk, nullptr, 1, n_low, t, mp, counters, st));
     }
     unsigned long long *dh = ds.n<unsigned long long>(HIST_BINS);
@@ -71,8 +71,8 @@ int merge_wide(const uint64_t *high_keys, const uint32_t *high_counts, uint64_t 
     if (n_ovf) CK(cudaMemcpyAsync(oh.data(), ovf, n_ovf * 4, cudaMemcpyDeviceToHost, st));
     const uint64_t n_copy = std::min(kept, out_cap);
     if (n_copy) {
-        CK(cudaMemcpyAsync(out_keys, sk, n_copy * nw * 8, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(out_counts, sc, n_copy * 4, cudaMemcpyDeviceToHost, st));
+        copy_out(out_keys, sk, n_copy * nw * 8, st);
+        copy_out(out_counts, sc, n_copy * 4, st);
     }
     CK(cudaStreamSynchronize(st));
     *n_out = kept;
@@ -122,8 +122,8 @@ extern "C" int kc_merge_records(const uint64_t *high_keys, const uint32_t *high_
         unsigned long long *hk = ds.n<unsigned long long>(std::max<uint64_t>(n_high, 1));
         uint32_t *hc = ds.n<uint32_t>(std::max<uint64_t>(n_high, 1));
         if (n_high) {
-            CK(cudaMemcpyAsync(hk, high_keys, n_high * 8, cudaMemcpyHostToDevice, st));
-            CK(cudaMemcpyAsync(hc, high_counts, n_high * 4, cudaMemcpyHostToDevice, st));
+            copy_in(hk, high_keys, n_high * 8, st);
+            copy_in(hc, high_counts, n_high * 4, st);
             CK(launch_insert_pairs(hk, hc, n_high, tr, mp, counters, st));
         }
         const uint64_t rec_cap = std::max<uint64_t>(n_high + n_low, 1);
@@ -135,7 +135,7 @@ extern "C" int kc_merge_records(const uint64_t *high_keys, const uint32_t *high_
         CK(cudaMemsetAsync(dh, 0, HIST_BINS * 8, st));
         if (n_low) {
             unsigned long long *lk = ds.n<unsigned long long>(n_low);
-            CK(cudaMemcpyAsync(lk, low_keys, n_low * 8, cudaMemcpyHostToDevice, st));
+            copy_in(lk, low_keys, n_low * 8, st);
             CK(launch_merge_low(lk, n_low, tr, mp, min_count, max_count, rk, rc, rec_cap, counters, st));
         }
         CK(launch_compact(tr, cap, count_max, min_count, max_count, rk, rc, rec_cap, dh, ovf, ovf_cap, counters, st));
@@ -156,8 +156,8 @@ extern "C" int kc_merge_records(const uint64_t *high_keys, const uint32_t *high_
         if (n_ovf) CK(cudaMemcpyAsync(oh.data(), ovf, n_ovf * 4, cudaMemcpyDeviceToHost, st));
         const uint64_t n_copy = std::min(n_rec, out_cap);
         if (n_copy) {
-            CK(cudaMemcpyAsync(out_keys, rk, n_copy * 8, cudaMemcpyDeviceToHost, st));
-            CK(cudaMemcpyAsync(out_counts, rc, n_copy * 4, cudaMemcpyDeviceToHost, st));
+            copy_out(out_keys, rk, n_copy * 8, st);
+            copy_out(out_counts, rc, n_copy * 4, st);
         }
         unsigned long long sort_flags = 0;
         CK(cudaMemcpyAsync(&sort_flags, counters + C_FLAGS, 8, cudaMemcpyDeviceToHost, st));
