@@ -124,18 +124,22 @@ constexpr uint32_t SLOT_CLAIMED = 1u << 31, SLOT_PUBLISHED = 1u << 30, SLOT_COUN
 // Counts one sub-bucket per block at a time.  The keys are inserted into an
 // open-addressing table in shared memory (a slot only changes from empty to a
 // key, by CAS; no barrier between tiles): every key looks at its home slot,
-// where most are found and counted; the others wait in the warp's queue until
-// there are 32 of them, so that a probe step (claim, count, or on to the next
-// slot and back into the queue) has all lanes busy.  (Each lane stepping its
-// own keys to the end left 16 of 32 lanes active and 198 warp instructions per
-// 32 keys; with the queue 23 and 172.  A ring that refilled each idle lane at
-// every step took 248: more bookkeeping than probing.)  Bound by instruction
-// issue (72%) and shared-memory wavefronts (63%): 2.4G k-mers of the 20M-read
-// job 18.5 -> 15.6 ms, 480M k-mers with every record kept 3.8 -> 3.15, 25M
-// mostly distinct ones 0.92 -> 0.49.  Then one sweep writes the kept
-// records to the front of the sub-bucket's place in the record arrays,
-// adds every count to the histogram and empties the table for the next
-// sub-bucket.  A table that fills up (more distinct k-mers than it holds) is
+// where most are found or find their place; the others wait in the warp's queue
+// until there are 32 of them, so that a probe step (claim, count, or on to the
+// next slot and back into the queue) has all lanes busy.  (Each lane stepping
+// its own keys to the end left 16 of 32 lanes active and 198 warp instructions
+// per 32 keys; with the queue 23 and 172.  A ring that refilled each idle lane
+// at every step took 248: more bookkeeping than probing.)  A home slot found
+// empty is claimed at once when most keys are distinct (25M k-mers 0.34 -> 0.32
+// ms; no difference at 3.3 occurrences each).  Then one sweep lists the used
+// slots and takes them 32 at a time, so that no lane handles an empty one (two
+// slots to a lane, a third of them used, the sweep was a fourth of all
+// instructions: 2.4G k-mers of the 20M-read job 15.8 -> 14.5 ms, 480M k-mers with
+// every record kept 3.21 -> 2.95): it writes the kept records to the front of the
+// sub-bucket's place in the record arrays, adds every count to the histogram and
+// empties the table for the next sub-bucket.  Bound by instruction issue (72%)
+// and shared-memory wavefronts (60%).
+// A table that fills up (more distinct k-mers than it holds) is
 // emptied and the sub-bucket counted in rounds over halves of its key range
 // (quarters, ... at most CP_MAX_ROUNDS), each round reading the keys again
 // from L2; a round's records lie after the earlier rounds' ones, and are a
@@ -190,10 +194,12 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
     __syncthreads();
     // the first tile of keys of a sub-bucket
     KeyN<N> kn[PER_THREAD];
+    constexpr uint32_t STEP = N == 1 ? 32 : THREADS;
+    const uint32_t first = N == 1 ? (uint32_t)(tid >> 5) * (32 * PER_THREAD) + (uint32_t)lane : (uint32_t)tid;
     auto load_first = [&](unsigned long long off, uint32_t cnt) {
 #pragma unroll
         for (uint32_t r = 0; r < PER_THREAD; ++r)
-            if (r * THREADS + tid < cnt) kn[r] = load_key<N>(a.keys, off + r * THREADS + tid, LoadStream());
+            if (first + STEP * r < cnt) kn[r] = load_key<N>(a.keys, off + first + STEP * r, LoadStream());
     };
     uint32_t sub = s_next, n = 0;
     unsigned long long base = 0;
@@ -305,20 +311,20 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
                 qn += (uint32_t)__popc(w);
                 __syncwarp();
             };
-            for (uint32_t t0 = 0; t0 < n; t0 += TILE_KEYS) {
+            for (uint32_t t0 = first; t0 - (N == 1 ? (uint32_t)lane : (uint32_t)tid) < n; t0 += TILE_KEYS) {
                 KeyN<N> k[PER_THREAD];
                 bool in[PER_THREAD];
 #pragma unroll
-                for (uint32_t r = 0; r < PER_THREAD; ++r) in[r] = t0 + r * THREADS + tid < n;
+                for (uint32_t r = 0; r < PER_THREAD; ++r) in[r] = t0 + STEP * r < n;
                 if (reread) {
 #pragma unroll
                     for (uint32_t r = 0; r < PER_THREAD; ++r)
-                        if (in[r]) k[r] = load_key<N>(a.keys, base + t0 + r * THREADS + tid, LoadL2());
+                        if (in[r]) k[r] = load_key<N>(a.keys, base + t0 + STEP * r, LoadL2());
                 } else {
 #pragma unroll
                     for (uint32_t r = 0; r < PER_THREAD; ++r) {
                         k[r] = kn[r];
-                        const uint32_t i = t0 + TILE_KEYS + r * THREADS + tid;
+                        const uint32_t i = t0 + TILE_KEYS + STEP * r;
                         if (i < n) kn[r] = load_key<N>(a.keys, base + i, LoadStream());
                     }
                 }
@@ -330,17 +336,28 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
                 // the home slots: most keys are there already and only counted
                 uint32_t slot[PER_THREAD];
                 bool hit[PER_THREAD];
+                unsigned long long cur[PER_THREAD];
 #pragma unroll
                 for (uint32_t r = 0; r < PER_THREAD; ++r) {
                     slot[r] = mix_of<N>(k[r]) >> hsh;
                     if constexpr (N == 1) {
-                        hit[r] = *(volatile unsigned long long *)&s_tk[slot[r]] == k[r].w[0];
+                        cur[r] = *(volatile unsigned long long *)&s_tk[slot[r]];
                     } else {
                         hit[r] = false;
                         if (in[r] && (*(volatile uint32_t *)&s_tc[slot[r]] & SLOT_PUBLISHED)) {
                             __threadfence_block();
                             hit[r] = load_key<N>(s_tk, slot[r], LoadPlain()) == k[r];
                         }
+                    }
+                }
+                if constexpr (N == 1) {
+#pragma unroll
+                    for (uint32_t r = 0; r < PER_THREAD; ++r) {
+                        if (in[r] && cur[r] == EMPTY_KEY) {
+                            cur[r] = atomicCAS(&s_tk[slot[r]], EMPTY_KEY, k[r].w[0]);
+                            if (cur[r] == EMPTY_KEY) cur[r] = k[r].w[0];
+                        }
+                        hit[r] = cur[r] == k[r].w[0];
                     }
                 }
 #pragma unroll
@@ -351,7 +368,7 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
                     if (wait) {
                         const uint32_t at = qn + (uint32_t)__popc(w & lt);
                         store_key<N>(q_key, at, k[r]);
-                        q_slot[at] = (uint16_t)slot[r];
+                        q_slot[at] = (uint16_t)(N == 1 ? (slot[r] + (mix_of<N>(k[r]) >> 3 | 1u)) & smask : slot[r]);
                     }
                     qn += (uint32_t)__popc(w);
                     // below 32 again before the next keys come (the queue holds 64)
@@ -386,67 +403,69 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
             }
             // the next sub-bucket's first keys arrive during the sweep
             if (rd + 1 == rounds) load_first(s_next_off, s_next < a.n_sub ? s_next_n : 0u);
-            // the sweep: records out, histogram, table emptied; two slots a thread
+            // the sweep: the used slots are listed (in the queue's memory, free
+            // now), four per lane at a time, and taken 32 at once: records out,
+            // histogram, slots emptied
             const unsigned long long out = base + off;
             const uint32_t cmax = cfg.count_max, keep_lo = cfg.min_count, keep_hi = cfg.max_count;
-            for (uint32_t i0 = 0; i0 <= smask; i0 += 2 * THREADS) {
-                const uint32_t i = i0 + 2 * tid;
-                uint32_t raw[2] = {0, 0}, c[2] = {0, 0};
-                bool keep[2] = {false, false};
-                KeyN<N> key[2];
-                bool used = false;
-                if constexpr (N == 1) {
-                    key[0].w[0] = key[1].w[0] = EMPTY_KEY;
-                    if (i <= smask) {
-                        const ulonglong2 kk = *reinterpret_cast<const ulonglong2 *>(&s_tk[i]);
-                        key[0].w[0] = kk.x;
-                        key[1].w[0] = kk.y;
+            uint16_t *used = reinterpret_cast<uint16_t *>(q_key);
+            static_assert(CP_QUEUE * 8 * N / 2 >= 128 + 31, "a list of the slots of one step and the rest of the last");
+            uint32_t un = 0;
+            auto take_used = [&](uint32_t m) {
+                __syncwarp();
+                un -= m;
+                uint32_t i = 0, c = 0;
+                bool keep = false;
+                KeyN<N> key;
+                if (lane < (int)m) {
+                    i = used[un + lane];
+                    const uint32_t raw = N > 1 ? s_tc[i] & SLOT_COUNT : s_tc[i];
+                    if constexpr (N == 1) key = load_key<N>(s_tk, i, LoadPlain());
+                    s_tc[i] = 0;
+                    if constexpr (N == 1) s_tk[i] = EMPTY_KEY;
+                    ++n_distinct;
+                    n_once += raw == 1;
+                    c = raw < cmax ? raw : cmax;
+                    if (c == 1) ++n_one;   // most k-mers of many inputs: one shared bin would serialize
+                    else if (c < CP_HIST) atomicAdd(&s_hist[c], 1u);
+                    else if (c < a.hist_bins) atomicAdd(&a.hist[(unsigned long long)s_group * a.hist_bins + c], 1ull);
+                    else {
+                        const unsigned long long q = atomicAdd(&a.counters[C_OVF_LEN], 1ull);
+                        if (q >= a.ovf_cap) atomicOr(&a.counters[C_FLAGS], ERR_HIST_OVERFLOW_FULL);
+                        else if (a.ovf64) a.ovf64[q] = ((unsigned long long)s_group << 32) | c;
+                        else a.ovf[q] = c;
                     }
-                    used = key[0].w[0] != EMPTY_KEY || key[1].w[0] != EMPTY_KEY;
+                    keep = c >= keep_lo && c <= keep_hi;
                 }
-                if (N == 1 ? used : i <= smask) {
-                    const uint2 r2 = *reinterpret_cast<const uint2 *>(&s_tc[i]);
-                    raw[0] = r2.x;
-                    raw[1] = r2.y;
-                }
-                if (raw[0] | raw[1]) {
-                    *reinterpret_cast<uint2 *>(&s_tc[i]) = make_uint2(0u, 0u);
-                    if constexpr (N == 1)
-                        *reinterpret_cast<ulonglong2 *>(&s_tk[i]) = make_ulonglong2(EMPTY_KEY, EMPTY_KEY);
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) {
-                        if (N > 1) raw[j] &= SLOT_COUNT;
-                        if (raw[j] == 0) continue;
-                        ++n_distinct;
-                        n_once += raw[j] == 1;
-                        c[j] = raw[j] < cmax ? raw[j] : cmax;
-                        if (c[j] == 1) ++n_one;   // most k-mers of many inputs: one shared bin would serialize
-                        else if (c[j] < CP_HIST) atomicAdd(&s_hist[c[j]], 1u);
-                        else if (c[j] < a.hist_bins) atomicAdd(&a.hist[(unsigned long long)s_group * a.hist_bins + c[j]], 1ull);
-                        else {
-                            const unsigned long long q = atomicAdd(&a.counters[C_OVF_LEN], 1ull);
-                            if (q >= a.ovf_cap) atomicOr(&a.counters[C_FLAGS], ERR_HIST_OVERFLOW_FULL);
-                            else if (a.ovf64) a.ovf64[q] = ((unsigned long long)s_group << 32) | c[j];
-                            else a.ovf[q] = c[j];
-                        }
-                        keep[j] = c[j] >= keep_lo && c[j] <= keep_hi;
-                    }
-                }
-                const uint32_t b0 = __ballot_sync(FULLW, keep[0]), b1 = __ballot_sync(FULLW, keep[1]);
-                if (b0 | b1) {
+                const uint32_t b = __ballot_sync(FULLW, keep);
+                if (b) {
                     uint32_t w = 0;
-                    if (lane == 0) w = atomicAdd(&s_out, (uint32_t)(__popc(b0) + __popc(b1)));
+                    if (lane == 0) w = atomicAdd(&s_out, (uint32_t)__popc(b));
                     w = __shfl_sync(FULLW, w, 0);
-                    const uint32_t at[2] = {w + (uint32_t)__popc(b0 & lt), w + (uint32_t)(__popc(b0) + __popc(b1 & lt))};
-#pragma unroll
-                    for (int j = 0; j < 2; ++j)
-                        if (keep[j]) {
-                            if (N > 1) key[j] = load_key<N>(s_tk, i + j, LoadPlain());
-                            store_key<N>(a.rec_keys, out + at[j], key[j]);
-                            a.rec_counts[out + at[j]] = c[j];
-                        }
+                    if (keep) {
+                        const unsigned long long at = out + w + (uint32_t)__popc(b & lt);
+                        if constexpr (N > 1) key = load_key<N>(s_tk, i, LoadPlain());
+                        store_key<N>(a.rec_keys, at, key);
+                        a.rec_counts[at] = c;
+                    }
                 }
+                __syncwarp();
+            };
+            for (uint32_t i0 = 0; i0 <= smask; i0 += 4 * THREADS) {
+                const uint32_t i = i0 + 4 * tid;
+                uint4 c4 = make_uint4(0, 0, 0, 0);
+                if (i <= smask) c4 = *reinterpret_cast<const uint4 *>(&s_tc[i]);
+                const uint32_t b0 = __ballot_sync(FULLW, c4.x != 0), b1 = __ballot_sync(FULLW, c4.y != 0);
+                const uint32_t b2 = __ballot_sync(FULLW, c4.z != 0), b3 = __ballot_sync(FULLW, c4.w != 0);
+                uint32_t at = un + (uint32_t)(__popc(b0 & lt) + __popc(b1 & lt) + __popc(b2 & lt) + __popc(b3 & lt));
+                if (c4.x) used[at++] = (uint16_t)i;
+                if (c4.y) used[at++] = (uint16_t)(i + 1);
+                if (c4.z) used[at++] = (uint16_t)(i + 2);
+                if (c4.w) used[at] = (uint16_t)(i + 3);
+                un += (uint32_t)(__popc(b0) + __popc(b1) + __popc(b2) + __popc(b3));
+                while (un >= 32) take_used(32);
             }
+            if (un) take_used(un);
             __syncthreads();
             const uint32_t len = s_out;
             __syncthreads();
