@@ -68,8 +68,8 @@ extern "C" {
 #define KC_INJECT_TABLE_FULL_ONCE 2u /* the first counting attempt reports its table full (plain jobs) or a
                                         sub-bucket table overflowed (Bloom jobs, shared-memory path): the
                                         job regrows / splits and counts again, with exact results */
-#define KC_INJECT_TABLE_FULL 4u      /* every counting attempt reports its table full: KC_ERR_DEVICE after
-                                        the retries (plain jobs of one table) */
+#define KC_INJECT_TABLE_FULL 4u      /* every counting attempt reports its table full, sub-bucket tables
+                                        first: KC_ERR_DEVICE after the retries (plain jobs of one table) */
 #define KC_INJECT_NOMEM 8u           /* the job's first device allocation fails as a failed cudaMalloc
                                         does: the job ends KC_ERR_NOMEM, the handle stays usable */
 
@@ -158,8 +158,8 @@ typedef struct {
     double phase_ms[KC_STAGES];
     uint64_t phase_launches[KC_STAGES];   /* kernel launches per stage */
     uint64_t low_len;             /* Bloom mode: FIRST occurrences */
-    uint64_t high_len;            /* occurrences counted in bucket or sub-bucket tables (Bloom mode: the
-                                     non-FIRST ones; large plain jobs: all); 0 for one table */
+    uint64_t high_len;            /* Bloom mode: the non-FIRST occurrences; large plain jobs: all; 0 for plain
+                                     jobs whose k-mers one table of at most 4M slots would hold */
     uint64_t input_bytes;         /* FASTQ bytes of the job */
     uint64_t n_records_total;     /* records on the device (also when keep_records = 0) */
     uint32_t passes;              /* counting passes over ranges of root prefixes (1: the whole job at once) */
@@ -184,7 +184,7 @@ typedef struct {
                                      default 1.6 */
     uint64_t sort_group_records;  /* records sorted together (kept in L2) by a batch's segmented sort;
                                      default 4M */
-    uint64_t bloom_smem;          /* Bloom jobs and plain jobs from 4 MiB of FASTQ on: 1 partitions the k-mers by
+    uint64_t bloom_smem;          /* 1 partitions the k-mers (of a job or a batch's samples) by
                                      their first bases and counts each sub-bucket in a shared-memory table
                                      (no filter: a FIRST occurrence is the one that makes its k-mer's table
                                      entry), 2 uses global-memory filters and tables; default 1 */

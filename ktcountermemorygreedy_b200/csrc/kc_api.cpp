@@ -8,14 +8,14 @@
 //
 // One job is the reference's counter run followed by its precise tools:
 //   upload (tile-aligned, zero padded)  -> newline census -> tile line numbers
-//   -> Bloom jobs and plain ones of some size (the prefix path): a sampled
-//      census -> scatter by the first bases, twice -> every sub-bucket counted
-//      in a shared-memory table, its records sorted on their own
-//      small plain jobs: SCAN (occurrences, HyperLogLog) -> INSERT into a table
-//      sized from the estimate -> compaction + histogram -> radix sort
-//      global-memory tables (kc_tuning.bloom_smem 2): SCAN with the Bloom
-//      pre-pass statistics -> root-prefix buckets -> the reference's filter
-//      -> insert, merge, compaction + histogram -> radix sort
+//   -> the prefix path: a census of the first four bases (sampled on larger
+//      inputs) -> scatter by them, then by the next ones -> every sub-bucket
+//      counted in a shared-memory table, its records sorted on their own
+//      global-memory tables (kc_tuning.bloom_smem 2, and k-mers that fit no
+//      sub-bucket table): SCAN (occurrences, HyperLogLog) -> INSERT into a table
+//      sized from the estimate -> compaction + histogram -> radix sort; large
+//      jobs by root-prefix buckets, Bloom jobs with the pre-pass statistics and
+//      the reference's filter before the insert
 //   -> queries -> host.
 // All device memory is stream-ordered (cudaMallocAsync on the worker stream)
 // from a pool that keeps freed memory for the next job.
@@ -92,9 +92,6 @@ kc_tuning default_tuning()
 // uploaded in chunks that the census, SCAN and partition follow.
 constexpr uint64_t STREAMED_UPLOAD_MIN_BYTES = 512ull << 20;
 
-// The prefix path (kc_tuning.bloom_smem = 1) takes every Bloom job and the
-// plain jobs of at least this many FASTQ bytes; smaller ones keep one table.
-constexpr uint64_t PREFIX_PATH_MIN_BYTES = 4ull << 20;
 
 // Most k-mers per sub-bucket of the prefix path, for its 8192-slot tables:
 // sub-buckets have half to all of it.
@@ -411,6 +408,7 @@ struct PrefixPass {
     std::vector<SubCfg> sc;             // per bucket: k, group and count limits
     uint32_t n_groups = 1, hist_bins = 0;
     unsigned long long *hist = nullptr; // hist_bins per group, added to
+    bool hist_zero = false;             // all zero so far
     uint32_t *ovf = nullptr;
     unsigned long long *ovf64 = nullptr;
     uint64_t ovf_cap = 0;
@@ -437,6 +435,7 @@ uint64_t prefix_list_cap(uint64_t n) { return n + n / 4 + 65536; }
 
 void count_by_prefix(PrefixPass &pp, DevScope &ds, HostStage &hs, PhaseClock &clk, const kc_tuning &tn, cudaStream_t st)
 {
+    if (pp.fault_inject & KC_INJECT_TABLE_FULL) throw SubTablesFull{};   // as if no table held its keys
     const uint32_t lo = pp.lo, hi = pp.hi, N = pp.words;
     unsigned long long *counters = pp.counters;
     const uint32_t shape = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(tn.count_shape, 4));
@@ -481,40 +480,44 @@ void count_by_prefix(PrefixPass &pp, DevScope &ds, HostStage &hs, PhaseClock &cl
             br.begin[b] = pp.cfg[b].key_base;
             br.len[b] = pp.cfg[b].key_len;
         }
-        SubCfg *d_sc = ds.n<SubCfg>(N_BUCKETS);
-        uint8_t *d_sb = ds.n<uint8_t>(n_sub);
-        uint32_t *sub_count = ds.n<uint32_t>(n_sub);
         uint32_t *sub_len = ds.n<uint32_t>(n_sub);
         unsigned long long *sub_off = ds.n<unsigned long long>(n_sub);
         unsigned long long *sub_cur = ds.n<unsigned long long>(n_sub);
         unsigned long long *sub_tmp = ds.n<unsigned long long>(scan_tmp_words(n_sub));
         unsigned int *sub_next = ds.n<unsigned int>(1);
-        uint32_t *bucket_ovf = ds.n<uint32_t>(N_BUCKETS);
+        // what starts at zero, cleared at once
+        const size_t zero_bytes = 3ull * pp.n_groups * 8 + N_BUCKETS * 4ull + n_sub * 4ull;
+        unsigned long long *totals = static_cast<unsigned long long *>(ds.get(zero_bytes));
+        uint32_t *bucket_ovf = reinterpret_cast<uint32_t *>(totals + 3 * pp.n_groups);
+        uint32_t *sub_count = bucket_ovf + N_BUCKETS;
+        // an attempt that fails leaves counts behind: they go to an array of
+        // their own unless nothing else is in the histogram
         const size_t hist_n = (size_t)pp.n_groups * pp.hist_bins;
-        unsigned long long *hist_sub = ds.n<unsigned long long>(hist_n);
-        unsigned long long *totals = ds.n<unsigned long long>(3 * pp.n_groups);
+        unsigned long long *hist_sub = pp.hist_zero ? pp.hist : ds.n<unsigned long long>(hist_n);
         const uint32_t unit_cap = 2 * n_sub + 4096;
         SubUnit *units = ds.n<SubUnit>((size_t)UNIT_CLASSES * unit_cap);
         const bool sampled = !exact_regions && !batch && pp.n_keys >= tn.sampled_region_keys;
         const uint32_t stride = sampled ? SUB_REGION_SAMPLE : 1;
-        // each bucket-major launch gets its 256 ranges, not a list of items
-        auto upload_ranges = [&](uint32_t &n_items, uint64_t item_keys) {
-            n_items = fill_item_starts_n(br, item_keys);
-            BucketRanges *d = ds.n<BucketRanges>(1);
-            CK(cudaMemcpyAsync(d, hs.up(&br, 1), sizeof(BucketRanges), cudaMemcpyHostToDevice, st));
-            return d;
-        };
-        uint32_t n_items = 0, n_sp_items = 0;
-        BucketRanges *d_br = upload_ranges(n_items, SUB_COUNT_KEYS * stride);
-        BucketRanges *d_bs = upload_ranges(n_sp_items, sub_scatter_item_keys(max_sub, N));
-        CK(cudaMemcpyAsync(d_sc, hs.up(pp.sc.data(), N_BUCKETS), N_BUCKETS * sizeof(SubCfg), cudaMemcpyHostToDevice, st));
-        CK(cudaMemcpyAsync(d_sb, hs.up(sb.data(), n_sub), n_sub, cudaMemcpyHostToDevice, st));
-        CK(cudaMemsetAsync(sub_count, 0, n_sub * 4ull, st));
-        CK(cudaMemsetAsync(bucket_ovf, 0, N_BUCKETS * 4, st));
-        CK(cudaMemsetAsync(hist_sub, 0, hist_n * 8, st));
-        CK(cudaMemsetAsync(totals, 0, 3ull * pp.n_groups * 8, st));
-        CK(cudaMemsetAsync(counters + C_SUB_OVF, 0, 2 * 8, st));   // C_SUB_OVF, C_REGION_OVF
-        CK(cudaMemsetAsync(counters + C_UNITS, 0, UNIT_CLASSES * 8, st));
+        // one upload: the 256 ranges of each bucket-major launch (not lists of
+        // items), the sub-buckets' settings and their buckets
+        constexpr size_t SC_BYTES = N_BUCKETS * sizeof(SubCfg);
+        static_assert(sizeof(BucketRanges) % 8 == 0 && SC_BYTES % 8 == 0, "layout of the upload");
+        const size_t up_bytes = 2 * sizeof(BucketRanges) + SC_BYTES + n_sub;
+        uint8_t *h_up = hs.n<uint8_t>(up_bytes), *d_up = ds.n<uint8_t>(up_bytes);
+        const uint32_t n_items = fill_item_starts_n(br, SUB_COUNT_KEYS * stride);
+        std::memcpy(h_up, &br, sizeof(br));
+        const uint32_t n_sp_items = fill_item_starts_n(br, sub_scatter_item_keys(max_sub, N));
+        std::memcpy(h_up + sizeof(br), &br, sizeof(br));
+        std::memcpy(h_up + 2 * sizeof(br), pp.sc.data(), SC_BYTES);
+        std::memcpy(h_up + 2 * sizeof(br) + SC_BYTES, sb.data(), n_sub);
+        CK(cudaMemcpyAsync(d_up, h_up, up_bytes, cudaMemcpyHostToDevice, st));
+        const BucketRanges *d_br = reinterpret_cast<const BucketRanges *>(d_up), *d_bs = d_br + 1;
+        const SubCfg *d_sc = reinterpret_cast<const SubCfg *>(d_br + 2);
+        const uint8_t *d_sb = reinterpret_cast<const uint8_t *>(d_sc + N_BUCKETS);
+        CK(cudaMemsetAsync(totals, 0, zero_bytes, st));
+        if (!pp.hist_zero) CK(cudaMemsetAsync(hist_sub, 0, hist_n * 8, st));
+        static_assert(C_REGION_OVF == C_SUB_OVF + 1 && C_UNITS > C_REGION_OVF, "cleared together");
+        CK(cudaMemsetAsync(counters + C_SUB_OVF, 0, (C_UNITS + UNIT_CLASSES - C_SUB_OVF) * 8, st));
         unsigned long long *sub_end = nullptr;
         clk.begin(9);
         if (sampled) {
@@ -569,6 +572,7 @@ void count_by_prefix(PrefixPass &pp, DevScope &ds, HostStage &hs, PhaseClock &cl
             std::vector<uint32_t> bo(N_BUCKETS);
             CK(cudaMemcpyAsync(bo.data(), bucket_ovf, N_BUCKETS * 4, cudaMemcpyDeviceToHost, st));
             CK(cudaMemcpyAsync(counters + C_OVF_LEN, ovf_len_saved, 8, cudaMemcpyDeviceToDevice, st));
+            if (pp.hist_zero) CK(cudaMemsetAsync(pp.hist, 0, hist_n * 8, st));
             CK(cudaStreamSynchronize(st));
             ds.rewind(m0);
             if (cs.v[C_REGION_OVF]) {
@@ -598,7 +602,7 @@ void count_by_prefix(PrefixPass &pp, DevScope &ds, HostStage &hs, PhaseClock &cl
         pp.n_rec = 0;
         for (uint32_t g = 0; g < pp.n_groups; ++g) pp.n_rec += pp.totals[3 * g + 2];
         clk.begin(6);
-        CK(launch_add_u64(pp.hist, hist_sub, hist_n, st));
+        if (!pp.hist_zero) CK(launch_add_u64(pp.hist, hist_sub, hist_n, st));
         pp.rec_keys = ds.n<unsigned long long>(std::max<uint64_t>(pp.n_rec, 1) * N);
         pp.rec_counts = ds.n<uint32_t>(std::max<uint64_t>(pp.n_rec, 1));
         // where each sub-bucket's records go; sub_cur is free again
@@ -661,14 +665,15 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
     // they go)
     ChunkedUpload cu;
     bool streamed = false;
-    // counted by printed-order prefix in shared memory
-    const auto by_prefix = [&](uint64_t bytes) {
-        return tn.bloom_smem == 1 && !global_tables && (P.bloom || bytes >= PREFIX_PATH_MIN_BYTES);
-    };
+    // counted by printed-order prefix in shared memory, also the smallest jobs:
+    // 30K distinct k-mers 0.70 -> 0.44 ms against one global-memory table (whose
+    // insert of 8 tiles takes 0.18 and whose eight sort passes 0.16), 200 reads
+    // 0.74 -> 0.57; 63-base k-mers of 200 reads 0.92 -> 0.62
+    const bool prefix = tn.bloom_smem == 1 && !global_tables;
     if (!in) {
         const std::vector<kc_buffer> files = inflate_inputs(job.files, inflated);
         streamed = !exact_census && files.size() == 1 && files[0].size >= STREAMED_UPLOAD_MIN_BYTES &&
-                   (P.bloom || by_prefix(files[0].size));
+                   (P.bloom || prefix);
         build_input(local, files.data(), (uint32_t)files.size(), st, &ds, tile_seg_host, nullptr,
                     streamed ? &cu : nullptr);
         in = &local;
@@ -676,7 +681,6 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
             fprintf(stderr, "[kc trace] job upload of %zu files enqueued after %.3f ms\n", job.files.size(),
                     now_ms() - th_start);
     }
-    const bool prefix = by_prefix(in->total_bytes);
     // small uploads and read-backs through pinned staging: a pageable copy
     // would hold the host (and, behind a streamed upload, wait for it)
     HostStage hs(st);
@@ -708,8 +712,12 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
     Seg *d_segs = ds.n<Seg>(std::max<uint32_t>(n_seg, 1));
     if (n_seg) CK(cudaMemcpyAsync(d_segs, hs.up(segs.data(), n_seg), n_seg * sizeof(Seg), cudaMemcpyHostToDevice, st));
 
-    unsigned long long *counters = ds.n<unsigned long long>(C_COUNT);
-    CK(cudaMemsetAsync(counters, 0, C_COUNT * 8, st));
+    // the counters, the occurrences and the bucket census: cleared at once and
+    // read back at once
+    constexpr uint32_t CENSUS_WORDS = C_COUNT + 1 + N_BUCKETS;
+    unsigned long long *counters = ds.n<unsigned long long>(CENSUS_WORDS);
+    unsigned long long *occ = counters + C_COUNT, *bucket_hist = occ + 1;
+    CK(cudaMemsetAsync(counters, 0, CENSUS_WORDS * 8, st));
 
     // ---- line numbers of tile starts --------------------------------------
     uint32_t *tile_nl = ds.n<uint32_t>(std::max<uint64_t>(T, 1));
@@ -758,10 +766,9 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
     }
 
     // ---- SCAN pass ---------------------------------------------------------
-    unsigned long long *occ = ds.n<unsigned long long>(1);
+    const bool want_hll = !P.bloom && !prefix;   // (no table, or tables sized from the non-FIRST occurrences)
     uint32_t *hll = ds.n<uint32_t>(HLL_M);
-    CK(cudaMemsetAsync(occ, 0, 8, st));
-    CK(cudaMemsetAsync(hll, 0, HLL_M * 4, st));
+    if (want_hll) CK(cudaMemsetAsync(hll, 0, HLL_M * 4, st));
     ExtractArgs a{};
     a.buf = in->buf;
     a.n_tiles = T;
@@ -774,14 +781,11 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
     a.hll_local = 1;
     uint32_t *prefix_hist = nullptr;
     unsigned long long *qual = nullptr;
-    unsigned long long *bucket_hist = nullptr;
+    a.bucket_hist = bucket_hist;
     clk.begin(1);
     if (P.bloom || prefix) {
-        a.hll = nullptr;   // no table, or tables sized from the non-FIRST occurrences
+        a.hll = nullptr;
         a.census_by_string = prefix;
-        bucket_hist = ds.n<unsigned long long>(N_BUCKETS);
-        CK(cudaMemsetAsync(bucket_hist, 0, N_BUCKETS * 8, st));
-        a.bucket_hist = bucket_hist;
         // the bucket census reads every 8th tile of large inputs; buckets get
         // regions with headroom and an outgrown region triggers an exact redo
         // (every 32nd from 512 MiB on, where no pre-pass statistics are needed)
@@ -823,28 +827,22 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
     } else {
         // plain jobs: an exact root-prefix census beside the distinct
         // estimate, for the partitioned path of large tables
-        bucket_hist = ds.n<unsigned long long>(N_BUCKETS);
-        CK(cudaMemsetAsync(bucket_hist, 0, N_BUCKETS * 8, st));
-        a.bucket_hist = bucket_hist;
         a.bucket_sample_mask = 0;
     }
     CK(launch_extract(MODE_SCAN, a, 0, st));
     clk.end();
     // the SCAN's results (and the bucket census) come back under one sync
-    unsigned long long *p_occ = hs.n<unsigned long long>(1);
+    unsigned long long *p_c0 = hs.n<unsigned long long>(CENSUS_WORDS), *p_occ = p_c0 + C_COUNT, *p_bh = p_occ + 1;
     uint32_t *p_hll = hs.n<uint32_t>(HLL_M);
     uint32_t *p_ph = hs.n<uint32_t>(256);
     unsigned long long *p_qh = hs.n<unsigned long long>(2);
-    unsigned long long *p_bh = hs.n<unsigned long long>(N_BUCKETS);
-    unsigned long long *p_c0 = hs.n<unsigned long long>(C_COUNT);
-    CK(cudaMemcpyAsync(p_occ, occ, 8, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(p_hll, hll, HLL_M * 4, cudaMemcpyDeviceToHost, st));
+    if (want_hll) CK(cudaMemcpyAsync(p_hll, hll, HLL_M * 4, cudaMemcpyDeviceToHost, st));
+    else std::fill(p_hll, p_hll + HLL_M, 0u);
     if (P.bloom && !prefix) {
         CK(cudaMemcpyAsync(p_ph, prefix_hist, 256 * 4, cudaMemcpyDeviceToHost, st));
         CK(cudaMemcpyAsync(p_qh, qual, 16, cudaMemcpyDeviceToHost, st));
     }
-    if (bucket_hist) CK(cudaMemcpyAsync(p_bh, bucket_hist, N_BUCKETS * 8, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(p_c0, counters, C_COUNT * 8, cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(p_c0, counters, CENSUS_WORDS * 8, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     std::vector<uint32_t> hll_h(p_hll, p_hll + HLL_M);
     unsigned long long O = *p_occ;
@@ -874,7 +872,7 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
     uint32_t *ovf = ds.n<uint32_t>(ovf_cap);
     unsigned long long *n_keys = ds.n<unsigned long long>(1);
     CK(cudaMemsetAsync(hist, 0, HIST_BINS * 8, st));
-    unsigned long long low_len = 0, high_len = 0;
+    unsigned long long low_len = 0, high_len = 0, plain_keys = 0;
     uint64_t table_cap = 0;
     // singletons that are no table entry (the global-memory filters' FIRST-only k-mers)
     uint64_t untabled = 0;
@@ -973,9 +971,9 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
         untabled += c2.v[C_LOW_ONLY];
     };
 
-    // a plain job whose table would not fit in L2 takes the partitioned path
-    // too (without the Bloom split): scattered by root prefix, every bucket's
-    // sub-table is filled while it sits in L2
+    // (in global-memory tables:) a plain job whose table would not fit in L2
+    // takes the partitioned path too (without the Bloom split): scattered by root
+    // prefix, every bucket's sub-table is filled while it sits in L2
     const bool plain_part = prefix || (!P.bloom && table_capacity_for(est, tn.table_factor) > PLAIN_PART_MIN_SLOTS);
     if (!P.bloom && !plain_part) {
         TableRef tr{};
@@ -1009,7 +1007,6 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
         // src/NewKmerTree.h:1488-1495): sizes from the SCAN census, one
         // scatter pass, then every bucket's Bloom filter and table slice is
         // processed while it sits in L2
-        if (!bucket_hist) throw KcError{KC_ERR_DEVICE, "partitioned job without a bucket census"};
         const std::vector<unsigned long long> bh(p_bh, p_bh + N_BUCKETS);
         std::vector<unsigned long long> region(N_BUCKETS);
         unsigned long long sampled = 0;
@@ -1090,20 +1087,21 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
                 list = keys;
             }
             BucketCfg *d_cfg_b = ds.n<BucketCfg>(N_BUCKETS);
-            unsigned long long *cursor = ds.n<unsigned long long>(N_BUCKETS);
-            unsigned long long *bbase = ds.n<unsigned long long>(2 * N_BUCKETS);
+            unsigned long long *bbase = ds.n<unsigned long long>(3 * N_BUCKETS);
+            unsigned long long *cursor = bbase + 2 * N_BUCKETS;
             unsigned long long *lh_cnt = ds.n<unsigned long long>(2 * N_BUCKETS);
             uint32_t *hll_high = ds.n<uint32_t>((size_t)N_BUCKETS * BUCKET_HLL_M);
             unsigned int *next_item = ds.n<unsigned int>(1);
-            std::vector<unsigned long long> bb(2 * N_BUCKETS, 0);
+            std::vector<unsigned long long> bb(3 * N_BUCKETS, 0);   // base, end and cursor (0) of each bucket
             for (uint32_t b = lo; b < hi; ++b) {
                 bb[b] = cfg[b].key_base;
                 bb[N_BUCKETS + b] = cfg[b].key_base + region[b];
             }
-            CK(cudaMemsetAsync(cursor, 0, N_BUCKETS * 8, st));
-            CK(cudaMemcpyAsync(bbase, hs.up(bb.data(), bb.size()), 2 * N_BUCKETS * 8, cudaMemcpyHostToDevice, st));
-            CK(cudaMemsetAsync(lh_cnt, 0, 2 * N_BUCKETS * 8, st));
-            CK(cudaMemsetAsync(hll_high, 0, (size_t)N_BUCKETS * BUCKET_HLL_M * 4, st));
+            CK(cudaMemcpyAsync(bbase, hs.up(bb.data(), bb.size()), bb.size() * 8, cudaMemcpyHostToDevice, st));
+            if (!prefix) {
+                CK(cudaMemsetAsync(lh_cnt, 0, 2 * N_BUCKETS * 8, st));
+                CK(cudaMemsetAsync(hll_high, 0, (size_t)N_BUCKETS * BUCKET_HLL_M * 4, st));
+            }
             a.hll = nullptr;
             a.prepass = 0;
             a.bucket_hist = nullptr;
@@ -1138,16 +1136,19 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
             clk.end();
             unsigned long long *p_fill = hs.n<unsigned long long>(N_BUCKETS);
             CK(cudaMemcpyAsync(p_fill, cursor, N_BUCKETS * 8, cudaMemcpyDeviceToHost, st));
-            CK(cudaStreamSynchronize(st));
-            const std::vector<unsigned long long> fill(p_fill, p_fill + N_BUCKETS);
+            // an exact census has the prefix path's buckets: it goes on without
+            // waiting, and they are compared once counted
+            const bool known = prefix && exact;
+            if (!known) CK(cudaStreamSynchronize(st));
             check_cancel(job, "after the partition");
             for (uint32_t b = lo; b < hi; ++b) {
-                if (fill[b] > region[b]) throw CensusOverflow{};
-                cfg[b].key_len = fill[b];
-                filled_total += fill[b];
+                if (!known && p_fill[b] > region[b]) throw CensusOverflow{};
+                cfg[b].key_len = known ? region[b] : p_fill[b];
+                filled_total += cfg[b].key_len;
             }
-            CK(cudaMemcpyAsync(d_cfg_b, hs.up(cfg.data(), N_BUCKETS), N_BUCKETS * sizeof(BucketCfg),
-                               cudaMemcpyHostToDevice, st));
+            if (!prefix)
+                CK(cudaMemcpyAsync(d_cfg_b, hs.up(cfg.data(), N_BUCKETS), N_BUCKETS * sizeof(BucketCfg),
+                                   cudaMemcpyHostToDevice, st));
             // each bucket-major launch gets its 256 ranges, not a list of items
             auto upload_ranges = [&](BucketRanges &r, uint32_t &n_items) {
                 n_items = fill_item_starts_n(r, WORK_ITEM_KEYS);
@@ -1177,12 +1178,16 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
                 pp.list = list;
                 pp.tmp_counts = tmp_counts;
                 pp.list_cap = list_cap;
-                pp.fault_inject = P.fault_inject;
+                pp.fault_inject = P.bloom ? P.fault_inject & ~KC_INJECT_TABLE_FULL : P.fault_inject;
                 pp.repartition = [&] {
                     CK(cudaMemsetAsync(cursor, 0, N_BUCKETS * 8, st));
                     CK(launch_part(PART_BY_STRING, k, a, st));
                 };
+                pp.hist_zero = lo == 0;
                 count_by_prefix(pp, ds, hs, clk, tn, st);
+                for (uint32_t b = lo; known && b < hi; ++b)
+                    if (p_fill[b] != region[b])
+                        throw KcError{KC_ERR_DEVICE, "partition does not add up to the occurrences"};
                 rec_keys = pp.rec_keys;
                 rec_counts = pp.rec_counts;
                 n_rec = pp.n_rec;
@@ -1195,7 +1200,7 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
                     low_len += pp.totals[0];
                     high_len += pp.n_keys - pp.totals[0];
                 } else {
-                    high_len += pp.n_keys;
+                    plain_keys += pp.n_keys;
                 }
                 table_cap = std::max(table_cap, pp.table_cap);
                 job.region_redos += pp.region_redos;
@@ -1231,7 +1236,6 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
                 ds.release(hll_high);
                 ds.release(lh_cnt);
                 ds.release(bbase);
-                ds.release(cursor);
                 ds.release(d_cfg_b);
                 if (P.bloom) {
                     ds.release(keys);
@@ -1377,16 +1381,32 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
     if (!reversed) CK(launch_pair_reverse(rec_keys, n_rec, st));
     clk.end();
 
+    // records to the host, after the job's last kernels
+    auto records_out = [&] {
+        CK(cudaEventRecord(ev1, st));
+        if (trace_host) fprintf(stderr, "[kc trace] records to host from %.3f ms (host clock)\n", now_ms() - th_start);
+        if (!P.keep_records) return;
+        job.recs.allocate(n_rec);
+        if (!n_rec) return;
+        CK(cudaMemcpyAsync(job.recs.keys(), rec_keys, n_rec * 8, cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(job.recs.counts(), rec_counts, n_rec * 4, cudaMemcpyDeviceToHost, st));
+    };
+
     // ---- histogram (with the counters, under one sync) ----------------------
     unsigned long long *p_c2 = hs.n<unsigned long long>(C_COUNT);
-    unsigned long long *p_hd = hs.n<unsigned long long>(HIST_BINS);
+    // (top-N thresholds look at any count, the histogram at its own range)
+    const uint32_t hist_lo = P.hist_min, hist_hi = std::max(P.hist_max, P.hist_min);
+    const uint32_t n_bins = P.top_n ? HIST_BINS : (uint32_t)std::min<uint64_t>(HIST_BINS, std::max(hist_hi, 1u) + 1ull);
+    unsigned long long *hd = hs.n<unsigned long long>(n_bins);
     CK(cudaMemcpyAsync(p_c2, counters, C_COUNT * 8, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(p_hd, hist, HIST_BINS * 8, cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(hd, hist, n_bins * 8, cudaMemcpyDeviceToHost, st));
+    // nothing more to compute: the records follow under the same sync
+    const bool last_work = !P.top_n && !P.want_le2 && !P.pack_high;
+    if (last_work) records_out();
     CK(cudaStreamSynchronize(st));
     Counters c2{};
     std::memcpy(c2.v, p_c2, sizeof(c2.v));
     check_flags(c2.v[C_FLAGS], "sort");
-    std::vector<unsigned long long> hd(p_hd, p_hd + HIST_BINS);
     const uint64_t n_ovf = std::min<uint64_t>(c2.v[C_OVF_LEN], ovf_cap);
     std::vector<uint32_t> ovf_h(n_ovf);
     if (n_ovf) {
@@ -1395,11 +1415,10 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
     }
     hd[1] += untabled;   // FIRST-only k-mers have count 1 (count_max >= 1)
     {
-        uint32_t lo = P.hist_min, hi = P.hist_max;
-        if (hi < lo) hi = lo;
+        const uint32_t lo = hist_lo, hi = hist_hi;
         uint64_t len = (uint64_t)hi - lo + 1;
         job.hist.assign(len, 0);
-        for (uint64_t c = std::max<uint64_t>(lo, 1); c < HIST_BINS && c <= hi; ++c) job.hist[c - lo] = (int64_t)hd[c];
+        for (uint64_t c = std::max<uint64_t>(lo, 1); c < n_bins && c <= hi; ++c) job.hist[c - lo] = (int64_t)hd[c];
         for (uint32_t c : ovf_h)
             if (c >= lo && c <= hi) job.hist[c - lo]++;
     }
@@ -1478,24 +1497,19 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
         clk.end();
     }
     if (P.pack_high) pack_high_on_device(job, ds, rec_keys, rec_counts, n_rec, st, clk);
-    CK(cudaEventRecord(ev1, st));
-
-    // ---- records to host ------------------------------------------------------
-    if (trace_host) fprintf(stderr, "[kc trace] records to host from %.3f ms (host clock)\n", now_ms() - th_start);
-    if (P.keep_records) {
-        job.recs.allocate(n_rec);
-        if (n_rec) {
-            CK(cudaMemcpyAsync(job.recs.keys(), rec_keys, n_rec * 8, cudaMemcpyDeviceToHost, st));
-            CK(cudaMemcpyAsync(job.recs.counts(), rec_counts, n_rec * 4, cudaMemcpyDeviceToHost, st));
-        }
+    if (!last_work) {
+        records_out();
+        CK(cudaStreamSynchronize(st));
     }
-    CK(cudaStreamSynchronize(st));
     if (trace_host) fprintf(stderr, "[kc trace] job done at %.3f ms (host clock)\n", now_ms() - th_start);
     float ms = 0;
     CK(cudaEventElapsedTime(&ms, ev0, ev1));
     job.device_ms = ms;
     clk.collect(job.phase_ms, job.phase_launches, ev0);
     job.low_len = low_len;
+    // plain jobs: 0 where one table small enough for L2 would hold the k-mers
+    if (plain_keys && table_capacity_for((double)job.distinct, tn.table_factor) > PLAIN_PART_MIN_SLOTS)
+        high_len = plain_keys;
     job.high_len = high_len;
     job.input_bytes = in->total_bytes;
     job.n_records_total = n_rec;
@@ -1506,10 +1520,10 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
 // src/main.cpp:617-633)
 // ---------------------------------------------------------------------------
 //
-// Jobs of some size take the prefix path with N-word string keys: a sampled
-// census per first four bases -> per pass over a range of those: partition ->
+// The prefix path with N-word string keys: a census per first four bases
+// (sampled on larger inputs) -> per pass over a range of those: partition ->
 // sub-buckets -> count and sort in shared memory.
-// The others: upload -> newline census -> SCAN (occurrences, HyperLogLog,
+// Global-memory tables: upload -> newline census -> SCAN (occurrences, HyperLogLog,
 // occurrences per root prefix) -> per pass over a range of root prefixes:
 // INSERT into an N-word table sized from the estimate (regrown when full) ->
 // compaction (count, then records + histogram) -> sort of all records in
@@ -1570,7 +1584,7 @@ void run_wide_job(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
         CK(launch_wait_flag(reinterpret_cast<const unsigned int *>(counters + C_COUNT - 1), 1024, counters + C_FLAGS,
                             st));
 
-    const bool prefix = tn.bloom_smem == 1 && !global_tables && in->total_bytes >= PREFIX_PATH_MIN_BYTES;
+    const bool prefix = tn.bloom_smem == 1 && !global_tables;
     job.smem_passes = job.smem_fallbacks = job.region_redos = 0;
     job.distinct = 0;
 
@@ -1741,6 +1755,7 @@ void run_wide_job(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
         pp.list_cap = list_cap;
         pp.fault_inject = P.fault_inject;
         pp.repartition = partition;
+        pp.hist_zero = rg.first == 0;
         count_by_prefix(pp, ds, hs, clk, tn, st);
         job.distinct += pp.totals[0];
         job.region_redos += pp.region_redos;
@@ -2196,6 +2211,7 @@ void run_batch_once(std::vector<std::shared_ptr<Job>> &jobs, cudaStream_t st, Wo
             pp.n_groups = ng;
             pp.hist = hist + (size_t)lo * HIST_BINS_BATCH;
             pp.hist_bins = HIST_BINS_BATCH;
+            pp.hist_zero = true;   // its samples' part
             pp.ovf64 = ovf;
             pp.ovf_cap = ovf_cap;
             pp.counters = counters;

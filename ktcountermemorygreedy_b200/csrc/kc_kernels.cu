@@ -1067,12 +1067,28 @@ __global__ void __launch_bounds__(1024) k_scan_top(unsigned long long *sums, uin
     }
 }
 
+// ALONE: the whole scan in this launch, each block adding up the items before
+// its own itself (they are in L2 and few).
+template <bool ALONE>
 __global__ void __launch_bounds__(256) k_scan_down(const uint32_t *in, uint64_t n, const unsigned long long *sums,
                                                    unsigned long long *out)
 {
     __shared__ unsigned long long s[8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t base = (uint64_t)blockIdx.x * SCAN_BLOCK;
+    unsigned long long before = 0;
+    if (ALONE) {
+        __shared__ unsigned long long s_before[8];
+#pragma unroll 8
+        for (uint64_t i = threadIdx.x; i < base; i += 256) before += in[i];
+        for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(FULL, before, o);
+        if (lane == 0) s_before[warp] = before;
+        __syncthreads();
+        before = 0;
+        for (int i = 0; i < 8; ++i) before += s_before[i];
+    } else {
+        before = sums[blockIdx.x];
+    }
     // each thread owns SCAN_ITEMS consecutive items
     uint32_t v[SCAN_ITEMS];
     unsigned long long local = 0;
@@ -1093,7 +1109,7 @@ __global__ void __launch_bounds__(256) k_scan_down(const uint32_t *in, uint64_t 
         for (int i = 0; i < 8; ++i) { unsigned long long t = s[i]; s[i] = c; c += t; }
     }
     __syncthreads();
-    unsigned long long run = sums[blockIdx.x] + s[warp] + x - local;
+    unsigned long long run = before + s[warp] + x - local;
     for (uint32_t j = 0; j < SCAN_ITEMS; ++j) {
         uint64_t i = base + threadIdx.x * SCAN_ITEMS + j;
         if (i < n) out[i] = run;
@@ -2255,6 +2271,11 @@ cudaError_t launch_extract(int mode, const ExtractArgs &a, int grid, cudaStream_
     }
 }
 
+// Up to this many blocks a scan is one launch instead of three (ALONE above): the
+// last block then reads at most 14K items of the others, 3 us, and two launches
+// are 7 us on the device and 5 on the host.
+constexpr uint64_t SCAN_ALONE_BLOCKS = 8;
+
 size_t scan_tmp_words(uint64_t n) { return (n + SCAN_BLOCK - 1) / SCAN_BLOCK + 1; }
 
 cudaError_t launch_scan_u32(const uint32_t *in, unsigned long long *out, uint64_t n, unsigned long long *tmp,
@@ -2263,11 +2284,15 @@ cudaError_t launch_scan_u32(const uint32_t *in, unsigned long long *out, uint64_
     if (!n) return cudaSuccess;
     uint64_t nb = (n + SCAN_BLOCK - 1) / SCAN_BLOCK;
     note_launch();
+    if (nb <= SCAN_ALONE_BLOCKS) {
+        k_scan_down<true><<<(unsigned)nb, 256, 0, st>>>(in, n, nullptr, out);
+        return cudaGetLastError();
+    }
     k_scan_reduce<<<(unsigned)nb, 256, 0, st>>>(in, n, tmp);
     note_launch();
     k_scan_top<<<1, 1024, 0, st>>>(tmp, nb);
     note_launch();
-    k_scan_down<<<(unsigned)nb, 256, 0, st>>>(in, n, tmp, out);
+    k_scan_down<false><<<(unsigned)nb, 256, 0, st>>>(in, n, tmp, out);
     return cudaGetLastError();
 }
 
@@ -2556,7 +2581,8 @@ cudaError_t preload_sort_in_scratch()
     const void *fns[] = {reinterpret_cast<const void *>(k_single_segment_tiles),
                          reinterpret_cast<const void *>(k_radix_count), reinterpret_cast<const void *>(k_radix_scatter),
                          reinterpret_cast<const void *>(k_scan_reduce), reinterpret_cast<const void *>(k_scan_top),
-                         reinterpret_cast<const void *>(k_scan_down)};
+                         reinterpret_cast<const void *>(k_scan_down<false>),
+                         reinterpret_cast<const void *>(k_scan_down<true>)};
     for (const void *f : fns) {
         const cudaError_t e = cudaFuncGetAttributes(&fa, f);
         if (e != cudaSuccess) return e;

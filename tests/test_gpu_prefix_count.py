@@ -1,5 +1,4 @@
-"""Counting by printed-order prefix in shared memory (Bloom jobs of any size and
-plain jobs from 4 MiB of FASTQ on), where it can go wrong: k below and at the
+"""Counting by printed-order prefix in shared memory, where it can go wrong: k below and at the
 bucket prefix, k-mers that share a long prefix (tables counted in rounds,
 buckets cut again, the global-memory fallback), one k-mer of very many
 occurrences, and sort units of every size class.  Integer work: exact
@@ -233,3 +232,18 @@ def test_batch_sample_of_one_prefix(counter, prefix, fallback):
     plain = ["".join(rnd.choice("ACGT") for _ in range(150)) for _ in range(300)]
     rs = _check_batch(counter, [plain, skew + skew[:999], plain[:50]], [21, 31, 32])
     assert all((r.smem_fallbacks > 0) == fallback and r.smem_passes == (0 if fallback else 1) for r in rs)
+
+
+@pytest.mark.parametrize("tiles", [1, 2, 2047, 2048, 2049, 16384, 16385])
+def test_line_numbers_at_scan_edges(counter, tiles):
+    """One record per 8 KiB tile, tile counts at the edges of one scan block and
+    of the one-launch scan: a wrong line number would count the quality lines
+    (letters) too."""
+    n = (8192 - 7) // 2
+    rec = b"@r\n" + b"A" * n + b"\n+\n" + b"C" * n + b"\n"
+    fq = (b"@" + b"r" * (8192 - len(rec) + 1) + rec[2:]) * tiles
+    assert len(fq) == 8192 * tiles
+    for bloom in (False, True):
+        r = counter.count([fq], k=31, count_max=U32, hist_max=10, **(dict(bloom=True, memory_gb=1) if bloom else {}))
+        assert r.occurrences == (n - 30) * tiles and r.distinct == 1
+        assert r.keys.tolist() == [0] and r.counts.tolist() == [(n - 30) * tiles]
