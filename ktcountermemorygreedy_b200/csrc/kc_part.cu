@@ -62,13 +62,16 @@ __device__ __forceinline__ uint32_t warp_inclusive(uint32_t v, int lane)
 // one bucket.  The next tile's bytes arrive while this one's k-mers are formed
 // and written (the tile buffer is free once classified).
 //
-// Bound by instruction issue (58%) and shared-memory wavefronts (56%).  A
+// String keys are rolled as complements, so that the smaller of the two is the
+// key itself.
+//
+// Bound by instruction issue (57%) and shared-memory wavefronts (57%).  A
 // kernel that staged the k-mers unsorted in shared memory first (stores 64
 // bytes apart, 16 to a bank), rolled chunks of 8 with 64-bit shifts by variable
 // amounts, read the file's data and line numbers when a tile had arrived and
 // checked every k-mer against its bucket's region took 172 warp instructions
-// per 32 k-mers at three blocks per SM, this one 122 at four: 2.4G k-mers of
-// 150-base reads 21.2 -> 13.7 ms, 480M 4.25 -> 2.74, 25M 0.23 -> 0.15.
+// per 32 k-mers at three blocks per SM, this one 117 at four: 2.4G k-mers of
+// 150-base reads 21.2 -> 13.3 ms, 480M 4.25 -> 2.67, 25M 0.23 -> 0.15.
 //
 // BY: what a bucket is (PartBy).  By sample all k-mers of a tile have one
 // bucket, and their places follow from a scan of the threads' counts.
@@ -192,17 +195,23 @@ __global__ void __launch_bounds__(PT_THREADS, 4) k_part(ExtractArgs a)
                 const bool half = (ch & 0x10000u) != 0;
                 // the window ending just before the chunk: forward word (base
                 // i at bit 64-2k+2i, stale bits below) and, from it, the
-                // reverse complement's
+                // reverse complement's; for string keys the complements of both
                 const uint32_t cw = half ? (uint32_t)(cur >> 32) : (uint32_t)cur;   // the chunk's 16 codes
                 uint32_t fh = half ? (uint32_t)cur : (uint32_t)(prev >> 32);
                 uint32_t fl = half ? (uint32_t)(prev >> 32) : (uint32_t)prev;
-                const uint64_t rc0 = ~(pair_reverse(((uint64_t)fh << 32) | fl) << fs) & topmask;
+                const uint64_t rev = pair_reverse(((uint64_t)fh << 32) | fl) << fs;
+                const uint64_t rc0 = STRING ? rev : ~rev & topmask;
                 uint32_t rh = (uint32_t)(rc0 >> 32), rl = (uint32_t)rc0;
-                // complemented codes at the bits where the roll takes them in
-                // (by sample with k <= 16 that is the upper half)
+                const uint32_t fw = STRING ? ~cw : cw;   // the forward word's codes, the reverse one's are their complements
+                if (STRING) {
+                    fh = ~fh;
+                    fl = ~fl;
+                }
+                // the reverse word's codes at the bits where the roll takes them
+                // in (by sample with k <= 16 that is the upper half)
                 const bool upper = SAMPLE && fs >= 32;
                 const uint32_t in_sh = !W || upper ? fs - 32 : fs;
-                const uint64_t nc = (uint64_t)(~cw) << in_sh;
+                const uint64_t nc = (uint64_t)(~fw) << in_sh;
                 const uint32_t nc_hi = (uint32_t)(nc >> 32), nc_lo = (uint32_t)nc;
                 const uint32_t in_mask = 3u << in_sh;
 #pragma unroll
@@ -219,18 +228,14 @@ __global__ void __launch_bounds__(PT_THREADS, 4) k_part(ExtractArgs a)
                     } else {
                         rh = (rh << 2) | in;
                     }
-                    fh = (fh >> 2) | ((cw << (30 - 2 * p)) & 0xC0000000u);
+                    fh = __funnelshift_r(fh, fw >> (2 * p), 2);
                     // the canonical word is the smaller one; the string key of
-                    // the canonical strand is the complement of the larger one
+                    // the canonical strand is the complement of the larger one:
+                    // the smaller complement
                     const uint32_t xh = W && !SAMPLE ? fh : fh & tm_hi, xl = W ? fl & tm_lo : 0u;
                     const bool less = W ? (((uint64_t)xh << 32) | xl) < (((uint64_t)rh << 32) | rl) : xh < rh;
-                    if (STRING) {
-                        kh[p] = W && !SAMPLE ? ~(less ? rh : xh) : ~(less ? rh : xh) & tm_hi;
-                        kl[p] = W ? ~(less ? rl : xl) & tm_lo : 0u;
-                    } else {
-                        kh[p] = less ? xh : rh;
-                        kl[p] = W ? (less ? xl : rl) : 0u;
-                    }
+                    kh[p] = less ? xh : rh;
+                    kl[p] = W ? (less ? xl : rl) : 0u;
                 }
                 if (!SAMPLE && !all_buckets) {
 #pragma unroll
