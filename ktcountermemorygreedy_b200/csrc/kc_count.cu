@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
 // records by comparing itself with the run's other keys: no lane waits for
 // another, unlike an insertion sort per run.  The counts are read where they
 // are written (a unit's counts stay in L1).
-template <uint32_t N, uint32_t THREADS, uint32_t CAP, uint32_t LGB>
+template <uint32_t THREADS, uint32_t CAP, uint32_t LGB>
 __global__ void __launch_bounds__(THREADS) k_unit_sort(const unsigned long long *tk, const uint32_t *tv,
                                                        const unsigned long long *sub_off,
                                                        const unsigned long long *sub_final, const SubUnit *units,
@@ -526,51 +526,36 @@ __global__ void __launch_bounds__(THREADS) k_unit_sort(const unsigned long long 
     static_assert(NB % THREADS == 0 && CAP <= 65536, "layout");
     extern __shared__ __align__(16) uint8_t us_smem[];
     unsigned long long *s_keys = reinterpret_cast<unsigned long long *>(us_smem);   // CAP keys
-    uint32_t *s_start = reinterpret_cast<uint32_t *>(s_keys + N * CAP);             // NB
+    uint32_t *s_start = reinterpret_cast<uint32_t *>(s_keys + CAP);             // NB
     uint16_t *s_idx = reinterpret_cast<uint16_t *>(s_start + NB);                   // CAP
-    __shared__ uint32_t s_warp[WARPS], s_xor[2 * N];
+    __shared__ uint32_t s_warp[WARPS], s_xor[2];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (uint32_t ui = blockIdx.x; ui < n_units; ui += gridDim.x) {
         const SubUnit u = units[ui];
         const uint32_t m = u.len < CAP ? u.len : CAP;
         const unsigned long long src = sub_off[u.sub] + u.off, dst = sub_final[u.sub] + u.off;
-        if (tid < 2 * (int)N) s_xor[tid] = 0;
+        if (tid < 2) s_xor[tid] = 0;
 #pragma unroll
         for (uint32_t j = 0; j < PER; ++j) s_start[j * THREADS + tid] = 0;
         __syncthreads();
         // common prefix: the bits in which no key differs from the first
-        const KeyN<N> k0 = load_key<N>(tk, src, LoadPlain());
-        unsigned long long x[N];
-#pragma unroll
-        for (uint32_t j = 0; j < N; ++j) x[j] = 0;
+        const unsigned long long k0 = tk[src];
+        unsigned long long x = 0;
 #pragma unroll 4
         for (uint32_t i = tid; i < m; i += THREADS) {
-            const KeyN<N> key = load_key<N>(tk, src + i, LoadStream());
-            store_key<N>(s_keys, i, key);
-#pragma unroll
-            for (uint32_t j = 0; j < N; ++j) x[j] |= key.w[j] ^ k0.w[j];
+            const unsigned long long key = __ldcs(tk + src + i);
+            s_keys[i] = key;
+            x |= key ^ k0;
         }
-#pragma unroll
-        for (uint32_t j = 0; j < N; ++j) {
-            const uint32_t xh = __reduce_or_sync(FULLW, (uint32_t)(x[j] >> 32)), xl = __reduce_or_sync(FULLW, (uint32_t)x[j]);
-            if (lane == 0) {
-                if (xh) atomicOr(&s_xor[2 * j], xh);
-                if (xl) atomicOr(&s_xor[2 * j + 1], xl);
-            }
+        const uint32_t xh = __reduce_or_sync(FULLW, (uint32_t)(x >> 32)), xl = __reduce_or_sync(FULLW, (uint32_t)x);
+        if (lane == 0) {
+            if (xh) atomicOr(&s_xor[0], xh);
+            if (xl) atomicOr(&s_xor[1], xl);
         }
         __syncthreads();
-        // the first word in which keys differ, and the digit below its common bits
-        uint32_t dw = 0;
-        unsigned long long diff = 0;
-#pragma unroll
-        for (uint32_t j = 0; j < N; ++j)
-            if (!diff) {
-                diff = ((unsigned long long)s_xor[2 * j] << 32) | s_xor[2 * j + 1];
-                dw = j;
-            }
-        const int pre = __clzll(diff);   // 64: one record
+        const int pre = __clzll(((unsigned long long)s_xor[0] << 32) | s_xor[1]);   // 64: one record
         const int dsh = 64 - pre - (int)LGB > 0 ? 64 - pre - (int)LGB : 0;
-        auto digit = [&](uint32_t i) { return (uint32_t)(s_keys[N * i + dw] >> dsh) & (NB - 1); };
+        auto digit = [&](uint32_t i) { return (uint32_t)(s_keys[i] >> dsh) & (NB - 1); };
         for (uint32_t i = tid; i < m; i += THREADS) atomicAdd(&s_start[digit(i)], 1u);
         __syncthreads();
         // exclusive scan of the NB counts, PER consecutive ones per thread
@@ -605,26 +590,156 @@ __global__ void __launch_bounds__(THREADS) k_unit_sort(const unsigned long long 
             const uint32_t i = s_idx[p], d = digit(i);
             const uint32_t lo = d ? s_start[d - 1] : 0u, hi = s_start[d];
             uint32_t rank = lo;
-            if constexpr (N == 1) {
-                const unsigned long long key = s_keys[i];
-                for (uint32_t j = lo; j < hi; ++j) rank += s_keys[s_idx[j]] < key ? 1u : 0u;
-            } else {
-                // the words before dw are the same in all keys
-                const unsigned long long kd = s_keys[N * i + dw];
-                for (uint32_t j = lo; j < hi; ++j) {
-                    const unsigned long long *o = s_keys + N * s_idx[j];
-                    bool less = o[dw] < kd;
-                    if (o[dw] == kd) {
-                        for (uint32_t w = dw + 1; w < N; ++w) {
-                            const unsigned long long ow = o[w], mw = s_keys[N * i + w];
-                            if (ow != mw) {
-                                less = ow < mw;
-                                break;
-                            }
-                        }
-                    }
-                    rank += less ? 1u : 0u;
+            const unsigned long long key = s_keys[i];
+            for (uint32_t j = lo; j < hi; ++j) rank += s_keys[s_idx[j]] < key ? 1u : 0u;
+            if (dst + rank < out_cap) {
+                out_k[dst + rank] = pair_reverse(key >> (64 - 2 * u.k));
+                out_v[dst + rank] = __ldg(&tv[src + i]);
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// 1 if the N-word number at p, its words `stride` apart and the first the most
+// significant, is less than o: the borrow of p - o.
+template <uint32_t N>
+__device__ __forceinline__ uint32_t words_less(const unsigned long long *p, uint32_t stride, const unsigned long long *o)
+{
+    uint32_t less;
+    if constexpr (N == 2)
+        asm("{ .reg .u64 t; sub.cc.u64 t, %1, %2; subc.cc.u64 t, %3, %4; subc.u32 %0, 0, 0; }"
+            : "=r"(less)
+            : "l"(p[stride]), "l"(o[1]), "l"(p[0]), "l"(o[0]));
+    else
+        asm("{ .reg .u64 t; sub.cc.u64 t, %1, %2; subc.cc.u64 t, %3, %4; subc.cc.u64 t, %5, %6; subc.cc.u64 t, %7, %8; "
+            "subc.u32 %0, 0, 0; }"
+            : "=r"(less)
+            : "l"(p[3 * stride]), "l"(o[3]), "l"(p[2 * stride]), "l"(o[2]), "l"(p[stride]), "l"(o[1]), "l"(p[0]), "l"(o[0]));
+    return less & 1u;
+}
+
+// The same for two- and four-word keys.  Word w of all keys lies together (keys
+// side by side, 32 bytes apart, put the same word of eight of them in one bank:
+// the shared-memory pipe was 90% busy, 60% of it conflicts).  Long k-mers of
+// reads come in runs of ten and more that start alike (the same position with
+// different errors further on): a run's records are compared whole, without
+// branches, by lanes next to one another, which read the same record at a time.
+// 29M 127-base k-mers of sequence covered 20 times 1.65 -> 1.03 ms (words apart
+// alone 1.46, with comparisons that stopped at the first difference).
+template <uint32_t N, uint32_t THREADS, uint32_t CAP, uint32_t LGB>
+__global__ void __launch_bounds__(THREADS) k_unit_sort_wide(const unsigned long long *tk, const uint32_t *tv,
+                                                            const unsigned long long *sub_off,
+                                                            const unsigned long long *sub_final, const SubUnit *units,
+                                                            uint32_t n_units, unsigned long long *out_k, uint32_t *out_v,
+                                                            uint64_t out_cap)
+{
+    constexpr uint32_t NB = 1u << LGB, PER = NB / THREADS, WARPS = THREADS / 32, OWN = CAP / THREADS;
+    static_assert(NB % THREADS == 0 && CAP % THREADS == 0 && CAP <= 65536, "layout");
+    extern __shared__ __align__(16) uint8_t us_smem[];
+    unsigned long long *s_keys = reinterpret_cast<unsigned long long *>(us_smem);   // N x CAP words
+    uint32_t *s_start = reinterpret_cast<uint32_t *>(s_keys + N * CAP);             // NB
+    uint16_t *s_idx = reinterpret_cast<uint16_t *>(s_start + NB);                   // CAP
+    __shared__ uint32_t s_warp[WARPS], s_xor[2 * N];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (uint32_t ui = blockIdx.x; ui < n_units; ui += gridDim.x) {
+        const SubUnit u = units[ui];
+        const uint32_t m = u.len < CAP ? u.len : CAP;
+        const unsigned long long src = sub_off[u.sub] + u.off, dst = sub_final[u.sub] + u.off;
+        if (tid < 2 * (int)N) s_xor[tid] = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < PER; ++j) s_start[j * THREADS + tid] = 0;
+        __syncthreads();
+        // common prefix: the bits in which no key differs from the first
+        const KeyN<N> k0 = load_key<N>(tk, src, LoadPlain());
+        unsigned long long x[N];
+#pragma unroll
+        for (uint32_t j = 0; j < N; ++j) x[j] = 0;
+#pragma unroll
+        for (uint32_t r = 0; r < OWN; ++r) {
+            const uint32_t i = r * THREADS + tid;
+            if (i < m) {
+                const KeyN<N> key = load_key<N>(tk, src + i, LoadStream());
+#pragma unroll
+                for (uint32_t j = 0; j < N; ++j) {
+                    s_keys[j * CAP + i] = key.w[j];
+                    x[j] |= key.w[j] ^ k0.w[j];
                 }
+            }
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < N; ++j) {
+            const uint32_t xh = __reduce_or_sync(FULLW, (uint32_t)(x[j] >> 32)), xl = __reduce_or_sync(FULLW, (uint32_t)x[j]);
+            if (lane == 0) {
+                if (xh) atomicOr(&s_xor[2 * j], xh);
+                if (xl) atomicOr(&s_xor[2 * j + 1], xl);
+            }
+        }
+        __syncthreads();
+        // the first word in which keys differ, and the digit below its common bits
+        uint32_t dw = 0;
+        unsigned long long diff = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < N; ++j)
+            if (!diff) {
+                diff = ((unsigned long long)s_xor[2 * j] << 32) | s_xor[2 * j + 1];
+                dw = j;
+            }
+        const int pre = __clzll(diff);   // 64: one record
+        const int dsh = 64 - pre - (int)LGB > 0 ? 64 - pre - (int)LGB : 0;
+        const unsigned long long *s_dw = s_keys + dw * CAP;
+        uint32_t d[OWN];
+#pragma unroll
+        for (uint32_t r = 0; r < OWN; ++r) {
+            const uint32_t i = r * THREADS + tid;
+            d[r] = 0;
+            if (i < m) {
+                d[r] = (uint32_t)(s_dw[i] >> dsh) & (NB - 1);
+                atomicAdd(&s_start[d[r]], 1u);
+            }
+        }
+        __syncthreads();
+        // exclusive scan of the NB counts, PER consecutive ones per thread
+        uint32_t c[PER], own = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < PER; ++j) {
+            c[j] = s_start[tid * PER + j];
+            own += c[j];
+        }
+        uint32_t inc = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULLW, inc, o);
+            if (lane >= o) inc += y;
+        }
+        if (lane == 31) s_warp[warp] = inc;
+        __syncthreads();
+        uint32_t run = inc - own;
+#pragma unroll
+        for (uint32_t w = 0; w < WARPS; ++w)
+            if ((int)w < warp) run += s_warp[w];
+#pragma unroll
+        for (uint32_t j = 0; j < PER; ++j) {
+            s_start[tid * PER + j] = run;
+            run += c[j];
+        }
+        __syncthreads();
+        // placing moves each start to its run's end: run d is [end of run d - 1, end of run d)
+#pragma unroll
+        for (uint32_t r = 0; r < OWN; ++r) {
+            const uint32_t i = r * THREADS + tid;
+            if (i < m) s_idx[atomicAdd(&s_start[d[r]], 1u)] = (uint16_t)i;
+        }
+        __syncthreads();
+        for (uint32_t p = tid; p < m; p += THREADS) {
+            const uint32_t i = s_idx[p], dg = (uint32_t)(s_dw[i] >> dsh) & (NB - 1);
+            const uint32_t lo = dg ? s_start[dg - 1] : 0u, hi = s_start[dg];
+            uint32_t rank = lo;
+            if (hi - lo > 1) {
+                unsigned long long own[N];
+#pragma unroll
+                for (uint32_t w = 0; w < N; ++w) own[w] = s_keys[w * CAP + i];
+                for (uint32_t j = lo; j < hi; ++j) rank += words_less<N>(s_keys + s_idx[j], CAP, own);
             }
             if (dst + rank < out_cap) {
                 // string order back to k-mer words: word w holds the 32 bases
@@ -636,10 +751,11 @@ __global__ void __launch_bounds__(THREADS) k_unit_sort(const unsigned long long 
                     unsigned long long v = 0;
                     if (b >= 0) {
                         const uint32_t o = 2 * (b & 31);
-                        v = s_keys[N * i + (b >> 5)] << o;
-                        if (o) v |= s_keys[N * i + (b >> 5) + 1] >> (64 - o);
+                        const unsigned long long *q = s_keys + (uint32_t)(b >> 5) * CAP + i;
+                        v = q[0] << o;
+                        if (o) v |= q[CAP] >> (64 - o);
                     } else if (b > -32) {
-                        v = s_keys[N * i] >> (-2 * b);
+                        v = s_keys[i] >> (-2 * b);
                     }
                     key.w[w] = pair_reverse(v);
                 }
@@ -678,7 +794,10 @@ cudaError_t launch_unit_sort_t(const unsigned long long *tk, const uint32_t *tv,
 {
     if (!n_units) return cudaSuccess;
     const size_t smem = (size_t)CAP * (8 * N + 2) + (size_t)(1u << LGB) * 4;
-    auto kern = k_unit_sort<N, THREADS, CAP, LGB>;
+    auto kern = [] {
+        if constexpr (N == 1) return k_unit_sort<THREADS, CAP, LGB>;
+        else return k_unit_sort_wide<N, THREADS, CAP, LGB>;
+    }();
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;

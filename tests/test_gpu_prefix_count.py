@@ -247,3 +247,21 @@ def test_line_numbers_at_scan_edges(counter, tiles):
         r = counter.count([fq], k=31, count_max=U32, hist_max=10, **(dict(bloom=True, memory_gb=1) if bloom else {}))
         assert r.occurrences == (n - 30) * tiles and r.distinct == 1
         assert r.keys.tolist() == [0] and r.counts.tolist() == [(n - 30) * tiles]
+
+
+@pytest.mark.parametrize("k,same", [(33, 20), (63, 31), (63, 33), (64, 60), (65, 40), (96, 64), (127, 70), (127, 100), (128, 124)])
+def test_wide_runs_that_start_alike(counter, k, same):
+    """Runs of k-mers with the same first `same` bases, told apart by any later
+    word: every place of a run's first difference, between the words too."""
+    rnd = random.Random(k + same)
+    seqs = []
+    for _ in range(300):
+        p = "A" + "".join(rnd.choice("ACGT") for _ in range(same - 1))
+        for _ in range(rnd.choice((1, 2, 3, 17, 40))):
+            seqs.append(p + "".join(rnd.choice("ACGT") for _ in range(k - same - 1)) + "A")
+    seqs += seqs[::3]
+    f = _fastq(seqs)
+    all_k, all_c = O.exact_records_wide([f], k)
+    r = counter.count([f], k=k, count_max=U32)
+    assert r.smem_passes == 1
+    assert np.array_equal(r.keys, all_k) and np.array_equal(r.counts, all_c)
