@@ -92,14 +92,18 @@ kc_tuning default_tuning()
 // uploaded in chunks that the census, SCAN and partition follow.
 constexpr uint64_t STREAMED_UPLOAD_MIN_BYTES = 512ull << 20;
 
-
 // Most k-mers per sub-bucket of the prefix path, for its 8192-slot tables:
-// sub-buckets have half to all of it.
-// At 16K the single large job's sub-buckets of 9K k-mers (2.7K distinct) fill
-// a third of a table: count 18.5 ms, scatter 21.0; 8K (half-empty tables swept
-// twice as often, runs of half the length in the scatter) 21.3 and 30.1, 24K
-// (tables that overflow into rounds) 25.3 and 17.1.
-constexpr uint64_t SUB_KEYS_TARGET = 16 * 1024;
+// sub-buckets have half to all of it.  Larger ones are written in longer runs
+// and swept less often, until their distinct k-mers overflow the tables into
+// rounds.  2.4G k-mers with 3.4 occurrences each: scatter and count 13.2 + 14.5 ms
+// at 16K, 12.2 + 14.4 at 20K, 15.2 + 16.9 at 8K; 480M (with every record kept) 2.04
+// + 2.95, 2.03 + 2.93, 2.14 + 3.40; 92M of 2.8 each 0.40 + 0.64, 0.40 + 0.68, 0.42 +
+// 0.72.  So 20K only from a billion k-mers on, where sequencing is deep.
+// Long k-mers catch more sequencing errors and repeat less: two-word ones (a
+// 63-base job of 176M) 1.30 + 3.41 at 16K, 1.32 + 2.41 at 10K, 1.36 + 2.48 at 8K,
+// four-word ones (127 bases, 34M) 0.68 + 1.86, 0.70 + 1.71, 0.70 + 1.60.
+constexpr uint64_t SUB_KEYS_TARGET = 16 * 1024, SUB_KEYS_DEEP = 20 * 1024, SUB_DEEP_PASS_KEYS = 1ull << 30;
+constexpr uint64_t SUB_KEYS_TWO_WORDS = 10 * 1024, SUB_KEYS_FOUR_WORDS = 8 * 1024;
 
 // The same where k-mers repeat little or sub-buckets are few: a batch's samples
 // (each sequenced far less deeply than a single large job's) and passes below
@@ -397,9 +401,10 @@ uint64_t default_pass_budget(Workspace &ws)
 // records, histograms and totals.  The buckets are cut into sub-buckets by the
 // next bases, each counted in a shared-memory table, and its records sorted on
 // their own.  A bucket (a batch's sample, base_bits 0) starts with at most
-// SUB_KEYS_TARGET or SUB_KEYS_SMALL k-mers per sub-bucket; one whose sub-buckets no number of rounds fits is cut into 16
-// times as many and the pass counted again, and a bucket that cannot be cut
-// further is reported by SubTablesFull.
+// the k-mers per sub-bucket that the pass's size and words call for; one whose
+// sub-buckets no number of rounds fits is cut into 16 times as many and the pass
+// counted again, and a bucket that cannot be cut further is reported by
+// SubTablesFull.
 struct PrefixPass {
     uint32_t words = 1;                 // 64-bit words per key
     uint32_t lo = 0, hi = 0;            // its buckets; their keys are cfg[b].key_base, key_len
@@ -443,8 +448,9 @@ void count_by_prefix(PrefixPass &pp, DevScope &ds, HostStage &hs, PhaseClock &cl
     for (uint32_t b = lo; b < hi; ++b) pass_keys += pp.cfg[b].key_len;
     const bool batch = pp.base_bits == 0;
     const bool small_subs = batch || (N == 1 && pass_keys < SUB_SMALL_PASS_KEYS);
-    const uint64_t keys_target =
-        (small_subs ? SUB_KEYS_SMALL : SUB_KEYS_TARGET) * sub_table_slots(N, shape) / sub_table_slots(1, 1);
+    const uint64_t one_word = small_subs ? SUB_KEYS_SMALL : (pass_keys < SUB_DEEP_PASS_KEYS ? SUB_KEYS_TARGET : SUB_KEYS_DEEP);
+    const uint64_t keys_target = (N == 1 ? one_word : (N == 2 ? SUB_KEYS_TWO_WORDS : SUB_KEYS_FOUR_WORDS)) *
+                                 sub_table_slots(N, shape) / sub_table_slots(1, 1);
     std::vector<uint32_t> nsub(N_BUCKETS, 0), max_nsub(N_BUCKETS, 1);
     for (uint32_t b = lo; b < hi; ++b) {
         const uint32_t word_bits = std::min(2 * pp.sc[b].k, 64u);
