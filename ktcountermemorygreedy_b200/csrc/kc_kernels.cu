@@ -11,10 +11,8 @@
 //                   bit-parallel run test; canonical words formed directly
 //                   from the packed codes.  The mode decides what happens to
 //                   each canonical k-mer: count + HyperLogLog (SCAN), insert
-//                   into the open-addressing table (INSERT), classify with the
-//                   reference's two-level Bloom filter (BLOOM) or append to a
+//                   into the open-addressing table (INSERT) or append to a
 //                   list (EMIT).
-//   k_insert_list   insert a k-mer list (Bloom non-FIRST occurrences)
 //   k_merge_low     add the FIRST occurrences back (exact merged counts)
 //   k_compact       table -> (string-order key, count) records + histogram
 //   radix sort      LSD, 8-bit digits, warp match ranking, stable
@@ -111,14 +109,6 @@ __device__ __forceinline__ void window_words(uint64_t prev, uint64_t cur, uint64
     else if (t >= 64) r = rprev;   // k = 32, q0 = 0
     else r = rcur << (-t);
     rc = r & kp.topmask;
-}
-
-__device__ __forceinline__ void hll_add(uint32_t *regs, unsigned long long key)
-{
-    uint64_t h = slot_hash(key ^ 0x5bd1e9955bd1e995ULL);
-    uint32_t r = (uint32_t)(h >> (64 - HLL_BITS));
-    uint32_t rank = __clzll((h << HLL_BITS) | (1ULL << (HLL_BITS - 1))) + 1;
-    if (rank > *(volatile uint32_t *)&regs[r]) atomicMax(&regs[r], rank);
 }
 
 // Batched jobs keep one register set per sample in global memory, shared by
@@ -319,8 +309,6 @@ __global__ void __launch_bounds__(EXT_THREADS, MODE == MODE_SCAN ? 5 : 3) k_extr
     __shared__ uint32_t s_hist[256];
     __shared__ uint32_t s_bhist[MODE == MODE_SCAN ? 256 : 1];
     __shared__ unsigned long long s_bcast[2];
-    __shared__ unsigned long long s_boff[MODE == MODE_BLOOM ? 256 : 1];
-    __shared__ unsigned long long s_bcap[MODE == MODE_BLOOM ? 256 : 1];
 
     const int tid = threadIdx.x, lane = tid & 31;
     // u walks the visited tiles (all tiles, or the SCAN subset a.visit)
@@ -340,10 +328,6 @@ __global__ void __launch_bounds__(EXT_THREADS, MODE == MODE_SCAN ? 5 : 3) k_extr
     }
     if (hll_local)
         for (uint32_t i = tid; i < HLL_M; i += EXT_THREADS) s_hll[i] = 0;
-    if (MODE == MODE_BLOOM) {
-        s_boff[tid] = a.bloom_off[tid];
-        s_bcap[tid] = a.bloom_cap[tid];
-    }
     __syncthreads();
     if (tid == 0) {
         mbar_expect_tx(&mbar[0], BUF_BYTES);
@@ -573,55 +557,6 @@ __global__ void __launch_bounds__(EXT_THREADS, MODE == MODE_SCAN ? 5 : 3) k_extr
                         if (b0 + i < a.list_cap) a.list[b0 + i] = s_stage[i];
                         else atomicOr(flags, ERR_LIST_FULL);
                     }
-                } else if (MODE == MODE_BLOOM) {
-                    uint32_t firsts = 0, highs = 0;
-                    for (uint32_t r = 0, i = tid; i < nr; ++r, i += EXT_THREADS) {
-                        unsigned long long key = s_stage[i];
-                        uint32_t p = (uint32_t)(key >> 56);
-                        uint64_t block, m;
-                        bloom_probe(key, s_bcap[p], block, m);
-                        unsigned long long *cell = a.bloom_bits + s_boff[p] + 2 * block;
-                        // ConcurrentBloomFilter::insert_prepared (src/BloomFilter.h:233-273)
-                        bool first_occ = false;
-                        unsigned long long bf1 = __ldcg(&cell[0]);
-                        if ((bf1 & m) != m) {
-                            unsigned long long bf2 = __ldcg(&cell[1]);
-                            if ((bf2 & m) == m) {
-                                atomicOr(&cell[0], (unsigned long long)m);
-                            } else {
-                                unsigned long long old2 = atomicOr(&cell[1], (unsigned long long)m);
-                                if ((old2 & m) == m) atomicOr(&cell[0], (unsigned long long)m);
-                                else first_occ = true;
-                            }
-                        }
-                        if (first_occ) firsts |= 1u << r;
-                        else {
-                            highs |= 1u << r;
-                            hll_add(a.hll_high, key);
-                        }
-                    }
-                    uint32_t tf, th;
-                    const uint32_t of = block_excl_scan(__popc(firsts), s_warp, tf);
-                    const uint32_t oh = block_excl_scan(__popc(highs), s_warp, th);
-                    if (tid == 0) {
-                        s_bcast[0] = atomicAdd(&a.counters[C_LOW_LEN], (unsigned long long)tf);
-                        s_bcast[1] = atomicAdd(&a.counters[C_HIGH_LEN], (unsigned long long)th);
-                    }
-                    __syncthreads();
-                    const unsigned long long lb = s_bcast[0] + of, hb = s_bcast[1] + oh;
-                    uint32_t nf = 0, nh = 0;
-                    for (uint32_t r = 0, i = tid; i < nr; ++r, i += EXT_THREADS) {
-                        unsigned long long key = s_stage[i];
-                        if ((firsts >> r) & 1u) {
-                            unsigned long long pos = lb + nf++;
-                            if (pos < a.list_cap) a.list[pos] = key;
-                            else atomicOr(flags, ERR_LIST_FULL);
-                        } else {
-                            unsigned long long pos = hb + nh++;
-                            if (pos < a.list_cap) a.list[a.list_cap - 1 - pos] = key;
-                            else atomicOr(flags, ERR_LIST_FULL);
-                        }
-                    }
                 }
                 __syncthreads();
             }
@@ -669,24 +604,6 @@ __global__ void k_count_keys(const Slot *slots, uint64_t n, unsigned long long *
         c += slots[i].key != EMPTY_KEY;
     c = __reduce_add_sync(FULL, c);
     if ((threadIdx.x & 31) == 0 && c) atomicAdd(out, (unsigned long long)c);
-}
-
-__global__ void k_fill_u64(unsigned long long *p, uint64_t n, unsigned long long v)
-{
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        p[i] = v;
-}
-
-__global__ void __launch_bounds__(256) k_insert_list(const unsigned long long *keys, uint64_t n, TableRef t,
-                                                     uint32_t max_probe, unsigned long long *counters)
-{
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    // whole warps iterate together so __match_any_sync sees all lanes
-    for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < n; base += stride) {
-        uint64_t i = base + (threadIdx.x & 31);
-        bool act = i < n;
-        warp_insert(act, act ? keys[i] : EMPTY_KEY, t, max_probe, &counters[C_FLAGS]);
-    }
 }
 
 __global__ void k_insert_pairs(const unsigned long long *keys, const uint32_t *counts, uint64_t n, TableRef t,
@@ -2265,7 +2182,6 @@ cudaError_t launch_extract(int mode, const ExtractArgs &a, int grid, cudaStream_
     switch (mode) {
     case MODE_SCAN: return launch_extract_t<MODE_SCAN>(a, grid, STAGE_CAP, st);
     case MODE_INSERT: return launch_extract_t<MODE_INSERT>(a, grid, STAGE_CAP, st);
-    case MODE_BLOOM: return launch_extract_t<MODE_BLOOM>(a, grid, STAGE_CAP, st);
     case MODE_EMIT: return launch_extract_t<MODE_EMIT>(a, grid, STAGE_CAP, st);
     default: return cudaErrorInvalidValue;
     }
@@ -2310,14 +2226,6 @@ cudaError_t launch_add_u64(unsigned long long *dst, const unsigned long long *sr
     return cudaGetLastError();
 }
 
-cudaError_t launch_fill_u64(unsigned long long *p, uint64_t n, unsigned long long v, cudaStream_t st)
-{
-    if (!n) return cudaSuccess;
-    note_launch();
-    k_fill_u64<<<grid_for(n, 256), 256, 0, st>>>(p, n, v);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_init_slots(Slot *slots, uint64_t n, cudaStream_t st)
 {
     if (!n) return cudaSuccess;
@@ -2331,15 +2239,6 @@ cudaError_t launch_count_keys(const Slot *slots, uint64_t n, unsigned long long 
     if (!n) return cudaSuccess;
     note_launch();
     k_count_keys<<<grid_for(n, 256), 256, 0, st>>>(slots, n, out);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_insert_list(const unsigned long long *keys, uint64_t n, TableRef t, uint32_t max_probe,
-                               unsigned long long *counters, cudaStream_t st)
-{
-    if (!n) return cudaSuccess;
-    note_launch();
-    k_insert_list<<<grid_for(n, 256), 256, 0, st>>>(keys, n, t, max_probe, counters);
     return cudaGetLastError();
 }
 

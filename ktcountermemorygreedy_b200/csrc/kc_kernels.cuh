@@ -30,8 +30,7 @@ constexpr unsigned long long ERR_HIST_OVERFLOW_FULL = 1ull << 4;
 // indexes into the per-job device counter block (unsigned long long each)
 enum Counter : int {
     C_FLAGS = 0,
-    C_LOW_LEN = 1,       // Bloom FIRST occurrences (low list, front of the list buffer)
-    C_HIGH_LEN = 2,      // other occurrences (back of the list buffer)
+    C_HIGH_LEN = 2,      // k > 32: occurrences inserted
     C_EMIT_LEN = 3,      // plain occurrence list (testing entry point)
     C_REC_LEN = 4,       // output records
     C_LOW_ONLY = 5,      // low k-mers absent from the table (final count 1); prefix path: k-mers seen once
@@ -100,12 +99,7 @@ struct ExtractArgs {
     // insert mode
     const TableRef *tables;         // per sample
     uint32_t max_probe;
-    // bloom mode (single sample)
-    const unsigned long long *bloom_off;   // 256 word offsets
-    const unsigned long long *bloom_cap;   // 256 capacities (blocks of two words)
-    unsigned long long *bloom_bits;
-    uint32_t *hll_high;             // HLL registers of the non-FIRST occurrences
-    // emit / bloom / part output list
+    // emit / part output list
     unsigned long long *list;
     unsigned long long list_cap;
     // buckets (single sample): SCAN counts, launch_part scatters
@@ -125,7 +119,7 @@ struct ExtractArgs {
     const unsigned long long *bucket_end;     // 256 end offsets in `list` (launch_part)
 };
 
-enum ExtractMode : int { MODE_SCAN = 0, MODE_INSERT = 1, MODE_BLOOM = 2, MODE_EMIT = 3 };
+enum ExtractMode : int { MODE_SCAN = 0, MODE_INSERT = 1, MODE_EMIT = 3 };
 
 constexpr uint32_t WORK_ITEM_KEYS = 2048;   // k-mers per work item (8 per thread)
 constexpr uint32_t BUCKET_HLL_BITS = 10;    // HyperLogLog registers per bucket = 2^10
@@ -210,10 +204,7 @@ cudaError_t launch_scan_u32(const uint32_t *in, unsigned long long *out, uint64_
 
 cudaError_t launch_init_slots(Slot *slots, uint64_t n, cudaStream_t st);
 cudaError_t launch_count_keys(const Slot *slots, uint64_t n, unsigned long long *out, cudaStream_t st);
-cudaError_t launch_fill_u64(unsigned long long *p, uint64_t n, unsigned long long v, cudaStream_t st);
 cudaError_t launch_add_u64(unsigned long long *dst, const unsigned long long *src, uint64_t n, cudaStream_t st);
-cudaError_t launch_insert_list(const unsigned long long *keys, uint64_t n, TableRef t, uint32_t max_probe,
-                               unsigned long long *counters, cudaStream_t st);
 cudaError_t launch_insert_pairs(const unsigned long long *keys, const uint32_t *counts, uint64_t n, TableRef t,
                                 uint32_t max_probe, unsigned long long *counters, cudaStream_t st);
 cudaError_t launch_merge_low(const unsigned long long *keys, uint64_t n, TableRef t, uint32_t max_probe,
@@ -292,11 +283,7 @@ constexpr uint64_t MSD_SORT_MIN_RECORDS = 1ull << 20;
 bool msd_sort_applies(uint64_t n, uint32_t bits);
 size_t msd_sort_tmp_bytes(uint64_t n, uint32_t bits);
 cudaError_t launch_msd_sort(unsigned long long *keys, uint32_t *vals, uint64_t n, uint32_t bits, void *tmp,
-                            cudaStream_t st, unsigned long long *flags, bool input_in_tmp, bool reverse_out = false,
-                            const uint32_t *hist16 = nullptr);
-// hist16: when not NULL, the records per value of the keys' top 16 bits
-// (key >> (bits - 16), 65536 counts) made while the records were written;
-// the sort then reads no key for its bucket histogram.
+                            cudaStream_t st, unsigned long long *flags, bool input_in_tmp, bool reverse_out = false);
 // Counts one kernel launch of this library (kernels launched outside kc_kernels.cu).
 void note_kernel_launch();
 

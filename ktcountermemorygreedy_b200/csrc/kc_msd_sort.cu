@@ -86,18 +86,6 @@ __global__ void __launch_bounds__(256) k_msd_hist(const unsigned long long *keys
         atomicAdd(&hb[(uint32_t)(__ldcs(&keys[i]) >> shift) & bmask], 1u);
 }
 
-// hb[b] = the 2^(16 - P) counts of hist16 under bucket b (the top P of the
-// key's top 16 bits).
-__global__ void k_msd_hist_fold(const uint32_t *hist16, uint32_t p_bits, uint32_t *hb)
-{
-    const uint32_t nb = 1u << p_bits, per = 1u << (16 - p_bits);
-    for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
-        uint32_t c = 0;
-        for (uint32_t j = 0; j < per; ++j) c += hist16[b * per + j];
-        hb[b] = c;
-    }
-}
-
 // Stable ranks of the items of one block among the items with the same digit,
 // in item order: items are blocked per warp (warp w holds items
 // w * per_warp + r * 32 + lane, r < steps), so per-warp digit counters taken
@@ -421,8 +409,7 @@ size_t msd_sort_tmp_bytes(uint64_t n, uint32_t bits)
 }
 
 cudaError_t launch_msd_sort(unsigned long long *keys, uint32_t *vals, uint64_t n, uint32_t bits, void *tmp,
-                            cudaStream_t st, unsigned long long *flags, bool input_in_tmp, bool reverse_out,
-                            const uint32_t *hist16)
+                            cudaStream_t st, unsigned long long *flags, bool input_in_tmp, bool reverse_out)
 {
     if (!msd_sort_applies(n, bits)) return cudaErrorInvalidValue;
     const uint32_t P = msd_prefix_bits(n, bits), P2 = P - 8;
@@ -460,10 +447,7 @@ cudaError_t launch_msd_sort(unsigned long long *keys, uint32_t *vals, uint64_t n
     if (e == cudaSuccess) e = cudaMemsetAsync(tile_ctr, 0, 16, st);
     if (e != cudaSuccess) return e;
     note_kernel_launch();
-    if (hist16 && P <= 16)
-        k_msd_hist_fold<<<(unsigned)((nb + 255) / 256), 256, 0, st>>>(hist16, P, hb);
-    else
-        k_msd_hist<<<n_sms() * 8, 256, 0, st>>>(ka, n, shift2, (uint32_t)(nb - 1), hb);
+    k_msd_hist<<<n_sms() * 8, 256, 0, st>>>(ka, n, shift2, (uint32_t)(nb - 1), hb);
     e = launch_scan_u32(hb, ob, nb, stmp, st);
     if (e != cudaSuccess) return e;
     // the bucket sizes come to the host once: the second pass's tiles follow
