@@ -180,12 +180,14 @@ typedef struct {
 typedef struct {
     double bucket_table_factor;   /* table slots per estimated key, per-bucket tables of the partitioned
                                      path (filled while in L2); default 3.0 */
-    double table_factor;          /* table slots per estimated key, one-table jobs and batched samples;
+    double table_factor;          /* table slots per estimated key, one-table jobs and batched samples in
+                                     global memory;
                                      default 1.6 */
-    uint64_t sort_group_records;  /* records sorted together (kept in L2) by a batch's segmented sort;
+    uint64_t sort_group_records;  /* records sorted together (kept in L2) by the segmented sort of a
+                                     batch counted in global-memory tables;
                                      default 4M */
-    uint64_t bloom_smem;          /* 1 partitions the k-mers (of a job or a batch's samples) by
-                                     their first bases and counts each sub-bucket in a shared-memory table
+    uint64_t bloom_smem;          /* 1 partitions the k-mers (of a job or a batch's samples) by their first
+                                     bases and counts each sub-bucket in a shared-memory table
                                      (no filter: a FIRST occurrence is the one that makes its k-mer's table
                                      entry), 2 uses global-memory filters and tables; default 1 */
     uint64_t record_sort;         /* records counted in global-memory tables, from 1M on: 1 sorts most
@@ -194,7 +196,7 @@ typedef struct {
     uint64_t sampled_region_keys; /* passes of the shared-memory path with at least this many k-mers size
                                      their sub-buckets from a 1-in-8 sample of the k-mers instead of
                                      counting them all (a sub-bucket that outgrows its estimate sends the
-                                     pass back to exact counts); default 64M */
+                                     pass back to exact counts; batches never do); default 64M */
     uint64_t count_shape;         /* block shape of the shared-memory count: 1, 3 = 512-thread blocks, two per
                                      SM, 8192-slot tables; 2, 4 = 256-thread blocks, four per SM, 4096-slot
                                      tables (sub-buckets of half the k-mers); default 1 */
@@ -245,8 +247,9 @@ int kc_release(kc_handle *h, kc_job_id id);
 int kc_cancel(kc_handle *h, kc_job_id id);
 
 /* Batched jobs: every job of the array is counted in one set of device passes
- * (one persistent extraction kernel over all samples' tiles, per-sample
- * tables in one arena); a batch larger than a worker's share of the
+ * (the samples are the buckets of one partition over all samples' tiles, up
+ * to 256 at a time; with kc_tuning.bloom_smem 2, per-sample tables in one
+ * arena); a batch larger than a worker's share of the
  * device-memory budget is cut into consecutive sub-batches of whole samples.
  * Bloom mode is not available here.  ids[i] is the id of jobs[i]; results
  * are read per id as for kc_submit. */
