@@ -112,9 +112,12 @@ constexpr uint64_t SUB_KEYS_TWO_WORDS = 10 * 1024, SUB_KEYS_FOUR_WORDS = 8 * 102
 // all are distinct, where 9K take a failed round and two more: count of a
 // 92M-k-mer batch 3.12 -> 2.26 ms, of 25M k-mers of reads 0.49 -> 0.36, of 20M of
 // assembled sequence 0.56 -> 0.31.  (92M k-mers of one job with 2.8 occurrences
-// each: 0.70 at 16K, 1.01 at 6144.)  A batch's sub-buckets are too small for
-// regions sized from a sample.
-constexpr uint64_t SUB_KEYS_SMALL = 6144, SUB_SMALL_PASS_KEYS = 32ull << 20;
+// each: 0.70 at 16K, 1.01 at 6144.)  A batch's sub-buckets are cut
+// from the whole printed order, whose first half holds three quarters of the
+// canonical k-mers (each is the smaller of two), so the first ones have twice the
+// mean: 4096 (the same batch's count 2.07 at 6144 and 8192's 2.50 -> 1.68 ms; 1.81 at
+// 3072).  They are too small for regions sized from a sample.
+constexpr uint64_t SUB_KEYS_SMALL = 6144, SUB_KEYS_BATCH = 4096, SUB_SMALL_PASS_KEYS = 32ull << 20;
 
 // A plain job whose table would hold more slots than this (64 MiB of slots,
 // half of L2) is counted through the root-prefix buckets.
@@ -397,6 +400,37 @@ uint64_t default_pass_budget(Workspace &ws)
     return (uint64_t)(0.7 * (double)(free_b + ws_free + pool_slack));
 }
 
+// The same for a job that needs `need` bytes in all.  What fits in 70% of the
+// workspace's unused part needs one pass whatever the device has free, and the
+// query of that takes 0.13 ms, a third of the smallest calls.
+uint64_t pass_budget(Workspace &ws, uint64_t need)
+{
+    const size_t ws_free = ws.capacity() > ws.mark().top ? ws.capacity() - ws.mark().top : 0;
+    return (double)need <= 0.7 * (double)ws_free ? need : default_pass_budget(ws);
+}
+
+// Passes over ranges of buckets that need nb[b] bytes each, within the budget
+// (the caller's, or 0: the worker's) or one bucket at least.
+std::vector<std::pair<uint32_t, uint32_t>> pass_ranges(Workspace &ws, const std::vector<uint64_t> &nb, uint64_t budget)
+{
+    uint64_t total = 0;
+    for (uint64_t n : nb) total += n;
+    if (!budget) budget = pass_budget(ws, total);
+    std::vector<std::pair<uint32_t, uint32_t>> ranges;
+    uint32_t lo = 0;
+    uint64_t need = 0;
+    for (uint32_t b = 0; b < N_BUCKETS; ++b) {
+        if (b > lo && need + nb[b] > budget) {
+            ranges.push_back({lo, b});
+            lo = b;
+            need = 0;
+        }
+        need += nb[b];
+    }
+    ranges.push_back({lo, N_BUCKETS});
+    return ranges;
+}
+
 // One counting pass of the prefix path: partitioned string keys -> sorted
 // records, histograms and totals.  The buckets are cut into sub-buckets by the
 // next bases, each counted in a shared-memory table, and its records sorted on
@@ -447,8 +481,10 @@ void count_by_prefix(PrefixPass &pp, DevScope &ds, HostStage &hs, PhaseClock &cl
     uint64_t pass_keys = 0;
     for (uint32_t b = lo; b < hi; ++b) pass_keys += pp.cfg[b].key_len;
     const bool batch = pp.base_bits == 0;
-    const bool small_subs = batch || (N == 1 && pass_keys < SUB_SMALL_PASS_KEYS);
-    const uint64_t one_word = small_subs ? SUB_KEYS_SMALL : (pass_keys < SUB_DEEP_PASS_KEYS ? SUB_KEYS_TARGET : SUB_KEYS_DEEP);
+    const uint64_t one_word = batch                              ? SUB_KEYS_BATCH
+                              : pass_keys < SUB_SMALL_PASS_KEYS ? SUB_KEYS_SMALL
+                              : pass_keys < SUB_DEEP_PASS_KEYS  ? SUB_KEYS_TARGET
+                                                                : SUB_KEYS_DEEP;
     const uint64_t keys_target = (N == 1 ? one_word : (N == 2 ? SUB_KEYS_TWO_WORDS : SUB_KEYS_FOUR_WORDS)) *
                                  sub_table_slots(N, shape) / sub_table_slots(1, 1);
     std::vector<uint32_t> nsub(N_BUCKETS, 0), max_nsub(N_BUCKETS, 1);
@@ -1036,26 +1072,13 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
         }
         // passes over ranges of buckets, each within the device-memory budget
         // of a pass (k-mer arrays, filters, tables, records of its buckets)
-        const uint64_t budget = P.pass_bytes ? P.pass_bytes : default_pass_budget(ws);
         // prefix path: two key arrays and the counts with room for estimated
         // sub-bucket regions (1.25 x (8 + 8 + 4)), then at most n / min count records
         const uint64_t per_occ =
             prefix ? 25 + (12 + std::max(P.min_count, 1u) - 1) / std::max(P.min_count, 1u) : (P.bloom ? 42 : 48);
-        std::vector<std::pair<uint32_t, uint32_t>> ranges;
-        {
-            uint32_t lo = 0;
-            uint64_t need = 0;
-            for (uint32_t b = 0; b < N_BUCKETS; ++b) {
-                const uint64_t nb = region[b] * per_occ + fcap[b] * 16;
-                if (b > lo && need + nb > budget) {
-                    ranges.push_back({lo, b});
-                    lo = b;
-                    need = 0;
-                }
-                need += nb;
-            }
-            ranges.push_back({lo, N_BUCKETS});
-        }
+        std::vector<uint64_t> nb(N_BUCKETS);
+        for (uint32_t b = 0; b < N_BUCKETS; ++b) nb[b] = region[b] * per_occ + fcap[b] * 16;
+        const auto ranges = pass_ranges(ws, nb, P.pass_bytes);
         const bool multi = ranges.size() > 1;
         if (streamed && multi) census_chunks(cu.ev.size());   // every pass reads every tile
         std::vector<std::unique_ptr<HostRecords>> spilled;
@@ -1650,27 +1673,15 @@ void run_wide_job(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
     // records); the final sort holds every record twice plus its temporaries
     const uint64_t slot_bytes = 8ull * nw + 8, rec_bytes = 8ull * nw + 4;
     const double factor = std::max(tn.table_factor, 1.25);
-    const uint64_t budget = P.pass_bytes ? P.pass_bytes : default_pass_budget(ws);
-    std::vector<std::pair<uint32_t, uint32_t>> ranges;
-    {
-        uint32_t lo = 0;
-        uint64_t need = 0;
-        for (uint32_t b = 0; b < N_BUCKETS; ++b) {
-            const double share = O ? (double)bh[b] / (double)O : 0.0;
-            // prefix path: two key arrays and the counts with room for
-            // estimated sub-bucket regions, then at most n / min count records
-            const uint64_t per_key = 20ull * nw + 5 + rec_bytes / std::max(P.min_count, 1u) + 1;
-            const uint64_t nb = prefix ? bh[b] * per_key + 4096
-                                       : (uint64_t)(share * est * (factor * slot_bytes + rec_bytes)) + 4096;
-            if (b > lo && need + nb > budget) {
-                ranges.push_back({lo, b});
-                lo = b;
-                need = 0;
-            }
-            need += nb;
-        }
-        ranges.push_back({lo, N_BUCKETS});
+    std::vector<uint64_t> nb(N_BUCKETS);
+    for (uint32_t b = 0; b < N_BUCKETS; ++b) {
+        const double share = O ? (double)bh[b] / (double)O : 0.0;
+        // prefix path: two key arrays and the counts with room for
+        // estimated sub-bucket regions, then at most n / min count records
+        const uint64_t per_key = 20ull * nw + 5 + rec_bytes / std::max(P.min_count, 1u) + 1;
+        nb[b] = prefix ? bh[b] * per_key + 4096 : (uint64_t)(share * est * (factor * slot_bytes + rec_bytes)) + 4096;
     }
+    const auto ranges = pass_ranges(ws, nb, P.pass_bytes);
     const bool multi = ranges.size() > 1;
     unsigned long long *hist = ds.n<unsigned long long>(HIST_BINS);
     CK(cudaMemsetAsync(hist, 0, HIST_BINS * 8, st));
@@ -2149,11 +2160,13 @@ void run_batch_once(std::vector<std::shared_ptr<Job>> &jobs, cudaStream_t st, Wo
         // sample is one bucket, and its k-mers' string keys are cut into
         // sub-buckets by their first bases
         HostStage hs(st);
-        const uint64_t budget = default_pass_budget(ws);
         const auto bytes_of = [&](uint32_t i) {
             const uint64_t m = std::max(jobs[i]->p.min_count, 1u);
             return occ_h[i] * (25 + (12 + m - 1) / m);
         };
+        uint64_t all = 0;
+        for (uint32_t i = 0; i < n; ++i) all += bytes_of(i);
+        const uint64_t budget = pass_budget(ws, all);
         for (uint32_t lo = 0; lo < n;) {
             uint64_t need = bytes_of(lo);
             if (need > budget) throw SubTablesFull{};   // its table of distinct k-mers may be smaller
