@@ -1479,36 +1479,53 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
                     if (c == 0) break;
                 }
             }
-            // the records above the threshold, and the first ones at it
-            unsigned long long *ak = ds.n<unsigned long long>(P.top_n);
-            uint32_t *ac = ds.n<uint32_t>(P.top_n);
-            unsigned long long *bk = ds.n<unsigned long long>(P.top_n);
-            uint32_t *bc = ds.n<uint32_t>(P.top_n);
-            const SelectRange at_thr{thr, thr, P.top_n, bk, bc, C_SEL_B};
-            const SelectRange sel[2] = {at_thr, SelectRange{thr + 1, 0xffffffffu, P.top_n, ak, ac, C_SEL_A}};
+            // the first records at the threshold, then those above it.  Of a
+            // top-N of ordinary size all places come back with their numbers
+            // under one wait (0.04 ms less than numbers first, then four copies)
+            const uint64_t q = std::min<uint64_t>(P.top_n, n_rec);
+            unsigned long long *sk = ds.n<unsigned long long>(2 * q);
+            uint32_t *sc = ds.n<uint32_t>(2 * q);
+            const SelectRange sel[2] = {SelectRange{thr, thr, q, sk, sc, C_SEL_B},
+                                        SelectRange{thr + 1, 0xffffffffu, q, sk + q, sc + q, C_SEL_A}};
             CK(cudaMemsetAsync(&counters[C_SEL_A], 0, 8, st));
             CK(launch_select(rec_keys, rec_counts, n_rec, sel, thr < 0xffffffffu ? 2 : 1, qtmp, counters, st));
-            const Counters ca = read_counters(counters, st);
-            const uint64_t n_above = std::min<uint64_t>(ca.v[C_SEL_A], P.top_n);
-            const uint64_t n_at = std::min<uint64_t>(ca.v[C_SEL_B], P.top_n - n_above);
-            std::vector<uint64_t> tk(n_above), tk2(n_at);
-            std::vector<uint32_t> tc(n_above), tc2(n_at);
-            if (n_above) {
-                CK(cudaMemcpyAsync(tk.data(), ak, n_above * 8, cudaMemcpyDeviceToHost, st));
-                CK(cudaMemcpyAsync(tc.data(), ac, n_above * 4, cudaMemcpyDeviceToHost, st));
+            const bool one_wait = q <= (1u << 16);
+            std::vector<unsigned long long> big_k;
+            std::vector<uint32_t> big_c;
+            unsigned long long *tk = nullptr, *n_sel = hs.n<unsigned long long>(C_COUNT);
+            uint32_t *tc = nullptr;
+            if (one_wait) {
+                tk = hs.n<unsigned long long>(2 * q);
+                tc = hs.n<uint32_t>(2 * q);
+                CK(cudaMemcpyAsync(tk, sk, 2 * q * 8, cudaMemcpyDeviceToHost, st));
+                CK(cudaMemcpyAsync(tc, sc, 2 * q * 4, cudaMemcpyDeviceToHost, st));
             }
-            if (n_at) {
-                CK(cudaMemcpyAsync(tk2.data(), bk, n_at * 8, cudaMemcpyDeviceToHost, st));
-                CK(cudaMemcpyAsync(tc2.data(), bc, n_at * 4, cudaMemcpyDeviceToHost, st));
-            }
+            CK(cudaMemcpyAsync(n_sel, counters, C_COUNT * 8, cudaMemcpyDeviceToHost, st));
             CK(cudaStreamSynchronize(st));
+            const uint64_t n_above = std::min<uint64_t>(n_sel[C_SEL_A], q);
+            const uint64_t n_at = std::min<uint64_t>(n_sel[C_SEL_B], q - n_above);
+            if (!one_wait) {
+                big_k.resize(2 * q);
+                big_c.resize(2 * q);
+                tk = big_k.data();
+                tc = big_c.data();
+                if (n_above) {
+                    CK(cudaMemcpyAsync(tk + q, sk + q, n_above * 8, cudaMemcpyDeviceToHost, st));
+                    CK(cudaMemcpyAsync(tc + q, sc + q, n_above * 4, cudaMemcpyDeviceToHost, st));
+                }
+                if (n_at) {
+                    CK(cudaMemcpyAsync(tk, sk, n_at * 8, cudaMemcpyDeviceToHost, st));
+                    CK(cudaMemcpyAsync(tc, sc, n_at * 4, cudaMemcpyDeviceToHost, st));
+                }
+                CK(cudaStreamSynchronize(st));
+            }
             // records above the threshold: count desc, then printed string asc
             // (they arrive in printed-string order; a stable sort keeps it)
             std::vector<size_t> idx(n_above);
             for (size_t i = 0; i < n_above; ++i) idx[i] = i;
-            std::stable_sort(idx.begin(), idx.end(), [&](size_t x, size_t y) { return tc[x] > tc[y]; });
-            for (size_t i : idx) { job.top_keys.push_back(tk[i]); job.top_counts.push_back(tc[i]); }
-            for (size_t i = 0; i < n_at; ++i) { job.top_keys.push_back(tk2[i]); job.top_counts.push_back(tc2[i]); }
+            std::stable_sort(idx.begin(), idx.end(), [&](size_t x, size_t y) { return tc[q + x] > tc[q + y]; });
+            for (size_t i : idx) { job.top_keys.push_back(tk[q + i]); job.top_counts.push_back(tc[q + i]); }
+            for (size_t i = 0; i < n_at; ++i) { job.top_keys.push_back(tk[i]); job.top_counts.push_back(tc[i]); }
         }
         if (P.want_le2 && n_rec) {
             unsigned long long *lk = ds.n<unsigned long long>(n_rec);

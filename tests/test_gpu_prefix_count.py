@@ -265,3 +265,18 @@ def test_wide_runs_that_start_alike(counter, k, same):
     r = counter.count([f], k=k, count_max=U32)
     assert r.smem_passes == 1
     assert np.array_equal(r.keys, all_k) and np.array_equal(r.counts, all_c)
+
+
+@pytest.mark.parametrize("top_n", [1, 65_535, 65_536, 65_537, 90_000, 200_000])
+def test_top_n_on_both_sides_of_one_wait(counter, top_n):
+    """Top-N lists up to 65536 come back with their lengths, longer ones after
+    them; lists shorter than N (fewer records) too."""
+    rng = np.random.default_rng(5)
+    bases = np.frombuffer(b"ACGT", np.uint8)
+    reads = bases[rng.integers(0, 4, size=(900, 150))]
+    fq = b"".join(b"@r\n" + r.tobytes() + b"\n+\n" + b"I" * 150 + b"\n" for i, r in enumerate(reads) for _ in range(1 + i % 3))
+    all_k, all_c = O.exact_records([fq], 31, U32)
+    assert 100_000 < len(all_c) < 200_000
+    order = np.argsort(-all_c.astype(np.int64), kind="stable")[:top_n]
+    r = counter.count([fq], k=31, count_max=U32, top_n=top_n)
+    assert np.array_equal(r.top_keys, all_k[order]) and np.array_equal(r.top_counts, all_c[order])
