@@ -501,7 +501,7 @@ void count_by_prefix(PrefixPass &pp, DevScope &ds, HostStage &hs, PhaseClock &cl
     // a large pass sizes the sub-buckets' regions from a sample of its keys
     // instead of counting them all; a sub-bucket that outgrows its region sends
     // the pass back to exact counts
-    bool exact_regions = false;
+    bool exact_regions = false, all_units = false;
     for (int attempt = 0;; ++attempt) {
         const DevScope::Mark m0 = ds.mark();
         std::vector<uint8_t> sb;
@@ -536,8 +536,8 @@ void count_by_prefix(PrefixPass &pp, DevScope &ds, HostStage &hs, PhaseClock &cl
         // their own unless nothing else is in the histogram
         const size_t hist_n = (size_t)pp.n_groups * pp.hist_bins;
         unsigned long long *hist_sub = pp.hist_zero ? pp.hist : ds.n<unsigned long long>(hist_n);
-        const uint32_t unit_cap = 2 * n_sub + 4096;
-        SubUnit *units = ds.n<SubUnit>((size_t)UNIT_CLASSES * unit_cap);
+        const UnitLists lists = unit_lists(pp.n_keys, n_sub, N, all_units);
+        SubUnit *units = ds.n<SubUnit>(lists.total);
         const bool sampled = !exact_regions && !batch && pp.n_keys >= tn.sampled_region_keys;
         const uint32_t stride = sampled ? SUB_REGION_SAMPLE : 1;
         // one upload: the 256 ranges of each bucket-major launch (not lists of
@@ -590,7 +590,7 @@ void count_by_prefix(PrefixPass &pp, DevScope &ds, HostStage &hs, PhaseClock &cl
         pc.rec_counts = pp.tmp_counts;
         pc.sub_len = sub_len;
         pc.units = units;
-        pc.unit_cap = unit_cap;
+        pc.lists = lists;
         pc.hist_bins = pp.hist_bins;
         pc.hist = hist_sub;
         pc.totals = totals;
@@ -610,7 +610,7 @@ void count_by_prefix(PrefixPass &pp, DevScope &ds, HostStage &hs, PhaseClock &cl
         CK(cudaMemcpyAsync(p_tot, totals, 3ull * pp.n_groups * 8, cudaMemcpyDeviceToHost, st));
         const Counters cs = read_counters(counters, st);
         check_flags(cs.v[C_FLAGS], "sub-bucket count");
-        if (cs.v[C_REGION_OVF] || cs.v[C_SUB_OVF]) {
+        if (cs.v[C_REGION_OVF] || cs.v[C_SUB_OVF] || cs.v[C_UNIT_OVF]) {
             std::vector<uint32_t> bo(N_BUCKETS);
             CK(cudaMemcpyAsync(bo.data(), bucket_ovf, N_BUCKETS * 4, cudaMemcpyDeviceToHost, st));
             CK(cudaMemcpyAsync(counters + C_OVF_LEN, ovf_len_saved, 8, cudaMemcpyDeviceToDevice, st));
@@ -622,6 +622,12 @@ void count_by_prefix(PrefixPass &pp, DevScope &ds, HostStage &hs, PhaseClock &cl
                 // leaves the keys alone): exact regions, same sub-buckets
                 exact_regions = true;
                 ++pp.region_redos;
+            } else if (!cs.v[C_SUB_OVF]) {
+                // more units than the lists hold: room for all there can be
+                all_units = true;
+                clk.begin(2);
+                pp.repartition();   // the records went over the partitioned keys
+                clk.end();
             } else {
                 // buckets with more distinct k-mers than 64 rounds of their
                 // sub-buckets hold: 16 times the sub-buckets
@@ -651,7 +657,7 @@ void count_by_prefix(PrefixPass &pp, DevScope &ds, HostStage &hs, PhaseClock &cl
         CK(launch_scan_u32(sub_len, sub_cur, n_sub, sub_tmp, st));
         uint32_t n_units[UNIT_CLASSES];
         for (uint32_t c = 0; c < UNIT_CLASSES; ++c) n_units[c] = (uint32_t)cs.v[C_UNITS + c];
-        CK(launch_unit_sort(N, pp.keys, pp.tmp_counts, sub_off, sub_cur, units, unit_cap, n_units, pp.rec_keys,
+        CK(launch_unit_sort(N, pp.keys, pp.tmp_counts, sub_off, sub_cur, units, lists, n_units, pp.rec_keys,
                             pp.rec_counts, pp.n_rec, st));
         clk.end();
         pp.n_sub = n_sub;

@@ -36,7 +36,6 @@ namespace {
 constexpr uint32_t FULLW = 0xffffffffu;
 constexpr uint32_t CP_HIST = 512;           // counts below this are histogrammed in shared memory
 constexpr uint32_t CP_QUEUE = 64;           // keys a warp has waiting for their next probe
-constexpr uint32_t CP_MAX_ROUNDS = 64;      // rounds a sub-bucket may be cut into
 
 __device__ __forceinline__ uint32_t lanes_below()
 {
@@ -141,7 +140,7 @@ constexpr uint32_t SLOT_CLAIMED = 1u << 31, SLOT_PUBLISHED = 1u << 30, SLOT_COUN
 // and shared-memory wavefronts (60%).
 // A table that fills up (more distinct k-mers than it holds) is
 // emptied and the sub-bucket counted in rounds over halves of its key range
-// (quarters, ... at most CP_MAX_ROUNDS), each round reading the keys again
+// (quarters, ... at most SUB_MAX_ROUNDS), each round reading the keys again
 // from L2; a round's records lie after the earlier rounds' ones, and are a
 // sort unit of their own.  The next sub-bucket's first keys are loaded before
 // the sweep.  Histogram and totals go to the sub-bucket's group.
@@ -398,7 +397,7 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
                 failed = true;
                 rounds *= 2;
                 rd *= 2;
-                if (rounds > CP_MAX_ROUNDS || (int)cfg.plen + (31 - __clz(rounds)) > 64) break;
+                if (rounds > SUB_MAX_ROUNDS || (int)cfg.plen + (31 - __clz(rounds)) > 64) break;
                 continue;
             }
             // the next sub-bucket's first keys arrive during the sweep
@@ -438,10 +437,10 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
                     keep = c >= keep_lo && c <= keep_hi;
                 }
                 const uint32_t b = __ballot_sync(FULLW, keep);
+                uint32_t at0 = 0;
+                if (lane == 0) at0 = atomicAdd(&s_out, (m << 16) + (uint32_t)__popc(b));
                 if (b) {
-                    uint32_t w = 0;
-                    if (lane == 0) w = atomicAdd(&s_out, (uint32_t)__popc(b));
-                    w = __shfl_sync(FULLW, w, 0);
+                    const uint32_t w = __shfl_sync(FULLW, at0, 0) & 0xFFFFu;
                     if (keep) {
                         const unsigned long long at = out + w + (uint32_t)__popc(b & lt);
                         if constexpr (N > 1) key = load_key<N>(s_tk, i, LoadPlain());
@@ -467,7 +466,8 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
             }
             if (un) take_used(un);
             __syncthreads();
-            const uint32_t len = s_out;
+            static_assert(SLOTS < 65536, "a round's distinct k-mers and records in one word");
+            const uint32_t len = s_out & 0xFFFFu, held = s_out >> 16;
             __syncthreads();
             if (tid == 0) {
                 s_out = 0;
@@ -475,13 +475,13 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
                     constexpr uint32_t CAP0 = unit_cap0(N);
                     const uint32_t cls = len <= CAP0 ? 0 : (len <= 2 * CAP0 ? 1 : (len <= 4 * CAP0 ? 2 : 3));
                     const unsigned long long u = atomicAdd(&a.counters[C_UNITS + cls], 1ull);
-                    if (u < a.unit_cap) a.units[cls * (uint64_t)a.unit_cap + u] = SubUnit{sub, off, len, cfg.k};
-                    else ++s_ovf;   // more sort units than the lists hold: counted as an overflow
+                    if (u < a.lists.cap[cls]) a.units[a.lists.base[cls] + u] = SubUnit{sub, off, len, cfg.k};
+                    else atomicOr(&a.counters[C_UNIT_OVF], 1ull);
                     s_kept += len;
                 }
             }
             off += len;
-            most = len > most ? len : most;
+            most = held > most ? held : most;
             ++rd;
         }
         const bool gave_up = rd < rounds;   // uniform
@@ -492,9 +492,16 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
                 atomicOr(&a.bucket_ovf[a.sub_bucket[sub]], 1u);
             }
         }
-        // sub-buckets are alike: the next one starts with as many rounds,
-        // or with half as many when no round came near the table's size
-        rounds0 = gave_up ? 1u : (rounds > 1 && most < SLOTS / 4 ? rounds / 2 : rounds);
+        // sub-buckets are alike: the next one starts with as many rounds, or with
+        // fewer when as large a share of its keys as were distinct here would
+        // fill no more than 7/8 of a table in any of them (a table takes about
+        // 94%, where a probe takes three steps on average).  Rounds that only
+        // came down below a quarter of a table stayed at four for sub-buckets
+        // of 8K to 16K distinct k-mers, which two hold.
+        rounds0 = gave_up || !n ? 1u : rounds;
+        while (rounds0 > 1 && (unsigned long long)most * rounds * s_next_n <=
+                                  (unsigned long long)(SLOTS - SLOTS / 8) * (rounds0 / 2) * n)
+            rounds0 /= 2;
         if (too_many) __syncthreads();   // thread 0 has taken the next sub-bucket
         if (gave_up) load_first(s_next_off, s_next < a.n_sub ? s_next_n : 0u);
         sub = s_next;
@@ -824,22 +831,22 @@ cudaError_t launch_unit_sort_t(const unsigned long long *tk, const uint32_t *tv,
 
 template <uint32_t N>
 cudaError_t launch_unit_sort_n(const unsigned long long *tk, const uint32_t *tv, const unsigned long long *sub_off,
-                               const unsigned long long *sub_final, const SubUnit *units, uint32_t unit_cap,
+                               const unsigned long long *sub_final, const SubUnit *units, const UnitLists &lists,
                                const uint32_t *n_units, unsigned long long *out_k, uint32_t *out_v, uint64_t out_cap,
                                cudaStream_t st)
 {
     constexpr uint32_t C = unit_cap0(N);
     static_assert(UNIT_CLASSES == 4, "one launch per class");
-    cudaError_t e = launch_unit_sort_t<N, 256, C, 9>(tk, tv, sub_off, sub_final, units, n_units[0], out_k, out_v, out_cap,
+    cudaError_t e = launch_unit_sort_t<N, 256, C, 9>(tk, tv, sub_off, sub_final, units + lists.base[0], n_units[0], out_k, out_v, out_cap,
                                                      st);
     if (e == cudaSuccess)
-        e = launch_unit_sort_t<N, 256, 2 * C, 10>(tk, tv, sub_off, sub_final, units + unit_cap, n_units[1], out_k, out_v,
+        e = launch_unit_sort_t<N, 256, 2 * C, 10>(tk, tv, sub_off, sub_final, units + lists.base[1], n_units[1], out_k, out_v,
                                                   out_cap, st);
     if (e == cudaSuccess)
-        e = launch_unit_sort_t<N, 512, 4 * C, 11>(tk, tv, sub_off, sub_final, units + 2ull * unit_cap, n_units[2], out_k,
+        e = launch_unit_sort_t<N, 512, 4 * C, 11>(tk, tv, sub_off, sub_final, units + lists.base[2], n_units[2], out_k,
                                                   out_v, out_cap, st);
     if (e == cudaSuccess)
-        e = launch_unit_sort_t<N, 512, 8 * C, 11>(tk, tv, sub_off, sub_final, units + 3ull * unit_cap, n_units[3], out_k,
+        e = launch_unit_sort_t<N, 512, 8 * C, 11>(tk, tv, sub_off, sub_final, units + lists.base[3], n_units[3], out_k,
                                                   out_v, out_cap, st);
     return e;
 }
@@ -859,14 +866,14 @@ cudaError_t launch_count_prefix(const PrefixCountArgs &a, uint32_t words, uint32
 
 cudaError_t launch_unit_sort(uint32_t words, const unsigned long long *tk, const uint32_t *tv,
                              const unsigned long long *sub_off, const unsigned long long *sub_final,
-                             const SubUnit *units, uint32_t unit_cap, const uint32_t *n_units,
+                             const SubUnit *units, const UnitLists &lists, const uint32_t *n_units,
                              unsigned long long *out_k, uint32_t *out_v, uint64_t out_cap, cudaStream_t st)
 {
     if (words == 1)
-        return launch_unit_sort_n<1>(tk, tv, sub_off, sub_final, units, unit_cap, n_units, out_k, out_v, out_cap, st);
+        return launch_unit_sort_n<1>(tk, tv, sub_off, sub_final, units, lists, n_units, out_k, out_v, out_cap, st);
     if (words == 2)
-        return launch_unit_sort_n<2>(tk, tv, sub_off, sub_final, units, unit_cap, n_units, out_k, out_v, out_cap, st);
-    return launch_unit_sort_n<4>(tk, tv, sub_off, sub_final, units, unit_cap, n_units, out_k, out_v, out_cap, st);
+        return launch_unit_sort_n<2>(tk, tv, sub_off, sub_final, units, lists, n_units, out_k, out_v, out_cap, st);
+    return launch_unit_sort_n<4>(tk, tv, sub_off, sub_final, units, lists, n_units, out_k, out_v, out_cap, st);
 }
 
 }  // namespace kc

@@ -41,6 +41,7 @@ enum Counter : int {
     C_SUB_OVF = 10,      // sub-buckets whose shared-memory table overflowed
     C_REGION_OVF = 11,   // nonzero: a sub-bucket outgrew its estimated region
     C_KEPT = 12,         // records a counting compaction pass would keep
+    C_UNIT_OVF = 13,     // nonzero: more sort units of a class than its list holds
     C_UNITS = 16,        // UNIT_CLASSES counts: sort units by size
     C_COUNT = 24
 };
@@ -341,18 +342,42 @@ cudaError_t launch_subpart_sizes(const unsigned long long *sub_off, const unsign
 // bucket's SubCfg) go to rec_keys / rec_counts from sub_off[s] on, unsorted
 // within each of its sort units; sub_len[s] receives their number.  A unit is
 // the run [off, off + len) of a sub-bucket's records; the units of size class c
-// (len <= unit_cap0(words) << c) are listed at units[c * unit_cap], C_UNITS + c
+// (len <= unit_cap0(words) << c) are listed from units[lists.base[c]] on, C_UNITS + c
 // of them.  Every k-mer's count goes to the group's histogram (hist_bins bins
 // at hist + group * hist_bins; larger counts to ovf, or with their group to
 // ovf64), totals to totals[3 * group ..]: distinct k-mers, k-mers seen once,
-// records.  Sub-buckets that no number of rounds fits, and more units than
-// unit_cap, are counted in C_SUB_OVF (and bucket_ovf[their bucket]): the
-// results are then incomplete.
+// records.  Sub-buckets that no number of rounds fits are counted in C_SUB_OVF
+// (and bucket_ovf[their bucket]), more units of a class than lists.cap[c] set
+// C_UNIT_OVF: the results are then incomplete.
 constexpr uint32_t UNIT_CLASSES = 4;
 __host__ __device__ constexpr uint32_t unit_cap0(uint32_t words) { return 1024u / words; }
 struct SubUnit {
     uint32_t sub, off, len, k;
 };
+constexpr uint32_t SUB_MAX_ROUNDS = 64;   // rounds a sub-bucket may be cut into, each a unit
+// Room for the units of n_keys keys in n_sub sub-buckets, class by class.  A
+// unit of a class from 1 on has more than unit_cap0 << (c - 1) records of keys of
+// its own, so their lists hold whatever comes.  Class 0 has room for two units a
+// sub-bucket; more of them (sub-buckets cut into many rounds, unevenly) set
+// C_UNIT_OVF, and `all` then gives each its SUB_MAX_ROUNDS.
+struct UnitLists {
+    uint64_t base[UNIT_CLASSES];
+    uint32_t cap[UNIT_CLASSES];
+    uint64_t total;
+};
+inline UnitLists unit_lists(uint64_t n_keys, uint32_t n_sub, uint32_t words, bool all)
+{
+    UnitLists u{};
+    for (uint32_t c = 0; c < UNIT_CLASSES; ++c) {
+        uint64_t n = c ? n_keys / (unit_cap0(words) << (c - 1)) + 1
+                       : (all ? (uint64_t)SUB_MAX_ROUNDS * n_sub : 2ull * n_sub + 4096);
+        n = n < 0xFFFFFFFFull ? n : 0xFFFFFFFFull;
+        u.base[c] = u.total;
+        u.cap[c] = (uint32_t)n;
+        u.total += n;
+    }
+    return u;
+}
 struct PrefixCountArgs {
     const unsigned long long *keys, *sub_off;
     const uint32_t *sub_count;
@@ -363,7 +388,8 @@ struct PrefixCountArgs {
     unsigned long long *rec_keys;
     uint32_t *rec_counts, *sub_len;
     SubUnit *units;
-    uint32_t unit_cap, hist_bins;
+    UnitLists lists;
+    uint32_t hist_bins;
     unsigned long long *hist, *totals;
     uint32_t *ovf;
     unsigned long long *ovf64;
@@ -385,7 +411,7 @@ inline uint32_t sub_table_slots(uint32_t words, uint32_t shape)
 // n_units: units per class (host values).
 cudaError_t launch_unit_sort(uint32_t words, const unsigned long long *tk, const uint32_t *tv,
                              const unsigned long long *sub_off, const unsigned long long *sub_final,
-                             const SubUnit *units, uint32_t unit_cap, const uint32_t *n_units,
+                             const SubUnit *units, const UnitLists &lists, const uint32_t *n_units,
                              unsigned long long *out_k, uint32_t *out_v, uint64_t out_cap, cudaStream_t st);
 cudaError_t launch_bloom_buckets(const unsigned long long *keys, const BucketRanges *rg, uint32_t n_items,
                                  unsigned int *next_item, const BucketCfg *cfg, unsigned long long *bits,
