@@ -153,8 +153,8 @@ typedef struct {
      * (plain) or scatter into the 256 buckets, [3] insert of the non-FIRST
      * k-mers, [4] merge of the FIRST k-mers, [5] compaction + histogram, [6]
      * sort of the records, [7] queries, [8] Bloom classification, [9] scatter
-     * of the buckets into sub-buckets and [10] their count in shared memory
-     * (prefix path), [11] packing of the high.bin records (kc_job.pack_high) */
+     * of the buckets into sub-buckets and [10] their count in shared memory,
+     * crowded ones' by sorting (prefix path), [11] packing of the high.bin records (kc_job.pack_high) */
     double phase_ms[KC_STAGES];
     uint64_t phase_launches[KC_STAGES];   /* kernel launches per stage */
     uint64_t low_len;             /* Bloom mode: FIRST occurrences */
@@ -163,9 +163,12 @@ typedef struct {
     uint64_t input_bytes;         /* FASTQ bytes of the job */
     uint64_t n_records_total;     /* records on the device (also when keep_records = 0) */
     uint32_t passes;              /* counting passes over ranges of root prefixes (1: the whole job at once) */
-    uint16_t smem_passes;         /* passes counted by printed-order prefix in shared memory */
-    uint16_t smem_fallbacks;      /* passes counted on global-memory tables because sub-buckets had more
-                                     distinct k-mers than their tables hold */
+    uint16_t smem_passes;         /* passes counted by printed-order prefix in shared memory (all but at
+                                     most an eighth of their k-mers) */
+    uint16_t smem_fallbacks;      /* passes of which more than an eighth of the k-mers were counted in global
+                                     memory, in sub-buckets with more distinct k-mers than a table holds
+                                     (sorted on their own), or all, where the device's memory is too small
+                                     for the partitioned k-mers (tables) */
     uint32_t region_redos;        /* shared-memory passes counted again because a sub-bucket outgrew the
                                      region estimated from a sample of the pass's keys */
     uint32_t batch_part;          /* batched jobs: the sub-batch (0, 1, ...) the sample was counted in; a

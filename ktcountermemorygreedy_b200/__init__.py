@@ -223,7 +223,7 @@ class Result:
     n_records_total: int = 0
     passes: int = 1
     smem_passes: int = 0      # passes counted per sub-bucket in shared memory
-    smem_fallbacks: int = 0   # passes counted on global-memory tables after sub-bucket tables overflowed
+    smem_fallbacks: int = 0   # passes with more than an eighth of their k-mers counted in global memory
     region_redos: int = 0     # shared-memory passes counted again after a sub-bucket outgrew its estimated region
     batch_part: int = 0       # batched jobs: the sub-batch the sample was counted in
 

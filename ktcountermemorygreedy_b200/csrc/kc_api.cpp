@@ -374,9 +374,8 @@ struct HostStage {
 // A bucket outgrew the region estimated from the sampled census.
 struct CensusOverflow {};
 
-// A sub-bucket of the prefix path holds more distinct k-mers than its rounds
-// can count and its bucket cannot be cut further: the job is counted again on
-// global-memory tables.
+// What the prefix path needs does not fit the device's memory (or its 32-bit
+// counts): the job is counted again on global-memory tables.
 struct SubTablesFull {};
 
 // Device memory one counting pass may use: 70% of the free device memory, the
@@ -435,10 +434,10 @@ std::vector<std::pair<uint32_t, uint32_t>> pass_ranges(Workspace &ws, const std:
 // records, histograms and totals.  The buckets are cut into sub-buckets by the
 // next bases, each counted in a shared-memory table, and its records sorted on
 // their own.  A bucket (a batch's sample, base_bits 0) starts with at most
-// the k-mers per sub-bucket that the pass's size and words call for; one whose
-// sub-buckets no number of rounds fits is cut into 16 times as many and the pass
-// counted again, and a bucket that cannot be cut further is reported by
-// SubTablesFull.
+// the k-mers per sub-bucket that the pass's size and words call for.  Sub-buckets
+// that fit no table (crowded ones) are counted by sorting their keys; when they
+// hold more than 1 in CROWD_SHARE of the pass's keys, their buckets are first cut
+// into 16 times as many, as long as they can be, and the pass counted again.
 struct PrefixPass {
     uint32_t words = 1;                 // 64-bit words per key
     uint32_t lo = 0, hi = 0;            // its buckets; their keys are cfg[b].key_base, key_len
@@ -465,12 +464,112 @@ struct PrefixPass {
     uint32_t *rec_counts = nullptr;
     uint64_t n_rec = 0, n_keys = 0, table_cap = 0, ovf_len = 0;
     uint32_t n_sub = 0, region_redos = 0;
+    bool crowded = false;               // more than 1 in CROWD_SHARE of its keys were sorted
     std::vector<unsigned long long> totals;   // per group: distinct k-mers, k-mers seen once, records
 };
+
+// Counting a pass again after a finer cut costs its partition, scatter and count
+// (480M k-mers 7.8 ms, 16 ps each), the sort of crowded sub-buckets' keys 140 to
+// 170 ps each (7.2M 31-mers 1.0 ms, 7.7M 1.3; 1.5M 63-mers 0.66, where launches
+// and waits count): from an eighth of the keys on the finer cut is tried.
+constexpr uint64_t CROWD_SHARE = 8;
+
+// Most keys sorted together: 64M take 3.7 GB (one word) to 8 GB (four).
+constexpr uint64_t CROWD_GROUP_KEYS = 64ull << 20;
 
 // Entries of a pass's arrays for n keys: room for the sub-buckets' estimated
 // regions (their sizes plus about 15% on a large pass).
 uint64_t prefix_list_cap(uint64_t n) { return n + n / 4 + 65536; }
+
+// Counts what the shared-memory count left of the crowded sub-buckets (listed on
+// the device at pc.crowd, n of them): pc's histogram, totals and record arrays
+// take their runs, sub_len their records, which are returned as a list (host
+// order: by sub-bucket) for launch_crowd_copy.
+std::vector<CrowdRecords> count_crowded(const PrefixPass &pp, const PrefixCountArgs &pc, uint64_t n, DevScope &ds,
+                                        HostStage &hs, cudaStream_t st)
+{
+    const uint32_t N = pp.words;
+    std::vector<CrowdSub> cs(n);
+    CK(cudaMemcpyAsync(cs.data(), pc.crowd, n * sizeof(CrowdSub), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    std::sort(cs.begin(), cs.end(), [](const CrowdSub &x, const CrowdSub &y) { return x.sub < y.sub; });
+    // working memory per key: gathered (and, of more words, sorted) keys and
+    // range numbers, the sort's, the runs'
+    const uint64_t per_key = N == 1 ? 60 : 16 * N + 66;
+    uint64_t largest = 0;
+    for (const CrowdSub &c : cs) largest = std::max<uint64_t>(largest, c.n);
+    const uint64_t memory = pass_budget(*ds.ws, std::max(largest, CROWD_GROUP_KEYS) * per_key);
+    if (largest * per_key > memory || largest >= 0xFFFFFFFFull) throw SubTablesFull{};
+    const uint64_t group_keys = std::max(largest, std::min(CROWD_GROUP_KEYS, memory / per_key));
+    static const bool trace = getenv("KC_TRACE") && getenv("KC_TRACE")[0] == '1';
+    if (trace) {
+        uint64_t all = 0;
+        for (const CrowdSub &c : cs) all += c.n;
+        fprintf(stderr, "[kc trace] %zu crowded sub-buckets of %llu keys, the largest %llu\n", cs.size(),
+                (unsigned long long)all, (unsigned long long)largest);
+    }
+    std::vector<CrowdRecords> recs;
+    uint64_t rec_total = 0;
+    for (size_t lo = 0; lo < n;) {
+        // one sample's or job's at a time: equal keys of two samples are different k-mers
+        uint64_t total = cs[lo].n;
+        size_t hi = lo + 1;
+        while (hi < n && total + cs[hi].n <= group_keys && pp.sc[cs[hi].bucket].group == pp.sc[cs[lo].bucket].group)
+            total += cs[hi++].n;
+        const uint32_t nr = (uint32_t)(hi - lo);
+        const SubCfg &cfg = pp.sc[cs[lo].bucket];
+        const DevScope::Mark mk = ds.mark();
+        CrowdRange *h_rg = hs.n<CrowdRange>(nr);
+        uint64_t at = 0;
+        for (uint32_t j = 0; j < nr; ++j) {
+            const CrowdSub &c = cs[lo + j];
+            const uint32_t lg = (uint32_t)__builtin_ctz(c.rounds);
+            h_rg[j] = CrowdRange{c.src, at, c.off, c.rd, c.rd ? 64 - pp.sc[c.bucket].plen - lg : 0, c.rounds - 1};
+            at += c.n;
+        }
+        CrowdRange *d_rg = ds.n<CrowdRange>(nr);
+        unsigned long long *first = ds.n<unsigned long long>(nr + 2), *cursor = first + nr + 1;
+        unsigned long long *keys = ds.n<unsigned long long>(total * N);
+        uint32_t *range = ds.n<uint32_t>(total);
+        CK(cudaMemcpyAsync(d_rg, h_rg, nr * sizeof(CrowdRange), cudaMemcpyHostToDevice, st));
+        CK(cudaMemsetAsync(first, 0, (nr + 2) * 8, st));
+        CK(launch_crowd_gather(N, pp.list, d_rg, nr, total, cfg.k, keys, range, cursor, st));
+        unsigned long long *h_m = hs.n<unsigned long long>(1);
+        CK(cudaMemcpyAsync(h_m, cursor, 8, cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        const uint64_t m = *h_m;
+        if (m > total) throw KcError{KC_ERR_DEVICE, "more keys gathered than the crowded sub-buckets hold"};
+        if (N == 1) {
+            void *tmp = ds.get(sort_tmp_bytes(m));
+            CK(launch_radix_sort(keys, range, m, 2 * cfg.k, tmp, st, pc.counters + C_FLAGS));
+            ds.release(tmp);
+        } else {
+            unsigned long long *sk = ds.n<unsigned long long>(m * N);
+            uint32_t *sr = ds.n<uint32_t>(m);
+            void *tmp = ds.get(wide_sort_tmp_bytes(m));
+            CK(launch_wide_sort(cfg.k, keys, range, m, sk, sr, tmp, pc.counters + C_FLAGS, st));
+            ds.release(tmp);
+            keys = sk;
+            range = sr;
+        }
+        CK(launch_crowd_runs(N, keys, range, m, d_rg, nr, cfg, pc, ds.get(crowd_runs_tmp_bytes(m)), first, st));
+        unsigned long long *h_first = hs.n<unsigned long long>(nr + 1);
+        CK(cudaMemcpyAsync(h_first, first, (nr + 1) * 8, cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        for (uint32_t j = 0; j < nr; ++j) {
+            const CrowdSub &c = cs[lo + j];
+            const uint64_t len = h_first[j + 1] - h_first[j];
+            if (h_first[j + 1] < h_first[j] || len > c.n)
+                throw KcError{KC_ERR_DEVICE, "the records of the crowded sub-buckets do not add up"};
+            if (!len) continue;
+            recs.push_back(CrowdRecords{c.src + c.off, rec_total, c.sub, c.off, (uint32_t)len, 0});
+            rec_total += len;
+        }
+        ds.rewind(mk);
+        lo = hi;
+    }
+    return recs;
+}
 
 void count_by_prefix(PrefixPass &pp, DevScope &ds, HostStage &hs, PhaseClock &clk, const kc_tuning &tn, cudaStream_t st)
 {
@@ -599,51 +698,55 @@ void count_by_prefix(PrefixPass &pp, DevScope &ds, HostStage &hs, PhaseClock &cl
         pc.ovf_cap = pp.ovf_cap;
         pc.counters = counters;
         pc.bucket_ovf = bucket_ovf;
+        pc.crowd = ds.n<CrowdSub>(n_sub);
         CK(launch_count_prefix(pc, N, shape, st));
         clk.end();
-        if (attempt == 0 && (pp.fault_inject & KC_INJECT_TABLE_FULL_ONCE)) {
-            // as if the first bucket's sub-bucket tables had overflowed
-            CK(cudaMemsetAsync(bucket_ovf + lo, 0x01, 1, st));
-            CK(launch_or_flags(counters + C_SUB_OVF, 1ull, st));
-        }
+        // (as if the first bucket's sub-buckets had been crowded)
+        const bool injected = attempt == 0 && (pp.fault_inject & KC_INJECT_TABLE_FULL_ONCE);
         unsigned long long *p_tot = hs.n<unsigned long long>(3 * pp.n_groups);
         CK(cudaMemcpyAsync(p_tot, totals, 3ull * pp.n_groups * 8, cudaMemcpyDeviceToHost, st));
-        const Counters cs = read_counters(counters, st);
+        Counters cs = read_counters(counters, st);
         check_flags(cs.v[C_FLAGS], "sub-bucket count");
-        if (cs.v[C_REGION_OVF] || cs.v[C_SUB_OVF] || cs.v[C_UNIT_OVF]) {
+        pp.crowded = !cs.v[C_REGION_OVF] && cs.v[C_CROWD_KEYS] * CROWD_SHARE > pp.n_keys;
+        // buckets of crowded sub-buckets that can be cut further: 16 times the
+        // sub-buckets
+        bool cut = false;
+        if (!cs.v[C_REGION_OVF] && (pp.crowded || injected)) {
             std::vector<uint32_t> bo(N_BUCKETS);
             CK(cudaMemcpyAsync(bo.data(), bucket_ovf, N_BUCKETS * 4, cudaMemcpyDeviceToHost, st));
+            CK(cudaStreamSynchronize(st));
+            for (uint32_t b = lo; b < hi; ++b) {
+                if (!(bo[b] || (injected && b == lo)) || nsub[b] * 2 > max_nsub[b]) continue;
+                nsub[b] = std::min(nsub[b] * 16, max_nsub[b]);
+                cut = true;
+            }
+        }
+        if (cs.v[C_REGION_OVF] || cs.v[C_UNIT_OVF] || cut) {
             CK(cudaMemcpyAsync(counters + C_OVF_LEN, ovf_len_saved, 8, cudaMemcpyDeviceToDevice, st));
             if (pp.hist_zero) CK(cudaMemsetAsync(pp.hist, 0, hist_n * 8, st));
-            CK(cudaStreamSynchronize(st));
             ds.rewind(m0);
             if (cs.v[C_REGION_OVF]) {
                 // a sub-bucket outgrew its estimated region (the count then
                 // leaves the keys alone): exact regions, same sub-buckets
                 exact_regions = true;
                 ++pp.region_redos;
-            } else if (!cs.v[C_SUB_OVF]) {
-                // more units than the lists hold: room for all there can be
-                all_units = true;
-                clk.begin(2);
-                pp.repartition();   // the records went over the partitioned keys
-                clk.end();
-            } else {
-                // buckets with more distinct k-mers than 64 rounds of their
-                // sub-buckets hold: 16 times the sub-buckets
-                bool cut = false;
-                for (uint32_t b = lo; b < hi; ++b) {
-                    if (!bo[b]) continue;
-                    if (nsub[b] * 2 > max_nsub[b]) throw SubTablesFull{};
-                    nsub[b] = std::min(nsub[b] * 16, max_nsub[b]);
-                    cut = true;
-                }
-                if (!cut) throw SubTablesFull{};
-                clk.begin(2);
-                pp.repartition();   // the records went over the partitioned keys
-                clk.end();
+                continue;
             }
+            if (cs.v[C_UNIT_OVF]) all_units = true;   // more units than the lists hold: room for all there can be
+            clk.begin(2);
+            pp.repartition();   // the records went over the partitioned keys
+            clk.end();
             continue;
+        }
+        std::vector<CrowdRecords> crowd;
+        if (cs.v[C_SUB_OVF]) {
+            clk.begin(10);
+            crowd = count_crowded(pp, pc, cs.v[C_SUB_OVF], ds, hs, st);
+            clk.end();
+            CK(cudaMemcpyAsync(p_tot, totals, 3ull * pp.n_groups * 8, cudaMemcpyDeviceToHost, st));
+            const Counters after = read_counters(counters, st);
+            check_flags(after.v[C_FLAGS], "count of crowded sub-buckets");
+            cs.v[C_OVF_LEN] = after.v[C_OVF_LEN];
         }
         pp.totals.assign(p_tot, p_tot + 3 * pp.n_groups);
         pp.ovf_len = cs.v[C_OVF_LEN];
@@ -654,11 +757,22 @@ void count_by_prefix(PrefixPass &pp, DevScope &ds, HostStage &hs, PhaseClock &cl
         pp.rec_keys = ds.n<unsigned long long>(std::max<uint64_t>(pp.n_rec, 1) * N);
         pp.rec_counts = ds.n<uint32_t>(std::max<uint64_t>(pp.n_rec, 1));
         // where each sub-bucket's records go; sub_cur is free again
+        const CrowdRecords *d_crowd = nullptr;
+        if (!crowd.empty()) {
+            CrowdRecords *d = ds.n<CrowdRecords>(crowd.size());
+            CK(cudaMemcpyAsync(d, hs.up(crowd.data(), crowd.size()), crowd.size() * sizeof(CrowdRecords),
+                               cudaMemcpyHostToDevice, st));
+            CK(launch_crowd_lens(d, (uint32_t)crowd.size(), sub_len, st));
+            d_crowd = d;
+        }
         CK(launch_scan_u32(sub_len, sub_cur, n_sub, sub_tmp, st));
         uint32_t n_units[UNIT_CLASSES];
         for (uint32_t c = 0; c < UNIT_CLASSES; ++c) n_units[c] = (uint32_t)cs.v[C_UNITS + c];
         CK(launch_unit_sort(N, pp.keys, pp.tmp_counts, sub_off, sub_cur, units, lists, n_units, pp.rec_keys,
                             pp.rec_counts, pp.n_rec, st));
+        if (d_crowd)
+            CK(launch_crowd_copy(N, d_crowd, (uint32_t)crowd.size(), crowd.back().start + crowd.back().len, pp.keys,
+                                 pp.tmp_counts, sub_cur, pp.rec_keys, pp.rec_counts, pp.n_rec, st));
         clk.end();
         pp.n_sub = n_sub;
         pp.table_cap = (uint64_t)n_sub * sub_table_slots(N, shape);
@@ -1239,7 +1353,7 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
                 }
                 table_cap = std::max(table_cap, pp.table_cap);
                 job.region_redos += pp.region_redos;
-                ++job.smem_passes;
+                ++(pp.crowded ? job.smem_fallbacks : job.smem_passes);
             }
             if (!prefix) {
                 std::vector<unsigned long long> lh(2 * N_BUCKETS, 0);
@@ -1799,7 +1913,7 @@ void run_wide_job(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
         count_by_prefix(pp, ds, hs, clk, tn, st);
         job.distinct += pp.totals[0];
         job.region_redos += pp.region_redos;
-        ++job.smem_passes;
+        ++(pp.crowded ? job.smem_fallbacks : job.smem_passes);
         table_cap = std::max(table_cap, pp.table_cap);
         if (multi) {
             park(pp.rec_keys, pp.rec_counts, pp.n_rec, mk);
@@ -2268,7 +2382,8 @@ void run_batch_once(std::vector<std::shared_ptr<Job>> &jobs, cudaStream_t st, Wo
                 caps[lo + b] = (uint64_t)pp.sc[b].n_sub * (pp.table_cap / std::max(pp.n_sub, 1u));
                 records_out(lo + b, pp.rec_keys + at, pp.rec_counts + at);
                 at += len_h[lo + b];
-                jobs[lo + b]->smem_passes = 1;
+                jobs[lo + b]->smem_passes = pp.crowded ? 0 : 1;
+                jobs[lo + b]->smem_fallbacks = pp.crowded ? 1 : 0;
             }
             const size_t n_ovf = (size_t)std::min<uint64_t>(pp.ovf_len, ovf_cap), o0 = ovf_h.size();
             if (n_ovf) {
@@ -2447,7 +2562,7 @@ void run_batch(std::vector<std::shared_ptr<Job>> &jobs, cudaStream_t st, Workspa
         run_batch_once(jobs, st, ws, true, tn);
         for (auto &j : jobs) {
             j->smem_passes = 0;
-            ++j->smem_fallbacks;
+            j->smem_fallbacks = 1;
         }
     }
 }

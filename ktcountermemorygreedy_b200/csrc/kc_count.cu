@@ -142,7 +142,9 @@ constexpr uint32_t SLOT_CLAIMED = 1u << 31, SLOT_PUBLISHED = 1u << 30, SLOT_COUN
 // emptied and the sub-bucket counted in rounds over halves of its key range
 // (quarters, ... at most SUB_MAX_ROUNDS), each round reading the keys again
 // from L2; a round's records lie after the earlier rounds' ones, and are a
-// sort unit of their own.  The next sub-bucket's first keys are loaded before
+// sort unit of their own.  A sub-bucket that no number of rounds fits, or that
+// would take one block too long, is listed with what is left of it (kc_crowd.cu
+// counts that).  The next sub-bucket's first keys are loaded before
 // the sweep.  Histogram and totals go to the sub-bucket's group.
 template <uint32_t N, uint32_t THREADS, uint32_t BPSM, uint32_t TBITS>
 __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs a)
@@ -158,8 +160,8 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
     uint16_t *q_slot = reinterpret_cast<uint16_t *>(s_hist + CP_HIST + 2 * N * CP_QUEUE * WARPS) +
                        (threadIdx.x >> 5) * CP_QUEUE;
     __shared__ uint32_t s_out, s_full, s_next, s_next_n;
-    __shared__ unsigned long long s_next_off, s_kept;   // s_kept, s_ovf, s_group: only thread 0 writes them
-    __shared__ uint32_t s_ovf, s_group;
+    __shared__ unsigned long long s_next_off, s_kept;   // s_kept, s_group: only thread 0 writes them
+    __shared__ uint32_t s_group;
     __shared__ SubCfg s_cfg[2];   // this sub-bucket's and the next one's
     const int tid = threadIdx.x, lane = tid & 31;
     const uint32_t lt = lanes_below();
@@ -186,7 +188,6 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
         s_out = 0;
         s_full = 0;
         s_kept = 0;
-        s_ovf = 0;
         take_next();
         s_group = s_next < a.n_sub ? s_cfg[0].group : 0u;
     }
@@ -248,7 +249,8 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
         const uint32_t smask = (1u << lg) - 1, hsh = 32 - lg;
         uint32_t rounds = rounds0, rd = 0, off = 0, most = 0;
         bool failed = false;
-        const bool too_many = N > 1 && n >= SLOT_COUNT;   // a count could run into the state bits
+        static_assert(SUB_MAX_KEYS < SLOT_COUNT, "a count would run into the state bits");
+        const bool too_many = n > SUB_MAX_KEYS;
         while (rd < rounds && !too_many) {
             const uint32_t rmask = rounds - 1;
             const int rsh = 64 - (int)cfg.plen - (31 - __clz(rounds));   // rounds == 1: unused
@@ -397,7 +399,8 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
                 failed = true;
                 rounds *= 2;
                 rd *= 2;
-                if (rounds > SUB_MAX_ROUNDS || (int)cfg.plen + (31 - __clz(rounds)) > 64) break;
+                if (rounds > SUB_MAX_ROUNDS || rounds * n > SUB_MAX_READS || (int)cfg.plen + (31 - __clz(rounds)) > 64)
+                    break;
                 continue;
             }
             // the next sub-bucket's first keys arrive during the sweep
@@ -488,8 +491,10 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
         if (tid == 0) {
             a.sub_len[sub] = off;
             if (gave_up) {
-                ++s_ovf;
-                atomicOr(&a.bucket_ovf[a.sub_bucket[sub]], 1u);
+                const uint32_t b = a.sub_bucket[sub];
+                atomicOr(&a.bucket_ovf[b], 1u);
+                atomicAdd(&a.counters[C_CROWD_KEYS], (unsigned long long)n);
+                a.crowd[atomicAdd(&a.counters[C_SUB_OVF], 1ull)] = CrowdSub{base, n, sub, off, rd, rounds, b};
             }
         }
         // sub-buckets are alike: the next one starts with as many rounds, or with
@@ -510,7 +515,6 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
         par ^= 1;
     }
     flush();
-    if (tid == 0 && s_ovf) atomicAdd(&a.counters[C_SUB_OVF], (unsigned long long)s_ovf);
 }
 
 // Sorts the records of one unit (a sub-bucket, or one round of it: at most

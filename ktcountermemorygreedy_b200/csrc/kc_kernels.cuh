@@ -38,10 +38,11 @@ enum Counter : int {
     C_OVF_LEN = 7,       // histogram counts >= HIST_BINS
     C_SEL_A = 8,         // query selections
     C_SEL_B = 9,
-    C_SUB_OVF = 10,      // sub-buckets whose shared-memory table overflowed
+    C_SUB_OVF = 10,      // crowded sub-buckets (CrowdSub), given up by the shared-memory count
     C_REGION_OVF = 11,   // nonzero: a sub-bucket outgrew its estimated region
     C_KEPT = 12,         // records a counting compaction pass would keep
     C_UNIT_OVF = 13,     // nonzero: more sort units of a class than its list holds
+    C_CROWD_KEYS = 14,   // keys of the crowded sub-buckets
     C_UNITS = 16,        // UNIT_CLASSES counts: sort units by size
     C_COUNT = 24
 };
@@ -346,15 +347,30 @@ cudaError_t launch_subpart_sizes(const unsigned long long *sub_off, const unsign
 // of them.  Every k-mer's count goes to the group's histogram (hist_bins bins
 // at hist + group * hist_bins; larger counts to ovf, or with their group to
 // ovf64), totals to totals[3 * group ..]: distinct k-mers, k-mers seen once,
-// records.  Sub-buckets that no number of rounds fits are counted in C_SUB_OVF
-// (and bucket_ovf[their bucket]), more units of a class than lists.cap[c] set
-// C_UNIT_OVF: the results are then incomplete.
+// records.  Sub-buckets that no number of rounds fits, or with more keys than
+// SUB_MAX_KEYS, are listed in crowd (C_SUB_OVF of them, C_CROWD_KEYS keys in all;
+// bucket_ovf[their bucket] is set): their finished rounds are counted and their
+// records in place, the rest is left to the caller.  More units of a class than
+// lists.cap[c] set C_UNIT_OVF: the results are then incomplete.
 constexpr uint32_t UNIT_CLASSES = 4;
 __host__ __device__ constexpr uint32_t unit_cap0(uint32_t words) { return 1024u / words; }
 struct SubUnit {
     uint32_t sub, off, len, k;
 };
 constexpr uint32_t SUB_MAX_ROUNDS = 64;   // rounds a sub-bucket may be cut into, each a unit
+// One block counts a sub-bucket, about 560 keys a microsecond and round: 256K keys
+// take it 0.5 ms, about what sorting them on the whole device takes with its dozen
+// launches and two waits, and from there on the sort gains (9.6M occurrences of
+// poly-A k-mers took 163 ms in one block).  The same bounds all rounds together,
+// with room for 64 rounds of 65K keys (7 ms): a table of 8192 slots then holds
+// whatever rounds can tell apart.
+constexpr uint32_t SUB_MAX_KEYS = 1u << 18, SUB_MAX_READS = 1u << 22;
+// A crowded sub-bucket: its keys [src, src + n); rounds 0 .. rd - 1 of `rounds`
+// are counted, with `off` records.
+struct CrowdSub {
+    unsigned long long src;
+    uint32_t n, sub, off, rd, rounds, bucket;
+};
 // Room for the units of n_keys keys in n_sub sub-buckets, class by class.  A
 // unit of a class from 1 on has more than unit_cap0 << (c - 1) records of keys of
 // its own, so their lists hold whatever comes.  Class 0 has room for two units a
@@ -396,6 +412,7 @@ struct PrefixCountArgs {
     uint64_t ovf_cap;
     unsigned long long *counters;
     uint32_t *bucket_ovf;
+    CrowdSub *crowd;   // n_sub entries
 };
 // shape (kc_tuning.count_shape): 1 and 3 run 512-thread blocks, two per SM,
 // with tables of 8192, 4096 or 2048 slots for keys of 1, 2 or 4 words; 2 and 4
@@ -413,6 +430,38 @@ cudaError_t launch_unit_sort(uint32_t words, const unsigned long long *tk, const
                              const unsigned long long *sub_off, const unsigned long long *sub_final,
                              const SubUnit *units, const UnitLists &lists, const uint32_t *n_units,
                              unsigned long long *out_k, uint32_t *out_v, uint64_t out_cap, cudaStream_t st);
+// Crowded sub-buckets counted by sorting (kc_crowd.cu), a group of them at a
+// time: the n_rg ranges of `total` keys, in order.  A range's keys [src, ..) are
+// the group's keys from `start` on; rd == 0: all are left to count, else those
+// with ((first word >> shift) & mask) >= rd.
+struct CrowdRange {
+    unsigned long long src, start;
+    uint32_t off, rd, shift, mask;
+};
+// The keys left, in the form the record sorts take (one word: right aligned;
+// more: k-mer words), with their range's number; *cursor counts them.
+cudaError_t launch_crowd_gather(uint32_t words, const unsigned long long *keys, const CrowdRange *rg, uint32_t n_rg,
+                                uint64_t total, uint32_t k, unsigned long long *out, uint32_t *out_range,
+                                unsigned long long *cursor, cudaStream_t st);
+// m keys sorted, equal ones a run: every run's count to the histogram, totals and
+// overflow list of a (group and limits: c), its records to a.rec_keys /
+// a.rec_counts from src + off of their range on, as k-mer words; first[j] =
+// records before range j, first[n_rg] = all.  m < 2^32 - 1.
+size_t crowd_runs_tmp_bytes(uint64_t m);
+cudaError_t launch_crowd_runs(uint32_t words, const unsigned long long *keys, const uint32_t *range, uint64_t m,
+                              const CrowdRange *rg, uint32_t n_rg, const SubCfg &c, const PrefixCountArgs &a, void *tmp,
+                              unsigned long long *first, cudaStream_t st);
+// len records from src on, the sub-bucket's from `off` on; start: records of the
+// list before them.
+struct CrowdRecords {
+    unsigned long long src, start;
+    uint32_t sub, off, len, pad;
+};
+cudaError_t launch_crowd_lens(const CrowdRecords *r, uint32_t n, uint32_t *sub_len, cudaStream_t st);
+cudaError_t launch_crowd_copy(uint32_t words, const CrowdRecords *r, uint32_t n_r, uint64_t total,
+                              const unsigned long long *rec_keys, const uint32_t *rec_counts,
+                              const unsigned long long *sub_final, unsigned long long *out_k, uint32_t *out_v,
+                              uint64_t out_cap, cudaStream_t st);
 cudaError_t launch_bloom_buckets(const unsigned long long *keys, const BucketRanges *rg, uint32_t n_items,
                                  unsigned int *next_item, const BucketCfg *cfg, unsigned long long *bits,
                                  unsigned long long *out, unsigned long long *low_cnt, unsigned long long *high_cnt,

@@ -60,3 +60,113 @@ def test_assembly_of_distinct_kmers(counter, shape):
     assert r.smem_passes == 1 and r.smem_fallbacks == 0
     assert np.array_equal(r.keys, want_k) and np.array_equal(r.counts, want_c)
     assert r.hist.tolist() == O.histogram(want_c, 1, 10).tolist()
+
+
+def _uniform(seed, n, length=150):
+    reads = BASES[np.random.default_rng(seed).integers(0, 4, size=(n, length), dtype=np.uint8)]
+    return [r.tobytes() for r in reads]
+
+
+def _repeat(seed, unit, n, sub, length=150):
+    """Reads of a repeated unit with substitutions."""
+    rng = np.random.default_rng(seed)
+    out = []
+    for _ in range(n):
+        s = np.resize(np.frombuffer(unit, np.uint8), length + len(unit))[rng.integers(0, len(unit)):][:length].copy()
+        at = np.nonzero(rng.random(length) < sub)[0]
+        s[at] = BASES[rng.integers(0, 4, len(at))]
+        out.append(s.tobytes())
+    return out
+
+
+def _fastq(seqs, seed=0):
+    seqs = list(seqs)
+    random.Random(seed).shuffle(seqs)
+    return b"".join(_record(s) for s in seqs)
+
+
+def _oracle(files, k):
+    return (O.exact_records if k <= 32 else O.exact_records_wide)(files, k, U32)
+
+
+def _check(c, files, k, min_count=1, max_count=U32, count_max=U32, **kw):
+    all_k, all_c = _oracle(files, k)
+    cc = np.minimum(all_c, count_max)
+    m = (cc >= min_count) & (cc <= max_count)
+    r = c.count(files, k=k, count_max=count_max, min_count=min_count, max_count=max_count, hist_max=300_000, top_n=20, **kw)
+    assert np.array_equal(r.keys, all_k[m]) and np.array_equal(r.counts, cc[m])
+    assert r.hist.tolist() == O.histogram(cc, 1, 300_000).tolist()
+    assert r.distinct == len(all_k) and r.occurrences == int(all_c.sum(dtype=np.uint64))
+    order = np.argsort(-cc[m].astype(np.int64), kind="stable")[:20]
+    assert np.array_equal(r.top_keys, all_k[m][order]) and np.array_equal(r.top_counts, cc[m][order])
+    return r
+
+
+@pytest.mark.parametrize("k", [16, 31, 32, 33, 63, 64, 96, 127])
+def test_reads_of_repeats_are_counted_in_the_pass(counter, k):
+    """Poly-A and microsatellites with errors: far more k-mers that start alike
+    than a table holds, in a few of the sub-buckets.  Those are counted on their
+    own, the pass stays where it is."""
+    seqs = _uniform(k, 20_000, 250)
+    for i, unit in enumerate((b"A", b"AC", b"GATA")):
+        seqs += _repeat(100 * k + i, unit, 700, 0.03, 250)
+    f = [_fastq(seqs, k)]
+    for kw in (dict(), dict(bloom=True, memory_gb=1, min_count=2), dict(count_max=3, min_count=2, max_count=3)):
+        r = _check(counter, f, k, **kw)
+        assert r.smem_passes == 1 and r.smem_fallbacks == 0
+
+
+@pytest.mark.parametrize("k", [31, 63, 127])
+@pytest.mark.parametrize("n", [262_143, 262_144, 262_145, 400_000])
+def test_one_kmer_at_the_edge_of_a_blocks_share(counter, k, n):
+    """n occurrences of one k-mer, at and around the number of keys that one
+    block counts (262144)."""
+    f = [_record(b"A" * (n + k - 1)) + _fastq(_uniform(n + k, 30_000, 250), 1)]
+    r = _check(counter, f, k)
+    assert r.smem_passes == 1 and r.smem_fallbacks == 0
+    assert int(r.counts.max()) >= n
+
+
+@pytest.mark.parametrize("shape", [1, 2])
+@pytest.mark.parametrize("k", [31, 47, 101])
+def test_crowded_after_finished_rounds(counter, k, shape):
+    """A sub-bucket whose first rounds fit and whose last ones do not: 20000
+    k-mers of one 10-base prefix spread evenly and 20000 more in its last part
+    that share 26 bases."""
+    rnd = random.Random(k)
+    tail = lambda n: "".join(rnd.choice("ACGT") for _ in range(n))
+    p = "AC" + tail(8)
+    even = {p + rnd.choice("AC") + tail(k - 12) + "A" for _ in range(20_000)}
+    q = p + "TT" + tail(14)
+    late = {q + tail(k - 27) + "A" for _ in range(20_000)} if k > 31 else {q + tail(4) + "A" for _ in range(300)} | {
+        p + "TTT" + tail(k - 14) + "A" for _ in range(20_000)}
+    seqs = [s.encode() for s in even | late]
+    seqs += seqs[::5] + _uniform(k, 6000, 300)
+    counter.set_tuning(count_shape=shape)
+    r = _check(counter, [_fastq(seqs, k)], k, min_count=1)
+    counter.set_tuning(count_shape=1)
+    assert r.smem_passes == 1 and r.smem_fallbacks == 0
+
+
+@pytest.mark.parametrize("k", [31, 63])
+def test_one_crowded_pass_of_several(counter, k):
+    """A job in passes whose k-mers crowd into one prefix in one of them: only
+    that pass counts most of its k-mers in global memory."""
+    seqs = _uniform(5, 30_000) + _repeat(6, b"A", 6000, 0.03)
+    f = [_fastq(seqs, 2)]
+    r = _check(counter, f, k, pass_bytes=16 << 20)
+    assert r.passes > 3 and r.smem_fallbacks == 1 and r.smem_passes == r.passes - 1
+
+
+def test_crowded_samples_of_a_batch(counter):
+    """Two samples with the same repeats and one without, k equal and not: each
+    has its own counts, and the batch stays in shared memory."""
+    seqs = [_uniform(i, 12_000) + (_repeat(9 + i // 2, b"A", 900, 0.03) if i < 3 else []) for i in range(4)]
+    files = [[_fastq(s, i)] for i, s in enumerate(seqs)]
+    ks = [31, 31, 25, 31]
+    rs = counter.count_batch(files, ks, count_max=U32, hist_max=200_000)
+    for f, k, r in zip(files, ks, rs):
+        all_k, all_c = _oracle(f, k)
+        assert np.array_equal(r.keys, all_k) and np.array_equal(r.counts, all_c)
+        assert r.hist.tolist() == O.histogram(all_c, 1, 200_000).tolist()
+        assert r.distinct == len(all_k) and r.smem_passes == 1 and r.smem_fallbacks == 0
