@@ -477,8 +477,22 @@ constexpr uint64_t CROWD_SHARE = 8;
 // Most keys sorted together: 64M take 3.7 GB (one word) to 8 GB (four).
 constexpr uint64_t CROWD_GROUP_KEYS = 64ull << 20;
 
+// Whether regions estimated from a sample (k_subpart_regions: each sub-bucket's
+// size m and 20 sqrt(m) + 64 more) fit the array: at most n + 20 sqrt(n n_sub) +
+// 64 n_sub in all, by Cauchy and Schwarz, and 1% for the estimates' own error.
+// One-word sub-buckets hold 8K keys and more from the default sampled_region_keys
+// on, and their regions (14 to 23% more) fit always.  Two-word ones (2.5K to 5K
+// keys: 30 to 43%) fit behind a sampled census, whose own margin is 15%, or not;
+// four-word ones (1K to 2K: 47 to 69%) never do: sampled all the same, 87M 127-base
+// k-mers were scattered twice, 3.3 ms instead of 1.9 with exact counts.
+bool sampled_regions_fit(uint64_t n_keys, uint32_t n_sub, uint64_t list_cap)
+{
+    const double n = (double)n_keys, m = (double)n_sub;
+    return 1.01 * (n + 20.0 * std::sqrt(n * m) + 64.0 * m) <= (double)list_cap;
+}
+
 // Entries of a pass's arrays for n keys: room for the sub-buckets' estimated
-// regions (their sizes plus about 15% on a large pass).
+// regions (sampled_regions_fit).
 uint64_t prefix_list_cap(uint64_t n) { return n + n / 4 + 65536; }
 
 // Counts what the shared-memory count left of the crowded sub-buckets (listed on
@@ -637,7 +651,8 @@ void count_by_prefix(PrefixPass &pp, DevScope &ds, HostStage &hs, PhaseClock &cl
         unsigned long long *hist_sub = pp.hist_zero ? pp.hist : ds.n<unsigned long long>(hist_n);
         const UnitLists lists = unit_lists(pp.n_keys, n_sub, N, all_units);
         SubUnit *units = ds.n<SubUnit>(lists.total);
-        const bool sampled = !exact_regions && !batch && pp.n_keys >= tn.sampled_region_keys;
+        const bool sampled = !exact_regions && !batch && pp.n_keys >= tn.sampled_region_keys &&
+                             (N == 1 || sampled_regions_fit(pp.n_keys, n_sub, pp.list_cap));
         const uint32_t stride = sampled ? SUB_REGION_SAMPLE : 1;
         // one upload: the 256 ranges of each bucket-major launch (not lists of
         // items), the sub-buckets' settings and their buckets

@@ -170,3 +170,18 @@ def test_crowded_samples_of_a_batch(counter):
         assert np.array_equal(r.keys, all_k) and np.array_equal(r.counts, all_c)
         assert r.hist.tolist() == O.histogram(all_c, 1, 200_000).tolist()
         assert r.distinct == len(all_k) and r.smem_passes == 1 and r.smem_fallbacks == 0
+
+
+@pytest.mark.parametrize("k", [63, 96, 127])
+@pytest.mark.parametrize("large", [False, True])
+def test_sampled_regions_of_long_kmers_fit(counter, k, large):
+    """Sub-buckets of two- and four-word k-mers are small, and regions estimated
+    from a sample leave each a margin that the key arrays have no room for, with
+    an exact census or (from 4 MiB on) a sampled one: such passes count exactly
+    instead of scattering twice."""
+    f = [_fastq(_uniform(k, 27_000 if large else 8_000, 250))]
+    assert (len(f[0]) > 4 << 20) == large
+    counter.set_tuning(sampled_region_keys=1)
+    r = _check(counter, f, k)
+    counter.set_tuning(sampled_region_keys=64 << 20)
+    assert r.smem_passes == 1 and r.region_redos == 0
