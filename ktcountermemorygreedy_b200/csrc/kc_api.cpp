@@ -510,18 +510,18 @@ std::vector<CrowdRecords> count_crowded(const PrefixPass &pp, const PrefixCountA
     // working memory per key: gathered (and, of more words, sorted) keys and
     // range numbers, the sort's, the runs'
     const uint64_t per_key = N == 1 ? 60 : 16 * N + 66;
-    uint64_t largest = 0;
-    for (const CrowdSub &c : cs) largest = std::max<uint64_t>(largest, c.n);
-    const uint64_t memory = pass_budget(*ds.ws, std::max(largest, CROWD_GROUP_KEYS) * per_key);
+    uint64_t largest = 0, all = 0;
+    for (const CrowdSub &c : cs) {
+        largest = std::max<uint64_t>(largest, c.n);
+        all += c.n;
+    }
+    const uint64_t memory = pass_budget(*ds.ws, std::min(all, std::max(largest, CROWD_GROUP_KEYS)) * per_key);
     if (largest * per_key > memory || largest >= 0xFFFFFFFFull) throw SubTablesFull{};
     const uint64_t group_keys = std::max(largest, std::min(CROWD_GROUP_KEYS, memory / per_key));
     static const bool trace = getenv("KC_TRACE") && getenv("KC_TRACE")[0] == '1';
-    if (trace) {
-        uint64_t all = 0;
-        for (const CrowdSub &c : cs) all += c.n;
+    if (trace)
         fprintf(stderr, "[kc trace] %zu crowded sub-buckets of %llu keys, the largest %llu\n", cs.size(),
                 (unsigned long long)all, (unsigned long long)largest);
-    }
     std::vector<CrowdRecords> recs;
     uint64_t rec_total = 0;
     for (size_t lo = 0; lo < n;) {
