@@ -822,42 +822,59 @@ void pack_high_on_device(Job &job, DevScope &ds, const unsigned long long *keys,
     job.has_packed = true;
 }
 
-void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, bool global_tables, const kc_tuning &tn)
-{
-    const kc_job &P = job.p;
-    const uint32_t k = P.k;
-    if (P.fault_inject & KC_INJECT_NOMEM) ws.fail_next_get();
-    DevScope ds(st, &ws);
-    std::vector<uint32_t> tile_seg_host;
-
-    // ---- input -----------------------------------------------------------
+// A job's FASTQ on the device: the caller's resident input, or the job's own
+// upload, which stays while the job is counted again (an outgrown census, tables
+// instead of the prefix path).
+struct JobInput {
+    const kc_input *in = nullptr;
     kc_input local;
-    const kc_input *in = job.input;
-    static const bool trace_host = getenv("KC_TRACE") && getenv("KC_TRACE")[0] == '1';
-    const double th_start = now_ms();
     std::vector<PinnedBlock> inflated;   // gzip files inflated on the host (kept until the job ends)
+    std::vector<uint32_t> tile_seg_host;
     // the one large host file of a prefix-path or Bloom job goes up in chunks
     // while the census, SCAN and partition work on the chunks that have arrived
     // (declared after the host and device buffers: it drains its copies before
     // they go)
     ChunkedUpload cu;
     bool streamed = false;
+
+    JobInput(const Job &job, bool may_stream, cudaStream_t st, DevScope &ds) : in(job.input)
+    {
+        if (in) return;
+        const std::vector<kc_buffer> files = inflate_inputs(job.files, inflated);
+        streamed = may_stream && files.size() == 1 && files[0].size >= STREAMED_UPLOAD_MIN_BYTES;
+        build_input(local, files.data(), (uint32_t)files.size(), st, &ds, tile_seg_host, nullptr,
+                    streamed ? &cu : nullptr);
+        in = &local;
+    }
+    JobInput(const JobInput &) = delete;
+    JobInput &operator=(const JobInput &) = delete;
+    // the rest of a streamed upload, all of it ahead of what follows on st
+    void finish(cudaStream_t st)
+    {
+        if (!streamed) return;
+        cu.enqueue(cu.ev.size());
+        for (cudaEvent_t e : cu.ev) CK(cudaStreamWaitEvent(st, e, 0));
+        streamed = false;
+    }
+};
+
+void run_job_once(Job &job, cudaStream_t st, Workspace &ws, DevScope &ds, JobInput &ji, bool exact_census,
+                  bool global_tables, const kc_tuning &tn)
+{
+    const kc_job &P = job.p;
+    const uint32_t k = P.k;
+
+    // ---- input -----------------------------------------------------------
+    const kc_input *in = ji.in;
+    ChunkedUpload &cu = ji.cu;
+    const bool streamed = ji.streamed;
+    static const bool trace_host = getenv("KC_TRACE") && getenv("KC_TRACE")[0] == '1';
+    const double th_start = now_ms();
     // counted by printed-order prefix in shared memory, also the smallest jobs:
     // 30K distinct k-mers 0.70 -> 0.44 ms against one global-memory table (whose
     // insert of 8 tiles takes 0.18 and whose eight sort passes 0.16), 200 reads
     // 0.74 -> 0.57; 63-base k-mers of 200 reads 0.92 -> 0.62
     const bool prefix = tn.bloom_smem == 1 && !global_tables;
-    if (!in) {
-        const std::vector<kc_buffer> files = inflate_inputs(job.files, inflated);
-        streamed = !exact_census && files.size() == 1 && files[0].size >= STREAMED_UPLOAD_MIN_BYTES &&
-                   (P.bloom || prefix);
-        build_input(local, files.data(), (uint32_t)files.size(), st, &ds, tile_seg_host, nullptr,
-                    streamed ? &cu : nullptr);
-        in = &local;
-        if (trace_host)
-            fprintf(stderr, "[kc trace] job upload of %zu files enqueued after %.3f ms\n", job.files.size(),
-                    now_ms() - th_start);
-    }
     // small uploads and read-backs through pinned staging: a pageable copy
     // would hold the host (and, behind a streamed upload, wait for it)
     HostStage hs(st);
@@ -1191,11 +1208,12 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
         const bool exact = a.bucket_sample_mask == 0;
         // SCAN counted the occurrences of the census tiles (all tiles when exact)
         if (sampled != O) throw KcError{KC_ERR_DEVICE, "bucket census does not add up to the occurrences"};
-        if (!exact && sampled < 65536) throw CensusOverflow{};   // too thin a sample
         // census tiles: t with (t & mask) == 0 among the tiles censused so far
         const double scale =
             exact ? 1.0
                   : (double)T / (double)((tiles_ready + a.bucket_sample_mask) / (a.bucket_sample_mask + 1));
+        // (15% and 8192 more are six standard deviations and up of a bucket's
+        // estimate from any sample, however thin)
         for (uint32_t b = 0; b < N_BUCKETS; ++b)
             region[b] = exact ? bh[b] : (unsigned long long)std::ceil((double)bh[b] * scale * 1.15) + 8192;
         std::vector<uint64_t> fcap(N_BUCKETS, 0);
@@ -1713,21 +1731,12 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
 // memory until the final sort.  The Bloom split (kc_job.bloom) only chooses
 // which occurrences the reference keeps in memory; the counts are exact
 // either way, so these jobs count every occurrence in the table.
-void run_wide_job(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, bool global_tables, const kc_tuning &tn)
+void run_wide_job(Job &job, cudaStream_t st, Workspace &ws, DevScope &ds, JobInput &ji, bool exact_census,
+                  bool global_tables, const kc_tuning &tn)
 {
     const kc_job &P = job.p;
     const uint32_t k = P.k, nw = key_words(k);
-    if (P.fault_inject & KC_INJECT_NOMEM) ws.fail_next_get();
-    DevScope ds(st, &ws);
-    std::vector<uint32_t> tile_seg_host;
-    kc_input local;
-    const kc_input *in = job.input;
-    std::vector<PinnedBlock> inflated;
-    if (!in) {
-        const std::vector<kc_buffer> files = inflate_inputs(job.files, inflated);
-        build_input(local, files.data(), (uint32_t)files.size(), st, &ds, tile_seg_host);
-        in = &local;
-    }
+    const kc_input *in = ji.in;
     HostStage hs(st);
     cudaEvent_t ev0, ev1;
     CK(cudaEventCreate(&ev0));
@@ -1812,7 +1821,6 @@ void run_wide_job(Job &job, cudaStream_t st, Workspace &ws, bool exact_census, b
     job.occurrences = O;
     check_cancel(job, "after the scan");
     const bool exact = !prefix || pa.bucket_sample_mask == 0;
-    if (!exact && O < 65536) throw CensusOverflow{};   // too thin a sample
     if (!exact)   // each bucket's region: its share of the census, and some
         for (auto &x : bh)
             x = (uint64_t)std::ceil((double)x * 1.15 * (double)T /
@@ -2186,11 +2194,19 @@ uint64_t reserve_for(const kc_job &p, uint64_t resident_bytes)
 
 void run_job(Job &job, cudaStream_t st, Workspace &ws, const kc_tuning &tn)
 {
+    static const bool trace = getenv("KC_TRACE") && getenv("KC_TRACE")[0] == '1';
+    if (job.p.fault_inject & KC_INJECT_NOMEM) ws.fail_next_get();
+    const double t0 = now_ms();
+    DevScope ds(st, &ws);
+    JobInput ji(job, job.p.k <= 32 && (job.p.bloom || tn.bloom_smem == 1), st, ds);
+    if (trace && !job.input)
+        fprintf(stderr, "[kc trace] job upload of %zu files enqueued after %.3f ms\n", job.files.size(), now_ms() - t0);
+    const DevScope::Mark uploaded = ds.mark();
     bool exact_census = false, global_tables = false;
     for (;;) {
         try {
-            if (job.p.k > 32) run_wide_job(job, st, ws, exact_census, global_tables, tn);
-            else run_job_once(job, st, ws, exact_census, global_tables, tn);
+            if (job.p.k > 32) run_wide_job(job, st, ws, ds, ji, exact_census, global_tables, tn);
+            else run_job_once(job, st, ws, ds, ji, exact_census, global_tables, tn);
             break;
         } catch (const CensusOverflow &) {
             // the sampled census missed a skewed bucket: count every tile instead
@@ -2199,8 +2215,8 @@ void run_job(Job &job, cudaStream_t st, Workspace &ws, const kc_tuning &tn)
             global_tables = true;
         }
         CK(cudaStreamSynchronize(st));
-        ws.end_job();
-        ws.begin_job();
+        ds.rewind(uploaded);
+        ji.finish(st);
     }
     if (global_tables) job.smem_fallbacks = job.passes;
 }

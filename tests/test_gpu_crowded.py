@@ -185,3 +185,58 @@ def test_sampled_regions_of_long_kmers_fit(counter, k, large):
     r = _check(counter, f, k)
     counter.set_tuning(sampled_region_keys=64 << 20)
     assert r.smem_passes == 1 and r.region_redos == 0
+
+
+def _tiles(seqs):
+    """One record per 8 KiB tile of the input."""
+    out = []
+    for s in seqs:
+        out.append(b"@rr\n" + s + b"\n+\n" + b"I" * 4092 + b"\n")
+        assert len(out[-1]) == 8192
+    return b"".join(out)
+
+
+@pytest.mark.parametrize("k", [31, 63, 127])
+@pytest.mark.parametrize("resident", [False, True])
+def test_census_sample_unlike_the_rest(counter, k, resident):
+    """Every eighth tile, those of the census sample, is unlike the others: the
+    buckets outgrow their regions, and the input that is on the device already
+    is counted again."""
+    rng = np.random.default_rng(k)
+    f = _tiles(BASES[rng.integers(0, 4, 4092)].tobytes() if i % 8 == 0 else np.resize(BASES[rng.integers(0, 4, 97)], 4092).tobytes()
+               for i in range(600))
+    want_k, want_c = _oracle([f], k)
+    kw = dict(k=k, count_max=U32, hist_max=10)
+    if resident:
+        inp = counter.upload([f])
+        r = counter.count(input=inp, **kw)
+        counter.free_input(inp)
+    else:
+        r = counter.count([f], **kw)
+    assert np.array_equal(r.keys, want_k) and np.array_equal(r.counts, want_c)
+    assert r.hist.tolist() == O.histogram(want_c, 1, 10).tolist()
+
+
+def test_streamed_upload_whose_first_quarter_is_unlike_the_rest(counter):
+    """A file that goes up in chunks: its first quarter, from which the bucket
+    regions come, has A and T only."""
+    rng = np.random.default_rng(8)
+    codes = rng.integers(0, 4, 280_000_000, dtype=np.uint8)
+    codes[: 70_000_000] = 3 * (codes[: 70_000_000] & 1)
+    f = _record(BASES[codes].tobytes())
+    assert len(f) > 512 << 20
+    want_k, want_c = _torch_records(codes, 31)
+    for kw in (dict(), dict(bloom=True, memory_gb=8)):
+        r = counter.count([f], k=31, count_max=U32, hist_max=10, **kw)
+        assert r.occurrences == len(codes) - 30
+        assert np.array_equal(r.keys, want_k) and np.array_equal(r.counts, want_c)
+
+
+@pytest.mark.parametrize("k,length", [(31, 34), (63, 66), (127, 130)])
+def test_few_kmers_in_many_tiles(counter, k, length):
+    """Reads hardly longer than k: the census sample of 600 tiles holds few
+    k-mers."""
+    n = 600 * 8192 // (2 * length + 7)
+    f = _fastq(_uniform(k, n // 2, length) + _uniform(k + 1, n - n // 2 + 100, min(length, k - 2)), 3)
+    r = _check(counter, [f], k)
+    assert r.smem_passes == 1 and r.smem_fallbacks == 0
