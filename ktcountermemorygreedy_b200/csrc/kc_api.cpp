@@ -408,6 +408,13 @@ uint64_t pass_budget(Workspace &ws, uint64_t need)
     return (double)need <= 0.7 * (double)ws_free ? need : default_pass_budget(ws);
 }
 
+// Whether a bucket alone needs more than the device has for a pass.
+bool bucket_too_large(Workspace &ws, const std::vector<uint64_t> &nb)
+{
+    const uint64_t most = *std::max_element(nb.begin(), nb.end());
+    return most > pass_budget(ws, most);
+}
+
 // Passes over ranges of buckets that need nb[b] bytes each, within the budget
 // (the caller's, or 0: the worker's) or one bucket at least.
 std::vector<std::pair<uint32_t, uint32_t>> pass_ranges(Workspace &ws, const std::vector<uint64_t> &nb, uint64_t budget)
@@ -592,7 +599,10 @@ void count_by_prefix(PrefixPass &pp, DevScope &ds, HostStage &hs, PhaseClock &cl
     unsigned long long *counters = pp.counters;
     const uint32_t shape = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(tn.count_shape, 4));
     uint64_t pass_keys = 0;
-    for (uint32_t b = lo; b < hi; ++b) pass_keys += pp.cfg[b].key_len;
+    for (uint32_t b = lo; b < hi; ++b) {
+        if (pp.cfg[b].key_len > 0xFFFFFFFFull) throw SubTablesFull{};   // a sub-bucket's keys are counted in 32 bits
+        pass_keys += pp.cfg[b].key_len;
+    }
     const bool batch = pp.base_bits == 0;
     const uint64_t one_word = batch                              ? SUB_KEYS_BATCH
                               : pass_keys < SUB_SMALL_PASS_KEYS ? SUB_KEYS_SMALL
@@ -1231,6 +1241,9 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, DevScope &ds, JobInp
             prefix ? 25 + (12 + std::max(P.min_count, 1u) - 1) / std::max(P.min_count, 1u) : (P.bloom ? 42 : 48);
         std::vector<uint64_t> nb(N_BUCKETS);
         for (uint32_t b = 0; b < N_BUCKETS; ++b) nb[b] = region[b] * per_occ + fcap[b] * 16;
+        // one bucket's occurrences larger than the device: tables of distinct
+        // k-mers may be smaller (plain jobs; a Bloom job's need the k-mers too)
+        if (prefix && !P.bloom && bucket_too_large(ws, nb)) throw SubTablesFull{};
         const auto ranges = pass_ranges(ws, nb, P.pass_bytes);
         const bool multi = ranges.size() > 1;
         if (streamed && multi) census_chunks(cu.ev.size());   // every pass reads every tile
@@ -1841,6 +1854,7 @@ void run_wide_job(Job &job, cudaStream_t st, Workspace &ws, DevScope &ds, JobInp
         const uint64_t per_key = 20ull * nw + 5 + rec_bytes / std::max(P.min_count, 1u) + 1;
         nb[b] = prefix ? bh[b] * per_key + 4096 : (uint64_t)(share * est * (factor * slot_bytes + rec_bytes)) + 4096;
     }
+    if (prefix && bucket_too_large(ws, nb)) throw SubTablesFull{};   // its table of distinct k-mers may be smaller
     const auto ranges = pass_ranges(ws, nb, P.pass_bytes);
     const bool multi = ranges.size() > 1;
     unsigned long long *hist = ds.n<unsigned long long>(HIST_BINS);

@@ -240,3 +240,32 @@ def test_few_kmers_in_many_tiles(counter, k, length):
     f = _fastq(_uniform(k, n // 2, length) + _uniform(k + 1, n - n // 2 + 100, min(length, k - 2)), 3)
     r = _check(counter, [f], k)
     assert r.smem_passes == 1 and r.smem_fallbacks == 0
+
+
+_LITTLE_MEMORY = """
+import sys
+import numpy as np, torch
+import ktcountermemorygreedy_b200 as kc
+k, n = int(sys.argv[1]), int(sys.argv[2])
+free, _ = torch.cuda.mem_get_info()
+held = torch.empty(free - (5 << 30), dtype=torch.uint8, device="cuda")
+with kc.KmerCounter(max_inflight_jobs=1) as c:
+    f = b"@r\\n" + b"A" * n + b"\\n+\\n" + b"I" * n + b"\\n"
+    r = c.count([f], k=k, count_max=kc.U32_MAX)
+    assert r.occurrences == n - k + 1 and r.distinct == 1, (r.occurrences, r.distinct)
+    assert r.counts.tolist() == [n - k + 1] and not r.keys.any()
+    assert r.smem_passes == 0 and r.smem_fallbacks == 1
+"""
+
+
+@pytest.mark.parametrize("k,n", [(31, 260_000_000), (63, 140_000_000)])
+def test_occurrences_that_do_not_fit_the_device(k, n):
+    """One k-mer's occurrences larger than the device memory left (5 GB, the
+    rest is held), its table a few slots: counted in global-memory tables."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    p = subprocess.run([sys.executable, "-c", _LITTLE_MEMORY, str(k), str(n)], cwd=root, capture_output=True, text=True,
+                       timeout=300)
+    assert p.returncode == 0, p.stderr[-2000:]
