@@ -601,6 +601,10 @@ def dump_text(keys: np.ndarray, counts: np.ndarray, k: int) -> str:
     return dump_bytes(keys, counts, k).decode("ascii")
 
 
+# a prototype of its own: pythonapi's function objects are the whole process's
+_new_bytes = C.PYFUNCTYPE(C.py_object, C.c_void_p, C.c_ssize_t)(("PyBytes_FromStringAndSize", C.pythonapi))
+
+
 def dump_bytes(keys: np.ndarray, counts: np.ndarray, k: int) -> bytes:
     keys = np.ascontiguousarray(keys, dtype=np.uint64)
     counts = np.ascontiguousarray(counts, dtype=np.uint32)
@@ -609,9 +613,7 @@ def dump_bytes(keys: np.ndarray, counts: np.ndarray, k: int) -> bytes:
     _check(lib().kc_dump_text(_ptr(keys), _ptr(counts), n, k, None, 0, C.byref(need)))
     # the text goes straight into a new bytes object of its size (nobody else
     # holds it yet): a second copy of 70 MB takes 29 ms
-    new_bytes = C.pythonapi.PyBytes_FromStringAndSize
-    new_bytes.restype, new_bytes.argtypes = C.py_object, [C.c_void_p, C.c_ssize_t]
-    out = new_bytes(None, need.value)
+    out = _new_bytes(None, need.value)
     got = C.c_uint64()
     _check(lib().kc_dump_text(_ptr(keys), _ptr(counts), n, k, C.cast(C.c_char_p(out), C.c_void_p), need.value,
                               C.byref(got)))
