@@ -605,6 +605,20 @@ def dump_text(keys: np.ndarray, counts: np.ndarray, k: int) -> str:
 _new_bytes = C.PYFUNCTYPE(C.py_object, C.c_void_p, C.c_ssize_t)(("PyBytes_FromStringAndSize", C.pythonapi))
 
 
+_madvise = C.CFUNCTYPE(C.c_int, C.c_void_p, C.c_size_t, C.c_int)(("madvise", C.CDLL(None)))
+
+
+def _advise_huge(addr: int, size: int):
+    """2 MiB pages for a new object nobody has touched yet, where the system gives
+    them on advice (the 17000 page faults of 4 KiB of a dump of 70 MB take 4 ms).
+    From 32 MiB on, where malloc always maps memory of its own: the advice goes
+    with the object."""
+    page, madv_hugepage = 2 << 20, 14
+    a, e = -(-addr // page) * page, (addr + size) // page * page
+    if size >= 32 << 20:
+        _madvise(a, e - a, madv_hugepage)   # advice: a refusal changes nothing
+
+
 def dump_bytes(keys: np.ndarray, counts: np.ndarray, k: int) -> bytes:
     keys = np.ascontiguousarray(keys, dtype=np.uint64)
     counts = np.ascontiguousarray(counts, dtype=np.uint32)
@@ -614,7 +628,8 @@ def dump_bytes(keys: np.ndarray, counts: np.ndarray, k: int) -> bytes:
     # the text goes straight into a new bytes object of its size (nobody else
     # holds it yet): a second copy of 70 MB takes 29 ms
     out = _new_bytes(None, need.value)
+    text = C.cast(C.c_char_p(out), C.c_void_p)
+    _advise_huge(text.value, need.value)
     got = C.c_uint64()
-    _check(lib().kc_dump_text(_ptr(keys), _ptr(counts), n, k, C.cast(C.c_char_p(out), C.c_void_p), need.value,
-                              C.byref(got)))
+    _check(lib().kc_dump_text(_ptr(keys), _ptr(counts), n, k, text, need.value, C.byref(got)))
     return out if got.value == need.value else out[: got.value]

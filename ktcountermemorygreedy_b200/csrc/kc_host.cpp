@@ -16,7 +16,6 @@
 #include <system_error>
 #include <thread>
 
-#include <sys/mman.h>
 #include <unistd.h>
 
 #include "kc_plan.h"
@@ -481,11 +480,6 @@ void copy_out(void *host, const void *dev, size_t bytes, cudaStream_t st)
         return;
     }
     CK(cudaStreamSynchronize(st));   // not with every thread waiting for the kernels
-    // a result array not yet touched: 2 MiB pages where the system gives them on
-    // advice (17000 page faults of 4 KiB take a dump of 70 MB 4 ms)
-    const uintptr_t page = uintptr_t(2) << 20, a = ((uintptr_t)host + page - 1) / page * page,
-                    e = ((uintptr_t)host + bytes) / page * page;
-    if (a < e) (void)madvise(reinterpret_cast<void *>(a), e - a, MADV_HUGEPAGE);
     StagedCopy c{static_cast<uint8_t *>(host), static_cast<uint8_t *>(const_cast<void *>(dev)), bytes, true, st};
     c.run();
 }
