@@ -1795,9 +1795,9 @@ void run_wide_job(Job &job, cudaStream_t st, Workspace &ws, DevScope &ds, JobInp
     // (prefix path: occurrences per first four bases of every 8th tile, every
     // 32nd from 512 MiB on)
     unsigned long long *scan_out = ds.n<unsigned long long>(1 + N_BUCKETS);   // occurrences, 256 bucket counts
-    uint32_t *hll = ds.n<uint32_t>(HLL_M);
+    uint32_t *hll = prefix ? nullptr : ds.n<uint32_t>(HLL_M);
     CK(cudaMemsetAsync(scan_out, 0, (1 + N_BUCKETS) * 8, st));
-    CK(cudaMemsetAsync(hll, 0, HLL_M * 4, st));
+    if (hll) CK(cudaMemsetAsync(hll, 0, HLL_M * 4, st));
     ExtractArgs pa{};
     pa.buf = in->buf;
     pa.n_tiles = T;
@@ -1825,12 +1825,12 @@ void run_wide_job(Job &job, cudaStream_t st, Workspace &ws, DevScope &ds, JobInp
     unsigned long long *h_scan = hs.n<unsigned long long>(1 + N_BUCKETS);
     uint32_t *h_hll = hs.n<uint32_t>(HLL_M);
     CK(cudaMemcpyAsync(h_scan, scan_out, (1 + N_BUCKETS) * 8, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(h_hll, hll, HLL_M * 4, cudaMemcpyDeviceToHost, st));
+    if (hll) CK(cudaMemcpyAsync(h_hll, hll, HLL_M * 4, cudaMemcpyDeviceToHost, st));
     Counters c0 = read_counters(counters, st);
     check_flags(c0.v[C_FLAGS], "scan");
     uint64_t O = h_scan[0];
     std::vector<uint64_t> bh(h_scan + 1, h_scan + 1 + N_BUCKETS);
-    const double est = hll_estimate(h_hll, HLL_M);
+    const double est = hll ? hll_estimate(h_hll, HLL_M) : 0.0;   // (the prefix path needs no table sizes)
     job.occurrences = O;
     check_cancel(job, "after the scan");
     const bool exact = !prefix || pa.bucket_sample_mask == 0;
@@ -2292,10 +2292,13 @@ void run_batch_once(std::vector<std::shared_ptr<Job>> &jobs, cudaStream_t st, Wo
     CK(launch_scan_u32(tile_nl, tile_prefix, T, scan_tmp, st));
     clk.end();
 
+    const bool prefix = tn.bloom_smem == 1 && !global_tables;
     unsigned long long *occ = ds.n<unsigned long long>(n);
-    uint32_t *hll = ds.n<uint32_t>((size_t)n * HLL_M);
+    // (the prefix path needs no table sizes)
+    const size_t hll_n = prefix ? 0 : (size_t)n * HLL_M;
+    uint32_t *hll = prefix ? nullptr : ds.n<uint32_t>(hll_n);
     CK(cudaMemsetAsync(occ, 0, (size_t)n * 8, st));
-    CK(cudaMemsetAsync(hll, 0, (size_t)n * HLL_M * 4, st));
+    if (hll) CK(cudaMemsetAsync(hll, 0, hll_n * 4, st));
     ExtractArgs a{};
     a.buf = in.buf;
     a.n_tiles = T;
@@ -2304,16 +2307,15 @@ void run_batch_once(std::vector<std::shared_ptr<Job>> &jobs, cudaStream_t st, Wo
     a.segs = d_segs;
     a.counters = counters;
     a.occ = occ;
-    const bool prefix = tn.bloom_smem == 1 && !global_tables;
-    a.hll = prefix ? nullptr : hll;   // the prefix path needs no table sizes
+    a.hll = hll;
     a.hll_local = n == 1;
     clk.begin(1);
     CK(launch_extract(MODE_SCAN, a, 0, st));
     clk.end();
     std::vector<unsigned long long> occ_h(n);
-    std::vector<uint32_t> hll_h((size_t)n * HLL_M);
+    std::vector<uint32_t> hll_h(hll_n);
     CK(cudaMemcpyAsync(occ_h.data(), occ, (size_t)n * 8, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(hll_h.data(), hll, (size_t)n * HLL_M * 4, cudaMemcpyDeviceToHost, st));
+    if (hll) CK(cudaMemcpyAsync(hll_h.data(), hll, hll_n * 4, cudaMemcpyDeviceToHost, st));
     Counters c0 = read_counters(counters, st);
     check_flags(c0.v[C_FLAGS], "scan");
 
