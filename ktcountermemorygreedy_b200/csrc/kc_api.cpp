@@ -1670,14 +1670,19 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, DevScope &ds, JobInp
             CK(cudaStreamSynchronize(st));
             const uint64_t n_above = std::min<uint64_t>(n_sel[C_SEL_A], q);
             const uint64_t n_at = std::min<uint64_t>(n_sel[C_SEL_B], q - n_above);
+            // (the records above the threshold lie behind those at it)
+            unsigned long long *above_k = one_wait ? tk + q : nullptr;
+            uint32_t *above_c = one_wait ? tc + q : nullptr;
             if (!one_wait) {
-                big_k.resize(2 * q);
-                big_c.resize(2 * q);
+                big_k.resize(n_at + n_above);
+                big_c.resize(n_at + n_above);
                 tk = big_k.data();
                 tc = big_c.data();
+                above_k = tk + n_at;
+                above_c = tc + n_at;
                 if (n_above) {
-                    CK(cudaMemcpyAsync(tk + q, sk + q, n_above * 8, cudaMemcpyDeviceToHost, st));
-                    CK(cudaMemcpyAsync(tc + q, sc + q, n_above * 4, cudaMemcpyDeviceToHost, st));
+                    CK(cudaMemcpyAsync(above_k, sk + q, n_above * 8, cudaMemcpyDeviceToHost, st));
+                    CK(cudaMemcpyAsync(above_c, sc + q, n_above * 4, cudaMemcpyDeviceToHost, st));
                 }
                 if (n_at) {
                     CK(cudaMemcpyAsync(tk, sk, n_at * 8, cudaMemcpyDeviceToHost, st));
@@ -1689,8 +1694,8 @@ void run_job_once(Job &job, cudaStream_t st, Workspace &ws, DevScope &ds, JobInp
             // (they arrive in printed-string order; a stable sort keeps it)
             std::vector<size_t> idx(n_above);
             for (size_t i = 0; i < n_above; ++i) idx[i] = i;
-            std::stable_sort(idx.begin(), idx.end(), [&](size_t x, size_t y) { return tc[q + x] > tc[q + y]; });
-            for (size_t i : idx) { job.top_keys.push_back(tk[q + i]); job.top_counts.push_back(tc[q + i]); }
+            std::stable_sort(idx.begin(), idx.end(), [&](size_t x, size_t y) { return above_c[x] > above_c[y]; });
+            for (size_t i : idx) { job.top_keys.push_back(above_k[i]); job.top_counts.push_back(above_c[i]); }
             for (size_t i = 0; i < n_at; ++i) { job.top_keys.push_back(tk[i]); job.top_counts.push_back(tc[i]); }
         }
         if (P.want_le2 && n_rec) {
