@@ -270,3 +270,43 @@ def test_occurrences_that_do_not_fit_the_device(k, n):
     p = subprocess.run([sys.executable, "-c", _LITTLE_MEMORY, str(k), str(n)], cwd=root, capture_output=True, text=True,
                        timeout=300)
     assert p.returncode == 0, p.stderr[-2000:]
+
+
+@pytest.mark.parametrize("k,n,shared", [(31, 7000, 24), (31, 7000, 16), (63, 3500, 42), (127, 1700, 42)])
+def test_sort_unit_of_one_run(counter, k, n, shared):
+    """A unit whose records all share the sort's digit but one: each is ranked
+    among all others.  24 shared bases of 31 leave 4096 k-mers that follow one
+    another, which crowd the table's slots too and may be counted apart."""
+    rnd = random.Random(k)
+    tail = lambda m: "".join(rnd.choice("ACGT") for _ in range(m))
+    p = "AC" + tail(shared - 2)
+    if shared == 24:
+        seqs = [p + "".join("ACGT"[(i >> 2 * j) & 3] for j in range(6)) + "A" for i in range(4096)]
+    else:
+        seqs = list({p + tail(k - shared - 1) + "A" for _ in range(n)})
+    seqs.append(p[:6] + ("T" if p[6] != "T" else "G") + tail(k - 8) + "A")
+    seqs += seqs[:100]
+    r = _check(counter, [_fastq([s.encode() for s in seqs])], k)
+    if shared != 24:
+        assert r.smem_passes == 1 and r.smem_fallbacks == 0
+
+
+def test_more_small_units_than_their_list(counter):
+    """128 sub-buckets that need all 64 rounds, 62 of them with a single k-mer:
+    more units of the smallest size than their list holds at first."""
+    rng = np.random.default_rng(6)
+    keys = []
+    for b in range(64):                       # buckets A...: with a last base A the forward strand is canonical
+        for sub in (1, 3):                    # of 4
+            r = np.concatenate([np.repeat(np.uint64([10, 11]), 5000), np.uint64([x for x in range(64) if x not in (10, 11)])])
+            t = rng.integers(0, 1 << 44, len(r), dtype=np.uint64) << np.uint64(2)
+            keys.append((np.uint64(b) << np.uint64(54)) | (np.uint64(sub) << np.uint64(52)) | (r << np.uint64(46)) | t)
+    keys = rng.permutation(np.unique(np.concatenate(keys)))
+    codes = (keys[:, None] >> np.arange(60, -2, -2, dtype=np.uint64)) & np.uint64(3)
+    seq = np.full((len(keys), 69), 10, np.uint8)   # @ r \n, 31 bases, \n + \n, 31 qualities, \n
+    seq[:, :3] = np.frombuffer(b"@r\n", np.uint8)
+    seq[:, 3:34] = BASES[codes]
+    seq[:, 34:37] = np.frombuffer(b"\n+\n", np.uint8)
+    seq[:, 37:68] = 73
+    r = _check(counter, [seq.tobytes()], 31)
+    assert len(r.counts) == len(keys) and r.smem_passes == 1 and r.smem_fallbacks == 0
