@@ -444,7 +444,9 @@ std::vector<std::pair<uint32_t, uint32_t>> pass_ranges(Workspace &ws, const std:
 // the k-mers per sub-bucket that the pass's size and words call for.  Sub-buckets
 // that fit no table (crowded ones) are counted by sorting their keys; when they
 // hold more than 1 in CROWD_SHARE of the pass's keys, their buckets are first cut
-// into 16 times as many, as long as they can be, and the pass counted again.
+// into 16 times as many, as long as they can be, and the pass counted again.  (Not
+// for sub-buckets of a large part of the pass: a few k-mers make those, which no
+// cut tells apart.)
 struct PrefixPass {
     uint32_t words = 1;                 // 64-bit words per key
     uint32_t lo = 0, hi = 0;            // its buckets; their keys are cfg[b].key_base, key_len
@@ -724,6 +726,7 @@ void count_by_prefix(PrefixPass &pp, DevScope &ds, HostStage &hs, PhaseClock &cl
         pc.counters = counters;
         pc.bucket_ovf = bucket_ovf;
         pc.crowd = ds.n<CrowdSub>(n_sub);
+        pc.max_keys = sub_max_keys(pp.n_keys);
         CK(launch_count_prefix(pc, N, shape, st));
         clk.end();
         // (as if the first bucket's sub-buckets had been crowded)
@@ -736,7 +739,7 @@ void count_by_prefix(PrefixPass &pp, DevScope &ds, HostStage &hs, PhaseClock &cl
         // buckets of crowded sub-buckets that can be cut further: 16 times the
         // sub-buckets
         bool cut = false;
-        if (!cs.v[C_REGION_OVF] && (pp.crowded || injected)) {
+        if (!cs.v[C_REGION_OVF] && (cs.v[C_CROWD_TRIED] * CROWD_SHARE > pp.n_keys || injected)) {
             std::vector<uint32_t> bo(N_BUCKETS);
             CK(cudaMemcpyAsync(bo.data(), bucket_ovf, N_BUCKETS * 4, cudaMemcpyDeviceToHost, st));
             CK(cudaStreamSynchronize(st));

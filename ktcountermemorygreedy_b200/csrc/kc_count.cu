@@ -247,10 +247,10 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
         uint32_t lg = n > 1 ? 33 - __clz(n - 1) : 1;
         lg = lg < 9 ? 9 : (lg > TBITS ? TBITS : lg);
         const uint32_t smask = (1u << lg) - 1, hsh = 32 - lg;
-        uint32_t rounds = rounds0, rd = 0, off = 0, most = 0;
+        uint32_t rounds = n > SUB_ROUNDS_KEYS ? 1 : rounds0, rd = 0, off = 0, most = 0;
         bool failed = false;
-        static_assert(SUB_MAX_KEYS < SLOT_COUNT, "a count would run into the state bits");
-        const bool too_many = n > SUB_MAX_KEYS;
+        static_assert(SUB_KEYS_CAP < SLOT_COUNT, "a count would run into the state bits");
+        const bool too_many = n > a.max_keys;
         while (rd < rounds && !too_many) {
             const uint32_t rmask = rounds - 1;
             const int rsh = 64 - (int)cfg.plen - (31 - __clz(rounds));   // rounds == 1: unused
@@ -399,7 +399,8 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
                 failed = true;
                 rounds *= 2;
                 rd *= 2;
-                if (rounds > SUB_MAX_ROUNDS || rounds * n > SUB_MAX_READS || (int)cfg.plen + (31 - __clz(rounds)) > 64)
+                if (rounds > SUB_MAX_ROUNDS || n > SUB_ROUNDS_KEYS || rounds * n > SUB_MAX_READS ||
+                    (int)cfg.plen + (31 - __clz(rounds)) > 64)
                     break;
                 continue;
             }
@@ -492,8 +493,11 @@ __global__ void __launch_bounds__(THREADS, BPSM) k_count_prefix(PrefixCountArgs 
             a.sub_len[sub] = off;
             if (gave_up) {
                 const uint32_t b = a.sub_bucket[sub];
-                atomicOr(&a.bucket_ovf[b], 1u);
                 atomicAdd(&a.counters[C_CROWD_KEYS], (unsigned long long)n);
+                if (!too_many) {
+                    atomicOr(&a.bucket_ovf[b], 1u);
+                    atomicAdd(&a.counters[C_CROWD_TRIED], (unsigned long long)n);
+                }
                 a.crowd[atomicAdd(&a.counters[C_SUB_OVF], 1ull)] = CrowdSub{base, n, sub, off, rd, rounds, b};
             }
         }

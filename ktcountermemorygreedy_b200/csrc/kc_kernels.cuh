@@ -43,6 +43,7 @@ enum Counter : int {
     C_KEPT = 12,         // records a counting compaction pass would keep
     C_UNIT_OVF = 13,     // nonzero: more sort units of a class than its list holds
     C_CROWD_KEYS = 14,   // keys of the crowded sub-buckets
+    C_CROWD_TRIED = 15,  // those of them that rounds were tried on
     C_UNITS = 16,        // UNIT_CLASSES counts: sort units by size
     C_COUNT = 24
 };
@@ -347,9 +348,9 @@ cudaError_t launch_subpart_sizes(const unsigned long long *sub_off, const unsign
 // of them.  Every k-mer's count goes to the group's histogram (hist_bins bins
 // at hist + group * hist_bins; larger counts to ovf, or with their group to
 // ovf64), totals to totals[3 * group ..]: distinct k-mers, k-mers seen once,
-// records.  Sub-buckets that no number of rounds fits, or with more keys than
-// SUB_MAX_KEYS, are listed in crowd (C_SUB_OVF of them, C_CROWD_KEYS keys in all;
-// bucket_ovf[their bucket] is set): their finished rounds are counted and their
+// records.  Sub-buckets that no number of rounds fits (bucket_ovf[their bucket] is
+// set, C_CROWD_TRIED keys in all), or with more keys than max_keys, are listed in
+// crowd (C_SUB_OVF of them, C_CROWD_KEYS keys in all): their finished rounds are counted and their
 // records in place, the rest is left to the caller.  More units of a class than
 // lists.cap[c] set C_UNIT_OVF: the results are then incomplete.
 constexpr uint32_t UNIT_CLASSES = 4;
@@ -360,11 +361,19 @@ struct SubUnit {
 constexpr uint32_t SUB_MAX_ROUNDS = 64;   // rounds a sub-bucket may be cut into, each a unit
 // One block counts a sub-bucket, about 560 keys a microsecond and round: 256K keys
 // take it 0.5 ms, about what sorting them on the whole device takes with its dozen
-// launches and two waits, and from there on the sort gains (9.6M occurrences of
-// poly-A k-mers took 163 ms in one block).  The same bounds all rounds together,
-// with room for 64 rounds of 65K keys (7 ms): a table of 8192 slots then holds
-// whatever rounds can tell apart.
-constexpr uint32_t SUB_MAX_KEYS = 1u << 18, SUB_MAX_READS = 1u << 22;
+// launches and two waits.  So sub-buckets of more keys get one round (a few
+// k-mers of very many occurrences fit it; 9.6M occurrences of poly-A k-mers with
+// errors took 163 ms in rounds), and none where they are also more than 1 in
+// SUB_PASS_SHARE of the pass's keys and would keep their block at it longer than
+// the 296 others at everything else.  All rounds of smaller ones read at most
+// SUB_MAX_READS keys, 64 rounds of 65K keys (7 ms).
+constexpr uint32_t SUB_ROUNDS_KEYS = 1u << 18, SUB_MAX_READS = 1u << 22, SUB_PASS_SHARE = 256;
+constexpr uint32_t SUB_KEYS_CAP = 1u << 29;   // two- and four-word counts share a word with two state bits
+inline uint32_t sub_max_keys(uint64_t n_keys)
+{
+    const uint64_t share = n_keys / SUB_PASS_SHARE;
+    return share < SUB_ROUNDS_KEYS ? SUB_ROUNDS_KEYS : (share < SUB_KEYS_CAP ? (uint32_t)share : SUB_KEYS_CAP);
+}
 // A crowded sub-bucket: its keys [src, src + n); rounds 0 .. rd - 1 of `rounds`
 // are counted, with `off` records.
 struct CrowdSub {
@@ -413,6 +422,7 @@ struct PrefixCountArgs {
     unsigned long long *counters;
     uint32_t *bucket_ovf;
     CrowdSub *crowd;   // n_sub entries
+    uint32_t max_keys;   // sub_max_keys(keys of the pass)
 };
 // shape (kc_tuning.count_shape): 1 and 3 run 512-thread blocks, two per SM,
 // with tables of 8192, 4096 or 2048 slots for keys of 1, 2 or 4 words; 2 and 4
