@@ -310,3 +310,23 @@ def test_more_small_units_than_their_list(counter):
     seq[:, 37:68] = 73
     r = _check(counter, [seq.tobytes()], 31)
     assert len(r.counts) == len(keys) and r.smem_passes == 1 and r.smem_fallbacks == 0
+
+
+def test_large_sub_buckets_of_a_large_pass(counter):
+    """150M k-mers, so that one block may count up to 586K keys, in one round
+    from 262144 on: two frequent k-mers (counted in it), a repeat with errors
+    (too many distinct ones for it) and a run beyond the limit."""
+    rng = np.random.default_rng(12)
+    codes = rng.integers(0, 4, 150_000_000, dtype=np.uint8)
+    codes[10_000_000:10_400_000] = 2                                   # G
+    codes[20_000_000:20_900_000] = np.resize(np.uint8([0, 1]), 900_000)   # AC and CA, 450K each
+    codes[30_000_000:31_000_000] = 0                                   # A, beyond the limit
+    errors = np.resize(np.uint8([0, 3]), 1_000_000)                    # AT with errors
+    at = rng.integers(0, len(errors), 30_000)
+    errors[at] = rng.integers(0, 4, len(at))
+    codes[40_000_000:41_000_000] = errors
+    want_k, want_c = _torch_records(codes, 31)
+    r = counter.count([_record(BASES[codes].tobytes())], k=31, count_max=U32, hist_max=2_000_000)
+    assert r.smem_passes == 1 and r.smem_fallbacks == 0
+    assert np.array_equal(r.keys, want_k) and np.array_equal(r.counts, want_c)
+    assert r.hist.tolist() == O.histogram(want_c, 1, 2_000_000).tolist()
