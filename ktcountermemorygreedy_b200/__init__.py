@@ -441,11 +441,11 @@ class KmerCounter:
     def set_tuning(self, bucket_table_factor: float = 0.0, table_factor: float = 0.0, sort_group_records: int = 0,
                    bloom_smem: int = 0, record_sort: int = 0, sampled_region_keys: int = 0, count_shape: int = 0,
                    part_shape: int = 0, scatter_shape: int = 0):
-        """0 (or less) keeps a setting.  bloom_smem: 1 counts Bloom and large
-        plain jobs per sub-bucket in shared memory, 2 on global-memory tables.
+        """0 (or less) keeps a setting.  bloom_smem: 1 counts jobs and
+        batches per sub-bucket in shared memory, 2 on global-memory tables.
         record_sort: 1 sorts those tables' records most significant bits first,
         2 with the LSD radix sort.  count_shape: the shared-memory count's
-        block shape, 1..4; part_shape: 1 or 2, no effect any more;
+        block shape, 1 or 2 (3 and 4 are the same); part_shape: 1 or 2, no effect any more;
         scatter_shape: the sub-bucket scatter's variant, 1 or 2 (kc_tuning in
         include/kc.h)."""
         t = kc_tuning()

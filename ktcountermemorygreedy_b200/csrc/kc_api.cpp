@@ -11,8 +11,9 @@
 //   -> the prefix path: a census of the first four bases (sampled on larger
 //      inputs) -> scatter by them, then by the next ones -> every sub-bucket
 //      counted in a shared-memory table, its records sorted on their own
-//      global-memory tables (kc_tuning.bloom_smem 2, and k-mers that fit no
-//      sub-bucket table): SCAN (occurrences, HyperLogLog) -> INSERT into a table
+//      (crowded sub-buckets, which no table holds: their keys sorted)
+//      global-memory tables (kc_tuning.bloom_smem 2, and buckets larger than
+//      the device's memory): SCAN (occurrences, HyperLogLog) -> INSERT into a table
 //      sized from the estimate -> compaction + histogram -> radix sort; large
 //      jobs by root-prefix buckets, Bloom jobs with the pre-pass statistics and
 //      the reference's filter before the insert
@@ -133,13 +134,13 @@ uint64_t table_capacity_for(double est, double factor = 1.6)
 
 int fail(int code, const std::string &msg) { return set_error(code, msg); }
 
+// Sub-bucket regions of a large pass (kc_tuning.sampled_region_keys) are
+// sized from a 1-in-SUB_REGION_SAMPLE sample of its keys, by lines of 16.
+constexpr uint32_t SUB_REGION_SAMPLE = 8;
+
 // Working memory of the sort of a job's n records (k-mers of k bases): the
 // MSD sort for large jobs, the LSD sort otherwise; both keep the alternate
 // arrays at the start (sort_tmp_alt).
-// Sub-bucket regions of a large pass (kc_tuning.sampled_region_keys) are
-// sized from a 1-in-SUB_REGION_SAMPLE sample of its work items.
-constexpr uint32_t SUB_REGION_SAMPLE = 8;
-
 size_t record_sort_bytes(uint64_t n, uint32_t k)
 {
     return msd_sort_applies(n, 2 * k) ? std::max(msd_sort_tmp_bytes(n, 2 * k), sort_tmp_bytes(n)) : sort_tmp_bytes(n);

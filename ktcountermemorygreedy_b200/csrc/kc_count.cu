@@ -17,13 +17,13 @@
 // Against the path it replaced (filter slices and 4096-slot tables per
 // sub-bucket of an XXH3 partition, global bucket tables for plain jobs, and a
 // sort of all records), on a B200: 20M reads (2.4G k-mers, 115M records,
-// min count 2) count 27.1 -> 18.5 ms and sort 7.1 -> 1.2 ms; 4M reads with
+// min count 2) count 27.1 -> 14.5 ms and sort 7.1 -> 1.1 ms; 4M reads with
 // every k-mer kept (480M k-mers, 145M records) insert + compaction 11.8 ms ->
-// scatter + count 6.8 ms, sort 11.9 -> 1.7 ms.
+// scatter + count 5.0 ms, sort 11.8 -> 1.6 ms.
 // k > 32, against an N-word table in HBM probed straight from the extraction and
-// one stable LSD sort per word: 2M reads at k = 63 (176M k-mers) scan, insert,
-// compaction and sort 26.2 ms -> census, partition, count and sort 7.0 ms; 500k
-// reads at k = 127 (29M records) 25.8 -> 5.1 ms.
+// one stable LSD sort per word: 2M reads at k = 63 (176M k-mers, min count 2) scan,
+// insert, compaction and sort 26.2 ms -> census, partition, scatter, count and sort
+// 6.0 ms; 500k reads at k = 127 (29M records) 25.8 -> 4.2 ms.
 #include <algorithm>
 
 #include "kc_device.cuh"

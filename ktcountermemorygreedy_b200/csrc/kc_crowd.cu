@@ -12,8 +12,8 @@
 //
 // When such sub-buckets sent the whole job (or batch) to global-memory tables: 960M
 // 31-mers of a 40 Mbp genome with 1% of poly-A and microsatellites 477 ms a call,
-// now 19.6 (17 crowded sub-buckets, 7.7M keys, 1.3 ms of it here; 17.1 without the
-// repeats), 176M 63-mers 73 -> 10.9, 48 samples with one of repeats 84 -> 18.6.
+// now 19.5 (17 crowded sub-buckets, 7.7M keys, 1.3 ms of it here; 17.1 without the
+// repeats), 176M 63-mers 73 -> 10.8, 48 samples with one of repeats 84 -> 18.4.
 #include <algorithm>
 
 #include "kc_device.cuh"

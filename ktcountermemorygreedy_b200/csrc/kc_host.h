@@ -165,8 +165,10 @@ uint64_t gzip_size_hint(const kc_buffer &b);
 std::vector<kc_buffer> inflate_inputs(const std::vector<kc_buffer> &files, std::vector<PinnedBlock> &hold);
 
 // Copies of a caller's arrays.  Pageable memory of some size goes through pinned
-// chunks filled or emptied by several threads; both return when done with the
-// host's side (copy_in: the device's too).
+// chunks filled or emptied by several threads.  copy_out returns when the array is
+// written.  copy_in returns when a pageable array has been read; a pinned one is
+// read by a copy that is only queued, and must stay as it is until the stream is
+// synchronised (the callers below do before they return).
 void copy_in(void *dev, const void *host, size_t bytes, cudaStream_t st);    // throws KcError
 void copy_out(void *host, const void *dev, size_t bytes, cudaStream_t st);   // throws KcError
 
