@@ -330,3 +330,20 @@ def test_large_sub_buckets_of_a_large_pass(counter):
     assert r.smem_passes == 1 and r.smem_fallbacks == 0
     assert np.array_equal(r.keys, want_k) and np.array_equal(r.counts, want_c)
     assert r.hist.tolist() == O.histogram(want_c, 1, 2_000_000).tolist()
+
+
+def test_crowded_jobs_side_by_side():
+    """Jobs with crowded sub-buckets on several workers of one handle: each has
+    the results it has alone."""
+    import ktcountermemorygreedy_b200 as kc
+    jobs = [(k, [_fastq(_uniform(i, 9000) + _repeat(50 + i, (b"A", b"AC", b"GATA")[i % 3], 800, 0.03), i)])
+            for i, k in enumerate((31, 63, 25, 127, 31, 47, 32, 31))]
+    with kc.KmerCounter(max_inflight_jobs=1) as c:
+        alone = [c.count(f, k=k, count_max=U32, hist_max=100) for k, f in jobs]
+    with kc.KmerCounter(max_inflight_jobs=4) as c:
+        ids = [c.submit(f, k=k, count_max=U32, hist_max=100) for _ in range(3) for k, f in jobs]
+        for i, (j, (k, _)) in enumerate(zip(ids, jobs * 3)):
+            c.wait(j)
+            r, want = c.result(j, k), alone[i % len(jobs)]
+            assert np.array_equal(r.keys, want.keys) and np.array_equal(r.counts, want.counts)
+            assert np.array_equal(r.hist, want.hist)
